@@ -196,27 +196,42 @@ inline TestHooks& test_hooks() {
   return hooks;
 }
 
+// The rare part of a bounded wait, out of line on purpose: inlined, its atomic and its clock arithmetic cost the loops
+// around a wait their register allocation (GEMM core: 1030 clocks per K block against 880, same source otherwise).
+static __device__ __noinline__ bool mbar_wait_expired(uint32_t start, volatile int* abort_flag, int* status, int code) {
+  if (*abort_flag) return true;
+  const int kiloclocks = abort_flag[1];
+  uint32_t budget = kiloclocks > 0 ? uint32_t(min(kiloclocks, 1 << 20)) << 10 : uint32_t(kWaitClockBudget);
+  // a producer that waits for a free slot waits for a consumer, which may itself be waiting: let the consumer report first
+  if (code == kStatusWaitSmemEmpty) budget *= 2;
+  if (uint32_t(clock()) - start <= budget) return false;
+  *abort_flag = 1;
+  if (status) atomicCAS(status, 0, code);
+  return true;
+}
+
 // Wait for `parity` of `bar`.  Gives up when the budget runs out or when another role of the
 // CTA has already raised the abort flag (`abort_flag` points at a WaitControl); on giving up it raises the
 // flag, records `code` in the global status word and returns false so that the caller can unwind.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long start = clock64();
-  const int kiloclocks = abort_flag[1];
-  const long long budget = kiloclocks > 0 ? (long long)kiloclocks << 10 : kWaitClockBudget;
-  uint32_t spins = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if ((++spins & 0x3ff) == 0) {
-      if (*abort_flag) return false;
-      if (clock64() - start > budget) {
-        *abort_flag = 1;
-        if (status) atomicCAS(status, 0, code);
-        return false;
-      }
+  const uint32_t start = clock();
+  for (uint32_t spins = 0; !mbar_try_wait(bar, parity);) {
+    if (++spins == 1024) {
+      if (mbar_wait_expired(start, abort_flag, status, code)) return false;
+      spins = 0;
     }
   }
   return true;
+}
+
+// ---- cp.async of one 32-bit word, and an arrival tied to the completion of a thread's copies --------------
+__device__ __forceinline__ void cp_async_4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+// Makes `bar` receive one (pre-counted) arrival from this thread once all its earlier cp.async copies have landed.
+__device__ __forceinline__ void cp_async_arrive_noinc(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // ---- TMA (bulk tensor copy global -> this CTA's shared memory, completion on an mbarrier) --
@@ -274,7 +289,6 @@ __device__ __forceinline__ void tcgen05_commit(uint64_t* bar) {
 __device__ __forceinline__ void tcgen05_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-
 // Shared-memory matrix descriptor of a K-major operand tile stored as rows of 128 bytes with
 // the 128-byte swizzle (what a SWIZZLE_128B TMA box of inner extent 128 B writes): 8-row
 // groups are 1024 B apart (stride byte offset), the leading byte offset is unused for this
@@ -378,6 +392,35 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, float* v) {
       : "memory");
 }
 
+// 32 lanes x 64 consecutive fp32 columns, complete on return, as 32 packed pairs (the operands of the packed fp32
+// instructions).  Load, wait and packing are one asm block: nothing can read a register before its load has landed.
+__device__ __forceinline__ void tmem_ld_wait_64(uint32_t taddr, uint64_t* v) {
+  asm volatile(
+      "{\n\t.reg .b32 r<64>;\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{r0, r1, r2, r3, r4, r5, r6, r7, r8, r9, r10, r11, r12, r13, r14, r15, "
+      "r16, r17, r18, r19, r20, r21, r22, r23, r24, r25, r26, r27, r28, r29, r30, r31}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{r32, r33, r34, r35, r36, r37, r38, r39, r40, r41, r42, r43, r44, r45, r46, r47, "
+      "r48, r49, r50, r51, r52, r53, r54, r55, r56, r57, r58, r59, r60, r61, r62, r63}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;\n\t"
+      "mov.b64 %0, {r0, r1}; mov.b64 %1, {r2, r3}; mov.b64 %2, {r4, r5}; mov.b64 %3, {r6, r7};\n\t"
+      "mov.b64 %4, {r8, r9}; mov.b64 %5, {r10, r11}; mov.b64 %6, {r12, r13}; mov.b64 %7, {r14, r15};\n\t"
+      "mov.b64 %8, {r16, r17}; mov.b64 %9, {r18, r19}; mov.b64 %10, {r20, r21}; mov.b64 %11, {r22, r23};\n\t"
+      "mov.b64 %12, {r24, r25}; mov.b64 %13, {r26, r27}; mov.b64 %14, {r28, r29}; mov.b64 %15, {r30, r31};\n\t"
+      "mov.b64 %16, {r32, r33}; mov.b64 %17, {r34, r35}; mov.b64 %18, {r36, r37}; mov.b64 %19, {r38, r39};\n\t"
+      "mov.b64 %20, {r40, r41}; mov.b64 %21, {r42, r43}; mov.b64 %22, {r44, r45}; mov.b64 %23, {r46, r47};\n\t"
+      "mov.b64 %24, {r48, r49}; mov.b64 %25, {r50, r51}; mov.b64 %26, {r52, r53}; mov.b64 %27, {r54, r55};\n\t"
+      "mov.b64 %28, {r56, r57}; mov.b64 %29, {r58, r59}; mov.b64 %30, {r60, r61}; mov.b64 %31, {r62, r63};\n\t"
+      "}"
+      : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]), "=l"(v[4]), "=l"(v[5]), "=l"(v[6]), "=l"(v[7]),
+        "=l"(v[8]), "=l"(v[9]), "=l"(v[10]), "=l"(v[11]), "=l"(v[12]), "=l"(v[13]), "=l"(v[14]), "=l"(v[15]),
+        "=l"(v[16]), "=l"(v[17]), "=l"(v[18]), "=l"(v[19]), "=l"(v[20]), "=l"(v[21]), "=l"(v[22]), "=l"(v[23]),
+        "=l"(v[24]), "=l"(v[25]), "=l"(v[26]), "=l"(v[27]), "=l"(v[28]), "=l"(v[29]), "=l"(v[30]), "=l"(v[31])
+      : "r"(taddr), "r"(taddr + 32)
+      : "memory");
+}
+
 // 32 lanes x 16 consecutive fp32 columns.
 __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, float* v) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);
@@ -417,6 +460,21 @@ __device__ __forceinline__ T cta1024_exclusive_scan(T value, T* warp_sums, T& to
   const T before = warp > 0 ? warp_sums[warp - 1] : T(0);
   __syncthreads();                      // warp_sums may be reused by the next scan
   return before + inc - value;
+}
+
+// Packed pairs of fp32: one instruction does both halves (each exactly as its scalar form would).
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+  uint64_t p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
+  return p;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t p, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
 }
 
 // ---- small numeric helpers ---------------------------------------------------------------

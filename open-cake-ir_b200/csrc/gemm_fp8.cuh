@@ -39,7 +39,7 @@ constexpr int kBytesA = kBM * kBK;                // 16 KiB
 constexpr int kBytesB = kBN * kBK;                // 32 KiB
 constexpr int kStageBytes = kBytesA + kBytesB;
 constexpr int kTailRows = 32;                    // box rows of the small A map
-constexpr int kControlWarps = 4;                  // one warpgroup: warp 0 TMA, warp 1 MMA, warps 2-3 idle
+constexpr int kControlWarps = 4;                  // one warpgroup: warp 0 TMA, warp 1 MMA, warp 2 scales, warp 3 idle
 constexpr int kEpilogueWarps = 8;                 // two warpgroups: 2 column groups x 4 TMEM lane quadrants
 constexpr int kThreads = (kControlWarps + kEpilogueWarps) * 32;
 // Register budget moved between the warpgroups once the roles split.  The pool setmaxnreg draws on
@@ -51,6 +51,13 @@ static_assert(kControlWarps * 32 * kControlRegs + kEpilogueWarps * 32 * kEpilogu
               "setmaxnreg budget exceeds the registers the launch allocates");
 constexpr int kMaxGroups = 512;
 constexpr int kItemSlots = 4;
+// The scales of block it + kScaleAhead are announced with the operands of block it, so that the epilogue can read a
+// block's scales from shared memory while it still works on the block before.  A slot is refilled when the shared-memory
+// stage of block it is handed back, i.e. when the MMAs of block it - kStages are done; those were issued after the epilogue
+// had read the scales of block it - kStages - kTmemStages.
+constexpr int kScaleAhead = 2;
+constexpr int kScaleSlots = 8;
+static_assert(kScaleSlots >= kStages + kTmemStages + kScaleAhead, "a slot's scales could be overwritten before they are read");
 
 enum Mode : int {
   kDense = 0,        // C bf16 [M, N]
@@ -82,6 +89,7 @@ struct Params {
 };
 
 struct Shared {
+  uint4 out_rows[kEpilogueWarps][128];                      // per epilogue warp: 32 rows of 64 bytes on their way out
   uint64_t full[kStages];
   uint64_t empty[kStages];
   uint64_t tmem_full[kTmemStages];
@@ -89,11 +97,30 @@ struct Shared {
   uint64_t exchange_done;                                   // kGateUp: all epilogue warps have published their amax
   uint64_t item_full[kItemSlots], item_empty[kItemSlots];   // hand-over of drawn work items from the TMA warp to the other roles
   int item_q[kItemSlots];
+  float scale_a[kScaleSlots][kBM];                          // sfa of the tile's rows for one K block
+  float scale_b[kScaleSlots][2];                            // sfb of the tile's two 128-column halves
   uint32_t tmem_base;
   WaitControl wait;
   int tile_prefix[kMaxGroups + 1];     // m tiles before group g
   float exchange[2][2][2][kBM];        // [item parity][term][column group][row] amax exchange for kGateUp
 };
+
+// A warp's 32 rows of 64 bytes (lane i holds row i) to global memory.  Through shared memory, so that a store instruction
+// writes whole 64-byte runs of eight rows: written straight from the registers it touches 16 bytes of each of 32 rows,
+// and the output of a tile then cost 110 clocks per K block (8192 x 4096 x 7168), 13 % of the whole.  The 16-byte chunk
+// index is XORed with the row pair, which keeps both sides free of bank conflicts.
+__device__ __forceinline__ void warp_store_64(uint4* scratch, const uint4 (&v)[4], uint8_t* dst, size_t stride, int rows, int lane) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) scratch[lane * 4 + (c ^ ((lane >> 1) & 3))] = v[c];
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = i * 8 + (lane >> 2), c = lane & 3;
+    const uint4 x = scratch[r * 4 + (c ^ ((r >> 1) & 3))];
+    if (r < rows) *reinterpret_cast<uint4*>(dst + size_t(r) * stride + c * 16) = x;
+  }
+  __syncwarp();
+}
 
 struct Item {
   int group, row0, rows_valid, n_tile;
@@ -126,16 +153,17 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a_tail,
                 const __grid_constant__ CUtensorMap map_b, const Params p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // by an offset, not by rounding the pointer as an integer: the compiler then still knows that it is shared memory
+  uint8_t* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   Shared* sh = reinterpret_cast<Shared*>(tiles + kStages * kStageBytes);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int n_tiles = (MODE == kGateUp) ? p.n / 128 : (p.n + kBN - 1) / kBN;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 1 + 32); mbar_init(&sh->empty[s], 1); }
     for (int s = 0; s < kTmemStages; ++s) { mbar_init(&sh->tmem_full[s], 1); mbar_init(&sh->tmem_empty[s], kEpilogueWarps); }
-    for (int s = 0; s < kItemSlots; ++s) { mbar_init(&sh->item_full[s], 1); mbar_init(&sh->item_empty[s], 1 + kEpilogueWarps); }
+    for (int s = 0; s < kItemSlots; ++s) { mbar_init(&sh->item_full[s], 1); mbar_init(&sh->item_empty[s], 2 + kEpilogueWarps); }
     mbar_init(&sh->exchange_done, kEpilogueWarps);
     sh->wait.abort_flag = 0;
     sh->wait.budget_kiloclocks = p.wait_kiloclocks;
@@ -268,6 +296,52 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
       }
     }
+  } else if (warp == 2) {
+    // ------------------------------ scale loader --------------------------------------
+    // Brings the scales of a K block (one per row of the tile, one per 128 columns) into a shared-memory ring and
+    // announces them with the operands of the block kScaleAhead before it: a complete partial product implies that the
+    // scales of the next one are there, so the epilogue waits once per block and reads them a block ahead.  (Each epilogue
+    // thread loading its own scales a few blocks ahead into registers paid one round trip to L2 per block, because handing
+    // a register on from block to block waits for the load behind it; a barrier of their own cost 150 clocks per block,
+    // and reading them when they are needed 75 to 170, since the reads queue behind the tensor core's operand reads.)
+    const int sfb_rows = p.b_rows_per_group / 128;
+    uint32_t it = 0, k = 0;
+    bool ok = true;
+    Item item;
+    for (int g = blockIdx.x; ok; g += gridDim.x, ++k) {
+      if (p.queue) {                   // the k-th item of this CTA, as drawn by the TMA warp
+        const int slot = k % kItemSlots;
+        ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
+        if (!ok) break;
+        g = sh->item_q[slot];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->item_empty[slot]);
+        if (g < 0) break;
+      }
+      if (!locate(sh, p, n_tiles, g, &item)) break;
+      // lanes 0 and 1 also fetch sfb: of x1 and x2 in the gate/up mode, else of the tile's two 128-column halves
+      const int sfb_row = MODE == kGateUp ? item.n_tile + (lane & 1) * (p.n / 128) : min(item.n_tile * 2 + (lane & 1), sfb_rows - 1);
+      const float* sfb = p.sfb + (size_t(item.group) * sfb_rows + sfb_row) * p.b_k_blocks;
+      for (int kb = 0; ok && kb < p.k_blocks; ++kb, ++it) {
+        ok = it < kScaleAhead || mbar_wait(&sh->empty[(it - kScaleAhead) % kStages], (((it - kScaleAhead) / kStages) & 1) ^ 1, abort_flag,
+                                           p.status, kStatusWaitSmemEmpty);
+        if (!ok) break;
+        int a_col = kb, b_col = kb;
+        if (p.interleave_hi_lo) { a_col = (kb & 1) * (p.k_blocks >> 1) + (kb >> 1); b_col = kb >> 1; }
+        const float* sfa = p.sfa + size_t(a_col) * p.row_capacity;
+        const int slot = it % kScaleSlots;
+#pragma unroll
+        for (int j = 0; j < kBM; j += 32)
+          cp_async_4(&sh->scale_a[slot][j + lane], sfa + min(item.row0 + j + lane, p.row_capacity - 1));
+        if (lane < 2) cp_async_4(&sh->scale_b[slot][lane], sfb + b_col);
+        if (it >= kScaleAhead) cp_async_arrive_noinc(&sh->full[(it - kScaleAhead) % kStages]);
+      }
+    }
+    for (uint32_t j = it < kScaleAhead ? 0 : it - kScaleAhead; ok && j < it; ++j) {       // the last blocks announce no further scales
+      ok = mbar_wait(&sh->empty[j % kStages], ((j / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
+      if (ok) cp_async_arrive_noinc(&sh->full[j % kStages]);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
@@ -281,7 +355,6 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     // columns; the other modes take 128 consecutive columns.
     const int seg_col0 = (MODE == kGateUp) ? cg * 64 : cg * 128;
     const int seg_col1 = (MODE == kGateUp) ? 128 + cg * 64 : cg * 128 + 64;
-    const int sfb_rows = p.b_rows_per_group / 128;
     uint32_t it = 0, k = 0;
     uint32_t exchanges = 0;                    // amax exchanges so far (phase of Shared::exchange_done)
     int parity = 0;
@@ -299,105 +372,61 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       }
       if (!locate(sh, p, n_tiles, g, &item)) break;
       const int row = item.row0 + r;
-      const int row_c = min(row, p.row_capacity - 1);
-      int sfb_row0, sfb_row1;
-      if (MODE == kGateUp) {
-        sfb_row0 = item.n_tile;
-        sfb_row1 = p.n / 128 + item.n_tile;
-      } else {
-        sfb_row0 = sfb_row1 = min(item.n_tile * 2 + cg, sfb_rows - 1);
-      }
-      const float* sfb0 = p.sfb + (size_t(item.group) * sfb_rows + sfb_row0) * p.b_k_blocks;
-      const float* sfb1 = p.sfb + (size_t(item.group) * sfb_rows + sfb_row1) * p.b_k_blocks;
-      float acc[128];
+      uint64_t acc2[64];                        // 128 fp32 accumulators as packed pairs
 #pragma unroll
-      for (int i = 0; i < 128; ++i) acc[i] = 0.f;
-      // Scales travel kScaleAhead K blocks ahead of their use: an L2 round trip under a full TMA
-      // stream is longer than one K block, and a scale that arrives late stalls the whole promotion.
-      constexpr int kScaleAhead = 3;
-      float sa_q[kScaleAhead], sb0_q[kScaleAhead], sb1_q[kScaleAhead];
-      auto fetch = [&](int kb, float& sa, float& sb0, float& sb1) {
-        int a_col = kb, b_col = kb;
-        if (p.interleave_hi_lo) { a_col = (kb & 1) * (p.k_blocks >> 1) + (kb >> 1); b_col = kb >> 1; }
-        sa = __ldg(p.sfa + size_t(a_col) * p.row_capacity + row_c);
-        sb0 = __ldg(sfb0 + b_col);
-        sb1 = __ldg(sfb1 + b_col);
+      for (int i = 0; i < 64; ++i) acc2[i] = 0;
+      float sa = 0.f, sb0 = 0.f, sb1 = 0.f;    // scales of the coming block
+      auto read_scales = [&](uint32_t block) {
+        sa = sh->scale_a[block % kScaleSlots][r];
+        sb0 = sh->scale_b[block % kScaleSlots][MODE == kGateUp ? 0 : cg];
+        if (MODE == kGateUp) sb1 = sh->scale_b[block % kScaleSlots][1];
       };
-#pragma unroll
-      for (int j = 0; j < kScaleAhead; ++j) {
-        sa_q[j] = sb0_q[j] = sb1_q[j] = 0.f;
-        if (j < p.k_blocks) fetch(j, sa_q[j], sb0_q[j], sb1_q[j]);
-      }
-      // A warp none of whose 32 rows exists (the tail tile of a group), or whose columns lie past N, only hands
-      // the accumulator stages back: no tensor-memory reads, no arithmetic.  Not in the gate/up mode: there the
-      // tail tile of a group runs beside the group's full tile on a neighbouring SM over the same 56 K blocks of
-      // weights, and a tail tile that skips its promotion runs so far ahead that the weights it fetched have left
-      // L2 again when the full tile asks for them (measured: 11 % more DRAM traffic and 10 % more time).
-      const bool warp_active = MODE == kGateUp || (quad * 32 < item.rows_valid && item.n_tile * kBN + cg * 128 < p.n);
-      for (int kb = 0; !warp_active && kb < p.k_blocks; ++kb, ++it) {
+      if (it > 0) read_scales(it);
+      for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
         const int t = it % kTmemStages;
-        ok = mbar_wait(&sh->tmem_full[t], (it / kTmemStages) & 1, abort_flag, p.status, kStatusWaitTmemFull);
-        if (!ok) break;
-        if (lane == 0) mbar_arrive(&sh->tmem_empty[t]);
-      }
-      for (int kb = 0; warp_active && kb < p.k_blocks; ++kb, ++it) {
-        const int t = it % kTmemStages;
-        const float s0 = sa_q[0] * sb0_q[0], s1 = sa_q[0] * sb1_q[0];
-#pragma unroll
-        for (int j = 0; j + 1 < kScaleAhead; ++j) { sa_q[j] = sa_q[j + 1]; sb0_q[j] = sb0_q[j + 1]; sb1_q[j] = sb1_q[j + 1]; }
-        if (kb + kScaleAhead < p.k_blocks) fetch(kb + kScaleAhead, sa_q[kScaleAhead - 1], sb0_q[kScaleAhead - 1], sb1_q[kScaleAhead - 1]);
         ok = mbar_wait(&sh->tmem_full[t], (it / kTmemStages) & 1, abort_flag, p.status, kStatusWaitTmemFull);
         if (!ok) break;
         tcgen05_fence_after();
         const uint32_t stage_addr = lane_base + t * kBN;
         // two round trips to tensor memory per K block, 64 columns each
-        float va[32], vb[32];
-        tmem_ld_32x32b_x32(stage_addr + seg_col0, va);
-        tmem_ld_32x32b_x32(stage_addr + seg_col0 + 32, vb);
-        tcgen05_wait_ld();
+        uint64_t v[32];
+        if (it == 0) read_scales(0);
+        const float s0 = sa * sb0, s1 = MODE == kGateUp ? sa * sb1 : s0;
+        tmem_ld_wait_64(stage_addr + seg_col0, v);
+        const uint64_t s0p = pack_f32x2(s0, s0);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          acc[i] = fmaf(va[i], s0, acc[i]);
-          acc[32 + i] = fmaf(vb[i], s0, acc[32 + i]);
-        }
-        tmem_ld_32x32b_x32(stage_addr + seg_col1, va);
-        tmem_ld_32x32b_x32(stage_addr + seg_col1 + 32, vb);
-        tcgen05_wait_ld();
+        for (int i = 0; i < 32; ++i) acc2[i] = fma_f32x2(v[i], s0p, acc2[i]);
+        tmem_ld_wait_64(stage_addr + seg_col1, v);
         tcgen05_fence_before();            // everything this warp needs has left tensor memory
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->tmem_empty[t]);
+        if (kb + 1 < p.k_blocks) read_scales(it + 1);
+        const uint64_t s1p = pack_f32x2(s1, s1);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          acc[64 + i] = fmaf(va[i], s1, acc[64 + i]);
-          acc[96 + i] = fmaf(vb[i], s1, acc[96 + i]);
-        }
+        for (int i = 0; i < 32; ++i) acc2[32 + i] = fma_f32x2(v[i], s1p, acc2[32 + i]);
       }
       if (!ok) break;
+      float acc[128];
+#pragma unroll
+      for (int i = 0; i < 64; ++i) unpack_f32x2(acc2[i], acc[2 * i], acc[2 * i + 1]);
       // rows past the group's end and, where N is an odd multiple of 128, the tile's second column group hold nothing
-      const bool valid = r < item.rows_valid && (MODE == kGateUp || item.n_tile * kBN + cg * 128 < p.n);
+      const bool columns_exist = MODE == kGateUp || item.n_tile * kBN + cg * 128 < p.n;
+      const bool valid = r < item.rows_valid && columns_exist;
 
-      if (MODE == kDense) {
-        if (valid) {
-          __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(row) * p.n + item.n_tile * kBN + cg * 128;
+      if (MODE == kDense || MODE == kDown) {
+        const float w = MODE == kDown && valid ? __ldg(p.row_weight + row) : 1.f;
+        uint8_t* out = reinterpret_cast<uint8_t*>(reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(item.row0 + quad * 32) * p.n + item.n_tile * kBN + cg * 128);
+        const int rows = columns_exist ? item.rows_valid - quad * 32 : 0;
 #pragma unroll
-          for (int i = 0; i < 128; i += 8) {
-            uint4 w;
-            w.x = pack_bf16x2(acc[i], acc[i + 1]); w.y = pack_bf16x2(acc[i + 2], acc[i + 3]);
-            w.z = pack_bf16x2(acc[i + 4], acc[i + 5]); w.w = pack_bf16x2(acc[i + 6], acc[i + 7]);
-            *reinterpret_cast<uint4*>(out + i) = w;
-          }
-        }
-      } else if (MODE == kDown) {
-        if (valid) {
-          const float w = __ldg(p.row_weight + row);
-          __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(row) * p.n + item.n_tile * kBN + cg * 128;
+        for (int c = 0; c < 4; ++c) {            // 32 columns = 64 bytes of each row at a time
+          uint4 v[4];
 #pragma unroll
-          for (int i = 0; i < 128; i += 8) {
-            uint4 v;
-            v.x = pack_bf16x2(acc[i] * w, acc[i + 1] * w); v.y = pack_bf16x2(acc[i + 2] * w, acc[i + 3] * w);
-            v.z = pack_bf16x2(acc[i + 4] * w, acc[i + 5] * w); v.w = pack_bf16x2(acc[i + 6] * w, acc[i + 7] * w);
-            *reinterpret_cast<uint4*>(out + i) = v;
+          for (int i = 0; i < 4; ++i) {
+            const float* a = acc + c * 32 + i * 8;
+            v[i].x = pack_bf16x2(a[0] * w, a[1] * w); v[i].y = pack_bf16x2(a[2] * w, a[3] * w);
+            v[i].z = pack_bf16x2(a[4] * w, a[5] * w); v[i].w = pack_bf16x2(a[6] * w, a[7] * w);
           }
+          warp_store_64(sh->out_rows[ew], v, out + c * 64, size_t(p.n) * 2, rows, lane);
         }
       } else {
         // SwiGLU on the 64 (x1, x2) pairs this thread holds, then e4m3 quantisation of the 128-wide
@@ -411,7 +440,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
         const int out_kb = p.n / 128;                      // K blocks of one term of the output
         const int terms = p.split_act ? 2 : 1;
-        uint8_t* out_base = reinterpret_cast<uint8_t*>(p.out) + size_t(row) * (size_t(p.n) * terms) + item.n_tile * 128 + cg * 64;
+        const size_t out_stride = size_t(p.n) * terms;
+        uint8_t* out = reinterpret_cast<uint8_t*>(p.out) + size_t(item.row0 + quad * 32) * out_stride + item.n_tile * 128 + cg * 64;
         for (int term = 0; term < terms; ++term, ++exchanges) {
           // The two column groups of a row meet through shared memory.  The hand-over is an mbarrier wait like
           // every other wait of the kernel: bounded, and given up when another role has raised the abort flag.
@@ -426,12 +456,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           uint32_t packed[16];
 #pragma unroll
           for (int i = 0; i < 64; i += 4) packed[i >> 2] = pack_e4m3x4(acc[i] * inv, acc[i + 1] * inv, acc[i + 2] * inv, acc[i + 3] * inv);
-          if (valid) {
-            uint4* dst = reinterpret_cast<uint4*>(out_base + size_t(term) * p.n);
+          uint4 v[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) dst[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
-            if (cg == 0) p.out_scale[size_t(term * out_kb + item.n_tile) * p.row_capacity + row] = scale;
-          }
+          for (int i = 0; i < 4; ++i) v[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+          warp_store_64(sh->out_rows[ew], v, out + size_t(term) * p.n, out_stride, item.rows_valid - quad * 32, lane);
+          if (valid && cg == 0) p.out_scale[size_t(term * out_kb + item.n_tile) * p.row_capacity + row] = scale;
           if (term + 1 < terms) {        // residual after the first term becomes the value to quantise
             amax = 0.f;
 #pragma unroll
