@@ -115,6 +115,24 @@ inline int sm_count(int device) {
 }
 
 #ifdef __CUDACC__
+// Launches `kernel` as a programmatic dependent of what the stream holds: it may become resident while that runs, and waits
+// for it on the device (griddepcontrol.wait), which takes a launch latency off the critical path.
+template <typename... Params, typename... Args>
+inline int launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = shared_bytes;
+  config.stream = stream;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  const cudaError_t err = cudaLaunchKernelEx(&config, kernel, args...);
+  return int(err != cudaSuccess ? err : cudaGetLastError());
+}
+
 // ---------------------------------------------------------------------------------------
 // Device helpers
 // ---------------------------------------------------------------------------------------
@@ -474,6 +492,12 @@ __device__ __forceinline__ void unpack_f32x2(uint64_t p, float& lo, float& hi) {
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 

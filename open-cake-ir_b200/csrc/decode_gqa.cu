@@ -22,6 +22,7 @@
 // a (sequence, KV head) merges the pieces and writes the output, so there is no reduce launch.
 #include "common.cuh"
 #include "prefill.cuh"
+#include "prefill_gqa.cuh"
 #include "../../include/cake_b200.h"
 #include <mutex>
 #include <new>
@@ -579,18 +580,7 @@ inline int launch(Params& p, int sms, cudaStream_t s) {
   gqa_plan_kernel<<<1, 1024, 0, s>>>(p);
   // The decode grid is a programmatic dependent: it may start while the plan kernel runs and waits
   // for it on the device, which takes the second launch latency off the critical path.
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(grid);
-  config.blockDim = dim3(kWarps * 32);
-  config.dynamicSmemBytes = kSmemBytes;
-  config.stream = s;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute[0].val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = attribute;
-  config.numAttrs = 1;
-  const cudaError_t err = cudaLaunchKernelEx(&config, gqa_decode_kernel, p);
-  return int(err != cudaSuccess ? err : cudaGetLastError());
+  return launch_dependent(gqa_decode_kernel, dim3(grid), dim3(kWarps * 32), kSmemBytes, s, p);
 }
 
 }  // namespace gqa
@@ -760,7 +750,25 @@ struct PrefillHandle {
   const int *qo_indptr, *kv_indptr_segments, *last_page_len;
   int *seq_start, *seq_tokens, *masked;
   int segments, total_q, kv_unit, nan_for_masked;
+  bool tiled;                      // query tiles that share KV tiles (prefill_gqa.cuh) instead of a decode sequence per query token
+  gqa_prefill::Params t;
 };
+
+// Which of the two forms a launch takes, from what the host knows (lengths live on the device; max_kv_len bounds them).
+// The tiled form works through ceil(kv / 128) KV tiles one after another, about 1.9 us each, on as many SMs as there are
+// (query tile, KV head) pairs; the decode form reads the KV rows once per query token, at about 7 TB/s once L2 holds
+// them, but spreads any amount of work over the whole GPU.  So the decode form stays the better one for a few query
+// rows behind a long prefix.
+inline bool use_tiles(const cake_b200_gqa_prefill_config& c) {
+  const double tiles = double((c.total_q + gqa_prefill::tokens_per_tile(c.num_qo_heads / c.num_kv_heads) - 1) / gqa_prefill::tokens_per_tile(c.num_qo_heads / c.num_kv_heads) + c.segments - 1) * c.num_kv_heads;
+  const double tiled_us = (tiles > 148 ? tiles / 148 : 1.0) * double((c.max_kv_len + 127) / 128) * 1.9;
+  const double decode_us = 10.0 + double(c.total_q) * double(c.max_kv_len) * c.num_kv_heads * 512 / 7e6;
+  return tiled_us <= decode_us;
+}
+inline size_t tile_list_bytes(const cake_b200_gqa_prefill_config& c) {
+  const size_t n = size_t(gqa_prefill::tile_capacity(c.total_q, c.segments, c.num_qo_heads / c.num_kv_heads));
+  return align256(n * sizeof(int4)) + align256((n + 1) * sizeof(int)) + align256(size_t(c.segments + 3) * sizeof(int));
+}
 }  // namespace gqa
 }  // namespace cake
 
@@ -780,7 +788,9 @@ static bool gqa_prefill_config_ok(const cake_b200_gqa_prefill_config& c, cake_b2
 extern "C" size_t cake_b200_gqa_prefill_workspace_bytes(const cake_b200_gqa_prefill_config* c) {
   cake_b200_gqa_decode_config d;
   if (!c || !gqa_prefill_config_ok(*c, &d)) return 0;
-  return cake_b200_gqa_decode_workspace_bytes(&d) + cake::prefill::table_bytes(c->total_q);
+  const size_t decode_form = cake_b200_gqa_decode_workspace_bytes(&d) + cake::prefill::table_bytes(c->total_q);
+  const size_t tiled_form = 512 + cake::gqa::tile_list_bytes(*c);
+  return decode_form > tiled_form ? decode_form : tiled_form;
 }
 
 extern "C" int cake_b200_gqa_prefill_create(void** buffers, const cake_b200_gqa_prefill_config* config, void** handle_out) {
@@ -827,9 +837,26 @@ extern "C" int cake_b200_gqa_prefill_create(void** buffers, const cake_b200_gqa_
   h->total_q = int(config->total_q);
   h->kv_unit = d.page_size;
   h->nan_for_masked = config->nan_for_masked;
+  h->tiled = gqa::use_tiles(*config);
+  gqa_prefill::Params& t = h->t;
+  t = gqa_prefill::Params{p.q, p.k_cache, p.v_cache, h->qo_indptr, h->kv_indptr_segments, p.kv_indices, h->last_page_len, p.sm_scale, p.out, p.lse};
+  t.status = p.status;
+  t.total_q = h->total_q;
+  t.segments = h->segments;
+  t.hq = p.hq;
+  t.hkv = p.hkv;
+  t.group = p.hq / p.hkv;
+  t.page_size = p.page_size;
+  t.nan_for_masked = h->nan_for_masked;
+  t.capacity = gqa_prefill::tile_capacity(t.total_q, t.segments, t.group);
+  t.tiles = reinterpret_cast<int4*>(ws);
+  t.tile_page = reinterpret_cast<int*>(ws + gqa::align256(size_t(t.capacity) * sizeof(int4)));
+  t.tile_count = t.tile_page + t.capacity;
+  t.prefix = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(t.tile_page) + gqa::align256(size_t(t.capacity + 1) * sizeof(int)));
   int sms = 0;
   int rc = gqa_sm_count(device, &sms);
   if (!rc) rc = int(cudaFuncSetAttribute(gqa::gqa_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gqa::kSmemBytes));
+  if (!rc) rc = int(cudaFuncSetAttribute(gqa_prefill::prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gqa_prefill::kSmemBytes)));
   if (rc) { delete h; return rc; }
   h->sms = sms < gqa::kMaxSms ? sms : gqa::kMaxSms;
   *handle_out = h;
@@ -845,6 +872,12 @@ extern "C" int cake_b200_gqa_prefill_launch(void* handle, void* cuda_stream) {
   if (device != h->device) return kErrWrongDevice;
   if (h->total_q == 0) return 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(cuda_stream);
+  if (h->tiled) {
+    gqa_prefill::Params t = h->t;
+    t.wait_kiloclocks = test_hooks().budget_kiloclocks;
+    gqa_prefill::plan_kernel<<<1, 1024, 0, s>>>(t);
+    return launch_dependent(gqa_prefill::prefill_kernel, dim3(unsigned(t.capacity) * t.hkv), dim3(gqa_prefill::kThreads), gqa_prefill::kSmemBytes, s, t);
+  }
   prefill::prefill_plan_kernel<<<(h->total_q + 255) / 256, 256, 0, s>>>(h->qo_indptr, h->kv_indptr_segments, h->last_page_len, h->segments,
                                                                        h->kv_unit, h->total_q, h->seq_start, h->seq_tokens, h->masked);
   gqa::Params p = h->p;
