@@ -876,7 +876,8 @@ extern "C" int cake_b200_gqa_prefill_launch(void* handle, void* cuda_stream) {
     gqa_prefill::Params t = h->t;
     t.wait_kiloclocks = test_hooks().budget_kiloclocks;
     gqa_prefill::plan_kernel<<<1, 1024, 0, s>>>(t);
-    return launch_dependent(gqa_prefill::prefill_kernel, dim3(unsigned(t.capacity) * t.hkv), dim3(gqa_prefill::kThreads), gqa_prefill::kSmemBytes, s, t);
+    const unsigned units = unsigned(t.capacity) * t.hkv;               // an upper bound: the list is made on the device
+    return launch_dependent(gqa_prefill::prefill_kernel, dim3(units < unsigned(h->sms) ? units : unsigned(h->sms)), dim3(gqa_prefill::kThreads), gqa_prefill::kSmemBytes, s, t);
   }
   prefill::prefill_plan_kernel<<<(h->total_q + 255) / 256, 256, 0, s>>>(h->qo_indptr, h->kv_indptr_segments, h->last_page_len, h->segments,
                                                                        h->kv_unit, h->total_q, h->seq_start, h->seq_tokens, h->masked);

@@ -1,7 +1,7 @@
 // Causal GQA prefill for sm_100a: query tiles against shared KV tiles on tcgen05 (flash attention, no split).
 //
 // Operator: the prefill branches of src/open_cake_ir/tasks/solx_fib/attention.py:132-183 (attention_specs.py:85-248), see
-// prefill.cuh for the masking rules.  A CTA owns one KV head and a tile of consecutive query tokens of one segment; the
+// prefill.cuh for the masking rules.  A unit of work is one KV head and a tile of consecutive query tokens of one segment; the
 // G = Hq/Hkv query heads that share the KV head are packed beside the tokens as rows, 128 / G tokens to an M = 128 tile,
 // two such tiles (A and B) to a CTA, so a 128-token K/V tile brought into shared memory serves 256 rows.
 //   S[128 x 128]  = Q . K^T      both from shared memory, K-major
@@ -14,8 +14,8 @@
 // and about 750 issue slots per warp.  Two row tiles with a softmax warpgroup each keep the pipe busy: the products of
 // one run while the other's softmax does ([P V of A(j), S of A(j+1)], [P V of B(j), S of B(j+1)], ...).
 // Running each query token as a decode sequence of its own read every KV row once per query token instead.
-// Roles: warp 0 issues the products, warps 1..3 gather K and V rows (cp.async through the page table, any page size; the
-// copies announce themselves on the stage's barrier), warps 4..7 and 8..11 are the softmax of tiles A and B.  Every wait
+// Roles: warp 0 issues the products, warps 4..7 gather Q, K and V rows (cp.async through the page table, any page size; the
+// copies announce themselves on the stage's barrier), warps 8..11 and 12..15 are the softmax of tiles A and B.  Every wait
 // is bounded and reports through the status word.
 #pragma once
 #include "common.cuh"
@@ -30,10 +30,11 @@ constexpr int kTile = 128;                       // KV rows per tile
 constexpr int kStages = 2;                       // K and V ring depth (each)
 constexpr int kSlabBytes = 128 * 128;            // 128 rows x 64 elements
 constexpr int kTileBytes = 2 * kSlabBytes;       // 32 KiB: 128 rows of 128 bf16
-constexpr int kLoaderWarps = 3;
-constexpr int kThreads = 384;
-constexpr int kControlRegs = 72, kSoftmaxRegs = 216;
-static_assert(128 * kControlRegs + 256 * kSoftmaxRegs <= (65536 / kThreads / 8 * 8) * kThreads, "setmaxnreg budget exceeds the launch's registers");
+constexpr int kLoaderWarp0 = 4, kLoaderWarps = 4;      // warp 0 issues the products; warps 1..3 only take part in the barriers
+constexpr int kSoftmaxWarp0 = 8;                 // two warpgroups: warp % 4 = TMEM lane quadrant
+constexpr int kThreads = 512;
+constexpr int kControlRegs = 72, kSoftmaxRegs = 184;
+static_assert(256 * kControlRegs + 256 * kSoftmaxRegs <= (65536 / kThreads / 8 * 8) * kThreads, "setmaxnreg budget exceeds the launch's registers");
 constexpr uint32_t kColS = 0, kColO = 256, kTmemColumns = 512;        // tile X: S at kColS + 128 X, O at kColO + 128 X
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleThreshold = 8.f;         // log2 units: O is rescaled when the running maximum grows by more
@@ -55,11 +56,12 @@ struct Params {
 
 struct Shared {
   uint64_t k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages];
-  uint64_t s_full[2], p_ready[2], o_done[2];     // per query tile
+  uint64_t q_full[2], q_empty[2], s_full[2], p_ready[2][2], o_done[2];     // per query tile; p_ready: per half of P
   uint32_t tmem_base;
   WaitControl wait;
 };
-constexpr size_t kSmemBytes = size_t(2 + 2 * kStages) * kTileBytes + sizeof(Shared) + 1024;
+constexpr int kOutBytes = 8 * 32 * 128;          // per softmax warp: 32 rows of 128 bytes on their way out
+constexpr size_t kSmemBytes = size_t(2 + 2 * kStages) * kTileBytes + kOutBytes + sizeof(Shared) + 1024;
 static_assert(kSmemBytes <= 232448, "the kernel's shared memory exceeds what a CTA may have on sm_100");
 
 inline int tokens_per_tile(int group) { return 2 * (kRows / group); }
@@ -136,6 +138,11 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool valid) {
   const int bytes = valid ? 16 : 0;              // 0 source bytes = zero fill
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -145,63 +152,70 @@ __device__ __forceinline__ uint32_t row_off(int row, int chunk) {
   return uint32_t((chunk >> 3) * kSlabBytes + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
 }
 
+// One unit of work as every role reads it from the list.
+struct Work {
+  int q0, rows, first_visible, kv_len, page_base, kvh;
+  int n_kv[2], n;                                  // KV tiles each query tile sees; the larger of the two
+};
+// The k-th unit of this CTA, false past the end.  CTA c takes entries c, 2g-1-c, 2g+c, ... of the (tile, KV head) list, which
+// is sorted by length: turning round every other time evens out what a CTA gets.
+__device__ __forceinline__ bool get_work(const Params& p, int units, int k, Work* w) {
+  const int g = gridDim.x;
+  const int u = k * g + ((k & 1) ? g - 1 - int(blockIdx.x) : int(blockIdx.x));
+  if (u >= units) return false;
+  const int index = u / p.hkv;
+  w->kvh = u - index * p.hkv;
+  const int4 tile = __ldg(p.tiles + index);
+  w->page_base = __ldg(p.tile_page + index);
+  w->q0 = tile.x; w->rows = tile.y; w->first_visible = tile.z; w->kv_len = tile.w;
+  const int per_half = kRows / p.group;
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    const int mine = min(w->rows - x * per_half, per_half);
+    const int last = mine > 0 ? min(w->kv_len, w->first_visible + x * per_half + mine - 1) : 0;
+    w->n_kv[x] = last > 0 ? (last + kTile - 1) / kTile : 0;
+  }
+  w->n = max(w->n_kv[0], w->n_kv[1]);
+  return true;
+}
+
 static __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t q_addr = smem_u32(base), k_addr = q_addr + 2 * kTileBytes, v_addr = k_addr + kStages * kTileBytes;
-  Shared* sh = reinterpret_cast<Shared*>(base + (2 + 2 * kStages) * kTileBytes);
+  uint8_t* out_rows = base + (2 + 2 * kStages) * kTileBytes;
+  Shared* sh = reinterpret_cast<Shared*>(out_rows + kOutBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.x % p.hkv, index = blockIdx.x / p.hkv;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&sh->k_full[s], kLoaderWarps * 32); mbar_init(&sh->k_empty[s], 1);
       mbar_init(&sh->v_full[s], kLoaderWarps * 32); mbar_init(&sh->v_empty[s], 1);
     }
-    for (int x = 0; x < 2; ++x) { mbar_init(&sh->s_full[x], 1); mbar_init(&sh->p_ready[x], 4); mbar_init(&sh->o_done[x], 1); }
+    for (int x = 0; x < 2; ++x) {
+      mbar_init(&sh->q_full[x], kLoaderWarps * 32); mbar_init(&sh->q_empty[x], 1);
+      mbar_init(&sh->s_full[x], 1); mbar_init(&sh->o_done[x], 1);
+      mbar_init(&sh->p_ready[x][0], 4); mbar_init(&sh->p_ready[x][1], 4);
+    }
     sh->wait.abort_flag = 0;
     sh->wait.budget_kiloclocks = p.wait_kiloclocks;
     fence_barrier_init();
   }
-  // launched as a programmatic dependent of the plan kernel: the list is read only after that grid has completed
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (index >= *p.tile_count) return;              // the whole CTA leaves together
-  const int4 tile = p.tiles[index];
-  const int page_base = p.tile_page[index];
-  const int q0 = tile.x, rows = tile.y, first_visible = tile.z, kv_len = tile.w;
-  const int per_half = kRows / p.group;            // query tokens per M tile
-  int n_kv[2];                                     // KV tiles each query tile sees
-#pragma unroll
-  for (int x = 0; x < 2; ++x) {
-    const int mine = min(rows - x * per_half, per_half);
-    const int last = mine > 0 ? min(kv_len, first_visible + x * per_half + mine - 1) : 0;
-    n_kv[x] = last > 0 ? (last + kTile - 1) / kTile : 0;
-  }
-  const int n = max(n_kv[0], n_kv[1]);
-
   if (warp == 0) {
     tmem_alloc(&sh->tmem_base, kTmemColumns);
     tmem_relinquish();
   }
-  // Q rows: token q0 + x * per_half + r / G, head kvh * G + r % G; rows without a token are zeros
-  if (n > 0) {
-    for (int i = threadIdx.x; i < 2 * kRows * 16; i += kThreads) {
-      const int x = i >> 11, r = (i >> 4) & 127, chunk = i & 15;
-      const int token = x * per_half + r / p.group;
-      const bool valid = r < per_half * p.group && token < rows;
-      const __nv_bfloat16* src = p.q + (size_t(q0 + (valid ? token : 0)) * p.hq + kvh * p.group + r % p.group) * kD + chunk * 8;
-      cp_async_16(q_addr + x * kTileBytes + row_off(r, chunk), src, valid);
-    }
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  fence_proxy_async_smem();
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   volatile int* abort_flag = &sh->wait.abort_flag;
+  const int per_half = kRows / p.group;            // query tokens per M tile
+  // launched as a programmatic dependent of the plan kernel: the list is read only after that grid has completed
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int units = *p.tile_count * p.hkv;
 
-  if (warp < 4) {
+  if (warp < kSoftmaxWarp0) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kControlRegs));
     if (warp == 0) {
       // ------------------------------ MMA issuer --------------------------------------
@@ -209,8 +223,11 @@ prefill_kernel(const Params p) {
         constexpr uint32_t idesc_qk = umma_idesc_ex(1 /* bf16 */, kRows, kTile, 0, 0);
         constexpr uint32_t idesc_pv = umma_idesc_ex(1 /* bf16 */, kRows, kD, 0, 1 /* V is MN-major */);
         bool ok = true;
-        auto issue_qk = [&](int x, int j) {
-          const uint64_t a = umma_desc_sw128(q_addr + x * kTileBytes), b = umma_desc_sw128(k_addr + (j % kStages) * kTileBytes);
+        uint32_t it = 0;                           // KV tiles so far
+        uint32_t products[2] = {0, 0}, loads[2] = {0, 0};      // per query tile: KV tiles and Q blocks so far
+        Work w;
+        auto issue_qk = [&](int x, uint32_t i) {
+          const uint64_t a = umma_desc_sw128(q_addr + x * kTileBytes), b = umma_desc_sw128(k_addr + (i % kStages) * kTileBytes);
 #pragma unroll
           for (int step = 0; step < kD / 16; ++step) {
             const uint64_t off = uint64_t(((step >> 2) * kSlabBytes + (step & 3) * 32) >> 4);
@@ -218,209 +235,259 @@ prefill_kernel(const Params p) {
           }
           tcgen05_commit(&sh->s_full[x]);
         };
-        auto k_ready = [&](int j) {
-          ok = mbar_wait(&sh->k_full[j % kStages], (j / kStages) & 1, abort_flag, p.status, kStatusWaitSmemFull);
+        auto k_ready = [&](uint32_t i) {
+          ok = mbar_wait(&sh->k_full[i % kStages], (i / kStages) & 1, abort_flag, p.status, kStatusWaitSmemFull);
           fence_proxy_async_smem();                // the rows were written through the generic proxy
           tcgen05_fence_after();
         };
-        if (n > 0) {
-          k_ready(0);
-          if (ok) {
-            for (int x = 0; x < 2; ++x) if (n_kv[x] > 0) issue_qk(x, 0);
-            tcgen05_commit(&sh->k_empty[0]);
-          }
-        }
-        for (int j = 0; ok && j < n; ++j) {
-          const int s = j % kStages;
-          ok = mbar_wait(&sh->v_full[s], (j / kStages) & 1, abort_flag, p.status, kStatusWaitSmemFull);
-          if (!ok) break;
-          fence_proxy_async_smem();
-          const uint64_t v_base = umma_desc_sw128_ex(v_addr + s * kTileBytes, kSlabBytes, 1024);
-          bool k_waited = false;
+        for (int k = 0; ok && get_work(p, units, k, &w); ++k) {
+          if (w.n == 0) continue;
+          k_ready(it);
+#pragma unroll 1
           for (int x = 0; ok && x < 2; ++x) {
-            if (j >= n_kv[x]) continue;
-            ok = mbar_wait(&sh->p_ready[x], j & 1, abort_flag, p.status, kStatusWaitFlag);
+            if (w.n_kv[x] == 0) continue;
+            ok = mbar_wait(&sh->q_full[x], loads[x]++ & 1, abort_flag, p.status, kStatusWaitSmemFull);
             if (!ok) break;
-            tcgen05_fence_after();
-#pragma unroll
-            for (int term = 0; term < 2; ++term)
-#pragma unroll
-              for (int ks = 0; ks < kTile / 16; ++ks)
-                umma_f16_a_tmem(tmem_base + kColO + x * kD, tmem_base + kColS + x * kTile + term * (kTile / 2) + ks * 8,
-                                v_base + uint64_t((ks * 2048) >> 4), idesc_pv, (j | term | ks) != 0);
-            tcgen05_commit(&sh->o_done[x]);
-            // The logits of the next tile go where P of this one lies: the pipe runs one thread's products in order
-            if (j + 1 < n_kv[x]) {
-              if (!k_waited) { k_ready(j + 1); k_waited = true; }
-              if (ok) issue_qk(x, j + 1);
-            }
+            fence_proxy_async_smem();
+            issue_qk(x, it);
+            if (w.n_kv[x] == 1) tcgen05_commit(&sh->q_empty[x]);
           }
           if (!ok) break;
-          tcgen05_commit(&sh->v_empty[s]);
-          if (k_waited) tcgen05_commit(&sh->k_empty[(j + 1) % kStages]);
+          tcgen05_commit(&sh->k_empty[it % kStages]);
+          for (int j = 0; ok && j < w.n; ++j, ++it) {
+            const int s = it % kStages;
+            ok = mbar_wait(&sh->v_full[s], (it / kStages) & 1, abort_flag, p.status, kStatusWaitSmemFull);
+            if (!ok) break;
+            fence_proxy_async_smem();
+            const uint64_t v_base = umma_desc_sw128_ex(v_addr + s * kTileBytes, kSlabBytes, 1024);
+            bool k_waited = false;
+#pragma unroll 1
+            for (int x = 0; ok && x < 2; ++x) {
+              if (j >= w.n_kv[x]) continue;
+              // P comes in two halves of 64 KV rows, so that the product starts while the second half is being made
+#pragma unroll
+              for (int half = 0; half < 2; ++half) {
+                ok = ok && mbar_wait(&sh->p_ready[x][half], products[x] & 1, abort_flag, p.status, kStatusWaitFlag);
+                if (!ok) break;
+                tcgen05_fence_after();
+#pragma unroll
+                for (int term = 0; term < 2; ++term)
+#pragma unroll
+                  for (int ks = half * 4; ks < half * 4 + 4; ++ks)
+                    umma_f16_a_tmem(tmem_base + kColO + x * kD, tmem_base + kColS + x * kTile + (ks >> 1) * 32 + term * 16 + (ks & 1) * 8,
+                                    v_base + uint64_t((ks * 2048) >> 4), idesc_pv, (j | half | term | (ks & 3)) != 0);
+              }
+              if (!ok) break;
+              ++products[x];
+              tcgen05_commit(&sh->o_done[x]);
+              // The logits of the next tile go where P of this one lies: the pipe runs one thread's products in order
+              if (j + 1 < w.n_kv[x]) {
+                if (!k_waited) { k_ready(it + 1); k_waited = true; }
+                if (ok) issue_qk(x, it + 1);
+                if (ok && j + 2 == w.n_kv[x]) tcgen05_commit(&sh->q_empty[x]);
+              }
+            }
+            if (!ok) break;
+            tcgen05_commit(&sh->v_empty[s]);
+            if (k_waited) tcgen05_commit(&sh->k_empty[(it + 1) % kStages]);
+          }
         }
       }
-    } else {
-      // ------------------------------ K/V loader --------------------------------------
-      // Row pairs (two rows of 256 bytes per instruction) go round the three warps.  A lane looks up the page of four rows
-      // of a tile, a tile ahead of their use, and hands the row numbers round by shuffle.
-      const int w = warp - 1;
-      auto lookup = [&](int j, int i) {
-        const int token = j * kTile + i * 32 + lane;
-        if (token >= kv_len) return -1;
-        if (!p.kv_indices) return page_base + token;
-        return __ldg(p.kv_indices + page_base + token / p.page_size) * p.page_size + token % p.page_size;      // < 2^31 rows
-      };
-      int row[4], next[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) row[i] = n > 0 ? lookup(0, i) : -1;
+    } else if (warp >= kLoaderWarp0) {
+      // ------------------------------ loader ------------------------------------------
+      // Row pairs (two rows of 256 bytes per instruction): a warp takes 32 of a tile's rows, whose pages its lanes look up a
+      // tile ahead of their use and hand round by shuffle.
+      const int lw = warp - kLoaderWarp0, chunk = lane & 15;
       bool ok = true;
-      const int chunk = lane & 15;
-      for (int j = 0; j < n; ++j) {
-        const int s = j % kStages;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) next[i] = j + 1 < n ? lookup(j + 1, i) : -1;
-#pragma unroll
-        for (int kv = 0; kv < 2; ++kv) {
-          ok = mbar_wait(kv ? &sh->v_empty[s] : &sh->k_empty[s], ((j / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
+      uint32_t it = 0, loads[2] = {0, 0};
+      Work w;
+      for (int k = 0; ok && get_work(p, units, k, &w); ++k) {
+        if (w.n == 0) continue;
+        auto lookup = [&](int j) {
+          const int token = j * kTile + lw * 32 + lane;
+          if (token >= w.kv_len) return -1;
+          if (!p.kv_indices) return w.page_base + token;
+          return __ldg(p.kv_indices + w.page_base + token / p.page_size) * p.page_size + token % p.page_size;      // < 2^31 rows
+        };
+        int row = lookup(0);
+        // Q rows: token q0 + x * per_half + r / G, head kvh * G + r % G; rows without a token are zeros
+        for (int x = 0; ok && x < 2; ++x) {
+          if (w.n_kv[x] == 0) continue;
+          ok = mbar_wait(&sh->q_empty[x], (loads[x]++ & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
           if (!ok) break;
-          const __nv_bfloat16* src = (kv ? p.v : p.k) + size_t(kvh) * kD + chunk * 8;
-          const uint32_t dst = (kv ? v_addr : k_addr) + s * kTileBytes;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
 #pragma unroll 4
-            for (int pair = (w + 3 - (i * 16) % 3) % 3; pair < 16; pair += kLoaderWarps) {
-              const int r = pair * 2 + (lane >> 4);
-              const int at = __shfl_sync(0xffffffffu, row[i], r);
-              cp_async_16(dst + row_off(i * 32 + r, chunk), src + size_t(at < 0 ? 0 : at) * p.hkv * kD, at >= 0);
-            }
+          for (int pair = lw * 16; pair < lw * 16 + 16; ++pair) {
+            const int r = pair * 2 + (lane >> 4), token = x * per_half + r / p.group;
+            const bool valid = r < per_half * p.group && token < w.rows;
+            cp_async_16(q_addr + x * kTileBytes + row_off(r, chunk),
+                        p.q + (size_t(w.q0 + (valid ? token : 0)) * p.hq + w.kvh * p.group + r % p.group) * kD + chunk * 8, valid);
           }
-          cp_async_arrive_noinc(kv ? &sh->v_full[s] : &sh->k_full[s]);
+          cp_async_arrive_noinc(&sh->q_full[x]);
         }
-        if (!ok) break;
+        for (int j = 0; ok && j < w.n; ++j, ++it) {
+          const int s = it % kStages;
+          const int next = j + 1 < w.n ? lookup(j + 1) : -1;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) row[i] = next[i];
+          for (int kv = 0; kv < 2; ++kv) {
+            ok = mbar_wait(kv ? &sh->v_empty[s] : &sh->k_empty[s], ((it / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
+            if (!ok) break;
+            const __nv_bfloat16* src = (kv ? p.v : p.k) + size_t(w.kvh) * kD + chunk * 8;
+            const uint32_t dst = (kv ? v_addr : k_addr) + s * kTileBytes;
+#pragma unroll
+            for (int pair = 0; pair < 16; ++pair) {
+              const int r = pair * 2 + (lane >> 4);
+              const int at = __shfl_sync(0xffffffffu, row, r);
+              cp_async_16(dst + row_off(lw * 32 + r, chunk), src + size_t(at < 0 ? 0 : at) * p.hkv * kD, at >= 0);
+            }
+            cp_async_arrive_noinc(kv ? &sh->v_full[s] : &sh->k_full[s]);
+          }
+          if (!ok) break;
+          row = next;
+        }
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
     // ------------------------------ softmax / output -------------------------------------
-    const int x = (warp - 4) >> 2, quad = warp & 3;
+    const int x = (warp - kSoftmaxWarp0) >> 2, quad = warp & 3;
     const int r = quad * 32 + lane;                // row of the query tile = TMEM lane
     const uint32_t lane_base = tmem_base + (uint32_t(quad * 32) << 16);
     const uint32_t s_col = lane_base + kColS + x * kTile, o_col = lane_base + kColO + x * kD;
     const float scale2 = __ldg(p.sm_scale) * kLog2e;
     const bool scale_positive = scale2 > 0.f;      // the contract's scales are; any other is applied to the logits first
     const float pre = scale_positive ? 1.f : scale2, post = scale_positive ? scale2 : 1.f;
-    const int token = x * per_half + r / p.group;
-    const bool exists = r < per_half * p.group && token < rows;
-    const int visible = exists ? min(kv_len, first_visible + token) : 0;      // KV rows this row sees
-    const int tiles = x ? n_kv[1] : n_kv[0];
-    float m_ref = -INFINITY, l = 0.f;
+    const int token = x * per_half + r / p.group, head_in_group = r % p.group;
+    const bool slot = r < per_half * p.group;
+    uint4* scratch = reinterpret_cast<uint4*>(out_rows + (warp - kSoftmaxWarp0) * (32 * 128));
     bool ok = true;
-    for (int j = 0; j < tiles; ++j) {
-      ok = mbar_wait(&sh->s_full[x], j & 1, abort_flag, p.status, kStatusWaitTmemFull);
-      if (!ok) break;
-      tcgen05_fence_after();
-      float sc[kTile];
+    uint32_t done = 0;                             // KV tiles so far
+    Work w;
+    for (int k = 0; ok && get_work(p, units, k, &w); ++k) {
+      const bool exists = slot && token < w.rows;
+      const int visible = exists ? min(w.kv_len, w.first_visible + token) : 0;      // KV rows this row sees
+      const int tiles = x ? w.n_kv[1] : w.n_kv[0];
+      float m_ref = -INFINITY, l = 0.f;
+      for (int j = 0; j < tiles; ++j, ++done) {
+        ok = mbar_wait(&sh->s_full[x], done & 1, abort_flag, p.status, kStatusWaitTmemFull);
+        if (!ok) break;
+        tcgen05_fence_after();
+        // The logits are read twice, once for the maximum and once for the weights, 32 columns at a time: all 128 in
+        // registers spill.  P of 32 KV rows (16 columns of values, 16 of residuals) goes over the logits it comes from.
+        const int limit = visible - j * kTile;     // columns at and past it are masked
+        const bool plain = !__any_sync(0xffffffffu, limit < kTile) && scale_positive;
+        float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int c = 0; c < kTile; c += 32) tmem_ld_32x32b_x32(s_col + c, sc + c);
-      tcgen05_wait_ld();
-      const int limit = visible - j * kTile;       // columns at and past it are masked
-      if (__any_sync(0xffffffffu, limit < kTile)) {
+        for (int c = 0; c < kTile; c += 64) {
+          float sc[64];
+          tmem_ld_32x32b_x32(s_col + c, sc);
+          tmem_ld_32x32b_x32(s_col + c + 32, sc + 32);
+          tcgen05_wait_ld();
+          if (!plain) {
 #pragma unroll
-        for (int c = 0; c < kTile; ++c) sc[c] = c < limit ? sc[c] * pre : -INFINITY;
-      } else if (!scale_positive) {
+            for (int i = 0; i < 64; ++i) sc[i] = c + i < limit ? sc[i] * pre : -INFINITY;
+          }
 #pragma unroll
-        for (int c = 0; c < kTile; ++c) sc[c] *= pre;
-      }
-      float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+          for (int i = 0; i < 64; i += 8) {
 #pragma unroll
-      for (int c = 0; c < kTile; c += 2) t4[(c >> 1) & 3] = fmaxf(t4[(c >> 1) & 3], fmaxf(sc[c], sc[c + 1]));
-      const float tmax = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * post;
-      if (j == 0) {
-        m_ref = tmax;
-      } else {
-        const bool need = tmax > m_ref + kRescaleThreshold;
-        if (__any_sync(0xffffffffu, need)) {       // O is about to be rescaled in tensor memory: the product before must have landed
-          ok = mbar_wait(&sh->o_done[x], (j - 1) & 1, abort_flag, p.status, kStatusWaitFlag);
-          if (!ok) break;
-          tcgen05_fence_after();
-          const float alpha = need ? exp2f(m_ref - tmax) : 1.f;
-          if (need) { m_ref = tmax; l *= alpha; }
-#pragma unroll 1
-          for (int c = 0; c < kD; c += 16) {
-            float o[16];
-            tmem_ld_32x32b_x16(o_col + c, o);
-            tcgen05_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] *= alpha;
-            tmem_st_32x32b_x16(o_col + c, reinterpret_cast<const uint32_t*>(o));
+            for (int q = 0; q < 4; ++q) t4[q] = max3(t4[q], sc[i + q], sc[i + 4 + q]);
           }
         }
-      }
-      const float m_use = m_ref == -INFINITY ? 0.f : m_ref;       // a row that sees nothing: weights 0, not NaN
-      const uint64_t post2 = pack_f32x2(post, post), minus_m = pack_f32x2(-m_use, -m_use), minus_one = pack_f32x2(-1.f, -1.f);
-      uint64_t sum2[2] = {0, 0};
+        const float tmax = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * post;
+        if (j == 0) {
+          m_ref = tmax;
+        } else {
+          const bool need = tmax > m_ref + kRescaleThreshold;
+          if (__any_sync(0xffffffffu, need)) {     // O is about to be rescaled in tensor memory: the product before must have landed
+            ok = mbar_wait(&sh->o_done[x], (done - 1) & 1, abort_flag, p.status, kStatusWaitFlag);
+            if (!ok) break;
+            tcgen05_fence_after();
+            const float alpha = need ? exp2f(m_ref - tmax) : 1.f;
+            if (need) { m_ref = tmax; l *= alpha; }
+#pragma unroll 1
+            for (int c = 0; c < kD; c += 16) {
+              float o[16];
+              tmem_ld_32x32b_x16(o_col + c, o);
+              tcgen05_wait_ld();
 #pragma unroll
-      for (int c = 0; c < kTile; c += 32) {
-        uint32_t hi[16], lo[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float a, b;
-          unpack_f32x2(fma_f32x2(pack_f32x2(sc[c + 2 * i], sc[c + 2 * i + 1]), post2, minus_m), a, b);
-          a = ex2(a); b = ex2(b);
-          const uint64_t pair = pack_f32x2(a, b);
-          sum2[i & 1] = add_f32x2(sum2[i & 1], pair);
-          hi[i] = pack_bf16x2(a, b);
-          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(hi[i] << 16), __uint_as_float(hi[i] & 0xffff0000u)), minus_one, pair), a, b);
-          lo[i] = pack_bf16x2(a, b);
+              for (int i = 0; i < 16; ++i) o[i] *= alpha;
+              tmem_st_32x32b_x16(o_col + c, reinterpret_cast<const uint32_t*>(o));
+            }
+          }
         }
-        tmem_st_32x32b_x16(s_col + c / 2, hi);
-        tmem_st_32x32b_x16(s_col + kTile / 2 + c / 2, lo);
-      }
-      tcgen05_wait_st();
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh->p_ready[x]);
-      float a, b;
-      unpack_f32x2(add_f32x2(sum2[0], sum2[1]), a, b);
-      l += a + b;
-    }
-    if (ok && tiles > 0) ok = mbar_wait(&sh->o_done[x], (tiles - 1) & 1, abort_flag, p.status, kStatusWaitFlag);
-    if (ok) {
-      tcgen05_fence_after();
-      // rows leave through this query tile's Q block (every product that read it has completed): 256 bytes of a row at a time
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      const bool nan = p.nan_for_masked && kv_len > 0 && visible <= 0;
-      uint4* scratch = reinterpret_cast<uint4*>(base + x * kTileBytes + quad * 32 * 256);
+        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;       // a row that sees nothing: weights 0, not NaN
+        const uint64_t post2 = pack_f32x2(post, post), minus_m = pack_f32x2(-m_use, -m_use), minus_one = pack_f32x2(-1.f, -1.f);
+        uint64_t sum2[2] = {0, 0};
 #pragma unroll
-      for (int c = 0; c < kD; c += 32) {
-        float o[32];
-        if (tiles > 0) {
-          tmem_ld_32x32b_x32(o_col + c, o);
+        for (int c = 0; c < kTile; c += 32) {
+          float sc[32];
+          tmem_ld_32x32b_x32(s_col + c, sc);
           tcgen05_wait_ld();
-        }
+          if (!plain) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint4 w;
-          w.x = pack_bf16x2(o[8 * i] * inv, o[8 * i + 1] * inv); w.y = pack_bf16x2(o[8 * i + 2] * inv, o[8 * i + 3] * inv);
-          w.z = pack_bf16x2(o[8 * i + 4] * inv, o[8 * i + 5] * inv); w.w = pack_bf16x2(o[8 * i + 6] * inv, o[8 * i + 7] * inv);
-          if (!(l > 0.f)) w = nan ? make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u) : make_uint4(0u, 0u, 0u, 0u);
-          scratch[lane * 16 + ((c / 8 + i) ^ (lane & 7))] = w;
+            for (int i = 0; i < 32; ++i) sc[i] = c + i < limit ? sc[i] * pre : -INFINITY;
+          }
+          uint32_t hi[16], lo[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float a, b;
+            unpack_f32x2(fma_f32x2(pack_f32x2(sc[2 * i], sc[2 * i + 1]), post2, minus_m), a, b);
+            a = ex2(a); b = ex2(b);
+            const uint64_t pair = pack_f32x2(a, b);
+            sum2[i & 1] = add_f32x2(sum2[i & 1], pair);
+            hi[i] = pack_bf16x2(a, b);
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(hi[i] << 16), __uint_as_float(hi[i] & 0xffff0000u)), minus_one, pair), a, b);
+            lo[i] = pack_bf16x2(a, b);
+          }
+          tmem_st_32x32b_x16(s_col + c, hi);
+          tmem_st_32x32b_x16(s_col + c + 16, lo);
+          if (c & 32) {                            // 64 KV rows of P are complete
+            tcgen05_wait_st();
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->p_ready[x][c >> 6]);
+          }
         }
+        float a, b;
+        unpack_f32x2(add_f32x2(sum2[0], sum2[1]), a, b);
+        l += a + b;
       }
-      __syncwarp();
-#pragma unroll 4
-      for (int i = 0; i < 16; ++i) {
-        const int rr = i * 2 + (lane >> 4), chunk = lane & 15;
-        const int row_r = quad * 32 + rr, row_token = x * per_half + row_r / p.group;
-        if (row_r < per_half * p.group && row_token < rows)
-          *reinterpret_cast<uint4*>(p.out + (size_t(q0 + row_token) * p.hq + kvh * p.group + row_r % p.group) * kD + chunk * 8) =
-              scratch[rr * 16 + (chunk ^ (rr & 7))];
+      if (ok && tiles > 0) ok = mbar_wait(&sh->o_done[x], (done - 1) & 1, abort_flag, p.status, kStatusWaitFlag);
+      if (!ok) break;
+      tcgen05_fence_after();
+      // rows leave through shared memory, 128 bytes of a row at a time
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const bool nan = p.nan_for_masked && w.kv_len > 0 && visible <= 0;
+#pragma unroll 1
+      for (int h = 0; h < kD; h += 64) {
+#pragma unroll
+        for (int c = 0; c < 64; c += 32) {
+          float o[32];
+          if (tiles > 0) {
+            tmem_ld_32x32b_x32(o_col + h + c, o);
+            tcgen05_wait_ld();
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            uint4 v;
+            v.x = pack_bf16x2(o[8 * i] * inv, o[8 * i + 1] * inv); v.y = pack_bf16x2(o[8 * i + 2] * inv, o[8 * i + 3] * inv);
+            v.z = pack_bf16x2(o[8 * i + 4] * inv, o[8 * i + 5] * inv); v.w = pack_bf16x2(o[8 * i + 6] * inv, o[8 * i + 7] * inv);
+            if (!(l > 0.f)) v = nan ? make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u) : make_uint4(0u, 0u, 0u, 0u);
+            scratch[lane * 8 + ((c / 8 + i) ^ (lane & 7))] = v;
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rr = i * 4 + (lane >> 3), chunk = lane & 7;
+          const int row_r = quad * 32 + rr, row_token = x * per_half + row_r / p.group;
+          if (row_r < per_half * p.group && row_token < w.rows)
+            *reinterpret_cast<uint4*>(p.out + (size_t(w.q0 + row_token) * p.hq + w.kvh * p.group + row_r % p.group) * kD + h + chunk * 8) =
+                scratch[rr * 8 + (chunk ^ (rr & 7))];
+        }
+        __syncwarp();
       }
-      if (exists) p.lse[size_t(q0 + token) * p.hq + kvh * p.group + r % p.group] = l > 0.f ? m_ref + log2f(l) : -INFINITY;
+      if (exists) p.lse[size_t(w.q0 + token) * p.hq + w.kvh * p.group + head_in_group] = l > 0.f ? m_ref + log2f(l) : -INFINITY;
     }
   }
 
