@@ -1,5 +1,6 @@
 // Dense block-scaled FP8 GEMM entry points (C ABI) on top of the shared tcgen05 core.
 #include "gemm_fp8.cuh"
+#include "gemm_skinny.cuh"
 #include "../../include/cake_b200.h"
 #include <new>
 
@@ -12,6 +13,8 @@ struct DenseHandle {
   gemm::Params params;
   int grid;
   int* status;
+  int skinny_grid, skinny_tiles, skinny_split;      // few rows: token tiles of eight and K split of skinny_kernel (0: the tcgen05 core)
+  skinny::Params skinny;
 };
 
 }  // namespace
@@ -63,6 +66,37 @@ extern "C" int cake_b200_block_scaled_gemm_create(void** buffers, const cake_b20
   const long long items = ((m + gemm::kBM - 1) / gemm::kBM) * ((n + gemm::kBN - 1) / gemm::kBN);
   const int sms = sm_count(device);
   h->grid = int(items < sms ? items : sms);
+  // Few rows go through the weight-streaming kernel.  Its cost is rounds x weight rows of a CTA, about 1.3 us per 32 rows of
+  // 7168 (the row tiles of 32 re-read the weights from L2); the tcgen05 core costs 0.45 us per K block and round whatever
+  // the number of rows.
+  h->skinny_tiles = m <= 8 ? 1 : m <= 16 ? 2 : 4;
+  const double row_tiles = double((m + 8 * h->skinny_tiles - 1) / (8 * h->skinny_tiles));
+  h->skinny_split = skinny::choose_split(row_tiles, int(n), p.k_blocks, sms);
+  const double features = 32.0 * (8 / h->skinny_split), skinny_items = row_tiles * double((n + int64_t(features) - 1) / int64_t(features));
+  const double skinny_us = 2.0 + double((long long)((skinny_items + sms - 1) / sms)) * features / 32 * p.k_blocks * 0.04;
+  const double core_us = double((items + sms - 1) / sms) * p.k_blocks * 0.45;
+  if (m > 1024 || skinny_us > core_us) h->skinny_tiles = 0;
+  if (h->skinny_tiles) {
+    skinny::Params& q = h->skinny;
+    q = skinny::Params{};
+    q.w = static_cast<const uint8_t*>(buffers[2]);
+    q.sw = p.sfb;
+    q.x = static_cast<const uint8_t*>(buffers[0]);
+    q.sx = p.sfa;
+    q.out = p.out;
+    q.status = h->status;
+    q.n = int(n);
+    q.k_blocks = q.w_k_blocks = p.k_blocks;
+    q.w_rows = int(n);
+    q.groups = 1;
+    q.dense_rows = int(m);
+    q.x_stride = int(k);
+    q.sx_stride = int(m);
+    q.terms = 1;
+    h->skinny_grid = int(skinny_items < sms ? skinny_items : sms);
+    rc = skinny::prepare_any<gemm::kDense>(h->skinny_tiles, h->skinny_split);
+    if (rc) { delete h; return rc; }
+  }
   *handle_out = h;
   return 0;
 }
@@ -75,6 +109,8 @@ extern "C" int cake_b200_block_scaled_gemm_launch(void* handle, void* cuda_strea
   CAKE_CUDA_OK(cudaGetDevice(&device));
   if (device != h->device) return kErrWrongDevice;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(cuda_stream);
+  if (h->skinny_tiles && !test_hooks().skip_load)
+    return skinny::launch_any<gemm::kDense>(h->skinny_tiles, h->skinny_split, h->skinny, h->skinny_grid, stream);
   CAKE_CUDA_OK(cudaMemsetAsync(h->status, 0, 8 * sizeof(int), stream));     // status word and work-item counter
   gemm::Params p = h->params;
   p.wait_kiloclocks = test_hooks().budget_kiloclocks;

@@ -84,6 +84,7 @@ struct Params {
   int split_act;               // kGateUp: 1 = also write the residual (lo) term
   int* status;                 // device status word (0 = ok)
   int* queue;                  // device counter, 0 at launch: work items are drawn from it (null: item i goes to CTA i mod grid)
+  int* drawn_out;              // device counter, 0 at launch, of CTAs that have drawn their last item: the last one clears both (null: the caller does)
   int wait_kiloclocks;         // budget of a bounded wait in units of 1024 clocks (0: the default, about a second)
   int skip_load;               // test hook: CTA 0's producer leaves out the loads of its second K block, once
 };
@@ -173,6 +174,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     tmem_alloc(&sh->tmem_base, kTmemColumns);
     tmem_relinquish();
   }
+  // launched as a programmatic dependent where the caller says so: everything above overlaps the kernel before
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (warp == kControlWarps) {   // m-tile prefix over groups (serial per lane chunk, then a warp scan)
     int running = 0;
     for (int base = 0; base < p.groups; base += 32) {
@@ -257,6 +261,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         g = drawn;
         ++k;
       }
+      if (p.drawn_out && atomicAdd(p.drawn_out, 1) == int(gridDim.x) - 1) { *p.queue = 0; *p.drawn_out = 0; }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------------------

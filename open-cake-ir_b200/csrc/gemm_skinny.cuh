@@ -1,0 +1,420 @@
+// Block-scaled FP8 (e4m3) GEMM for few rows per group on sm_100a: weights stream through, a handful of tokens stays.
+//
+// The same products as gemm_fp8.cuh, C[m, n] = sum_kb (sum_{k in kb} A[m, k] B[n, k]) sfa[kb, m] sfb[n/128, kb], for decode
+// steps, where a group (an expert, or the whole dense problem) has at most a few dozen rows.  What bounds it is the weight
+// stream: 2 x 32 rows of products per weight byte at most.  The tcgen05 core pays for 128 rows whatever the group holds, in
+// tensor time, in tensor-memory round trips per K block (about 0.4 us, one after another) and in power, and needs 256
+// columns to a CTA, so a small problem occupies a few SMs.  Here every warp is on its own: it streams 32 weight rows
+// through a ring of its own (cp.async, one 128-wide K block of weights, token rows and scales per slot, several slots in
+// flight, no CTA-wide barrier in the main loop), multiplies with mma.m16n8k32 (weights are the 16 rows, tokens the 8
+// columns; exact products, fp32 sums, 1.06 clocks per instruction and SM) into a fresh partial sum per K block and
+// promotes that with the block's scales in registers.
+//
+// A CTA of eight warps covers WM = 8 / WK sub-tiles of 32 weight rows, each by WK warps that take every WK-th K block and
+// meet once per item in shared memory (in warp order).  WK = 1 for many groups (a whole 128-feature quantisation group
+// of the gate/up product lies in one CTA and is quantised here); WK = 4, 8 where items would not fill the GPU, the
+// gate/up result then leaves as fp32 for quantize_kernel.
+// K order inside a block is free as long as both operands use the same: lane quad q takes bytes [32 q, 32 q + 32) of a row,
+// so that fragments of all four k-steps are two 16-byte shared-memory reads per row instead of eight 4-byte ones.
+#pragma once
+#include "gemm_fp8.cuh"
+
+namespace cake {
+namespace skinny {
+
+using gemm::kDense;
+using gemm::kDown;
+using gemm::kGateUp;
+constexpr int kWarps = 8, kThreads = kWarps * 32;
+constexpr int kSubRows = 32;                       // weight rows of a warp: two MMA tiles (gate/up: 16 of x1, 16 of x2)
+constexpr int kWeightBytes = kSubRows * 128;       // of one K block
+constexpr int kMaxGroups = gemm::kMaxGroups;
+
+struct Params {
+  const uint8_t* w;            // [groups, w_rows, 128 * w_k_blocks]
+  const float* sw;             // [groups, w_rows / 128, w_k_blocks]
+  const uint8_t* x;            // rows of x_stride bytes
+  const float* sx;             // [k_blocks, sx_stride]
+  const int* row_map;          // sorted row -> pair, token = pair / map_div, which names the row of x and sx (null: the sorted row does)
+  const int* offsets;          // [groups + 1] rows before a group (null: one group of dense_rows rows)
+  const float* row_weight;     // kDown: route weight of a pair (by row_map_weight)
+  const int* weight_map;       // kDown: sorted row -> pair
+  void* out;                   // kGateUp: e4m3 [rows, n * terms] (WK = 1) or fp32 [rows, n]; else bf16 [rows, n]
+  float* out_scale;            // kGateUp, WK = 1: [n / 128 * terms, row_capacity]
+  int* status;                 // status word to clear (null: someone else does); nothing here waits, so nothing ever sets it
+  int n, k_blocks, w_k_blocks, w_rows, groups, dense_rows, x_stride, sx_stride, map_div, row_capacity, terms;
+  int interleave_hi_lo;        // 1: K block kb is token column block (kb & 1) * (k_blocks / 2) + kb / 2, weight column block kb / 2
+};
+
+template <int NT, int WK>
+struct Shape {
+  static constexpr int kTokens = NT * 8;
+  static constexpr int kSlotBytes = kWeightBytes + kTokens * 128 + 256;        // + the block's scales
+  static constexpr int kReduceBytes = WK > 1 ? kWarps * NT * 4 * 32 * 4 : 0;    // one MMA tile's sums of every warp
+  static constexpr int kSlots = (232448 - 8192 - kReduceBytes) / (kWarps * kSlotBytes) > 6 ? 6 : (232448 - 8192 - kReduceBytes) / (kWarps * kSlotBytes);
+  static constexpr int kSmemBytes = kSlots * kWarps * kSlotBytes + kReduceBytes;
+};
+
+__device__ __forceinline__ void cp_async_16_hint(uint32_t dst, const void* src, uint64_t policy) {
+  asm volatile("cp.async.cg.shared.global.L2::cache_hint.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void cp_async_16_zfill(uint32_t dst, const void* src, bool valid) {
+  const int bytes = valid ? 16 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_4_zfill(uint32_t dst, const void* src, bool valid) {
+  const int bytes = valid ? 4 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ float2 lds64f(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void mma_e4m3(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+struct Item {
+  int group, feature0, row0, rows;                 // first feature of the CTA's sub-tiles; first sorted row; rows of it (<= 8 NT)
+};
+
+template <int MODE, int NT, int WK>
+__global__ void __launch_bounds__(kThreads, 1)
+skinny_kernel(const Params p) {
+  using S = Shape<NT, WK>;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ int tile_prefix[kMaxGroups + 1];      // row tiles before a group
+  __shared__ float group_amax[2][kWarps][S::kTokens];
+  constexpr int WM = kWarps / WK;
+  constexpr int kSubFeatures = MODE == kGateUp ? 16 : 32;
+  constexpr int kItemFeatures = WM * kSubFeatures;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wm = warp / WK, wk = warp % WK;
+  const int g8 = lane >> 2, q = lane & 3;
+  const uint32_t ring = smem_u32(smem) + warp * (S::kSlots * S::kSlotBytes);
+  float* reduce = reinterpret_cast<float*>(smem + S::kSlots * kWarps * S::kSlotBytes);
+  const uint64_t stream = l2_policy_evict_first();
+  asm volatile("griddepcontrol.wait;" ::: "memory");         // everything above overlaps the kernel before
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (p.status && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;
+
+  if (warp == 0) {
+    int running = 0;
+    for (int base = 0; base < p.groups; base += 32) {
+      const int g = base + lane;
+      const int count = g < p.groups ? (p.offsets ? p.offsets[g + 1] - p.offsets[g] : p.dense_rows) : 0;
+      const int tiles = (count + S::kTokens - 1) / S::kTokens;
+      int incl = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (g < p.groups) tile_prefix[g] = running + incl - tiles;
+      running += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) tile_prefix[p.groups] = running;
+  }
+  __syncthreads();
+  const int n_tiles = (p.n + kItemFeatures - 1) / kItemFeatures;
+  const int items = tile_prefix[p.groups] * n_tiles;
+  // item i: groups in order, feature tiles of a group in order, row tiles of a feature tile next to each other (the second
+  // one finds the weights in L2)
+  auto locate = [&](int i, Item* it) {
+    int lo = 0, hi = p.groups;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (tile_prefix[mid] * n_tiles <= i) lo = mid; else hi = mid;
+    }
+    const int m_tiles = tile_prefix[lo + 1] - tile_prefix[lo], idx = i - tile_prefix[lo] * n_tiles;
+    const int begin = p.offsets ? p.offsets[lo] : 0, end = p.offsets ? p.offsets[lo + 1] : p.dense_rows;
+    it->group = lo;
+    it->feature0 = idx / m_tiles * kItemFeatures;
+    it->row0 = begin + idx % m_tiles * S::kTokens;
+    it->rows = min(S::kTokens, end - it->row0);
+  };
+  // a warp whose features lie past n (n is a multiple of 128, an item may cover 256) streams the last ones again, to no effect
+  auto sub_feature = [&](const Item& it) { return min(it.feature0 + wm * kSubFeatures, p.n - kSubFeatures); };
+
+  // ---- load side: the stream of (item, K block) pairs of this warp, some slots ahead of the compute side
+  int load_item = blockIdx.x, load_kb = wk, load_slot = 0;
+  const uint8_t *w_lo = nullptr, *w_hi = nullptr;  // this lane's first weight row of each MMA tile, at its 16-byte chunk
+  const float* sw_ptr = nullptr;                   // lanes 0, 1: the scale row of each MMA tile
+  const uint8_t* x_ptr[2 * NT];                    // this lane's token rows (null: no such row)
+  const float* sx_ptr = nullptr;                   // this lane's token's scales
+  int load_tiles = 0;                              // token tiles of eight in the item
+  const size_t w_stride = size_t(p.w_k_blocks) * 128;
+  auto open_item = [&]() {
+    if (load_item >= items) return;
+    Item it;
+    locate(load_item, &it);
+    const int f = sub_feature(it);
+    const uint8_t* w = p.w + (size_t(it.group) * p.w_rows + f + (lane >> 3)) * w_stride + (lane & 7) * 16;
+    w_lo = w;
+    w_hi = w + size_t(MODE == kGateUp ? p.n : 16) * w_stride;
+    sw_ptr = p.sw + (size_t(it.group) * (p.w_rows / 128) + f / 128 + (MODE == kGateUp ? (lane & 1) * (p.n / 128) : 0)) * p.w_k_blocks;
+    load_tiles = (it.rows + 7) >> 3;
+#pragma unroll
+    for (int i = 0; i < 2 * NT; ++i) {
+      const int r = i * 4 + (lane >> 3);
+      x_ptr[i] = nullptr;
+      if (r < it.rows) {
+        const int row = p.row_map ? __ldg(p.row_map + it.row0 + r) / p.map_div : it.row0 + r;
+        x_ptr[i] = p.x + size_t(row) * p.x_stride + (lane & 7) * 16;
+      }
+    }
+    sx_ptr = nullptr;
+    if (lane < it.rows) sx_ptr = p.sx + (p.row_map ? __ldg(p.row_map + it.row0 + lane) / p.map_div : it.row0 + lane);
+  };
+  auto load_next = [&]() {                         // one slot; an empty copy group past the end, so that the group count stays
+    if (load_item < items) {
+      int x_col = load_kb, w_col = load_kb;
+      if (p.interleave_hi_lo) { x_col = (load_kb & 1) * (p.k_blocks >> 1) + (load_kb >> 1); w_col = load_kb >> 1; }
+      const uint32_t dst = ring + load_slot * S::kSlotBytes + (lane >> 3) * 128;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {                // four rows of 128 bytes per instruction
+        const uint8_t* src = (i < 4 ? w_lo : w_hi) + size_t(w_col) * 128 + size_t(i & 3) * 4 * w_stride;
+        cp_async_16_hint(dst + i * 512 + (((lane & 7) ^ ((i * 4 + (lane >> 3)) & 7)) << 4), src, stream);
+      }
+#pragma unroll
+      for (int i = 0; i < 2 * NT; ++i)
+        if (i < 2 * load_tiles)
+          cp_async_16_zfill(dst + kWeightBytes + i * 512 + (((lane & 7) ^ ((i * 4 + (lane >> 3)) & 7)) << 4),
+                            x_ptr[i] ? x_ptr[i] + size_t(x_col) * 128 : p.x, x_ptr[i] != nullptr);
+      const uint32_t scales = ring + load_slot * S::kSlotBytes + kWeightBytes + S::kTokens * 128;
+      if (lane < S::kTokens) cp_async_4_zfill(scales + lane * 4, sx_ptr ? sx_ptr + size_t(x_col) * p.sx_stride : p.sx, sx_ptr != nullptr);
+      if (lane < 2) cp_async_4_zfill(scales + 128 + lane * 4, sw_ptr + w_col, true);
+      load_kb += WK;
+      if (load_kb >= p.k_blocks) { load_kb = wk; load_item += gridDim.x; open_item(); }
+      load_slot = load_slot + 1 == S::kSlots ? 0 : load_slot + 1;
+    }
+    cp_async_commit();
+  };
+  // a warp without a K block of its own (fewer K blocks than warps share) has nothing to load
+  if (wk >= p.k_blocks) load_item = items;
+  open_item();
+#pragma unroll
+  for (int s = 0; s < S::kSlots - 1; ++s) load_next();
+
+  int slot = 0, flip = 0;
+  for (int i = blockIdx.x; i < items; i += gridDim.x) {
+    Item it;
+    locate(i, &it);
+    const int tiles = (it.rows + 7) >> 3;
+    float acc[2][NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[0][n][e] = acc[1][n][e] = 0.f;
+    for (int kb = wk; kb < p.k_blocks; kb += WK) {
+      cp_async_wait<S::kSlots - 2>();
+      __syncwarp();                                // the slot has landed for every lane; every lane is done with the one before
+      load_next();
+      const uint32_t s = ring + slot * S::kSlotBytes, scales = s + kWeightBytes + S::kTokens * 128;
+      uint32_t a[2][2][8];                         // [MMA tile][row g / g + 8][k-step pair words]
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = t * 16 + h * 8 + g8;
+          const uint4 lo = lds128(s + r * 128 + (((2 * q) ^ g8) << 4)), hi = lds128(s + r * 128 + (((2 * q + 1) ^ g8) << 4));
+          a[t][h][0] = lo.x; a[t][h][1] = lo.y; a[t][h][2] = lo.z; a[t][h][3] = lo.w;
+          a[t][h][4] = hi.x; a[t][h][5] = hi.y; a[t][h][6] = hi.z; a[t][h][7] = hi.w;
+        }
+      const float2 sw = lds64f(scales + 128);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        if (n >= tiles) break;
+        const uint32_t xr = s + kWeightBytes + (n * 8 + g8) * 128;
+        const uint4 lo = lds128(xr + (((2 * q) ^ g8) << 4)), hi = lds128(xr + (((2 * q + 1) ^ g8) << 4));
+        const uint32_t b[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        const float2 sx = lds64f(scales + (n * 8 + q * 2) * 4);
+        float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+            mma_e4m3(d[t], a[t][0][2 * ks], a[t][1][2 * ks], a[t][0][2 * ks + 1], a[t][1][2 * ks + 1], b[2 * ks], b[2 * ks + 1]);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const float w = t == 0 ? sw.x : sw.y, s0 = w * sx.x, s1 = w * sx.y;
+          acc[t][n][0] = fmaf(d[t][0], s0, acc[t][n][0]); acc[t][n][1] = fmaf(d[t][1], s1, acc[t][n][1]);
+          acc[t][n][2] = fmaf(d[t][2], s0, acc[t][n][2]); acc[t][n][3] = fmaf(d[t][3], s1, acc[t][n][3]);
+        }
+      }
+      slot = slot + 1 == S::kSlots ? 0 : slot + 1;
+    }
+
+    const bool exists = it.feature0 + wm * kSubFeatures < p.n;
+    const int f = sub_feature(it);
+    // One accumulator of each MMA tile: token 8 n + 2 q + (e & 1) of the item, feature f + g + 8 (e >> 1) (+ 16 in tile 1)
+    auto emit = [&](int n, int e, float v0, float v1) {
+      const int token = n * 8 + q * 2 + (e & 1);
+      if (!exists || token >= it.rows) return;
+      const size_t at = size_t(it.row0 + token) * p.n + f + g8 + 8 * (e >> 1);
+      if (MODE == kGateUp) {
+        reinterpret_cast<float*>(p.out)[at] = v0 * (v1 / (1.f + __expf(-v1)));
+      } else {
+        const float w = MODE == kDown ? __ldg(p.row_weight + __ldg(p.weight_map + it.row0 + token)) : 1.f;
+        reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(v0 * w);
+        reinterpret_cast<__nv_bfloat16*>(p.out)[at + 16] = __float2bfloat16_rn(v1 * w);
+      }
+    };
+    if (WK > 1) {
+      // the sub-tile's warps add their sums in warp order; each of them finishes a share of the accumulators
+      constexpr int kMine = (NT * 4 + WK - 1) / WK;
+      float sum[2][kMine];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+#pragma unroll
+        for (int j = 0; j < NT * 4; ++j) reduce[(warp * NT * 4 + j) * 32 + lane] = acc[t][j >> 2][j & 3];
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < kMine; ++m) {
+          const int j = wk + m * WK;
+          float v = 0.f;
+          if (j < NT * 4) {
+#pragma unroll
+            for (int k = 0; k < WK; ++k) v += reduce[((wm * WK + k) * NT * 4 + j) * 32 + lane];
+          }
+          sum[t][m] = v;
+        }
+        __syncthreads();
+      }
+#pragma unroll
+      for (int m = 0; m < kMine; ++m) {
+        const int j = wk + m * WK;
+        if (j < NT * 4) emit(j >> 2, j & 3, sum[0][m], sum[1][m]);
+      }
+    } else if (MODE != kGateUp) {
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) emit(n, e, acc[0][n][e], acc[1][n][e]);
+    } else {
+      // SwiGLU, then e4m3 quantisation over the item's 128 features (16 of each warp): the warps' maxima meet in shared memory
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[0][n][e] *= acc[1][n][e] / (1.f + __expf(-acc[1][n][e]));
+      for (int term = 0; term < p.terms; ++term, flip ^= 1) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float m = fmaxf(fabsf(acc[0][n][e]), fabsf(acc[0][n][e + 2]));
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            if (g8 == 0) group_amax[flip][warp][n * 8 + q * 2 + e] = m;
+          }
+        __syncthreads();
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          float scale[2], inv[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float m = 0.f;
+#pragma unroll
+            for (int k = 0; k < kWarps; ++k) m = fmaxf(m, group_amax[flip][k][n * 8 + q * 2 + e]);
+            scale[e] = m > 0.f ? m / 448.f : 1.f;
+            inv[e] = 1.f / scale[e];
+          }
+          const uint32_t packed = pack_e4m3x4(acc[0][n][0] * inv[0], acc[0][n][1] * inv[1], acc[0][n][2] * inv[0], acc[0][n][3] * inv[1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int token = n * 8 + q * 2 + (e & 1);
+            const uint8_t byte = uint8_t(packed >> (8 * e));
+            if (token < it.rows) {
+              reinterpret_cast<uint8_t*>(p.out)[size_t(it.row0 + token) * (size_t(p.n) * p.terms) + size_t(term) * p.n + f + g8 + 8 * (e >> 1)] = byte;
+              if (warp == 0 && g8 == 0 && e < 2) p.out_scale[size_t(term * (p.n / 128) + it.feature0 / 128) * p.row_capacity + it.row0 + token] = scale[e];
+            }
+            acc[0][n][e] -= e4m3_to_float(byte) * scale[e & 1];      // what a second term has to carry
+          }
+        }
+      }
+    }
+  }
+  cp_async_wait<0>();
+}
+
+// fp32 [rows, n] -> e4m3 [rows, n * terms] + scales [n / 128 * terms, row_capacity]: one warp per (row, 128 features).
+static __global__ void __launch_bounds__(256)
+quantize_kernel(const float* __restrict__ in, const int* __restrict__ rows_ptr, uint8_t* __restrict__ out, float* __restrict__ out_scale,
+                int n, int terms, int row_capacity) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int lane = threadIdx.x & 31, blocks = n / 128;
+  const int total = *rows_ptr * blocks;
+  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < total; i += gridDim.x * 8) {
+    const int row = i / blocks, b = i - row * blocks;
+    float4 v = *reinterpret_cast<const float4*>(in + size_t(row) * n + b * 128 + lane * 4);
+    for (int term = 0; term < terms; ++term) {
+      const float m = warp_max(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+      const float scale = m > 0.f ? m / 448.f : 1.f, inv = 1.f / scale;
+      const uint32_t packed = pack_e4m3x4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
+      reinterpret_cast<uint32_t*>(out + size_t(row) * (size_t(n) * terms) + size_t(term) * n + b * 128)[lane] = packed;
+      if (lane == 0) out_scale[size_t(term * blocks + b) * row_capacity + row] = scale;
+      v.x -= e4m3_to_float(uint8_t(packed)) * scale; v.y -= e4m3_to_float(uint8_t(packed >> 8)) * scale;
+      v.z -= e4m3_to_float(uint8_t(packed >> 16)) * scale; v.w -= e4m3_to_float(uint8_t(packed >> 24)) * scale;
+    }
+  }
+}
+
+template <int MODE, int NT, int WK>
+inline int launch(const Params& p, int grid, cudaStream_t s) {
+  return launch_dependent(skinny_kernel<MODE, NT, WK>, dim3(grid), dim3(kThreads), Shape<NT, WK>::kSmemBytes, s, p);
+}
+template <int MODE, int NT, int WK>
+inline int prepare() {
+  return int(cudaFuncSetAttribute(skinny_kernel<MODE, NT, WK>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<NT, WK>::kSmemBytes));
+}
+
+// The three shapes of K split, for `nt` token tiles of eight: a kernel's entry points by run-time numbers.
+template <int MODE, int NT>
+inline int launch_wk(int wk, const Params& p, int grid, cudaStream_t s) {
+  return wk == 1 ? launch<MODE, NT, 1>(p, grid, s) : wk == 4 && MODE != kGateUp ? launch<MODE, NT, MODE == kGateUp ? 8 : 4>(p, grid, s) : launch<MODE, NT, 8>(p, grid, s);
+}
+template <int MODE>
+inline int launch_any(int nt, int wk, const Params& p, int grid, cudaStream_t s) {
+  return nt == 1 ? launch_wk<MODE, 1>(wk, p, grid, s) : nt == 2 ? launch_wk<MODE, 2>(wk, p, grid, s) : launch_wk<MODE, 4>(wk, p, grid, s);
+}
+template <int MODE, int NT>
+inline int prepare_wk(int wk) {
+  return wk == 1 ? prepare<MODE, NT, 1>() : wk == 4 && MODE != kGateUp ? prepare<MODE, NT, MODE == kGateUp ? 8 : 4>() : prepare<MODE, NT, 8>();
+}
+template <int MODE>
+inline int prepare_any(int nt, int wk) {
+  return nt == 1 ? prepare_wk<MODE, 1>(wk) : nt == 2 ? prepare_wk<MODE, 2>(wk) : prepare_wk<MODE, 4>(wk);
+}
+
+// Token tiles of eight per item, so that most groups of a layer fit one item: 8, 16 or 32 rows for an average of 3, 9 or more.
+inline int token_tiles(double rows_per_group) { return rows_per_group <= 3 ? 1 : rows_per_group <= 9 ? 2 : 4; }
+
+// How many warps share a sub-tile's K blocks: fewest rounds of the GPU, counted in weight rows a CTA streams one after
+// another; on a tie the smaller split, which meets less often.  `row_tiles`: row tiles of all groups together.
+inline int choose_split(double row_tiles, int n, int k_blocks, int sms) {
+  int best = 1;
+  double best_cost = 1e30;
+  for (int wk = 1; wk <= 8; wk *= 2) {
+    if (wk == 2 || wk > k_blocks) continue;
+    const int features = 32 * (kWarps / wk);
+    const double items = row_tiles * ((n + features - 1) / features);
+    const double rounds = items <= sms ? 1 : items > 8 * sms ? items / sms : double((long long)(items / sms + 0.999));
+    if (rounds * features < best_cost * 0.999) { best_cost = rounds * features; best = wk; }
+  }
+  return best;
+}
+
+}  // namespace skinny
+}  // namespace cake

@@ -4,7 +4,7 @@
 // Operator and layouts: src/open_cake_ir/tasks/solx_fib/moe.py:13-20 (tensor ABI), :122-155
 // (oracle), :275-287 (routing).  The grouped GEMMs run on the tcgen05 core in gemm_fp8.cuh; the
 // small integer kernels here are warp-level (top-k by 64-bit ordered keys, ballot prefix scans).
-#include "gemm_fp8.cuh"
+#include "gemm_skinny.cuh"
 #include "../../include/cake_b200.h"
 #include <new>
 
@@ -40,6 +40,8 @@ routing_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict
                float* __restrict__ route_weights, int tokens, int experts, int top_k, int n_group,
                int topk_group, int mode) {
   __shared__ float group_scores[4][32];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int token = blockIdx.x * 4 + warp;
   if (token >= tokens) return;
@@ -139,85 +141,71 @@ routing_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict
   }
 }
 
-// ---- permute: histogram, scan, stable placement -------------------------------------------
-__global__ void histogram_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_ptr,
-                                 int* __restrict__ counts, int* __restrict__ inv_perm, int pairs, int local_experts) {
-  const int offset = __ldg(offset_ptr);
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < pairs; p += gridDim.x * blockDim.x) {
-    const int e = expert_ids[p] - offset;
-    if (e >= 0 && e < local_experts) atomicAdd(counts + e, 1);
-    else inv_perm[p] = -1;
-  }
-}
-
-__global__ void __launch_bounds__(1024)
-scan_kernel(const int* __restrict__ counts, int* __restrict__ offsets, int local_experts) {
-  __shared__ int warp_totals[32];
-  __shared__ int carry;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < local_experts; base += blockDim.x) {
-    const int e = base + threadIdx.x;
-    const int c = e < local_experts ? counts[e] : 0;
-    int incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    if (lane == 31) warp_totals[warp] = incl;
-    __syncthreads();
-    int before = carry;
-    for (int w = 0; w < warp; ++w) before += warp_totals[w];
-    if (e < local_experts) offsets[e] = before + incl - c;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = before + incl;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) offsets[local_experts] = carry;
-}
-
-// One CTA of eight warps per local expert.  Each warp owns a contiguous eighth of the pairs: a first
-// pass counts its matches, a prefix over the eight warps gives every warp its starting position, a
-// second pass places the pairs by ballot rank -- ascending pair order inside the expert, so the
-// permutation is the stable sort by expert.  Eight loads per lane are in flight per step.
+// ---- permute: stable placement ---------------------------------------------------------------
+// One CTA of eight warps per local expert, and nothing before it: the CTA counts the pairs of its expert and those of the
+// local experts before it (its offset) in one pass over the ids, so no histogram, scan or counter to clear is needed.  Each
+// warp owns a contiguous eighth of the pairs; a prefix over the warps gives every warp its starting position, and a second
+// pass places the pairs by ballot rank -- ascending pair order inside the expert, so the permutation is the stable sort
+// by expert.  Eight loads per lane are in flight per step.  Pairs of other ranks get inv_perm -1 (each step's by one CTA).
+// `clear` (may be null): `clear_words` counters of the kernels that follow.
 constexpr int kPlaceWarps = 8;
 constexpr int kPlaceStep = 256;      // pairs one warp looks at per step
 __global__ void __launch_bounds__(kPlaceWarps * 32)
-place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_ptr,
-             const int* __restrict__ offsets, int* __restrict__ sorted_pairs, int* __restrict__ inv_perm,
-             int pairs, int local_experts) {
-  __shared__ int warp_count[kPlaceWarps];
+place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_ptr, int* __restrict__ counts,
+             int* __restrict__ offsets, int* __restrict__ sorted_pairs, int* __restrict__ inv_perm, int pairs, int local_experts,
+             int* __restrict__ clear, int clear_words) {
+  __shared__ int warp_count[kPlaceWarps], warp_before[kPlaceWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int e = blockIdx.x;
-  const int want = e + __ldg(offset_ptr);
-  const int first = offsets[e];
-  if (offsets[e + 1] == first) return;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int offset = __ldg(offset_ptr), want = e + offset;
+  if (e == 0 && clear && threadIdx.x < clear_words) clear[threadIdx.x] = 0;
   const int per_warp = ((pairs + kPlaceWarps - 1) / kPlaceWarps + kPlaceStep - 1) / kPlaceStep * kPlaceStep;
   const int begin = warp * per_warp, end = min(pairs, begin + per_warp);
   const uint32_t below = (1u << lane) - 1u;
-  int count = 0;
+  int count = 0, before = 0;
   for (int base = begin; base < end; base += kPlaceStep) {
     int ids[kPlaceStep / 32];
 #pragma unroll
     for (int i = 0; i < kPlaceStep / 32; ++i) {
       const int p = base + 32 * i + lane;
-      ids[i] = p < end ? __ldg(expert_ids + p) : -1;
+      ids[i] = p < end ? expert_ids[p] : want - 1 - e;        // one below the local ids
     }
 #pragma unroll
-    for (int i = 0; i < kPlaceStep / 32; ++i) count += __popc(__ballot_sync(0xffffffffu, ids[i] == want));
+    for (int i = 0; i < kPlaceStep / 32; ++i) {
+      count += __popc(__ballot_sync(0xffffffffu, ids[i] == want));
+      before += __popc(__ballot_sync(0xffffffffu, ids[i] >= offset && ids[i] < want));
+    }
+    if ((base / kPlaceStep) % local_experts == e) {
+#pragma unroll
+      for (int i = 0; i < kPlaceStep / 32; ++i) {
+        const int p = base + 32 * i + lane;
+        if (p < end && (ids[i] < offset || ids[i] >= offset + local_experts)) inv_perm[p] = -1;
+      }
+    }
   }
-  if (lane == 0) warp_count[warp] = count;
+  if (lane == 0) { warp_count[warp] = count; warp_before[warp] = before; }
   __syncthreads();
-  int cursor = first;
-  for (int w = 0; w < warp; ++w) cursor += warp_count[w];
+  int first = 0, total = 0, cursor = 0;
+  for (int w = 0; w < kPlaceWarps; ++w) {
+    first += warp_before[w];
+    if (w < warp) cursor += warp_count[w];
+    total += warp_count[w];
+  }
+  cursor += first;
+  if (threadIdx.x == 0) {
+    counts[e] = total;
+    offsets[e] = first;
+    if (e == local_experts - 1) offsets[local_experts] = first + total;
+  }
+  if (count == 0) return;
   for (int base = begin; base < end; base += kPlaceStep) {
     int ids[kPlaceStep / 32];
 #pragma unroll
     for (int i = 0; i < kPlaceStep / 32; ++i) {
       const int p = base + 32 * i + lane;      // lane-contiguous loads keep ballots in ascending pair order
-      ids[i] = p < end ? __ldg(expert_ids + p) : -1;
+      ids[i] = p < end ? expert_ids[p] : want - 1 - e;
     }
 #pragma unroll
     for (int i = 0; i < kPlaceStep / 32; ++i) {
@@ -243,7 +231,9 @@ gather_kernel(const uint8_t* __restrict__ hidden, const float* __restrict__ hidd
               float* __restrict__ row_weight, int tokens, int hidden_width, int top_k, int local_experts,
               int capacity) {
   const int lane = threadIdx.x & 31;
-  const int n_local = __ldg(offsets + local_experts);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int n_local = offsets[local_experts];
   for (int pos = blockIdx.x * 8 + (threadIdx.x >> 5); pos < n_local; pos += gridDim.x * 8) {
     const int pair = __ldg(sorted_pairs + pos);
     const int token = pair / top_k;
@@ -262,6 +252,8 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ inv_
                int hidden_width, int top_k) {
   const int token = blockIdx.x;
   __shared__ int rows[32];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x < top_k) rows[threadIdx.x] = inv_perm[size_t(token) * top_k + threadIdx.x];
   __syncthreads();
   for (int c = threadIdx.x * 8; c < hidden_width; c += blockDim.x * 8) {
@@ -287,18 +279,18 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ inv_
 }
 
 template <int EPL>
-void launch_routing_t(const float* logits, const __nv_bfloat16* bias, const float* factor, int* ids, float* w,
+int launch_routing_t(const float* logits, const __nv_bfloat16* bias, const float* factor, int* ids, float* w,
                       int tokens, int experts, int top_k, int n_group, int topk_group, int mode, cudaStream_t s) {
-  routing_kernel<EPL><<<(tokens + 3) / 4, 128, 0, s>>>(logits, bias, factor, ids, w, tokens, experts, top_k, n_group,
-                                                      topk_group, mode);
+  return launch_dependent(routing_kernel<EPL>, dim3((tokens + 3) / 4), dim3(128), 0, s, logits, bias, factor, ids, w, tokens, experts,
+                          top_k, n_group, topk_group, mode);
 }
-inline void launch_routing(const float* logits, const __nv_bfloat16* bias, const float* factor, int* ids, float* w,
+inline int launch_routing(const float* logits, const __nv_bfloat16* bias, const float* factor, int* ids, float* w,
                            int tokens, int experts, int top_k, int n_group, int topk_group, int mode, cudaStream_t s) {
   const int epl = (experts + 31) / 32;
-  if (epl <= 2) launch_routing_t<2>(logits, bias, factor, ids, w, tokens, experts, top_k, n_group, topk_group, mode, s);
-  else if (epl <= 4) launch_routing_t<4>(logits, bias, factor, ids, w, tokens, experts, top_k, n_group, topk_group, mode, s);
-  else if (epl <= 8) launch_routing_t<8>(logits, bias, factor, ids, w, tokens, experts, top_k, n_group, topk_group, mode, s);
-  else launch_routing_t<16>(logits, bias, factor, ids, w, tokens, experts, top_k, n_group, topk_group, mode, s);
+  if (epl <= 2) return launch_routing_t<2>(logits, bias, factor, ids, w, tokens, experts, top_k, n_group, topk_group, mode, s);
+  if (epl <= 4) return launch_routing_t<4>(logits, bias, factor, ids, w, tokens, experts, top_k, n_group, topk_group, mode, s);
+  if (epl <= 8) return launch_routing_t<8>(logits, bias, factor, ids, w, tokens, experts, top_k, n_group, topk_group, mode, s);
+  return launch_routing_t<16>(logits, bias, factor, ids, w, tokens, experts, top_k, n_group, topk_group, mode, s);
 }
 
 inline bool routing_config_ok(int64_t tokens, int experts, int top_k, int n_group, int topk_group, int mode) {
@@ -314,19 +306,9 @@ struct PermuteArgs {
   int *counts, *offsets, *sorted_pairs, *inv_perm;
   int pairs, local_experts;
 };
-inline int launch_permute(const PermuteArgs& a, cudaStream_t s) {
-  CAKE_CUDA_OK(cudaMemsetAsync(a.counts, 0, sizeof(int) * a.local_experts, s));
-  if (a.pairs > 0) {
-    const int blocks = (a.pairs + 255) / 256;
-    histogram_kernel<<<blocks < 1024 ? blocks : 1024, 256, 0, s>>>(a.expert_ids, a.local_offset, a.counts, a.inv_perm,
-                                                                  a.pairs, a.local_experts);
-  }
-  const int scan_threads = a.local_experts >= 1024 ? 1024 : ((a.local_experts + 31) / 32) * 32;
-  scan_kernel<<<1, scan_threads, 0, s>>>(a.counts, a.offsets, a.local_experts);
-  if (a.pairs > 0)
-    place_kernel<<<a.local_experts, kPlaceWarps * 32, 0, s>>>(a.expert_ids, a.local_offset, a.offsets, a.sorted_pairs,
-                                                          a.inv_perm, a.pairs, a.local_experts);
-  return int(cudaGetLastError());
+inline int launch_permute(const PermuteArgs& a, cudaStream_t s, int* clear = nullptr, int clear_words = 0) {
+  return launch_dependent(place_kernel, dim3(a.local_experts), dim3(kPlaceWarps * 32), 0, s, a.expert_ids, a.local_offset, a.counts,
+                          a.offsets, a.sorted_pairs, a.inv_perm, a.pairs, a.local_experts, clear, clear_words);
 }
 
 struct RoutingHandle {
@@ -343,8 +325,9 @@ inline size_t align_up(size_t v, size_t a = 256) { return (v + a - 1) / a * a; }
 
 struct Layout {     // byte offsets inside the workspace
   size_t status, expert_ids, route_weights, counts, offsets, sorted_pairs, inv_perm, row_weight, x_perm, sx_perm,
-      act, act_scale, y, total;
+      act, act_scale, y, act32, total;
   int capacity, terms;
+  int token_tiles, split1, split2;       // few rows per expert: token tiles of eight and K splits of the weight-streaming kernel (0: the tcgen05 core)
 };
 inline Layout make_layout(const cake_b200_moe_config& c) {
   Layout l{};
@@ -366,6 +349,18 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
   l.act = take(size_t(l.capacity) * c.intermediate * l.terms);
   l.act_scale = take(size_t(c.intermediate / 128) * l.terms * l.capacity * 4);
   l.y = take(size_t(l.capacity) * c.hidden * 2);
+  // The weight-streaming kernel up to 20 rows per expert on average (beyond, an expert needs a second tile of 32 rows often
+  // enough, and products begin to cost more than the weights' way from memory).
+  const double per_expert = double(pairs) / c.experts;
+  if (per_expert <= 20) {
+    l.token_tiles = skinny::token_tiles(per_expert);
+    double missed = 1;                   // experts that get a row: those not missed by every token
+    for (int64_t t = 0; t < c.tokens && missed > 1e-3; ++t) missed *= 1.0 - double(c.top_k) / c.experts;
+    const double touched = c.local_experts * (1 - missed);
+    l.split1 = touched * (c.intermediate / 128) >= 2 * 148 || c.hidden / 128 < 8 ? 1 : 8;
+    l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128 * l.terms, 148);
+    if (l.split1 > 1) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation
+  }
   l.total = at;
   return l;
 }
@@ -381,6 +376,7 @@ struct MoeHandle {
   int* expert_ids; float* route_weights;       // in the workspace, or the caller's when routing is external
   CUtensorMap map_a1, map_a1_tail, map_b1, map_a2, map_a2_tail, map_b2;
   gemm::Params p1, p2;
+  skinny::Params s1, s2;
   int grid;
 };
 
@@ -417,9 +413,8 @@ extern "C" int cake_b200_moe_routing_launch(void* handle, void* cuda_stream) {
   CAKE_CUDA_OK(cudaGetDevice(&device));
   if (device != h->device) return kErrWrongDevice;
   if (h->cfg.tokens == 0) return 0;
-  moe::launch_routing(h->logits, h->bias, h->factor, h->ids, h->weights, int(h->cfg.tokens), h->cfg.experts, h->cfg.top_k,
-                      h->cfg.n_group, h->cfg.topk_group, h->cfg.mode, reinterpret_cast<cudaStream_t>(cuda_stream));
-  return int(cudaGetLastError());
+  return moe::launch_routing(h->logits, h->bias, h->factor, h->ids, h->weights, int(h->cfg.tokens), h->cfg.experts, h->cfg.top_k,
+                             h->cfg.n_group, h->cfg.topk_group, h->cfg.mode, reinterpret_cast<cudaStream_t>(cuda_stream));
 }
 extern "C" int cake_b200_moe_routing_destroy(void* handle) {
   delete static_cast<cake::moe::RoutingHandle*>(handle);
@@ -535,6 +530,7 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
   p1.out_scale = reinterpret_cast<float*>(h->ws + l.act_scale);
   p1.split_act = l.terms == 2;
   p1.status = status;
+  p1.drawn_out = status + 11;
   p1.queue = status + 9;                 // GEMM1: items drawn from a counter too: the two row tiles of an expert then start together on two SMs
                                          // and the second reads the weights from L2 (DRAM reads 1.12 -> 1.00 x algorithmic, 2 % less time)
   gemm::Params& p2 = h->p2;
@@ -552,9 +548,54 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
   p2.out = h->ws + l.y;
   p2.row_weight = reinterpret_cast<const float*>(h->ws + l.row_weight);
   p2.status = status;
+  p2.drawn_out = status + 10;
   p2.queue = status + 8;                 // GEMM2: items are drawn from a counter inside the 256-byte status block (12 % faster: short
                                          // items, 16 K blocks each, so an SM that runs slower should simply take fewer)
   h->grid = sm_count(device);
+  if (l.token_tiles) {
+    const int* sorted_pairs = reinterpret_cast<const int*>(h->ws + l.sorted_pairs);
+    skinny::Params& s1 = h->s1;            // token rows straight from hidden_states: no gather
+    s1 = skinny::Params{};
+    s1.w = static_cast<const uint8_t*>(buffers[4]);
+    s1.sw = p1.sfb;
+    s1.x = h->hidden;
+    s1.sx = h->hidden_scale;
+    s1.row_map = sorted_pairs;
+    s1.map_div = c.top_k;
+    s1.offsets = offsets;
+    s1.out = l.split1 > 1 ? static_cast<void*>(h->ws + l.act32) : p1.out;
+    s1.out_scale = p1.out_scale;
+    s1.n = inter;
+    s1.k_blocks = s1.w_k_blocks = hidden / 128;
+    s1.w_rows = 2 * inter;
+    s1.groups = c.local_experts;
+    s1.x_stride = hidden;
+    s1.sx_stride = int(c.tokens);
+    s1.row_capacity = l.capacity;
+    s1.terms = l.terms;
+    skinny::Params& s2 = h->s2;
+    s2 = skinny::Params{};
+    s2.w = static_cast<const uint8_t*>(buffers[6]);
+    s2.sw = p2.sfb;
+    s2.x = h->ws + l.act;
+    s2.sx = p2.sfa;
+    s2.offsets = offsets;
+    s2.row_weight = h->route_weights;
+    s2.weight_map = sorted_pairs;
+    s2.out = p2.out;
+    s2.n = hidden;
+    s2.k_blocks = p2.k_blocks;
+    s2.w_k_blocks = p2.b_k_blocks;
+    s2.w_rows = hidden;
+    s2.groups = c.local_experts;
+    s2.x_stride = inter * l.terms;
+    s2.sx_stride = s2.row_capacity = l.capacity;
+    s2.terms = 1;
+    s2.interleave_hi_lo = p2.interleave_hi_lo;
+    rc = skinny::prepare_any<gemm::kGateUp>(l.token_tiles, l.split1);
+    if (!rc) rc = skinny::prepare_any<gemm::kDown>(l.token_tiles, l.split2);
+    if (rc) { delete h; return rc; }
+  }
   *handle_out = h;
   return 0;
 }
@@ -570,40 +611,44 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
                       reinterpret_cast<int*>(h->ws + l.inv_perm), tokens * c.top_k, c.local_experts};
   switch (stage) {
     case 0: {
-      CAKE_CUDA_OK(cudaMemsetAsync(h->ws + l.status, 0, 256, s));
       if (!c.external_routing)
-        moe::launch_routing(h->logits, h->bias, h->factor, h->expert_ids, h->route_weights, tokens, c.experts, c.top_k,
-                            c.n_group, c.topk_group, c.routing_mode, s);
-      if (int rc = moe::launch_permute(pa, s)) return rc;
+        if (int rc = moe::launch_routing(h->logits, h->bias, h->factor, h->expert_ids, h->route_weights, tokens, c.experts, c.top_k,
+                                         c.n_group, c.topk_group, c.routing_mode, s))
+          return rc;
+      // the status word and the GEMMs' counters start at 0
+      if (int rc = moe::launch_permute(pa, s, reinterpret_cast<int*>(h->ws + l.status), 64)) return rc;
+      if (l.token_tiles) return 0;
       const int gather_blocks = (l.capacity + 7) / 8;
-      moe::gather_kernel<<<gather_blocks < 4096 ? gather_blocks : 4096, 256, 0, s>>>(
-          h->hidden, h->hidden_scale, h->route_weights, pa.sorted_pairs, pa.offsets, h->ws + l.x_perm,
-          reinterpret_cast<float*>(h->ws + l.sx_perm), reinterpret_cast<float*>(h->ws + l.row_weight), tokens, c.hidden,
-          c.top_k, c.local_experts, l.capacity);
-      break;
+      return launch_dependent(moe::gather_kernel, dim3(gather_blocks < 4096 ? gather_blocks : 4096), dim3(256), 0, s,
+                              h->hidden, h->hidden_scale, h->route_weights, pa.sorted_pairs, pa.offsets, h->ws + l.x_perm,
+                              reinterpret_cast<float*>(h->ws + l.sx_perm), reinterpret_cast<float*>(h->ws + l.row_weight), tokens, c.hidden,
+                              c.top_k, c.local_experts, l.capacity);
     }
     case 1: {
-      if (h->p1.queue) CAKE_CUDA_OK(cudaMemsetAsync(h->p1.queue, 0, sizeof(int), s));     // the work-item counter starts at 0
+      if (l.token_tiles) {
+        if (int rc = skinny::launch_any<gemm::kGateUp>(l.token_tiles, l.split1, h->s1, h->grid, s)) return rc;
+        if (l.split1 == 1) return 0;
+        const int64_t rows = int64_t(l.capacity) * (c.intermediate / 128);
+        return launch_dependent(skinny::quantize_kernel, dim3(unsigned(rows < 8 * 592 ? (rows + 7) / 8 : 592)), dim3(256), 0, s,
+                                reinterpret_cast<const float*>(h->ws + l.act32), pa.offsets + c.local_experts, h->ws + l.act,
+                                h->p1.out_scale, c.intermediate, l.terms, l.capacity);
+      }
       gemm::Params p = h->p1;
       p.wait_kiloclocks = test_hooks().budget_kiloclocks;
-      gemm::gemm_fp8_kernel<gemm::kGateUp><<<h->grid, gemm::kThreads, gemm::kSmemBytes, s>>>(h->map_a1, h->map_a1_tail, h->map_b1, p);
-      break;
+      return launch_dependent(gemm::gemm_fp8_kernel<gemm::kGateUp>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a1, h->map_a1_tail, h->map_b1, p);
     }
     case 2: {
-      if (h->p2.queue) CAKE_CUDA_OK(cudaMemsetAsync(h->p2.queue, 0, sizeof(int), s));
+      if (l.token_tiles) return skinny::launch_any<gemm::kDown>(l.token_tiles, l.split2, h->s2, h->grid, s);
       gemm::Params p = h->p2;
       p.wait_kiloclocks = test_hooks().budget_kiloclocks;
-      gemm::gemm_fp8_kernel<gemm::kDown><<<h->grid, gemm::kThreads, gemm::kSmemBytes, s>>>(h->map_a2, h->map_a2_tail, h->map_b2, p);
-      break;
+      return launch_dependent(gemm::gemm_fp8_kernel<gemm::kDown>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a2, h->map_a2_tail, h->map_b2, p);
     }
     case 3:
-      moe::combine_kernel<<<tokens, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(h->ws + l.y), pa.inv_perm, h->output,
-                                                 c.hidden, c.top_k);
-      break;
+      return launch_dependent(moe::combine_kernel, dim3(tokens), dim3(256), 0, s, reinterpret_cast<const __nv_bfloat16*>(h->ws + l.y), pa.inv_perm,
+                              h->output, c.hidden, c.top_k);
     default:
       return kErrBadArgument;
   }
-  return int(cudaGetLastError());
 }
 
 extern "C" int cake_b200_moe_launch_stage(void* handle, int stage, void* cuda_stream) {
