@@ -207,7 +207,7 @@ class NativeHandle:
         self.calls = 0
 
     def launch(self, stream: int) -> None:
-        code = self._launch(self.handle, c_void_p(stream))
+        code = self._launch(self.handle, stream)        # argtypes convert the integer
         if code != 0:
             raise CakeError(f"cake_b200_{self.stem}_launch", code)
         self.calls += 1

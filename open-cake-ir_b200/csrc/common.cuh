@@ -116,21 +116,28 @@ inline int sm_count(int device) {
 
 #ifdef __CUDACC__
 // Launches `kernel` as a programmatic dependent of what the stream holds: it may become resident while that runs, and waits
-// for it on the device (griddepcontrol.wait), which takes a launch latency off the critical path.
+// for it on the device (griddepcontrol.wait), which takes a launch latency off the critical path.  `cluster` > 1: in
+// clusters of that many CTAs.
 template <typename... Params, typename... Args>
-inline int launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, const Args&... args) {
-  cudaLaunchAttribute attribute[1];
+inline int launch_dependent_cluster(int cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute attribute[2];
   attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  attribute[1].id = cudaLaunchAttributeClusterDimension;
+  attribute[1].val.clusterDim = {unsigned(cluster), 1, 1};
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
   config.dynamicSmemBytes = shared_bytes;
   config.stream = stream;
   config.attrs = attribute;
-  config.numAttrs = 1;
+  config.numAttrs = cluster > 1 ? 2 : 1;
   const cudaError_t err = cudaLaunchKernelEx(&config, kernel, args...);
   return int(err != cudaSuccess ? err : cudaGetLastError());
+}
+template <typename... Params, typename... Args>
+inline int launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, const Args&... args) {
+  return launch_dependent_cluster(1, kernel, grid, block, shared_bytes, stream, args...);
 }
 
 // ---------------------------------------------------------------------------------------

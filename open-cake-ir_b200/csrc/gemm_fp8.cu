@@ -11,7 +11,7 @@ struct DenseHandle {
   int device;
   CUtensorMap map_a, map_a_tail, map_b;
   gemm::Params params;
-  int grid;
+  int grid, split;                     // CTAs of a cluster that share a tile's K (1: none)
   int* status;
   int skinny_grid, skinny_tiles, skinny_split;      // few rows: token tiles of eight and K split of skinny_kernel (0: the tcgen05 core)
   skinny::Params skinny;
@@ -65,17 +65,22 @@ extern "C" int cake_b200_block_scaled_gemm_create(void** buffers, const cake_b20
   p.queue = h->status + 4;               // work-item counter, inside the 256-byte status block
   const long long items = ((m + gemm::kBM - 1) / gemm::kBM) * ((n + gemm::kBN - 1) / gemm::kBN);
   const int sms = sm_count(device);
-  h->grid = int(items < sms ? items : sms);
-  // Few rows go through the weight-streaming kernel.  Its cost is rounds x weight rows of a CTA, about 1.3 us per 32 rows of
-  // 7168 (the row tiles of 32 re-read the weights from L2); the tcgen05 core costs 0.45 us per K block and round whatever
-  // the number of rows.
-  h->skinny_tiles = m <= 8 ? 1 : m <= 16 ? 2 : 4;
-  const double row_tiles = double((m + 8 * h->skinny_tiles - 1) / (8 * h->skinny_tiles));
-  h->skinny_split = skinny::choose_split(row_tiles, int(n), p.k_blocks, sms);
-  const double features = 32.0 * (8 / h->skinny_split), skinny_items = row_tiles * double((n + int64_t(features) - 1) / int64_t(features));
-  const double skinny_us = 2.0 + double((long long)((skinny_items + sms - 1) / sms)) * features / 32 * p.k_blocks * 0.04;
-  const double core_us = double((items + sms - 1) / sms) * p.k_blocks * 0.45;
-  if (m > 1024 || skinny_us > core_us) h->skinny_tiles = 0;
+  // Where tiles leave SMs idle, two or four CTAs of a cluster share a tile's K, at least four K blocks each (64 x 4096 x 7168:
+  // 28.7 us unsplit, 22.1 at two, 15.6 at four; 23 at eight, where the exchange of the sums costs more than the K blocks saved).
+  h->split = 1;
+  for (int s = 4; s > 1 && h->split == 1; s >>= 1)
+    if (items * s <= sms && p.k_blocks >= 4 * s) h->split = s;
+  if (h->split > 1) {
+    p.queue = nullptr;
+    rc = int(cudaFuncSetAttribute(gemm::gemm_fp8_kernel<gemm::kDense, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemm::kSmemBytes)));
+    if (rc) { delete h; return rc; }
+  }
+  h->grid = h->split > 1 ? int(items) * h->split : int(items < sms ? items : sms);
+  // At most 16 rows go through the weight-streaming kernel (4096 x 7168: 8.9 us at 1 row, 10.5 at 16; 14.4 for a split tile
+  // of the core).  Beyond, its second tile of 16 rows reads the weights again.
+  h->skinny_tiles = m > 16 ? 0 : m <= 8 ? 1 : 2;
+  h->skinny_split = skinny::choose_split(1.0, int(n), p.k_blocks, sms);
+  const int64_t skinny_items = (n + 32 * (8 / h->skinny_split) - 1) / (32 * (8 / h->skinny_split));
   if (h->skinny_tiles) {
     skinny::Params& q = h->skinny;
     q = skinny::Params{};
@@ -111,10 +116,13 @@ extern "C" int cake_b200_block_scaled_gemm_launch(void* handle, void* cuda_strea
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(cuda_stream);
   if (h->skinny_tiles && !test_hooks().skip_load)
     return skinny::launch_any<gemm::kDense>(h->skinny_tiles, h->skinny_split, h->skinny, h->skinny_grid, stream);
-  CAKE_CUDA_OK(cudaMemsetAsync(h->status, 0, 8 * sizeof(int), stream));     // status word and work-item counter
   gemm::Params p = h->params;
   p.wait_kiloclocks = test_hooks().budget_kiloclocks;
   p.skip_load = test_hooks().skip_load;
+  if (h->split > 1)
+    return launch_dependent_cluster(h->split, gemm::gemm_fp8_kernel<gemm::kDense, true>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes,
+                                    stream, h->map_a, h->map_a_tail, h->map_b, p);
+  CAKE_CUDA_OK(cudaMemsetAsync(h->status, 0, 8 * sizeof(int), stream));     // status word and work-item counter
   gemm::gemm_fp8_kernel<gemm::kDense><<<h->grid, gemm::kThreads, gemm::kSmemBytes, stream>>>(h->map_a, h->map_a_tail, h->map_b, p);
   return int(cudaGetLastError());
 }

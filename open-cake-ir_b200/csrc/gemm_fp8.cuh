@@ -149,7 +149,21 @@ __device__ __forceinline__ bool locate(const Shared* sh, const Params& p, int n_
   return true;
 }
 
-template <int MODE>
+// Two CTA-wide rendezvous of a cluster.  Hardware barriers: every CTA gets to them, since every wait before is bounded.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float4 load_cluster(uint32_t local_addr, uint32_t rank) {
+  float4 v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(local_addr), "r"(rank) : "memory");
+  return v;
+}
+
+// SPLIT (dense only): the CTAs of a cluster share one output tile, each a part of K.  A problem of few tiles otherwise runs
+// its K blocks, about 0.45 us each, one after another on a handful of SMs (64 x 4096 x 7168: 16 SMs).  The parts meet
+// through distributed shared memory: CTA r finishes columns [256 r / S, 256 (r + 1) / S) of the tile.
+template <int MODE, bool SPLIT = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a_tail,
                 const __grid_constant__ CUtensorMap map_b, const Params p) {
@@ -159,6 +173,14 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   Shared* sh = reinterpret_cast<Shared*>(tiles + kStages * kStageBytes);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  uint32_t rank = 0, split = 1;
+  if (SPLIT) {
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(split));
+  }
+  const int first_item = SPLIT ? blockIdx.x / split : blockIdx.x;
+  const int k_begin = SPLIT ? int(rank * uint32_t(p.k_blocks) / split) : 0;                  // this CTA's K blocks
+  const int k_count = SPLIT ? int((rank + 1) * uint32_t(p.k_blocks) / split) - k_begin : p.k_blocks;
   const int n_tiles = (MODE == kGateUp) ? p.n / 128 : (p.n + kBN - 1) / kBN;
 
   if (threadIdx.x == 0) {
@@ -177,6 +199,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   // launched as a programmatic dependent where the caller says so: everything above overlaps the kernel before
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (SPLIT && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;      // long before any wait can run out
   if (warp == kControlWarps) {   // m-tile prefix over groups (serial per lane chunk, then a warp scan)
     int running = 0;
     for (int base = 0; base < p.groups; base += 32) {
@@ -219,7 +242,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       uint32_t it = 0, k = 0;
       bool ok = true;
       Item item;
-      int g = blockIdx.x;
+      int g = first_item;
       while (ok) {
         const bool valid = locate(sh, p, n_tiles, g, &item);
         int drawn = g + int(gridDim.x);
@@ -239,14 +262,14 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // there; their products land in accumulator rows that no one reads.
         const bool tail = item.rows_valid <= kTailRows;
         const uint32_t stage_tx = tail ? uint32_t(kTailRows * kBK + kBytesB) : uint32_t(kStageBytes);
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        for (int kb = 0; kb < k_count; ++kb, ++it) {
           const int s = it % kStages;
           ok = mbar_wait(&sh->empty[s], ((it / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
           if (!ok) break;
           if (p.skip_load && blockIdx.x == 0 && it == 1) continue;      // test hook: this ring slot is never filled
           uint8_t* a_dst = tiles + s * kStageBytes;
           uint8_t* b_dst = a_dst + kBytesA;
-          int a_col = kb, b_col = kb;
+          int a_col = k_begin + kb, b_col = k_begin + kb;
           if (p.interleave_hi_lo) { a_col = (kb & 1) * (p.k_blocks >> 1) + (kb >> 1); b_col = kb >> 1; }
           mbar_arrive_expect_tx(&sh->full[s], stage_tx);
           tma_load_2d_hint(a_dst, tail ? &map_a_tail : &map_a, a_col * kBK, item.row0, &sh->full[s], keep);
@@ -270,7 +293,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       uint32_t it = 0, k = 0;
       bool ok = true;
       Item item;
-      for (int g = blockIdx.x; ok; g += gridDim.x, ++k) {
+      for (int g = first_item; ok; g += gridDim.x, ++k) {
         if (p.queue) {                 // the k-th item of this CTA, as drawn by the TMA warp
           const int slot = k % kItemSlots;
           ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
@@ -280,7 +303,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           if (g < 0) break;
         }
         if (!locate(sh, p, n_tiles, g, &item)) break;
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        for (int kb = 0; kb < k_count; ++kb, ++it) {
           const int s = it % kStages;
           const int t = it % kTmemStages;
           ok = mbar_wait(&sh->full[s], (it / kStages) & 1, abort_flag, p.status, kStatusWaitSmemFull) &&
@@ -313,7 +336,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     uint32_t it = 0, k = 0;
     bool ok = true;
     Item item;
-    for (int g = blockIdx.x; ok; g += gridDim.x, ++k) {
+    for (int g = first_item; ok; g += gridDim.x, ++k) {
       if (p.queue) {                   // the k-th item of this CTA, as drawn by the TMA warp
         const int slot = k % kItemSlots;
         ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
@@ -327,11 +350,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       // lanes 0 and 1 also fetch sfb: of x1 and x2 in the gate/up mode, else of the tile's two 128-column halves
       const int sfb_row = MODE == kGateUp ? item.n_tile + (lane & 1) * (p.n / 128) : min(item.n_tile * 2 + (lane & 1), sfb_rows - 1);
       const float* sfb = p.sfb + (size_t(item.group) * sfb_rows + sfb_row) * p.b_k_blocks;
-      for (int kb = 0; ok && kb < p.k_blocks; ++kb, ++it) {
+      for (int kb = 0; ok && kb < k_count; ++kb, ++it) {
         ok = it < kScaleAhead || mbar_wait(&sh->empty[(it - kScaleAhead) % kStages], (((it - kScaleAhead) / kStages) & 1) ^ 1, abort_flag,
                                            p.status, kStatusWaitSmemEmpty);
         if (!ok) break;
-        int a_col = kb, b_col = kb;
+        int a_col = k_begin + kb, b_col = k_begin + kb;
         if (p.interleave_hi_lo) { a_col = (kb & 1) * (p.k_blocks >> 1) + (kb >> 1); b_col = kb >> 1; }
         const float* sfa = p.sfa + size_t(a_col) * p.row_capacity;
         const int slot = it % kScaleSlots;
@@ -348,6 +371,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   }
+  if (SPLIT) { cluster_sync(); cluster_sync(); }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
     // ------------------------------ epilogue / promotion ------------------------------
@@ -363,9 +387,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     uint32_t it = 0, k = 0;
     uint32_t exchanges = 0;                    // amax exchanges so far (phase of Shared::exchange_done)
     int parity = 0;
-    bool ok = true;
+    bool ok = true, met = false;               // met: SPLIT, this thread has been at the cluster's barriers
     Item item;
-    for (int g = blockIdx.x; ok; g += gridDim.x, parity ^= 1, ++k) {
+    for (int g = first_item; ok; g += gridDim.x, parity ^= 1, ++k) {
       if (p.queue) {                   // the k-th item of this CTA, as drawn by the TMA warp
         const int slot = k % kItemSlots;
         ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
@@ -387,7 +411,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (MODE == kGateUp) sb1 = sh->scale_b[block % kScaleSlots][1];
       };
       if (it > 0) read_scales(it);
-      for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+      for (int kb = 0; kb < k_count; ++kb, ++it) {
         const int t = it % kTmemStages;
         ok = mbar_wait(&sh->tmem_full[t], (it / kTmemStages) & 1, abort_flag, p.status, kStatusWaitTmemFull);
         if (!ok) break;
@@ -405,10 +429,55 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         tcgen05_fence_before();            // everything this warp needs has left tensor memory
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->tmem_empty[t]);
-        if (kb + 1 < p.k_blocks) read_scales(it + 1);
+        if (kb + 1 < k_count) read_scales(it + 1);
         const uint64_t s1p = pack_f32x2(s1, s1);
 #pragma unroll
         for (int i = 0; i < 32; ++i) acc2[32 + i] = fma_f32x2(v[i], s1p, acc2[32 + i]);
+      }
+      if (SPLIT) {
+        // This CTA's products are done, so its operand ring is idle: the sums go there, [chunk of 4 columns][row], and every
+        // CTA reads its own columns of all of them.  Each starts with its own part and goes round from there, so that the
+        // CTAs of a cluster read from different ones at a time (pushed to their owners, all in the same order, the sums took
+        // 14 us at eight CTAs).
+        const int chunks = 64 / int(split);
+        float4* sums = reinterpret_cast<float4*>(tiles);
+        if (ok) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            float4 v;
+            unpack_f32x2(acc2[2 * i], v.x, v.y);
+            unpack_f32x2(acc2[2 * i + 1], v.z, v.w);
+            sums[(cg * 32 + i) * kBM + r] = v;
+          }
+        }
+        cluster_sync();
+        if (ok) {
+          const int rows = (item.rows_valid + 31) & ~31, column0 = item.n_tile * kBN + int(rank) * chunks * 4;
+          for (int i = threadIdx.x - kControlWarps * 32; i < rows * chunks / 2; i += kEpilogueWarps * 32) {
+            const int row_i = i % rows, c = i / rows * 2;
+            const uint32_t from = smem_u32(sums + (int(rank) * chunks + c) * kBM + row_i);
+            float4 v[8][2];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              if (k < int(split)) {
+                const uint32_t peer = (rank + k) & (split - 1);
+                v[k][0] = load_cluster(from, peer);
+                v[k][1] = load_cluster(from + kBM * 16, peer);
+              }
+            float4 sum[2] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              if (k < int(split))
+#pragma unroll
+                for (int h = 0; h < 2; ++h) { sum[h].x += v[k][h].x; sum[h].y += v[k][h].y; sum[h].z += v[k][h].z; sum[h].w += v[k][h].w; }
+            if (row_i < item.rows_valid && column0 + c * 4 < p.n)
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(item.row0 + row_i) * p.n + column0 + c * 4) =
+                  make_uint4(pack_bf16x2(sum[0].x, sum[0].y), pack_bf16x2(sum[0].z, sum[0].w), pack_bf16x2(sum[1].x, sum[1].y), pack_bf16x2(sum[1].z, sum[1].w));
+          }
+        }
+        cluster_sync();                          // the sums stay until every CTA of the cluster has read them
+        met = true;
+        break;
       }
       if (!ok) break;
       float acc[128];
@@ -479,6 +548,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (!ok) break;
       }
     }
+    if (SPLIT && !met) { cluster_sync(); cluster_sync(); }
   }
 
   // ------------------------------ teardown ---------------------------------------------

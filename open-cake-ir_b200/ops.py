@@ -41,6 +41,12 @@ def _no_alias(outputs: dict, everything: dict) -> None:
                 raise ValueError(f"output {out_name} aliases {name}")
 
 
+# A launch is a microsecond of device work at the small end, and the public forms of these two cost three: the current
+# device's index and the handle of its current stream, straight from the bindings behind torch.cuda.
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 def _stream(stream) -> int:
     if stream is None:
         return torch.cuda.current_stream().cuda_stream
@@ -82,7 +88,13 @@ class _Operator:
             self.native = _lib.NativeHandle(self.stem, pointers, config)
 
     def launch(self, stream=None) -> None:
-        with torch.cuda.device(self.device):
+        index = self.device.index
+        if _current_device() != index:
+            with torch.cuda.device(self.device):
+                self.native.launch(_stream(stream))
+        elif stream is None:
+            self.native.launch(_raw_stream(index))
+        else:
             self.native.launch(_stream(stream))
 
     def status(self, stream=None) -> int:
