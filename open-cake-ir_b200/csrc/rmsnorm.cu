@@ -63,6 +63,10 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
   __shared__ float partial[2][kThreads / 32];
   const int vectors = width >> 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // A chain of launches: each is resident while the one before runs and lets the next one in at once, so a norm of a few
+  // rows costs its own work and not a launch's round trip.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   uint4 w[VPT];
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
@@ -151,6 +155,63 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
   }
 }
 
+// Narrow rows (at most 2048 elements): one warp per row, four rows to a CTA, no barrier; a row's vectors are all in flight
+// at once.  A CTA per row leaves most of its threads without a vector (64 of 256 at 512 columns).
+template <int VPL, int MODE>
+__global__ void __launch_bounds__(128)
+rmsnorm_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
+                    const __nv_bfloat16* __restrict__ weight, __nv_bfloat16* __restrict__ out,
+                    __nv_bfloat16* __restrict__ residual_out, int rows, int width, float eps) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int lane = threadIdx.x & 31, vectors = width >> 3;
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  uint4 raw[VPL], res[MODE ? VPL : 1], w[VPL];
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    const int idx = lane + i * 32;
+    raw[i] = idx < vectors ? ld_stream(reinterpret_cast<const uint4*>(x + size_t(row) * width) + idx) : make_uint4(0, 0, 0, 0);
+    if (MODE) res[MODE ? i : 0] = idx < vectors ? ld_stream(reinterpret_cast<const uint4*>(residual + size_t(row) * width) + idx) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    const int idx = lane + i * 32;
+    w[i] = idx < vectors ? __ldg(reinterpret_cast<const uint4*>(weight) + idx) : make_uint4(0, 0, 0, 0);
+  }
+  float z[VPL][8], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    unpack8(raw[i], z[i]);
+    if (MODE) {
+      float r[8];
+      unpack8(res[MODE ? i : 0], r);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) z[i][j] += r[j];
+    }
+    if (MODE == 2) {                       // the rounding seam: the bf16 sum is returned and normalised
+      uint4 q;
+      q.x = pack_bf16x2(z[i][0], z[i][1]); q.y = pack_bf16x2(z[i][2], z[i][3]); q.z = pack_bf16x2(z[i][4], z[i][5]); q.w = pack_bf16x2(z[i][6], z[i][7]);
+      unpack8(q, z[i]);
+      if (lane + i * 32 < vectors) st_stream(reinterpret_cast<uint4*>(residual_out + size_t(row) * width) + lane + i * 32, q);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss = fmaf(z[i][j], z[i][j], ss);
+  }
+  const float inverse = 1.f / sqrtf(warp_sum(ss) * (1.f / float(width)) + eps);
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    float wf[8];
+    unpack8(w[i], wf);
+    uint4 o;
+    o.x = pack_bf16x2(z[i][0] * inverse * wf[0], z[i][1] * inverse * wf[1]);
+    o.y = pack_bf16x2(z[i][2] * inverse * wf[2], z[i][3] * inverse * wf[3]);
+    o.z = pack_bf16x2(z[i][4] * inverse * wf[4], z[i][5] * inverse * wf[5]);
+    o.w = pack_bf16x2(z[i][6] * inverse * wf[6], z[i][7] * inverse * wf[7]);
+    if (lane + i * 32 < vectors) st_stream(reinterpret_cast<uint4*>(out + size_t(row) * width) + lane + i * 32, o);
+  }
+}
+
 struct Handle {
   int device;
   const __nv_bfloat16 *x, *residual, *weight;
@@ -163,21 +224,24 @@ struct Handle {
 
 inline void choose_shape(Handle* h, int device) {
   const int vectors = h->width / 8;
-  // shape class: 0 = 256 threads x 1 vector; 1..4 = 512 threads x 1, 2, 4, 8 vectors
+  // shape class: 0 = a warp per row; 1..4 = 512 threads x 1, 2, 4, 8 vectors
   h->vpt = vectors <= 256 ? 0 : vectors <= 512 ? 1 : vectors <= 1024 ? 2 : vectors <= 2048 ? 3 : 4;
   // persistent CTAs: as many as are resident at once, each walking rows with a stride of the grid
-  const int resident = sm_count(device) * (h->vpt == 0 ? 6 : h->vpt == 1 ? 3 : h->vpt == 2 ? 2 : 1);
-  h->grid = h->rows < 1 ? 1 : (h->rows < resident ? h->rows : resident);
+  const int resident = sm_count(device) * (h->vpt == 1 ? 3 : h->vpt == 2 ? 2 : 1);
+  if (h->vpt == 0) h->grid = (h->rows + 3) / 4;
+  else h->grid = h->rows < 1 ? 1 : (h->rows < resident ? h->rows : resident);
 }
 
 template <int kThreads, int VPT>
-void launch(const Handle* h, cudaStream_t stream) {
-  if (h->residual_out)
-    rmsnorm_kernel<kThreads, VPT, 2><<<h->grid, kThreads, 0, stream>>>(h->x, h->residual, h->weight, h->out, h->residual_out, h->rows, h->width, h->eps);
-  else if (h->residual)
-    rmsnorm_kernel<kThreads, VPT, 1><<<h->grid, kThreads, 0, stream>>>(h->x, h->residual, h->weight, h->out, nullptr, h->rows, h->width, h->eps);
-  else
-    rmsnorm_kernel<kThreads, VPT, 0><<<h->grid, kThreads, 0, stream>>>(h->x, nullptr, h->weight, h->out, nullptr, h->rows, h->width, h->eps);
+int launch(const Handle* h, cudaStream_t stream) {
+  auto* kernel = h->residual_out ? rmsnorm_kernel<kThreads, VPT, 2> : h->residual ? rmsnorm_kernel<kThreads, VPT, 1> : rmsnorm_kernel<kThreads, VPT, 0>;
+  return launch_dependent(kernel, dim3(h->grid), dim3(kThreads), 0, stream, h->x, h->residual, h->weight, h->out, h->residual_out, h->rows, h->width, h->eps);
+}
+
+template <int VPL>
+int launch_warps(const Handle* h, cudaStream_t stream) {
+  auto* kernel = h->residual_out ? rmsnorm_warp_kernel<VPL, 2> : h->residual ? rmsnorm_warp_kernel<VPL, 1> : rmsnorm_warp_kernel<VPL, 0>;
+  return launch_dependent(kernel, dim3(h->grid), dim3(128), 0, stream, h->x, h->residual, h->weight, h->out, h->residual_out, h->rows, h->width, h->eps);
 }
 
 }  // namespace
@@ -224,13 +288,12 @@ static int rmsnorm_launch_any(void* handle, void* cuda_stream) {
   if (h->rows == 0) return 0;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(cuda_stream);
   switch (h->vpt) {
-    case 0: launch<256, 1>(h, stream); break;
-    case 1: launch<512, 1>(h, stream); break;
-    case 2: launch<512, 2>(h, stream); break;
-    case 3: launch<512, 4>(h, stream); break;
-    default: launch<512, 8>(h, stream); break;
+    case 0: return h->width <= 512 ? launch_warps<2>(h, stream) : h->width <= 1024 ? launch_warps<4>(h, stream) : launch_warps<8>(h, stream);
+    case 1: return launch<512, 1>(h, stream);
+    case 2: return launch<512, 2>(h, stream);
+    case 3: return launch<512, 4>(h, stream);
+    default: return launch<512, 8>(h, stream);
   }
-  return int(cudaGetLastError());
 }
 
 extern "C" int cake_b200_rmsnorm_launch(void* handle, void* cuda_stream) { return rmsnorm_launch_any(handle, cuda_stream); }
