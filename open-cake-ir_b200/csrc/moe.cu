@@ -20,110 +20,105 @@ __device__ __forceinline__ uint32_t ordered_bits(float v) {
   if ((b << 1) == 0) b = 0;
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
-__device__ __forceinline__ unsigned long long make_key(float score, int id) {
-  return (static_cast<unsigned long long>(ordered_bits(score)) << 32) | (0xffffffffu - uint32_t(id));
-}
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long other = __shfl_xor_sync(0xffffffffu, v, o);
-    v = other > v ? other : v;
-  }
-  return v;
-}
-
-// One warp per token.  Lane l holds experts j*32 + l.
+// Routing of one token by one warp; lane l holds experts j*32 + l.  Returns selection k's expert and weight in lane k.
 template <int EPL>
-__global__ void __launch_bounds__(128)
-routing_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ bias,
-               const float* __restrict__ factor_ptr, int* __restrict__ expert_ids,
-               float* __restrict__ route_weights, int tokens, int experts, int top_k, int n_group,
-               int topk_group, int mode) {
-  __shared__ float group_scores[4][32];
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int token = blockIdx.x * 4 + warp;
-  if (token >= tokens) return;
-  const float factor = __ldg(factor_ptr);
+__device__ __forceinline__ void route_token(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ bias, float factor,
+                                            int experts, int top_k, int n_group, int topk_group, int mode,
+                                            int& picked_id, float& weight) {
+  const int lane = threadIdx.x & 31;
   float raw[EPL], choice[EPL];   // raw = value the weight is made from; choice = value ranked
 #pragma unroll
   for (int j = 0; j < EPL; ++j) {
     const int id = j * 32 + lane;
-    float x = id < experts ? __ldg(logits + size_t(token) * experts + id) : -INFINITY;
+    raw[j] = id < experts ? __ldg(logits + id) : -INFINITY;
+    choice[j] = mode == 0 && id < experts ? __bfloat162float(bias[id]) : 0.f;
+  }
+#pragma unroll
+  for (int j = 0; j < EPL; ++j) {
+    const bool exists = j * 32 + lane < experts;
     if (mode == 0) {
-      const float s = id < experts ? 1.f / (1.f + expf(-x)) : -INFINITY;
-      raw[j] = s;
-      choice[j] = id < experts ? s + __bfloat162float(bias[id]) : -INFINITY;
+      raw[j] = exists ? 1.f / (1.f + expf(-raw[j])) : -INFINITY;
+      choice[j] = exists ? raw[j] + choice[j] : -INFINITY;
     } else {
-      raw[j] = x;
-      choice[j] = x;
+      choice[j] = raw[j];
     }
   }
   if (mode == 0 && n_group > 1) {
     const int group_size = experts / n_group;
-    for (int g = 0; g < n_group; ++g) {
-      float m1 = -INFINITY, m2 = -INFINITY;      // this lane's two best of group g
+    float mine = -INFINITY;                       // lane g: score of group g = sum of its two best
+    auto best_two = [&](float& m1, float& m2) {   // disjoint halves: merging two top-2 sets is exact
 #pragma unroll
-      for (int j = 0; j < EPL; ++j) {
-        const int id = j * 32 + lane;
-        if (id < experts && id / group_size == g) {
-          const float v = choice[j];
-          if (v > m1) { m2 = m1; m1 = v; } else if (v > m2) { m2 = v; }
+      for (int o = 16; o > 0; o >>= 1) {
+        const float p1 = __shfl_xor_sync(0xffffffffu, m1, o), p2 = __shfl_xor_sync(0xffffffffu, m2, o);
+        const float hi = fmaxf(m1, p1), lo = fmaxf(fminf(m1, p1), fmaxf(m2, p2));
+        m1 = hi; m2 = lo;
+      }
+    };
+    if (group_size == 32 && n_group == EPL) {     // group j is slot j of every lane: the groups' reductions are independent of one another
+      float m1[EPL], m2[EPL];
+#pragma unroll
+      for (int j = 0; j < EPL; ++j) { m1[j] = choice[j]; m2[j] = -INFINITY; }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) {
+          const float p1 = __shfl_xor_sync(0xffffffffu, m1[j], o), p2 = __shfl_xor_sync(0xffffffffu, m2[j], o);
+          const float hi = fmaxf(m1[j], p1), lo = fmaxf(fminf(m1[j], p1), fmaxf(m2[j], p2));
+          m1[j] = hi; m2[j] = lo;
         }
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {          // disjoint halves: merging two top-2 sets is exact
-        const float p1 = __shfl_xor_sync(0xffffffffu, m1, o);
-        const float p2 = __shfl_xor_sync(0xffffffffu, m2, o);
-        const float hi = fmaxf(m1, p1);
-        const float lo = fmaxf(fminf(m1, p1), fmaxf(m2, p2));
-        m1 = hi; m2 = lo;
-      }
-      if (lane == 0) group_scores[warp][g] = m1 + m2;
-    }
-    __syncwarp();
-    bool keep = false;
-    if (lane < n_group) {
-      const float mine = group_scores[warp][lane];
-      int rank = 0;
+      for (int j = 0; j < EPL; ++j) if (lane == j) mine = m1[j] + m2[j];
+    } else {
       for (int g = 0; g < n_group; ++g) {
-        const float other = group_scores[warp][g];
-        rank += (other > mine) || (other == mine && g < lane);
+        float m1 = -INFINITY, m2 = -INFINITY;      // this lane's two best of group g
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) {
+          const int id = j * 32 + lane;
+          if (id < experts && id / group_size == g) {
+            const float v = choice[j];
+            if (v > m1) { m2 = m1; m1 = v; } else if (v > m2) { m2 = v; }
+          }
+        }
+        best_two(m1, m2);
+        if (lane == g) mine = m1 + m2;
       }
-      keep = rank < topk_group;
     }
-    const uint32_t kept = __ballot_sync(0xffffffffu, keep);
+    int rank = 0;
+    for (int g = 0; g < n_group; ++g) {
+      const float other = __shfl_sync(0xffffffffu, mine, g);
+      rank += (other > mine) || (other == mine && g < lane);
+    }
+    const uint32_t kept = __ballot_sync(0xffffffffu, lane < n_group && rank < topk_group);
 #pragma unroll
     for (int j = 0; j < EPL; ++j) {
       const int id = j * 32 + lane;
       if (id < experts && !((kept >> (id / group_size)) & 1u)) choice[j] = -INFINITY;
     }
   }
-  unsigned long long keys[EPL];
+  // Ordered score bits, 0 = absent or taken; the largest over the warp by one reduction, its lowest expert id by another.
+  uint32_t keys[EPL];
 #pragma unroll
-  for (int j = 0; j < EPL; ++j) {
-    const int id = j * 32 + lane;
-    keys[j] = id < experts ? make_key(choice[j], id) : 0ull;
-  }
+  for (int j = 0; j < EPL; ++j) keys[j] = j * 32 + lane < experts ? ordered_bits(choice[j]) : 0u;
   float picked = 0.f;      // lane k keeps the raw value of the k-th selection
-  int picked_id = 0;
+  picked_id = 0;
   for (int k = 0; k < top_k; ++k) {
-    unsigned long long best = 0ull;
+    uint32_t best = 0;
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) best = keys[j] > best ? keys[j] : best;
-    best = warp_max_u64(best);
-    const int id = int(0xffffffffu - uint32_t(best & 0xffffffffull));
-    const int owner = id & 31, slot = id >> 5;
+    for (int j = 0; j < EPL; ++j) best = max(best, keys[j]);
+    best = __reduce_max_sync(0xffffffffu, best);
+    int id = 0x7fffffff;
     float value = 0.f;
 #pragma unroll
-    for (int j = 0; j < EPL; ++j)
-      if (j == slot) { value = raw[j]; if (lane == owner) keys[j] = 0ull; }
-    value = __shfl_sync(0xffffffffu, value, owner);
-    if (lane == k) { picked = value; picked_id = id; }
+    for (int j = EPL - 1; j >= 0; --j)             // descending: the lane's lowest id wins its ties
+      if (keys[j] == best && j * 32 + lane < experts) { id = j * 32 + lane; value = raw[j]; }
+    const int chosen = __reduce_min_sync(0xffffffffu, id);
+    value = __shfl_sync(0xffffffffu, value, chosen & 31);
+#pragma unroll
+    for (int j = 0; j < EPL; ++j) if (j * 32 + lane == chosen) keys[j] = 0u;
+    if (lane == k) { picked = value; picked_id = chosen; }
   }
   // weights over the selected experts, in selection order
-  float weight;
   if (mode == 0) {
     float total = 0.f;
     for (int k = 0; k < top_k; ++k) total += __shfl_sync(0xffffffffu, picked, k);
@@ -135,8 +130,25 @@ routing_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict
     for (int k = 0; k < top_k; ++k) total += __shfl_sync(0xffffffffu, e, k);
     weight = e / total * factor;
   }
+}
+
+// One warp per token.
+template <int EPL>
+__global__ void __launch_bounds__(128)
+routing_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ bias,
+               const float* __restrict__ factor_ptr, int* __restrict__ expert_ids,
+               float* __restrict__ route_weights, int tokens, int experts, int top_k, int n_group,
+               int topk_group, int mode) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int token = blockIdx.x * 4 + warp;
+  if (token >= tokens) return;
+  int id;
+  float weight;
+  route_token<EPL>(logits + size_t(token) * experts, bias, __ldg(factor_ptr), experts, top_k, n_group, topk_group, mode, id, weight);
   if (lane < top_k) {
-    expert_ids[size_t(token) * top_k + lane] = picked_id;
+    expert_ids[size_t(token) * top_k + lane] = id;
     route_weights[size_t(token) * top_k + lane] = weight;
   }
 }
@@ -222,6 +234,55 @@ place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_
   }
 }
 
+// Routing and permute of a step of at most 32 tokens in one CTA, a warp per token: two launches less, and the pairs never
+// leave shared memory.  A pair's position is the number of local pairs before it in (expert, pair) order, counted directly.
+constexpr int kSmallTokens = 32;
+template <int EPL>
+__global__ void __launch_bounds__(kSmallTokens * 32)
+route_place_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ bias, const float* __restrict__ factor_ptr,
+                   const int* __restrict__ offset_ptr, int* __restrict__ expert_ids, float* __restrict__ route_weights,
+                   int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ sorted_pairs, int* __restrict__ inv_perm,
+                   int tokens, int experts, int top_k, int n_group, int topk_group, int mode, int local_experts,
+                   int* __restrict__ clear, int clear_words) {
+  __shared__ int local_id[kSmallTokens * 32];        // -1: another rank's
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int offset = __ldg(offset_ptr);
+  int id;
+  float weight;
+  route_token<EPL>(logits + size_t(warp) * experts, bias, __ldg(factor_ptr), experts, top_k, n_group, topk_group, mode, id, weight);
+  if (lane < top_k) {
+    const int p = warp * top_k + lane;
+    expert_ids[p] = id;
+    route_weights[p] = weight;
+    local_id[p] = id >= offset && id < offset + local_experts ? id - offset : -1;
+  }
+  for (int i = threadIdx.x; i < clear_words; i += blockDim.x) clear[i] = 0;
+  __syncthreads();
+  const int pairs = tokens * top_k;
+  if (threadIdx.x < pairs) {
+    const int p = threadIdx.x, mine = local_id[p];
+    int at = 0;
+    for (int q = 0; q < pairs; ++q) {
+      const int other = local_id[q];
+      at += other >= 0 && (other < mine || (other == mine && q < p));
+    }
+    inv_perm[p] = mine < 0 ? -1 : at;
+    if (mine >= 0) sorted_pairs[at] = p;
+  }
+  for (int e = threadIdx.x; e <= local_experts; e += blockDim.x) {
+    int before = 0, count = 0;
+    for (int q = 0; q < pairs; ++q) {
+      const int other = local_id[q];
+      before += other >= 0 && other < e;
+      count += other == e;
+    }
+    offsets[e] = before;
+    if (e < local_experts) counts[e] = count;
+  }
+}
+
 // Copies each routed row (e4m3 hidden state + its K-block scales + its route weight) to its
 // sorted position.  One warp per destination row.
 __global__ void __launch_bounds__(256)
@@ -246,36 +307,38 @@ gather_kernel(const uint8_t* __restrict__ hidden, const float* __restrict__ hidd
   }
 }
 
-// out[t,:] = bf16( fp32 sum over the token's local slots, in slot order, of the bf16 rows y[inv_perm[t,slot],:] ).
+// out[t,:] = bf16( fp32 sum over the token's local slots, in slot order, of the bf16 rows y[inv_perm[t,slot],:] ).  A thread
+// owns eight columns of a token; the rows of eight slots are asked for before the first is added.
 __global__ void __launch_bounds__(256)
 combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ inv_perm, __nv_bfloat16* __restrict__ out,
-               int hidden_width, int top_k) {
-  const int token = blockIdx.x;
-  __shared__ int rows[32];
+               int hidden_width, int top_k, int parts) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (threadIdx.x < top_k) rows[threadIdx.x] = inv_perm[size_t(token) * top_k + threadIdx.x];
-  __syncthreads();
-  for (int c = threadIdx.x * 8; c < hidden_width; c += blockDim.x * 8) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int s = 0; s < top_k; ++s) {
-      const int row = rows[s];
-      if (row >= 0) {
-        const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(y + size_t(row) * hidden_width + c));
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const int token = blockIdx.x / parts, c = ((blockIdx.x % parts) * 256 + threadIdx.x) * 8;
+  if (c >= hidden_width) return;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int s0 = 0; s0 < top_k; s0 += 8) {
+    uint4 raw[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = __bfloat1622float2(h[i]);
-          acc[2 * i] += f.x;
-          acc[2 * i + 1] += f.y;
-        }
+    for (int i = 0; i < 8; ++i) {
+      const int row = s0 + i < top_k ? inv_perm[size_t(token) * top_k + s0 + i] : -1;
+      raw[i] = row >= 0 ? __ldcs(reinterpret_cast<const uint4*>(y + size_t(row) * hidden_width + c)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[i]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(h[j]);
+        acc[2 * j] += f.x;
+        acc[2 * j + 1] += f.y;
       }
     }
-    uint4 o;
-    o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]);
-    o.z = pack_bf16x2(acc[4], acc[5]); o.w = pack_bf16x2(acc[6], acc[7]);
-    *reinterpret_cast<uint4*>(out + size_t(token) * hidden_width + c) = o;
   }
+  uint4 o;
+  o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]);
+  o.z = pack_bf16x2(acc[4], acc[5]); o.w = pack_bf16x2(acc[6], acc[7]);
+  *reinterpret_cast<uint4*>(out + size_t(token) * hidden_width + c) = o;
 }
 
 template <int EPL>
@@ -611,12 +674,19 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
                       reinterpret_cast<int*>(h->ws + l.inv_perm), tokens * c.top_k, c.local_experts};
   switch (stage) {
     case 0: {
+      int* const clear = reinterpret_cast<int*>(h->ws + l.status);      // the status word and the GEMMs' counters start at 0
+      if (!c.external_routing && tokens <= moe::kSmallTokens && l.token_tiles) {
+        const int epl = (c.experts + 31) / 32;
+        auto* kernel = epl <= 2 ? moe::route_place_kernel<2> : epl <= 4 ? moe::route_place_kernel<4> : epl <= 8 ? moe::route_place_kernel<8> : moe::route_place_kernel<16>;
+        return launch_dependent(kernel, dim3(1), dim3(32 * tokens), 0, s, h->logits, h->bias, h->factor, h->local_offset, h->expert_ids, h->route_weights,
+                                pa.counts, pa.offsets, pa.sorted_pairs, pa.inv_perm, tokens, c.experts, c.top_k, c.n_group, c.topk_group,
+                                c.routing_mode, c.local_experts, clear, 64);
+      }
       if (!c.external_routing)
         if (int rc = moe::launch_routing(h->logits, h->bias, h->factor, h->expert_ids, h->route_weights, tokens, c.experts, c.top_k,
                                          c.n_group, c.topk_group, c.routing_mode, s))
           return rc;
-      // the status word and the GEMMs' counters start at 0
-      if (int rc = moe::launch_permute(pa, s, reinterpret_cast<int*>(h->ws + l.status), 64)) return rc;
+      if (int rc = moe::launch_permute(pa, s, clear, 64)) return rc;
       if (l.token_tiles) return 0;
       const int gather_blocks = (l.capacity + 7) / 8;
       return launch_dependent(moe::gather_kernel, dim3(gather_blocks < 4096 ? gather_blocks : 4096), dim3(256), 0, s,
@@ -644,8 +714,11 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
       return launch_dependent(gemm::gemm_fp8_kernel<gemm::kDown>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a2, h->map_a2_tail, h->map_b2, p);
     }
     case 3:
-      return launch_dependent(moe::combine_kernel, dim3(tokens), dim3(256), 0, s, reinterpret_cast<const __nv_bfloat16*>(h->ws + l.y), pa.inv_perm,
-                              h->output, c.hidden, c.top_k);
+    {
+      const int parts = (c.hidden + 2047) / 2048;
+      return launch_dependent(moe::combine_kernel, dim3(unsigned(tokens) * parts), dim3(256), 0, s, reinterpret_cast<const __nv_bfloat16*>(h->ws + l.y),
+                              pa.inv_perm, h->output, c.hidden, c.top_k, parts);
+    }
     default:
       return kErrBadArgument;
   }
