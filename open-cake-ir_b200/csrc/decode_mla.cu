@@ -67,6 +67,8 @@ struct Params {
   float* lse;             // [B, H] (null: not asked for)
   float* part_o;          // [2 * workers, rows, 512]   partial results of sequences that a range boundary cuts (see slot_of)
   float* part_lse;        // [2 * workers, rows]
+  int4* cuts;             // [workers] sequences that a range boundary cuts: {sequence, first and last range, slot of its first piece}
+  int* cut_count;
   int* tile_prefix;       // [sequences + 1] work units (tiles + start-up shares) before a sequence, written by the plan kernel
   int* status;
   int sequences, heads, page_size, workers;
@@ -153,6 +155,22 @@ __device__ __forceinline__ int sequence_at(const Params& p, int count, int unit)
   return lo;
 }
 
+// Lists the cut sequences for the reduce kernel (all threads of a plan CTA, once the prefix is complete).
+__device__ __forceinline__ void list_cuts(const Params& p, int count, int total) {
+  __shared__ int listed;
+  if (threadIdx.x == 0) listed = 0;
+  __syncthreads();                                 // also makes the prefix visible
+  const int per = units_per_worker(p, total);
+  for (int b = threadIdx.x; b < count; b += blockDim.x) {
+    const int begin = p.tile_prefix[b], end = p.tile_prefix[b + 1];
+    if (end == begin) continue;
+    const int first = (begin + p.seq_cost) / per, last = (end - 1) / per;
+    if (first < last) p.cuts[atomicAdd(&listed, 1)] = make_int4(b, first, last, slot_of(first, begin, per));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *p.cut_count = listed;
+}
+
 // One CTA: tile_prefix[b] = units before sequence b (exclusive scan), tile_prefix[B] = all units.
 static __global__ void __launch_bounds__(1024)
 mla_plan_kernel(const Params p) {
@@ -171,6 +189,7 @@ mla_plan_kernel(const Params p) {
     before += batch_total;
   }
   if (threadIdx.x == 0) p.tile_prefix[p.sequences] = before;
+  list_cuts(p, p.sequences, before);
 }
 
 // The same for a causal prefill: cuts the query rows of every segment into sequences of up to `pack` tokens first.  Rows
@@ -228,6 +247,7 @@ mla_prefill_plan_kernel(const Params p) {
     units += all;
   }
   if (tid == 0) { p.tile_prefix[count] = units; *p.seq_count = count; *p.status = 0; }
+  list_cuts(p, count, units);
 }
 
 // A piece of a sequence as every role of a cluster reads it off the list.
@@ -278,9 +298,11 @@ __device__ __forceinline__ bool next_piece(const Params& p, int range_end, Curso
 __device__ __forceinline__ void cluster_sync() {           // hardware barrier: every CTA gets to it, since every wait before is bounded
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
-// An arrival on CTA `rank`'s barrier at the same place as `bar` here.
+// An arrival on CTA `rank`'s barrier at the same place as `bar` here.  What it announces lies in this CTA's shared memory and is
+// read by the tensor core, in front of which every writer has put a proxy fence; a release at cluster scope on top of that
+// took 1060 clocks.
 __device__ __forceinline__ void arrive_at(uint64_t* bar, uint32_t rank) {
-  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tmbarrier.arrive.release.cluster.shared::cluster.b64 _, [a];\n\t}"
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tmbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
                ::"r"(smem_u32(bar)), "r"(rank) : "memory");
 }
 // mbar_wait for a barrier that the other CTA arrives on: what it wrote before is visible after.
@@ -312,15 +334,10 @@ __device__ __forceinline__ void commit_pair(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(smem_u32(bar)), "h"(uint16_t(3)) : "memory");
 }
-// A row's 32 values as bf16: 64 bytes.
-__device__ __forceinline__ void store_row_bf16(__nv_bfloat16* dst, const float* v, float scale) {
-#pragma unroll
-  for (int i = 0; i < 32; i += 8) {
-    uint4 w;
-    w.x = pack_bf16x2(v[i] * scale, v[i + 1] * scale); w.y = pack_bf16x2(v[i + 2] * scale, v[i + 3] * scale);
-    w.z = pack_bf16x2(v[i + 4] * scale, v[i + 5] * scale); w.w = pack_bf16x2(v[i + 6] * scale, v[i + 7] * scale);
-    *reinterpret_cast<uint4*>(dst + i) = w;
-  }
+// 32 bytes at once: a lane has a row of its own, and a whole sector per store leaves twice as fast as halves of one.
+__device__ __forceinline__ void store_32(void* dst, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 
 template <bool SPARSE>
@@ -674,12 +691,22 @@ mla_decode_kernel(const Params p) {
         }
         if (!exists) continue;
         if (w.whole) {
-          store_row_bf16(p.out + out_row * kCkv + dim, o, l > 0.f ? inv : 1.f);
-        } else {
-          float* dst = p.part_o + slot_row * kCkv + dim;
+          const float by = l > 0.f ? inv : 1.f;
 #pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            *reinterpret_cast<float4*>(dst + i) = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
+          for (int h = 0; h < 32; h += 16) {
+            uint32_t v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = pack_bf16x2(o[h + 2 * i] * by, o[h + 2 * i + 1] * by);
+            store_32(p.out + out_row * kCkv + dim + h, v);
+          }
+        } else {
+#pragma unroll
+          for (int h = 0; h < 32; h += 8) {
+            uint32_t v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = __float_as_uint(o[h + i] * inv);
+            store_32(p.part_o + slot_row * kCkv + dim + h, v);
+          }
         }
       }
       if (exists && half == 0) {
@@ -696,45 +723,47 @@ mla_decode_kernel(const Params p) {
   if (warp == kMmaWarp) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemColumns) : "memory");
 }
 
-// Merges the pieces of a cut sequence: CTA (x, w) looks after the sequence whose first piece ends at the end of range w (if
-// there is one) and four of its rows, 128 threads x 4 dims each.
-static __global__ void __launch_bounds__(512)
+// Merges the pieces of the cut sequences: CTA (x, y) two rows of the y-th, 128 threads x 4 dims each, the results of four
+// pieces in flight (most sequences have two to four; eight in flight take registers from half of the resident rows).
+static __global__ void __launch_bounds__(256, 4)
 mla_reduce_kernel(const Params p) {
   // launched as a programmatic dependent of the decode kernel: resident early, reads after it has completed
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int count = sequence_count(p), total = p.tile_prefix[count], per = units_per_worker(p, total);
-  const int w = blockIdx.y, cut = (w + 1) * per;
-  if (cut >= total) return;
-  const int b = sequence_at(p, count, cut);
-  const int seq_begin = p.tile_prefix[b], first = (seq_begin + p.seq_cost) / per, last = (p.tile_prefix[b + 1] - 1) / per;
-  if (first != w || last == w) return;
+  if (int(blockIdx.y) >= *p.cut_count) return;
+  const int4 cut = p.cuts[blockIdx.y];
+  const int b = cut.x, first = cut.y, last = cut.z;
   const int4 s = p.seq ? p.seq[b] : make_int4(b, 1, 0, 0);
-  const int row = blockIdx.x * 4 + (threadIdx.x >> 7), d = (threadIdx.x & 127) * 4;
+  const int row = blockIdx.x * 2 + (threadIdx.x >> 7), d = (threadIdx.x & 127) * 4;
   if (row >= s.y * p.heads) return;
-  const int slot0 = slot_of(first, seq_begin, per);
-  auto slot_row = [&](int k) { return size_t(k == first ? slot0 : 2 * k) * p.rows + row; };
-  float mm = -INFINITY;
-  for (int k = first; k <= last; ++k) mm = fmaxf(mm, p.part_lse[slot_row(k)]);
-  float weight = 0.f;
+  auto slot_row = [&](int k) { return size_t(k == first ? cut.w : 2 * k) * p.rows + row; };
+  float mm = -INFINITY, weight = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (mm > -INFINITY) {
-    for (int k0 = first; k0 <= last; k0 += 8) {      // eight pieces in flight
-      float ls[8];
-      float4 v[8];
+  for (int k0 = first; k0 <= last; k0 += 4) {
+    float ls[4];
+    float4 v[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const size_t at = slot_row(min(k0 + i, last));
-        ls[i] = p.part_lse[at];
-        v[i] = *reinterpret_cast<const float4*>(p.part_o + at * kCkv + d);
+    for (int i = 0; i < 4; ++i)
+      if (k0 + i <= last) {
+        const size_t at = slot_row(k0 + i);
+        ls[i] = __ldcg(p.part_lse + at);
+        v[i] = __ldcg(reinterpret_cast<const float4*>(p.part_o + at * kCkv + d));
       }
+    float m_new = mm;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float wt = k0 + i <= last ? exp2f(ls[i] - mm) : 0.f;
+    for (int i = 0; i < 4; ++i) if (k0 + i <= last) m_new = fmaxf(m_new, ls[i]);
+    if (m_new == -INFINITY) continue;              // nothing seen so far
+    const float rescale = exp2f(mm - m_new);       // 0 the first time
+    mm = m_new;
+    weight *= rescale;
+    acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (k0 + i <= last) {
+        const float wt = exp2f(ls[i] - mm);
         weight += wt;
         acc.x += wt * v[i].x; acc.y += wt * v[i].y; acc.z += wt * v[i].z; acc.w += wt * v[i].w;
       }
-    }
   }
   const size_t out_row = size_t(s.x) * p.heads + row;
   uint2 packed = make_uint2(0u, 0u);
@@ -755,13 +784,13 @@ struct Handle {
 
 constexpr int kMaxWorkers = 96;                            // pairs of SMs the workspace is sized for
 
-// Workspace behind the 256-byte status block: tile_prefix [sequences + 1] int | part_o [slots, rows, 512] f32 | part_lse [slots, rows],
+// Workspace behind the 256-byte status block: tile_prefix [sequences + 1] int | cuts [kMaxWorkers] int4, their number | part_o [slots, rows, 512] f32 | part_lse [slots, rows],
 // and for the prefill form seq [sequences] int4 | seq_page [sequences] | segment_prefix [segments + 3] | seq_count [1]
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 inline int head_blocks(int rows) { return (rows + kHeads - 1) / kHeads; }
 inline size_t slots_for(int rows) { const int n = kMaxWorkers / head_blocks(rows); return 2 * size_t(n > 0 ? n : 1); }
 inline size_t part_bytes(int rows) { return align256(slots_for(rows) * rows * kCkv * sizeof(float)) + align256(slots_for(rows) * rows * sizeof(float)); }
-inline size_t workspace(int64_t sequences, int rows) { return 256 + align256((size_t(sequences) + 1) * sizeof(int)) + part_bytes(rows) + 256; }
+inline size_t workspace(int64_t sequences, int rows) { return 256 + align256((size_t(sequences) + 1) * sizeof(int)) + align256((kMaxWorkers + 1) * sizeof(int4)) + part_bytes(rows) + 256; }
 // Tokens of a sequence in the prefill form, and how many sequences total_q rows of `segments` segments make at most.
 inline int pack_tokens(int heads) { return heads <= kHeads / 2 ? kHeads / heads : 1; }
 inline int64_t prefill_sequences(const cake_b200_mla_prefill_config& c) { return c.total_q / pack_tokens(c.num_qo_heads) + c.segments + 3; }
@@ -779,6 +808,9 @@ inline uint8_t* carve(Params& p, void* buffer) {
   ws += (256 - (reinterpret_cast<uintptr_t>(ws) & 255)) & 255;
   p.tile_prefix = reinterpret_cast<int*>(ws);
   ws += align256((size_t(p.sequences) + 1) * sizeof(int));
+  p.cuts = reinterpret_cast<int4*>(ws);
+  p.cut_count = reinterpret_cast<int*>(p.cuts + kMaxWorkers);
+  ws += align256((kMaxWorkers + 1) * sizeof(int4));
   p.part_o = reinterpret_cast<float*>(ws);
   p.part_lse = reinterpret_cast<float*>(ws + align256(slots_for(p.rows) * p.rows * kCkv * sizeof(float)));
   return ws + part_bytes(p.rows);
@@ -804,7 +836,7 @@ inline int launch(const Handle* h, cudaStream_t s) {
   if (int rc = launch_dependent_cluster(2, p.sparse_indices ? mla_decode_kernel<true> : mla_decode_kernel<false>, grid, dim3(kThreads), kSmemBytes, s, p))
     return rc;
   if (p.workers == 1) return 0;                              // nothing is ever cut
-  return launch_dependent(mla_reduce_kernel, dim3((p.rows + 3) / 4, p.workers - 1), dim3(512), 0, s, p);
+  return launch_dependent(mla_reduce_kernel, dim3((p.rows + 1) / 2, p.workers - 1 < p.sequences ? p.workers - 1 : p.sequences), dim3(256), 0, s, p);
 }
 
 }  // namespace mla
