@@ -63,6 +63,7 @@ struct Params {
   int* done;                     // [B, Hkv] finished items
   int* status;                   // library status word (may be null)
   int batch, hq, hkv, page_size, capacity, ranges;
+  int merge_kernel;              // pieces are merged by gqa_merge_kernel instead of the pair that finishes a sequence's last one
   // Explicit sequence table (causal prefill, where every query token is a sequence of its own over a prefix of its
   // segment's rows): sequence b holds seq_tokens[b] tokens whose page list starts at kv_indices[seq_start[b]];
   // null = sequences come from kv_indptr / kv_last_page_len.  With kv_indices null the page list is the
@@ -141,13 +142,20 @@ __device__ __forceinline__ void load_half(const __nv_bfloat16* __restrict__ cach
 // resets the counters and writes the results of empty sequences (zeros, lse = -inf), which no
 // piece covers.
 constexpr int kPieceCost = 32;
+constexpr int kMaxSms = 192;             // SM count the workspace is sized for
+constexpr int kMaxRanges = kMaxSms * kHeads;
 __global__ void __launch_bounds__(1024)
 gqa_plan_kernel(const Params p) {
   __shared__ long long sums64[32];
   __shared__ int sums32[32];
+  __shared__ long long starts[1024];               // of 1024 sequences at a time: where the tokens begin, in units,
+  __shared__ int lens[1024], firsts[1024];         // how many there are, and the list index of the first piece
+  __shared__ int range_first[kMaxRanges], range_last[kMaxRanges];
   const int tid = threadIdx.x;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0 && p.status) *p.status = 0;
-  for (int r = tid; r < p.ranges; r += 1024) { p.range_first[r] = 0x7fffffff; p.range_count[r] = 0; }
+  for (int r = tid; r < p.ranges; r += 1024) { range_first[r] = 0x7fffffff; range_last[r] = -1; }
   const int len0 = tid < p.batch ? seq_len(p, tid) : 0;              // the first 1024 lengths stay in registers
   long long mine = len0 > 0 ? len0 + kPieceCost : 0, all_units = 0;
   for (int b = tid + 1024; b < p.batch; b += 1024) { const int n = seq_len(p, b); mine += n > 0 ? n + kPieceCost : 0; }
@@ -161,30 +169,46 @@ gqa_plan_kernel(const Params p) {
     const int len = base == 0 ? len0 : (b < p.batch ? seq_len(p, b) : 0);
     long long batch_units;
     const long long start = units_before + cta1024_exclusive_scan((long long)(len > 0 ? len + kPieceCost : 0), sums64, batch_units) + kPieceCost;
-    const int first_range = int(start / per);                          // `start`: where the sequence's tokens begin
-    const int n = len > 0 ? int((start + len - 1) / per) - first_range + 1 : 0;
+    const int n = len > 0 ? int((start + len - 1) / per) - int(start / per) + 1 : 0;
     int batch_entries;
     const int first = entries_before + cta1024_exclusive_scan(n, sums32, batch_entries);
+    starts[tid] = start; lens[tid] = len; firsts[tid] = first;
     if (b < p.batch) {
-      const int page_base = p.seq_start ? p.seq_start[b] : p.kv_indptr[b];
-      for (int k = 0; k < n; ++k) {
-        const long long range_start = (long long)(first_range + k) * per;
-        const long long piece_begin = max(start, range_start), piece_end = min(start + len, range_start + per);
-        p.items[first + k] = make_int4(b | (n << 16), int(piece_begin - start), first, int(piece_end - start));
-        p.item_page[first + k] = page_base;
-        atomicMin(p.range_first + first_range + k, first + k);
-        atomicAdd(p.range_count + first_range + k, 1);
-      }
-      for (int h = 0; h < p.hkv; ++h) p.done[size_t(b) * p.hkv + h] = 0;
+      // finished pieces per KV head; for the merge kernel the sequence's first piece and their number instead
+      if (p.merge_kernel) p.done[size_t(b) * p.hkv] = first | (n << 17);
+      else for (int h = 0; h < p.hkv; ++h) p.done[size_t(b) * p.hkv + h] = 0;
       if (len == 0) {
         for (int h = 0; h < p.hq; ++h) {
           p.lse[size_t(b) * p.hq + h] = -INFINITY;
-          for (int d = 0; d < kD; ++d) p.out[(size_t(b) * p.hq + h) * kD + d] = __float2bfloat16(0.f);
+          for (int d = 0; d < kD; d += 8) *reinterpret_cast<uint4*>(p.out + (size_t(b) * p.hq + h) * kD + d) = make_uint4(0u, 0u, 0u, 0u);
         }
       }
     }
+    __syncthreads();
+    // the pieces of these sequences, a thread each: largest sequence whose first piece is not behind piece e
+    const int here = min(1024, p.batch - base);
+    for (int e = entries_before + tid; e < entries_before + batch_entries; e += 1024) {
+      int lo = 0, hi = here;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (firsts[mid] <= e) lo = mid; else hi = mid;
+      }
+      const long long s0 = starts[lo];
+      const int count = int((s0 + lens[lo] - 1) / per) - int(s0 / per) + 1, range = int(s0 / per) + e - firsts[lo];
+      const long long range_start = (long long)range * per;
+      const long long piece_begin = max(s0, range_start), piece_end = min(s0 + lens[lo], range_start + per);
+      p.items[e] = make_int4((base + lo) | (count << 16), int(piece_begin - s0), firsts[lo], int(piece_end - s0));
+      p.item_page[e] = p.seq_start ? p.seq_start[base + lo] : p.kv_indptr[base + lo];
+      atomicMin(range_first + range, e);
+      atomicMax(range_last + range, e);
+    }
+    __syncthreads();
     units_before += batch_units;
     entries_before += batch_entries;
+  }
+  for (int r = tid; r < p.ranges; r += 1024) {
+    p.range_first[r] = range_first[r];
+    p.range_count[r] = range_last[r] < 0 ? 0 : range_last[r] - range_first[r] + 1;
   }
 }
 
@@ -467,34 +491,110 @@ gqa_decode_kernel(const Params p) {
     }
     pair_barrier(pair);                 // the parked state has been read
     if (part == 0) {
-      // partial result of this item: normalised rows and base-2 log-sum-exp
-      const size_t slot0 = size_t(idx / p.hkv) * p.hq + kvh * group;
+      if (chunks == 1) {                  // the whole sequence: this is the result
+        const size_t row0 = size_t(b) * p.hq + kvh * group;
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        const int dim = n * 16 + row;
-        if (quad * 2 < group) {
-          store_keep(p.part_o + (slot0 + quad * 2) * kD + dim, o[n][0], keep_policy);
-          store_keep(p.part_o + (slot0 + quad * 2) * kD + dim + 8, o[n][2], keep_policy);
+        for (int n = 0; n < 8; ++n) {
+          const int dim = n * 16 + row;
+          if (quad * 2 < group) {
+            p.out[(row0 + quad * 2) * kD + dim] = __float2bfloat16_rn(o[n][0]);
+            p.out[(row0 + quad * 2) * kD + dim + 8] = __float2bfloat16_rn(o[n][2]);
+          }
+          if (quad * 2 + 1 < group) {
+            p.out[(row0 + quad * 2 + 1) * kD + dim] = __float2bfloat16_rn(o[n][1]);
+            p.out[(row0 + quad * 2 + 1) * kD + dim + 8] = __float2bfloat16_rn(o[n][3]);
+          }
         }
-        if (quad * 2 + 1 < group) {
-          store_keep(p.part_o + (slot0 + quad * 2 + 1) * kD + dim, o[n][1], keep_policy);
-          store_keep(p.part_o + (slot0 + quad * 2 + 1) * kD + dim + 8, o[n][3], keep_policy);
+        if (row < group && quad == 0) p.lse[row0 + row] = m + log2f(l);
+      } else {
+        // partial result of this item: normalised rows and base-2 log-sum-exp
+        const size_t slot0 = size_t(idx / p.hkv) * p.hq + kvh * group;
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+          const int dim = n * 16 + row;
+          if (quad * 2 < group) {
+            store_keep(p.part_o + (slot0 + quad * 2) * kD + dim, o[n][0], keep_policy);
+            store_keep(p.part_o + (slot0 + quad * 2) * kD + dim + 8, o[n][2], keep_policy);
+          }
+          if (quad * 2 + 1 < group) {
+            store_keep(p.part_o + (slot0 + quad * 2 + 1) * kD + dim, o[n][1], keep_policy);
+            store_keep(p.part_o + (slot0 + quad * 2 + 1) * kD + dim + 8, o[n][3], keep_policy);
+          }
         }
-      }
-      if (row < group && quad == 0) store_keep(p.part_lse + slot0 + row, m + log2f(l), keep_policy);
-      // The pair that completes the last item of (b, kvh) merges the chunks.
-      __threadfence();
-      __syncwarp();
-      int last_item = 0;
-      if (lane == 0) last_item = atomicAdd(p.done + size_t(b) * p.hkv + kvh, 1) == chunks - 1;
-      if (__shfl_sync(0xffffffffu, last_item, 0)) {
-        __threadfence();
-        merge_chunks(p, b, kvh, rec.z, chunks, group, lane);
+        if (row < group && quad == 0) store_keep(p.part_lse + slot0 + row, m + log2f(l), keep_policy);
+        if (!p.merge_kernel) {
+          // The pair that completes the last item of (b, kvh) merges the chunks.
+          __threadfence();
+          __syncwarp();
+          int last_item = 0;
+          if (lane == 0) last_item = atomicAdd(p.done + size_t(b) * p.hkv + kvh, 1) == chunks - 1;
+          if (__shfl_sync(0xffffffffu, last_item, 0)) {
+            __threadfence();
+            merge_chunks(p, b, kvh, rec.z, chunks, group, lane);
+          }
+        }
       }
     }
     idx = nxt_idx; rec = nxt_rec; page_base = nxt_page;
   }
   cp_async_wait<0>();
+}
+
+// Merges the pieces of sequences that are cut into many: one CTA per (head, sequence), each of its eight warps every eighth
+// piece, four in flight, a float4 of the row to a lane.
+constexpr int kMergeWarps = 8;
+__global__ void __launch_bounds__(kMergeWarps * 32)
+gqa_merge_kernel(const Params p) {
+  __shared__ float4 sums[kMergeWarps][32];
+  __shared__ float2 stats[kMergeWarps];            // maximum, weight
+  const int head = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int packed = p.done[size_t(b) * p.hkv], first = packed & 0x1ffff, count = packed >> 17;
+  if (count < 2) return;                           // empty, or written by the decode kernel
+  float mm = -INFINITY, weight = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k0 = warp; k0 < count; k0 += 4 * kMergeWarps) {
+    float ls[4];
+    float4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const size_t at = size_t(first + min(k0 + i * kMergeWarps, count - 1)) * p.hq + head;
+      ls[i] = k0 + i * kMergeWarps < count ? __ldcg(p.part_lse + at) : -INFINITY;
+      v[i] = __ldcg(reinterpret_cast<const float4*>(p.part_o + at * kD) + lane);
+    }
+    const float m_new = fmaxf(fmaxf(fmaxf(ls[0], ls[1]), fmaxf(ls[2], ls[3])), mm);       // finite: ls[0] is
+    const float rescale = exp2f(mm - m_new);       // 0 the first time
+    mm = m_new;
+    weight *= rescale;
+    acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float w = exp2f(ls[i] - mm);
+      weight += w;
+      acc.x += w * v[i].x; acc.y += w * v[i].y; acc.z += w * v[i].z; acc.w += w * v[i].w;
+    }
+  }
+  sums[warp][lane] = acc;
+  if (lane == 0) stats[warp] = make_float2(mm, weight);
+  __syncthreads();
+  if (warp) return;
+  mm = -INFINITY;
+#pragma unroll
+  for (int k = 0; k < kMergeWarps; ++k) mm = fmaxf(mm, stats[k].x);
+  weight = 0.f;
+  acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < kMergeWarps; ++k) {
+    const float w = exp2f(stats[k].x - mm);        // a warp without a piece: 0
+    const float4 v = sums[k][lane];
+    weight += w * stats[k].y;
+    acc.x += w * v.x; acc.y += w * v.y; acc.z += w * v.z; acc.w += w * v.w;
+  }
+  const float inv = 1.f / weight;
+  *reinterpret_cast<uint2*>(p.out + (size_t(b) * p.hq + head) * kD + lane * 4) =
+      make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
+  if (lane == 0) p.lse[size_t(b) * p.hq + head] = mm + log2f(weight);
 }
 
 struct Handle {
@@ -516,7 +616,6 @@ inline void geometry(int hkv, int sms, int* ranges, int* grid) {
     *grid = sms;
   }
 }
-constexpr int kMaxSms = 192;             // SM count the workspace is sized for
 
 // A range holds a piece of every sequence it touches: at most ranges + batch pieces in all.
 inline size_t entries_for(const cake_b200_gqa_decode_config& c, int sms) {
@@ -577,10 +676,16 @@ inline int fill_params(Params& p, void** buffers, const cake_b200_gqa_decode_con
 inline int launch(Params& p, int sms, cudaStream_t s) {
   int grid;
   geometry(p.hkv, sms, &p.ranges, &grid);
-  gqa_plan_kernel<<<1, 1024, 0, s>>>(p);
+  // A sequence cut into more than a handful of pieces is merged by a kernel of its own: the one warp that merges it inside
+  // the decode kernel reads four pieces at a time, 14 us for the 50 to 90 pieces of each of three long sequences, against
+  // 3 us for the launch.  At eight ranges a sequence the two cost the same.
+  p.merge_kernel = p.batch * 8 <= p.ranges;
+  if (int rc = launch_dependent(gqa_plan_kernel, dim3(1), dim3(1024), 0, s, p)) return rc;
   // The decode grid is a programmatic dependent: it may start while the plan kernel runs and waits
   // for it on the device, which takes the second launch latency off the critical path.
-  return launch_dependent(gqa_decode_kernel, dim3(grid), dim3(kWarps * 32), kSmemBytes, s, p);
+  if (int rc = launch_dependent(gqa_decode_kernel, dim3(grid), dim3(kWarps * 32), kSmemBytes, s, p)) return rc;
+  if (!p.merge_kernel) return 0;
+  return launch_dependent(gqa_merge_kernel, dim3(p.hq, p.batch), dim3(kMergeWarps * 32), 0, s, p);
 }
 
 }  // namespace gqa
