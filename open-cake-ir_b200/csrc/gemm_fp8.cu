@@ -91,7 +91,7 @@ extern "C" int cake_b200_block_scaled_gemm_create(void** buffers, const cake_b20
     q.out = p.out;
     q.status = h->status;
     q.n = int(n);
-    q.k_blocks = q.w_k_blocks = p.k_blocks;
+    q.k_blocks = p.k_blocks;
     q.w_rows = int(n);
     q.groups = 1;
     q.dense_rows = int(m);
@@ -99,7 +99,7 @@ extern "C" int cake_b200_block_scaled_gemm_create(void** buffers, const cake_b20
     q.sx_stride = int(m);
     q.terms = 1;
     h->skinny_grid = int(skinny_items < sms ? skinny_items : sms);
-    rc = skinny::prepare_any<gemm::kDense>(h->skinny_tiles, h->skinny_split);
+    rc = skinny::prepare_any<gemm::kDense>(h->skinny_tiles, h->skinny_split, 1);
     if (rc) { delete h; return rc; }
   }
   *handle_out = h;
@@ -115,7 +115,7 @@ extern "C" int cake_b200_block_scaled_gemm_launch(void* handle, void* cuda_strea
   if (device != h->device) return kErrWrongDevice;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(cuda_stream);
   if (h->skinny_tiles && !test_hooks().skip_load)
-    return skinny::launch_any<gemm::kDense>(h->skinny_tiles, h->skinny_split, h->skinny, h->skinny_grid, stream);
+    return skinny::launch_any<gemm::kDense>(h->skinny_tiles, h->skinny_split, 1, h->skinny, h->skinny_grid, stream);
   gemm::Params p = h->params;
   p.wait_kiloclocks = test_hooks().budget_kiloclocks;
   p.skip_load = test_hooks().skip_load;

@@ -18,6 +18,7 @@
 // so that fragments of all four k-steps are two 16-byte shared-memory reads per row instead of eight 4-byte ones.
 #pragma once
 #include "gemm_fp8.cuh"
+#include <type_traits>
 
 namespace cake {
 namespace skinny {
@@ -31,10 +32,10 @@ constexpr int kWeightBytes = kSubRows * 128;       // of one K block
 constexpr int kMaxGroups = gemm::kMaxGroups;
 
 struct Params {
-  const uint8_t* w;            // [groups, w_rows, 128 * w_k_blocks]
-  const float* sw;             // [groups, w_rows / 128, w_k_blocks]
+  const uint8_t* w;            // [groups, w_rows, 128 * k_blocks]
+  const float* sw;             // [groups, w_rows / 128, k_blocks]
   const uint8_t* x;            // rows of x_stride bytes
-  const float* sx;             // [k_blocks, sx_stride]
+  const float* sx;             // [k_blocks * TERMS, sx_stride]
   const int* row_map;          // sorted row -> pair, token = pair / map_div, which names the row of x and sx (null: the sorted row does)
   const int* offsets;          // [groups + 1] rows before a group (null: one group of dense_rows rows)
   const float* row_weight;     // kDown: route weight of a pair (by row_map_weight)
@@ -42,14 +43,16 @@ struct Params {
   void* out;                   // kGateUp: e4m3 [rows, n * terms] (WK = 1) or fp32 [rows, n]; else bf16 [rows, n]
   float* out_scale;            // kGateUp, WK = 1: [n / 128 * terms, row_capacity]
   int* status;                 // status word to clear (null: someone else does); nothing here waits, so nothing ever sets it
-  int n, k_blocks, w_k_blocks, w_rows, groups, dense_rows, x_stride, sx_stride, map_div, row_capacity, terms;
-  int interleave_hi_lo;        // 1: K block kb is token column block (kb & 1) * (k_blocks / 2) + kb / 2, weight column block kb / 2
+  int n, k_blocks, w_rows, groups, dense_rows, x_stride, sx_stride, map_div, row_capacity, terms;
 };
 
-template <int NT, int WK>
+// TERMS: e4m3 terms of a token row (value, residual), one row of k_blocks after the other; a weight block meets both.
+template <int NT, int WK, int TERMS>
 struct Shape {
   static constexpr int kTokens = NT * 8;
-  static constexpr int kSlotBytes = kWeightBytes + kTokens * 128 + 256;        // + the block's scales
+  static constexpr int kTermBytes = kTokens * 128;
+  static constexpr int kScaleOffset = kWeightBytes + TERMS * kTermBytes;        // 128 bytes of sx per term, then sw
+  static constexpr int kSlotBytes = kScaleOffset + TERMS * 128 + 128;
   static constexpr int kReduceBytes = WK > 1 ? kWarps * NT * 4 * 32 * 4 : 0;    // one MMA tile's sums of every warp
   static constexpr int kSlots = (232448 - 8192 - kReduceBytes) / (kWarps * kSlotBytes) > 6 ? 6 : (232448 - 8192 - kReduceBytes) / (kWarps * kSlotBytes);
   static constexpr int kSmemBytes = kSlots * kWarps * kSlotBytes + kReduceBytes;
@@ -89,10 +92,10 @@ struct Item {
   int group, feature0, row0, rows;                 // first feature of the CTA's sub-tiles; first sorted row; rows of it (<= 8 NT)
 };
 
-template <int MODE, int NT, int WK>
+template <int MODE, int NT, int WK, int TERMS>
 __global__ void __launch_bounds__(kThreads, 1)
 skinny_kernel(const Params p) {
-  using S = Shape<NT, WK>;
+  using S = Shape<NT, WK, TERMS>;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ int tile_prefix[kMaxGroups + 1];      // row tiles before a group
   __shared__ float group_amax[2][kWarps][S::kTokens];
@@ -154,7 +157,7 @@ skinny_kernel(const Params p) {
   const uint8_t* x_ptr[2 * NT];                    // this lane's token rows (null: no such row)
   const float* sx_ptr = nullptr;                   // this lane's token's scales
   int load_tiles = 0;                              // token tiles of eight in the item
-  const size_t w_stride = size_t(p.w_k_blocks) * 128;
+  const size_t w_stride = size_t(p.k_blocks) * 128;
   auto open_item = [&]() {
     if (load_item >= items) return;
     Item it;
@@ -163,7 +166,7 @@ skinny_kernel(const Params p) {
     const uint8_t* w = p.w + (size_t(it.group) * p.w_rows + f + (lane >> 3)) * w_stride + (lane & 7) * 16;
     w_lo = w;
     w_hi = w + size_t(MODE == kGateUp ? p.n : 16) * w_stride;
-    sw_ptr = p.sw + (size_t(it.group) * (p.w_rows / 128) + f / 128 + (MODE == kGateUp ? (lane & 1) * (p.n / 128) : 0)) * p.w_k_blocks;
+    sw_ptr = p.sw + (size_t(it.group) * (p.w_rows / 128) + f / 128 + (MODE == kGateUp ? (lane & 1) * (p.n / 128) : 0)) * p.k_blocks;
     load_tiles = (it.rows + 7) >> 3;
 #pragma unroll
     for (int i = 0; i < 2 * NT; ++i) {
@@ -179,22 +182,24 @@ skinny_kernel(const Params p) {
   };
   auto load_next = [&]() {                         // one slot; an empty copy group past the end, so that the group count stays
     if (load_item < items) {
-      int x_col = load_kb, w_col = load_kb;
-      if (p.interleave_hi_lo) { x_col = (load_kb & 1) * (p.k_blocks >> 1) + (load_kb >> 1); w_col = load_kb >> 1; }
       const uint32_t dst = ring + load_slot * S::kSlotBytes + (lane >> 3) * 128;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {                // four rows of 128 bytes per instruction
-        const uint8_t* src = (i < 4 ? w_lo : w_hi) + size_t(w_col) * 128 + size_t(i & 3) * 4 * w_stride;
+        const uint8_t* src = (i < 4 ? w_lo : w_hi) + size_t(load_kb) * 128 + size_t(i & 3) * 4 * w_stride;
         cp_async_16_hint(dst + i * 512 + (((lane & 7) ^ ((i * 4 + (lane >> 3)) & 7)) << 4), src, stream);
       }
+      const uint32_t scales = ring + load_slot * S::kSlotBytes + S::kScaleOffset;
 #pragma unroll
-      for (int i = 0; i < 2 * NT; ++i)
-        if (i < 2 * load_tiles)
-          cp_async_16_zfill(dst + kWeightBytes + i * 512 + (((lane & 7) ^ ((i * 4 + (lane >> 3)) & 7)) << 4),
-                            x_ptr[i] ? x_ptr[i] + size_t(x_col) * 128 : p.x, x_ptr[i] != nullptr);
-      const uint32_t scales = ring + load_slot * S::kSlotBytes + kWeightBytes + S::kTokens * 128;
-      if (lane < S::kTokens) cp_async_4_zfill(scales + lane * 4, sx_ptr ? sx_ptr + size_t(x_col) * p.sx_stride : p.sx, sx_ptr != nullptr);
-      if (lane < 2) cp_async_4_zfill(scales + 128 + lane * 4, sw_ptr + w_col, true);
+      for (int term = 0; term < TERMS; ++term) {
+        const int x_col = term * p.k_blocks + load_kb;
+#pragma unroll
+        for (int i = 0; i < 2 * NT; ++i)
+          if (i < 2 * load_tiles)
+            cp_async_16_zfill(dst + kWeightBytes + term * S::kTermBytes + i * 512 + (((lane & 7) ^ ((i * 4 + (lane >> 3)) & 7)) << 4),
+                              x_ptr[i] ? x_ptr[i] + size_t(x_col) * 128 : p.x, x_ptr[i] != nullptr);
+        if (lane < S::kTokens) cp_async_4_zfill(scales + term * 128 + lane * 4, sx_ptr ? sx_ptr + size_t(x_col) * p.sx_stride : p.sx, sx_ptr != nullptr);
+      }
+      if (lane < 2) cp_async_4_zfill(scales + TERMS * 128 + lane * 4, sw_ptr + load_kb, true);
       load_kb += WK;
       if (load_kb >= p.k_blocks) { load_kb = wk; load_item += gridDim.x; open_item(); }
       load_slot = load_slot + 1 == S::kSlots ? 0 : load_slot + 1;
@@ -212,6 +217,10 @@ skinny_kernel(const Params p) {
     Item it;
     locate(i, &it);
     const int tiles = (it.rows + 7) >> 3;
+    // the route weight of token `lane`, asked for before the products: asked for where it is used, its two dependent loads
+    // took longer than the products of a short K
+    float token_weight = 0.f;
+    if (MODE == kDown && lane < it.rows) token_weight = __ldg(p.row_weight + __ldg(p.weight_map + it.row0 + lane));
     float acc[2][NT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n)
@@ -221,7 +230,7 @@ skinny_kernel(const Params p) {
       cp_async_wait<S::kSlots - 2>();
       __syncwarp();                                // the slot has landed for every lane; every lane is done with the one before
       load_next();
-      const uint32_t s = ring + slot * S::kSlotBytes, scales = s + kWeightBytes + S::kTokens * 128;
+      const uint32_t s = ring + slot * S::kSlotBytes, scales = s + S::kScaleOffset;
       uint32_t a[2][2][8];                         // [MMA tile][row g / g + 8][k-step pair words]
 #pragma unroll
       for (int t = 0; t < 2; ++t)
@@ -232,14 +241,15 @@ skinny_kernel(const Params p) {
           a[t][h][0] = lo.x; a[t][h][1] = lo.y; a[t][h][2] = lo.z; a[t][h][3] = lo.w;
           a[t][h][4] = hi.x; a[t][h][5] = hi.y; a[t][h][6] = hi.z; a[t][h][7] = hi.w;
         }
-      const float2 sw = lds64f(scales + 128);
+      const float2 sw = lds64f(scales + TERMS * 128);
 #pragma unroll
-      for (int n = 0; n < NT; ++n) {
+      for (int m = 0; m < NT * TERMS; ++m) {
+        const int n = m / TERMS, term = m % TERMS;
         if (n >= tiles) break;
-        const uint32_t xr = s + kWeightBytes + (n * 8 + g8) * 128;
+        const uint32_t xr = s + kWeightBytes + term * S::kTermBytes + (n * 8 + g8) * 128;
         const uint4 lo = lds128(xr + (((2 * q) ^ g8) << 4)), hi = lds128(xr + (((2 * q + 1) ^ g8) << 4));
         const uint32_t b[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-        const float2 sx = lds64f(scales + (n * 8 + q * 2) * 4);
+        const float2 sx = lds64f(scales + term * 128 + (n * 8 + q * 2) * 4);
         float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
@@ -261,12 +271,12 @@ skinny_kernel(const Params p) {
     // One accumulator of each MMA tile: token 8 n + 2 q + (e & 1) of the item, feature f + g + 8 (e >> 1) (+ 16 in tile 1)
     auto emit = [&](int n, int e, float v0, float v1) {
       const int token = n * 8 + q * 2 + (e & 1);
+      const float w = MODE == kDown ? __shfl_sync(0xffffffffu, token_weight, token) : 1.f;
       if (!exists || token >= it.rows) return;
       const size_t at = size_t(it.row0 + token) * p.n + f + g8 + 8 * (e >> 1);
       if (MODE == kGateUp) {
         reinterpret_cast<float*>(p.out)[at] = v0 * (v1 / (1.f + __expf(-v1)));
       } else {
-        const float w = MODE == kDown ? __ldg(p.row_weight + __ldg(p.weight_map + it.row0 + token)) : 1.f;
         reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(v0 * w);
         reinterpret_cast<__nv_bfloat16*>(p.out)[at + 16] = __float2bfloat16_rn(v1 * w);
       }
@@ -305,12 +315,15 @@ skinny_kernel(const Params p) {
     } else {
       // SwiGLU, then e4m3 quantisation over the item's 128 features (16 of each warp): the warps' maxima meet in shared memory
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
+      for (int n = 0; n < NT; ++n) {
+        if (n >= tiles) break;
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[0][n][e] *= acc[1][n][e] / (1.f + __expf(-acc[1][n][e]));
+      }
       for (int term = 0; term < p.terms; ++term, flip ^= 1) {
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+        for (int n = 0; n < NT; ++n) {
+          if (n >= tiles) break;
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             float m = fmaxf(fabsf(acc[0][n][e]), fabsf(acc[0][n][e + 2]));
@@ -318,9 +331,11 @@ skinny_kernel(const Params p) {
             for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
             if (g8 == 0) group_amax[flip][warp][n * 8 + q * 2 + e] = m;
           }
+        }
         __syncthreads();
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
+          if (n >= tiles) break;
           float scale[2], inv[2];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
@@ -371,49 +386,53 @@ quantize_kernel(const float* __restrict__ in, const int* __restrict__ rows_ptr, 
   }
 }
 
-template <int MODE, int NT, int WK>
-inline int launch(const Params& p, int grid, cudaStream_t s) {
-  return launch_dependent(skinny_kernel<MODE, NT, WK>, dim3(grid), dim3(kThreads), Shape<NT, WK>::kSmemBytes, s, p);
-}
-template <int MODE, int NT, int WK>
-inline int prepare() {
-  return int(cudaFuncSetAttribute(skinny_kernel<MODE, NT, WK>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<NT, WK>::kSmemBytes));
-}
-
-// The three shapes of K split, for `nt` token tiles of eight: a kernel's entry points by run-time numbers.
-template <int MODE, int NT>
-inline int launch_wk(int wk, const Params& p, int grid, cudaStream_t s) {
-  return wk == 1 ? launch<MODE, NT, 1>(p, grid, s) : wk == 4 && MODE != kGateUp ? launch<MODE, NT, MODE == kGateUp ? 8 : 4>(p, grid, s) : launch<MODE, NT, 8>(p, grid, s);
-}
-template <int MODE>
-inline int launch_any(int nt, int wk, const Params& p, int grid, cudaStream_t s) {
-  return nt == 1 ? launch_wk<MODE, 1>(wk, p, grid, s) : nt == 2 ? launch_wk<MODE, 2>(wk, p, grid, s) : launch_wk<MODE, 4>(wk, p, grid, s);
-}
-template <int MODE, int NT>
-inline int prepare_wk(int wk) {
-  return wk == 1 ? prepare<MODE, NT, 1>() : wk == 4 && MODE != kGateUp ? prepare<MODE, NT, MODE == kGateUp ? 8 : 4>() : prepare<MODE, NT, 8>();
+// A kernel's entry points by run-time numbers: token tiles of eight, K split, terms (two in the down mode only).
+template <int MODE, typename F>
+inline int with_shape(int nt, int wk, int terms, F f) {
+  auto by_terms = [&](auto tiles, auto split) {
+    if constexpr (MODE == kDown) { if (terms == 2) return f(tiles, split, std::integral_constant<int, 2>()); }
+    return f(tiles, split, std::integral_constant<int, 1>());
+  };
+  auto by_split = [&](auto tiles) {
+    if (wk == 1) return by_terms(tiles, std::integral_constant<int, 1>());
+    if constexpr (MODE != kGateUp) { if (wk == 4) return by_terms(tiles, std::integral_constant<int, 4>()); }
+    return by_terms(tiles, std::integral_constant<int, 8>());
+  };
+  return nt == 1 ? by_split(std::integral_constant<int, 1>()) : nt == 2 ? by_split(std::integral_constant<int, 2>()) : by_split(std::integral_constant<int, 4>());
 }
 template <int MODE>
-inline int prepare_any(int nt, int wk) {
-  return nt == 1 ? prepare_wk<MODE, 1>(wk) : nt == 2 ? prepare_wk<MODE, 2>(wk) : prepare_wk<MODE, 4>(wk);
+inline int launch_any(int nt, int wk, int terms, const Params& p, int grid, cudaStream_t s) {
+  return with_shape<MODE>(nt, wk, terms, [&](auto tiles, auto split, auto t) {
+    return launch_dependent(skinny_kernel<MODE, tiles(), split(), t()>, dim3(grid), dim3(kThreads), Shape<tiles(), split(), t()>::kSmemBytes, s, p);
+  });
+}
+template <int MODE>
+inline int prepare_any(int nt, int wk, int terms) {
+  return with_shape<MODE>(nt, wk, terms, [](auto tiles, auto split, auto t) {
+    return int(cudaFuncSetAttribute(skinny_kernel<MODE, tiles(), split(), t()>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<tiles(), split(), t()>::kSmemBytes));
+  });
 }
 
 // Token tiles of eight per item, so that most groups of a layer fit one item: 8, 16 or 32 rows for an average of 3, 9 or more.
 inline int token_tiles(double rows_per_group) { return rows_per_group <= 3 ? 1 : rows_per_group <= 9 ? 2 : 4; }
 
-// How many warps share a sub-tile's K blocks: fewest rounds of the GPU, counted in weight rows a CTA streams one after
-// another; on a tie the smaller split, which meets less often.  `row_tiles`: row tiles of all groups together.
+// Time of a launch in units of a warp's K block (32 weight rows x 128): rounds of the GPU times an item's K blocks and what
+// it costs beside them.  `features`: of an item, `row_tiles`: row tiles of all groups together.
+inline double cost(double row_tiles, int n, int features, int k_blocks, int wk, int sms) {
+  const double items = row_tiles * ((n + features - 1) / features);
+  const double rounds = items <= sms ? 1 : items > 8 * sms ? items / sms : double((long long)(items / sms + 0.999));
+  return rounds * ((k_blocks + wk - 1) / wk + 3);
+}
+// How many warps share a sub-tile's K blocks; on a tie the smaller split, which meets less often.
 inline int choose_split(double row_tiles, int n, int k_blocks, int sms) {
   int best = 1;
-  double best_cost = 1e30;
-  for (int wk = 1; wk <= 8; wk *= 2) {
-    if (wk == 2 || wk > k_blocks) continue;
-    const int features = 32 * (kWarps / wk);
-    const double items = row_tiles * ((n + features - 1) / features);
-    const double rounds = items <= sms ? 1 : items > 8 * sms ? items / sms : double((long long)(items / sms + 0.999));
-    if (rounds * features < best_cost * 0.999) { best_cost = rounds * features; best = wk; }
-  }
+  for (int wk : {4, 8})
+    if (wk <= k_blocks && cost(row_tiles, n, 32 * (kWarps / wk), k_blocks, wk, sms) < 0.999 * cost(row_tiles, n, 32 * (kWarps / best), k_blocks, best, sms)) best = wk;
   return best;
+}
+// The same for the gate/up product (16 features to a sub-tile), where a split means that quantize_kernel runs after it.
+inline int choose_split_gate_up(double row_tiles, int n, int k_blocks, int sms) {
+  return k_blocks >= 8 && cost(row_tiles, n, 16, k_blocks, 8, sms) + 5 < cost(row_tiles, n, 128, k_blocks, 1, sms) ? 8 : 1;
 }
 
 }  // namespace skinny

@@ -420,8 +420,8 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
     double missed = 1;                   // experts that get a row: those not missed by every token
     for (int64_t t = 0; t < c.tokens && missed > 1e-3; ++t) missed *= 1.0 - double(c.top_k) / c.experts;
     const double touched = c.local_experts * (1 - missed);
-    l.split1 = touched * (c.intermediate / 128) >= 2 * 148 || c.hidden / 128 < 8 ? 1 : 8;
-    l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128 * l.terms, 148);
+    l.split1 = skinny::choose_split_gate_up(touched > 1 ? touched : 1, c.intermediate, c.hidden / 128, 148);
+    l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128, 148);
     if (l.split1 > 1) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation
   }
   l.total = at;
@@ -629,7 +629,7 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
     s1.out = l.split1 > 1 ? static_cast<void*>(h->ws + l.act32) : p1.out;
     s1.out_scale = p1.out_scale;
     s1.n = inter;
-    s1.k_blocks = s1.w_k_blocks = hidden / 128;
+    s1.k_blocks = hidden / 128;
     s1.w_rows = 2 * inter;
     s1.groups = c.local_experts;
     s1.x_stride = hidden;
@@ -647,16 +647,14 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
     s2.weight_map = sorted_pairs;
     s2.out = p2.out;
     s2.n = hidden;
-    s2.k_blocks = p2.k_blocks;
-    s2.w_k_blocks = p2.b_k_blocks;
+    s2.k_blocks = p2.b_k_blocks;
     s2.w_rows = hidden;
     s2.groups = c.local_experts;
     s2.x_stride = inter * l.terms;
     s2.sx_stride = s2.row_capacity = l.capacity;
     s2.terms = 1;
-    s2.interleave_hi_lo = p2.interleave_hi_lo;
-    rc = skinny::prepare_any<gemm::kGateUp>(l.token_tiles, l.split1);
-    if (!rc) rc = skinny::prepare_any<gemm::kDown>(l.token_tiles, l.split2);
+    rc = skinny::prepare_any<gemm::kGateUp>(l.token_tiles, l.split1, 1);
+    if (!rc) rc = skinny::prepare_any<gemm::kDown>(l.token_tiles, l.split2, l.terms);
     if (rc) { delete h; return rc; }
   }
   *handle_out = h;
@@ -696,7 +694,7 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
     }
     case 1: {
       if (l.token_tiles) {
-        if (int rc = skinny::launch_any<gemm::kGateUp>(l.token_tiles, l.split1, h->s1, h->grid, s)) return rc;
+        if (int rc = skinny::launch_any<gemm::kGateUp>(l.token_tiles, l.split1, 1, h->s1, h->grid, s)) return rc;
         if (l.split1 == 1) return 0;
         const int64_t rows = int64_t(l.capacity) * (c.intermediate / 128);
         return launch_dependent(skinny::quantize_kernel, dim3(unsigned(rows < 8 * 592 ? (rows + 7) / 8 : 592)), dim3(256), 0, s,
@@ -708,7 +706,7 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
       return launch_dependent(gemm::gemm_fp8_kernel<gemm::kGateUp>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a1, h->map_a1_tail, h->map_b1, p);
     }
     case 2: {
-      if (l.token_tiles) return skinny::launch_any<gemm::kDown>(l.token_tiles, l.split2, h->s2, h->grid, s);
+      if (l.token_tiles) return skinny::launch_any<gemm::kDown>(l.token_tiles, l.split2, l.terms, h->s2, h->grid, s);
       gemm::Params p = h->p2;
       p.wait_kiloclocks = test_hooks().budget_kiloclocks;
       return launch_dependent(gemm::gemm_fp8_kernel<gemm::kDown>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a2, h->map_a2_tail, h->map_b2, p);
