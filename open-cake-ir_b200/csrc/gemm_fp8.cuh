@@ -199,7 +199,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   // launched as a programmatic dependent where the caller says so: everything above overlaps the kernel before
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (SPLIT && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;      // long before any wait can run out
+  if (MODE == kDense && !p.queue && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;      // long before any wait can run out
   if (warp == kControlWarps) {   // m-tile prefix over groups (serial per lane chunk, then a warp scan)
     int running = 0;
     for (int base = 0; base < p.groups; base += 32) {
