@@ -92,8 +92,7 @@ struct Params {
 };
 
 struct Shared {
-  uint64_t k_full[kStages], v_full[kStages];             // this CTA's rows have landed
-  uint64_t peer_k_full[kStages], peer_v_full[kStages];   // CTA 0: those of CTA 1 have
+  uint64_t k_full[kStages], v_full[kStages];             // this CTA's rows have landed (CTA 0: and CTA 1's, by its relay)
   uint64_t k_empty[kStages], v_empty[kStages], q_empty;  // by commit, in both CTAs
   uint64_t s_full[2], o_full;                            // by commit, in both CTAs
   uint64_t p_ready, o_empty;                             // CTA 0: four warps of each CTA
@@ -305,34 +304,21 @@ __device__ __forceinline__ void arrive_at(uint64_t* bar, uint32_t rank) {
   asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tmbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
                ::"r"(smem_u32(bar)), "r"(rank) : "memory");
 }
-// mbar_wait for a barrier that the other CTA arrives on: what it wrote before is visible after.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  const uint32_t start = clock();
-  for (uint32_t spins = 0;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred P;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, P;\n\t}"
-        : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    if (done) return true;
-    if (++spins == 1024) {
-      if (mbar_wait_expired(start, abort_flag, status, code)) return false;
-      spins = 0;
-    }
-  }
-}
-__device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+// The whole warp runs the issuing loop and one lane of it (`leader`) issues: with uniform control flow the compiler keeps
+// addresses in uniform registers, where these instructions want them (750 clocks for the 36 products of S otherwise).
+__device__ __forceinline__ void mma_pair(uint32_t leader, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 // Arrives on `bar` of both CTAs when every product issued so far has completed.
-__device__ __forceinline__ void commit_pair(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"(uint16_t(3)) : "memory");
+__device__ __forceinline__ void commit_pair(uint32_t leader, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+               ::"r"(smem_u32(bar)), "h"(uint16_t(3)), "r"(leader) : "memory");
 }
 // 32 bytes at once: a lane has a row of its own, and a whole sector per store leaves twice as fast as halves of one.
 __device__ __forceinline__ void store_32(void* dst, const uint32_t (&v)[8]) {
@@ -380,8 +366,7 @@ mla_decode_kernel(const Params p) {
   Shared* sh = reinterpret_cast<Shared*>(base + kQBytes + kStages * (kKBytes + kVBytes) + 2 * kPBytes);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(&sh->k_full[s], kLoaderThreads); mbar_init(&sh->v_full[s], kLoaderThreads);
-      mbar_init(&sh->peer_k_full[s], 1); mbar_init(&sh->peer_v_full[s], 1);
+      mbar_init(&sh->k_full[s], kLoaderThreads + 1 - rank); mbar_init(&sh->v_full[s], kLoaderThreads + 1 - rank);
       mbar_init(&sh->k_empty[s], 1); mbar_init(&sh->v_empty[s], 1);
       mbar_init(&sh->s_full[s], 1);
       mbar_init(&sh->pair[s], 2);
@@ -413,12 +398,20 @@ mla_decode_kernel(const Params p) {
     // A warp gathers eight of this CTA's 32 tokens (all of a row, for K) and the same tokens and eight of the other CTA's
     // (this CTA's dims, for V).  Lanes 0..7 look up the rows of the own tokens, lanes 8..15 of the others, a tile ahead.
     const bool skip = p.skip_load != 0;
-    auto lookup = [&](int j) -> long long {
+    // The page number stays as it was loaded until its rows are asked for (`resolve`): worked on at once, each lookup held the
+    // warp for its trip to L2.
+    struct Lookup { int page, offset; };           // offset -1: no such token
+    auto lookup = [&](int j) -> Lookup {
       const int half = lane < 8 ? rank : rank ^ 1;
       const int tok = w.begin + j * kTile + half * kOwn + warp * 8 + (lane & 7);
-      if (lane >= 16 || tok >= w.end) return -1;
-      if (SPARSE) return (long long)__ldg(p.sparse_indices + w.page_base + tok);
-      return (long long)__ldg(p.kv_indices + w.page_base + tok / p.page_size) * p.page_size + tok % p.page_size;
+      if (lane >= 16 || tok >= w.end) return {0, -1};
+      if (SPARSE) return {__ldg(p.sparse_indices + w.page_base + tok), 0};
+      const int page = tok / p.page_size;
+      return {__ldg(p.kv_indices + w.page_base + page), tok - page * p.page_size};
+    };
+    auto resolve = [&](Lookup l) -> long long {
+      asm volatile("" : "+r"(l.page));             // not before this point
+      return l.offset < 0 ? -1 : (long long)l.page * p.page_size + l.offset;
     };
     auto load_k = [&](uint32_t i, long long rows) {
       const uint32_t dst = k_addr + (i % kStages) * kKBytes;
@@ -447,7 +440,8 @@ mla_decode_kernel(const Params p) {
       }
     };
     for (; ok && next_piece<SPARSE>(p, range_end, &cursor, &w); ++pieces) {
-      long long rows = lookup(0), ahead = w.tiles > 1 ? lookup(1) : -1;
+      long long rows = resolve(lookup(0)), next = -1;
+      Lookup ahead = w.tiles > 1 ? lookup(1) : Lookup{0, -1};
       auto k_tile = [&](uint32_t i, long long r) {
         ok = ok && mbar_wait(&sh->k_empty[i % kStages], ((i / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
         if (!ok || (skip && pieces == 0 && i == 2)) return;      // test hook: never filled
@@ -467,39 +461,40 @@ mla_decode_kernel(const Params p) {
       }
       k_tile(it, rows);
       for (int j = 0; ok && j < w.tiles; ++j, ++it) {
-        const long long further = j + 2 < w.tiles ? lookup(j + 2) : -1;
-        if (j + 1 < w.tiles) k_tile(it + 1, ahead);
+        const Lookup further = j + 2 < w.tiles ? lookup(j + 2) : Lookup{0, -1};
+        next = resolve(ahead);
+        if (j + 1 < w.tiles) k_tile(it + 1, next);
         ok = ok && mbar_wait(&sh->v_empty[it % kStages], ((it / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
         if (!ok) break;
         load_v(it, rows);
         cp_async_arrive_noinc(&sh->v_full[it % kStages]);
-        rows = ahead;
+        rows = next;
         ahead = further;
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == kMmaWarp) {
-    if (rank == 0 && elect_one()) {
+    if (rank == 0) {
       // ------------------------------ MMA issuer --------------------------------------
       constexpr uint32_t idesc_qk = umma_idesc_ex(1 /* bf16 */, kHeads, kTile, 0, 0);
       constexpr uint32_t idesc_pv = umma_idesc_ex(1 /* bf16 */, kHeads, 256, 0, 1 /* V is MN-major */);
+      const uint32_t leader = elect_one();
       auto issue_qk = [&](uint32_t i, bool last) {
         const int s = i % kStages;
         const uint32_t parity = (i / kStages) & 1;
         // S buffer i mod 2 needs no wait: the softmax has read it before it announced P(i - 2), which O(i - 2) waited for
-        ok = mbar_wait(&sh->k_full[s], parity, abort_flag, p.status, kStatusWaitSmemFull) &&
-             mbar_wait_cluster(&sh->peer_k_full[s], parity, abort_flag, p.status, kStatusWaitSmemFull);
+        ok = mbar_wait(&sh->k_full[s], parity, abort_flag, p.status, kStatusWaitSmemFull);
         if (!ok) return;
         fence_proxy_async_smem();                  // rows were written by cp.async (generic proxy), the products read them through the async proxy
         tcgen05_fence_after();
         const uint64_t a = umma_desc_sw128(q_addr), b = umma_desc_sw128(k_addr + s * kKBytes);
 #pragma unroll
         for (int step = 0; step < kRow / 16; ++step)
-          mma_pair(tmem_base + kColS + (i & 1) * 32, a + uint64_t(((step >> 2) * kQSlabBytes + (step & 3) * 32) >> 4),
+          mma_pair(leader, tmem_base + kColS + (i & 1) * 32, a + uint64_t(((step >> 2) * kQSlabBytes + (step & 3) * 32) >> 4),
                    b + uint64_t(((step >> 2) * kKSlabBytes + (step & 3) * 32) >> 4), idesc_qk, step != 0);
-        commit_pair(&sh->s_full[i & 1]);
-        commit_pair(&sh->k_empty[s]);
-        if (last) commit_pair(&sh->q_empty);
+        commit_pair(leader, &sh->s_full[i & 1]);
+        commit_pair(leader, &sh->k_empty[s]);
+        if (last) commit_pair(leader, &sh->q_empty);
       };
       for (; ok && next_piece<SPARSE>(p, range_end, &cursor, &w); ++pieces) {
         issue_qk(it, w.tiles == 1);
@@ -508,9 +503,8 @@ mla_decode_kernel(const Params p) {
           const int s = it % kStages;
           const uint32_t parity = (it / kStages) & 1;
           ok = ok && mbar_wait(&sh->v_full[s], parity, abort_flag, p.status, kStatusWaitSmemFull) &&
-               mbar_wait_cluster(&sh->peer_v_full[s], parity, abort_flag, p.status, kStatusWaitSmemFull) &&
-               (j > 0 || mbar_wait_cluster(&sh->o_empty, (pieces & 1) ^ 1, abort_flag, p.status, kStatusWaitTmemEmpty)) &&
-               mbar_wait_cluster(&sh->p_ready, it & 1, abort_flag, p.status, kStatusWaitFlag);
+               (j > 0 || mbar_wait(&sh->o_empty, (pieces & 1) ^ 1, abort_flag, p.status, kStatusWaitTmemEmpty)) &&
+               mbar_wait(&sh->p_ready, it & 1, abort_flag, p.status, kStatusWaitFlag);
           if (!ok) break;
           fence_proxy_async_smem();
           tcgen05_fence_after();
@@ -523,25 +517,25 @@ mla_decode_kernel(const Params p) {
             for (int term = 0; term < 2; ++term)
 #pragma unroll
               for (int ks = 0; ks < kTile / 16; ++ks)
-                mma_pair(tmem_base + kColO + half * 128, a + uint64_t((term * kPBytes + ks * 32) >> 4),
+                mma_pair(leader, tmem_base + kColO + half * 128, a + uint64_t((term * kPBytes + ks * 32) >> 4),
                          v + uint64_t((half * 2 * kVSlabBytes + ks * 2048) >> 4), idesc_pv, (j | term | ks) != 0);
-          commit_pair(&sh->v_empty[s]);
-          if (j + 1 == w.tiles) commit_pair(&sh->o_full);
+          commit_pair(leader, &sh->v_empty[s]);
+          if (j + 1 == w.tiles) commit_pair(leader, &sh->o_full);
         }
       }
     } else if (rank == 1 && elect_one()) {
       // ------------------------------ relay -------------------------------------------
-      auto relay = [&](uint64_t* full, uint64_t* peer, uint32_t i) {
+      auto relay = [&](uint64_t* full, uint32_t i) {
         ok = ok && mbar_wait(&full[i % kStages], (i / kStages) & 1, abort_flag, p.status, kStatusWaitSmemFull);
         if (!ok) return;
         fence_proxy_async_smem();
-        arrive_at(&peer[i % kStages], 0);
+        arrive_at(&full[i % kStages], 0);
       };
       for (; ok && next_piece<SPARSE>(p, range_end, &cursor, &w); ++pieces) {
-        relay(sh->k_full, sh->peer_k_full, it);
+        relay(sh->k_full, it);
         for (int j = 0; ok && j < w.tiles; ++j, ++it) {
-          if (j + 1 < w.tiles) relay(sh->k_full, sh->peer_k_full, it + 1);
-          relay(sh->v_full, sh->peer_v_full, it);
+          if (j + 1 < w.tiles) relay(sh->k_full, it + 1);
+          relay(sh->v_full, it);
         }
       }
     }
