@@ -11,7 +11,7 @@ struct DenseHandle {
   int device;
   CUtensorMap map_a, map_a_tail, map_b;
   gemm::Params params;
-  int grid, split;                     // CTAs of a cluster that share a tile's K (1: none)
+  int grid, split;                     // CTAs that share a tile of 128 columns (0: tiles of 256, the whole of K to a CTA)
   int* status;
   int skinny_grid, skinny_tiles, skinny_split;      // few rows: token tiles of eight and K split of skinny_kernel (0: the tcgen05 core)
   skinny::Params skinny;
@@ -44,7 +44,15 @@ extern "C" int cake_b200_block_scaled_gemm_create(void** buffers, const cake_b20
   h->device = device;
   int rc = make_tensor_map_u8_sw128(&h->map_a, buffers[0], uint64_t(m), uint64_t(k), gemm::kBM);
   if (!rc) rc = make_tensor_map_u8_sw128(&h->map_a_tail, buffers[0], uint64_t(m), uint64_t(k), gemm::kTailRows);
-  if (!rc) rc = make_tensor_map_u8_sw128(&h->map_b, buffers[2], uint64_t(n), uint64_t(k), gemm::kBN);
+  // Where tiles of 128 columns leave SMs idle, two or four CTAs of a cluster share a tile's K, at least four K blocks each
+  // (64 x 4096 x 7168: 28.7 us as 16 tiles of 256 columns, 15.5 at four CTAs to each of them, 12.1 at four CTAs to each of 32
+  // tiles of 128; clusters of eight do not all fit the GPU at a time).
+  const int sms = sm_count(device), row_tiles = int((m + gemm::kBM - 1) / gemm::kBM);
+  const int64_t narrow = row_tiles * (n / 128);
+  h->split = 0;
+  for (int s = 4; s > 1 && !h->split; s >>= 1)
+    if (narrow * s <= sms && k / gemm::kBK >= 4 * s) h->split = s;
+  if (!rc) rc = make_tensor_map_u8_sw128(&h->map_b, buffers[2], uint64_t(n), uint64_t(k), h->split ? 128 : gemm::kBN);
   if (!rc) rc = int(cudaFuncSetAttribute(gemm::gemm_fp8_kernel<gemm::kDense>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemm::kSmemBytes)));
   if (rc) { delete h; return rc; }
@@ -63,21 +71,15 @@ extern "C" int cake_b200_block_scaled_gemm_create(void** buffers, const cake_b20
   h->status = static_cast<int*>(buffers[5]);
   p.status = h->status;
   p.queue = h->status + 4;               // work-item counter, inside the 256-byte status block
-  const long long items = ((m + gemm::kBM - 1) / gemm::kBM) * ((n + gemm::kBN - 1) / gemm::kBN);
-  const int sms = sm_count(device);
-  // Where tiles leave SMs idle, two or four CTAs of a cluster share a tile's K, at least four K blocks each (64 x 4096 x 7168:
-  // 28.7 us unsplit, 22.1 at two, 15.6 at four; 23 at eight, where the exchange of the sums costs more than the K blocks saved).
-  h->split = 1;
-  for (int s = 4; s > 1 && h->split == 1; s >>= 1)
-    if (items * s <= sms && p.k_blocks >= 4 * s) h->split = s;
+  const long long items = row_tiles * ((n + gemm::kBN - 1) / gemm::kBN);
   // Drawing items from a counter evens out SMs of different speed, 2 % of a long launch, but the counter has to be cleared in
   // front of the kernel, 4 us: not for a few rounds of the GPU (346 x 6272 x 640, one round: 12.3 -> 7.5 us).
   if (items <= 6 * sms) p.queue = nullptr;
-  if (h->split > 1) {
+  if (h->split) {
     rc = int(cudaFuncSetAttribute(gemm::gemm_fp8_kernel<gemm::kDense, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemm::kSmemBytes)));
     if (rc) { delete h; return rc; }
   }
-  h->grid = h->split > 1 ? int(items) * h->split : int(items < sms ? items : sms);
+  h->grid = h->split ? int(narrow) * h->split : int(items < sms ? items : sms);
   // At most 16 rows go through the weight-streaming kernel (4096 x 7168: 8.9 us at 1 row, 10.5 at 16; 14.4 for a split tile
   // of the core).  Beyond, its second tile of 16 rows reads the weights again.
   h->skinny_tiles = m > 16 ? 0 : m <= 8 ? 1 : 2;
@@ -121,7 +123,7 @@ extern "C" int cake_b200_block_scaled_gemm_launch(void* handle, void* cuda_strea
   gemm::Params p = h->params;
   p.wait_kiloclocks = test_hooks().budget_kiloclocks;
   p.skip_load = test_hooks().skip_load;
-  if (h->split > 1)
+  if (h->split)
     return launch_dependent_cluster(h->split, gemm::gemm_fp8_kernel<gemm::kDense, true>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes,
                                     stream, h->map_a, h->map_a_tail, h->map_b, p);
   if (p.queue) CAKE_CUDA_OK(cudaMemsetAsync(h->status, 0, 8 * sizeof(int), stream));     // status word and work-item counter

@@ -44,9 +44,10 @@ constexpr int kEpilogueWarps = 8;                 // two warpgroups: 2 column gr
 constexpr int kThreads = (kControlWarps + kEpilogueWarps) * 32;
 // Register budget moved between the warpgroups once the roles split.  The pool setmaxnreg draws on
 // is what the launch allocated, 168 registers x 384 threads = 64512, not the SM's 65536: an
-// increase that asks for more than the pool ever holds blocks for good.  128 x 40 + 256 x 232 = 64512.
-constexpr int kControlRegs = 40;
-constexpr int kEpilogueRegs = 232;
+// increase that asks for more than the pool ever holds blocks for good.  128 x 56 + 256 x 224 = 64512 (at 40 and 232 the kernel spilled
+// a few registers: the MoE layer 2 % slower).
+constexpr int kControlRegs = 56;
+constexpr int kEpilogueRegs = 224;
 static_assert(kControlWarps * 32 * kControlRegs + kEpilogueWarps * 32 * kEpilogueRegs <= (65536 / kThreads / 8 * 8) * kThreads,
               "setmaxnreg budget exceeds the registers the launch allocates");
 constexpr int kMaxGroups = 512;
@@ -160,9 +161,9 @@ __device__ __forceinline__ float4 load_cluster(uint32_t local_addr, uint32_t ran
   return v;
 }
 
-// SPLIT (dense only): the CTAs of a cluster share one output tile, each a part of K.  A problem of few tiles otherwise runs
-// its K blocks, about 0.45 us each, one after another on a handful of SMs (64 x 4096 x 7168: 16 SMs).  The parts meet
-// through distributed shared memory: CTA r finishes columns [256 r / S, 256 (r + 1) / S) of the tile.
+// SPLIT (dense only): tiles of 128 columns, each shared by the CTAs of a cluster (two or four), a part of K to each.  A
+// problem of few tiles otherwise runs its K blocks, about 0.45 us each, one after another on a handful of SMs (64 x 4096 x
+// 7168: 16 SMs).  The parts meet through distributed shared memory: CTA r finishes columns [128 r / S, 128 (r + 1) / S).
 template <int MODE, bool SPLIT = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a_tail,
@@ -181,7 +182,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const int first_item = SPLIT ? blockIdx.x / split : blockIdx.x;
   const int k_begin = SPLIT ? int(rank * uint32_t(p.k_blocks) / split) : 0;                  // this CTA's K blocks
   const int k_count = SPLIT ? int((rank + 1) * uint32_t(p.k_blocks) / split) - k_begin : p.k_blocks;
-  const int n_tiles = (MODE == kGateUp) ? p.n / 128 : (p.n + kBN - 1) / kBN;
+  constexpr int kCols = SPLIT ? 128 : kBN;         // columns of a tile
+  const int n_tiles = (MODE == kGateUp) ? p.n / 128 : (p.n + kCols - 1) / kCols;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 1 + 32); mbar_init(&sh->empty[s], 1); }
@@ -261,7 +263,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // draw, so every byte not fetched shortens it.  Rows of the stage beyond them keep what an earlier tile left
         // there; their products land in accumulator rows that no one reads.
         const bool tail = item.rows_valid <= kTailRows;
-        const uint32_t stage_tx = tail ? uint32_t(kTailRows * kBK + kBytesB) : uint32_t(kStageBytes);
+        const uint32_t stage_tx = uint32_t((tail ? kTailRows * kBK : kBytesA) + kCols * kBK);
         for (int kb = 0; kb < k_count; ++kb, ++it) {
           const int s = it % kStages;
           ok = mbar_wait(&sh->empty[s], ((it / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
@@ -278,7 +280,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + item.n_tile * 128, &sh->full[s]);
             tma_load_2d(b_dst + 128 * kBK, &map_b, b_col * kBK, b_row0 + p.n + item.n_tile * 128, &sh->full[s]);
           } else {
-            tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + item.n_tile * kBN, &sh->full[s]);
+            tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + item.n_tile * kCols, &sh->full[s]);
           }
         }
         g = drawn;
@@ -289,7 +291,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------------------
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc(0 /* e4m3 */, kBM, kBN);
+      constexpr uint32_t idesc = umma_idesc(0 /* e4m3 */, kBM, kCols);
       uint32_t it = 0, k = 0;
       bool ok = true;
       Item item;
@@ -348,7 +350,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       }
       if (!locate(sh, p, n_tiles, g, &item)) break;
       // lanes 0 and 1 also fetch sfb: of x1 and x2 in the gate/up mode, else of the tile's two 128-column halves
-      const int sfb_row = MODE == kGateUp ? item.n_tile + (lane & 1) * (p.n / 128) : min(item.n_tile * 2 + (lane & 1), sfb_rows - 1);
+      const int sfb_row = MODE == kGateUp ? item.n_tile + (lane & 1) * (p.n / 128) : SPLIT ? item.n_tile : min(item.n_tile * 2 + (lane & 1), sfb_rows - 1);
       const float* sfb = p.sfb + (size_t(item.group) * sfb_rows + sfb_row) * p.b_k_blocks;
       for (int kb = 0; ok && kb < k_count; ++kb, ++it) {
         ok = it < kScaleAhead || mbar_wait(&sh->empty[(it - kScaleAhead) % kStages], (((it - kScaleAhead) / kStages) & 1) ^ 1, abort_flag,
@@ -382,7 +384,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const uint32_t lane_base = tmem_base + (uint32_t(quad * 32) << 16);
     // Two 64-column segments per thread: gate/up takes 64 x1 columns and the matching 64 x2
     // columns; the other modes take 128 consecutive columns.
-    const int seg_col0 = (MODE == kGateUp) ? cg * 64 : cg * 128;
+    const int seg_col0 = (MODE == kGateUp || SPLIT) ? cg * 64 : cg * 128;
     const int seg_col1 = (MODE == kGateUp) ? 128 + cg * 64 : cg * 128 + 64;
     uint32_t it = 0, k = 0;
     uint32_t exchanges = 0;                    // amax exchanges so far (phase of Shared::exchange_done)
@@ -407,7 +409,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       float sa = 0.f, sb0 = 0.f, sb1 = 0.f;    // scales of the coming block
       auto read_scales = [&](uint32_t block) {
         sa = sh->scale_a[block % kScaleSlots][r];
-        sb0 = sh->scale_b[block % kScaleSlots][MODE == kGateUp ? 0 : cg];
+        sb0 = sh->scale_b[block % kScaleSlots][MODE == kGateUp || SPLIT ? 0 : cg];
         if (MODE == kGateUp) sb1 = sh->scale_b[block % kScaleSlots][1];
       };
       if (it > 0) read_scales(it);
@@ -425,11 +427,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const uint64_t s0p = pack_f32x2(s0, s0);
 #pragma unroll
         for (int i = 0; i < 32; ++i) acc2[i] = fma_f32x2(v[i], s0p, acc2[i]);
-        tmem_ld_wait_64(stage_addr + seg_col1, v);
+        if (!SPLIT) tmem_ld_wait_64(stage_addr + seg_col1, v);
         tcgen05_fence_before();            // everything this warp needs has left tensor memory
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->tmem_empty[t]);
         if (kb + 1 < k_count) read_scales(it + 1);
+        if (SPLIT) continue;                   // 64 columns to a thread
         const uint64_t s1p = pack_f32x2(s1, s1);
 #pragma unroll
         for (int i = 0; i < 32; ++i) acc2[32 + i] = fma_f32x2(v[i], s1p, acc2[32 + i]);
@@ -439,20 +442,20 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // CTA reads its own columns of all of them.  Each starts with its own part and goes round from there, so that the
         // CTAs of a cluster read from different ones at a time (pushed to their owners, all in the same order, the sums took
         // 14 us at eight CTAs).
-        const int chunks = 64 / int(split);
+        const int chunks = 32 / int(split);
         float4* sums = reinterpret_cast<float4*>(tiles);
         if (ok) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < 16; ++i) {
             float4 v;
             unpack_f32x2(acc2[2 * i], v.x, v.y);
             unpack_f32x2(acc2[2 * i + 1], v.z, v.w);
-            sums[(cg * 32 + i) * kBM + r] = v;
+            sums[(cg * 16 + i) * kBM + r] = v;
           }
         }
         cluster_sync();
         if (ok) {
-          const int rows = (item.rows_valid + 31) & ~31, column0 = item.n_tile * kBN + int(rank) * chunks * 4;
+          const int rows = (item.rows_valid + 31) & ~31, column0 = item.n_tile * kCols + int(rank) * chunks * 4;
           for (int i = threadIdx.x - kControlWarps * 32; i < rows * chunks / 2; i += kEpilogueWarps * 32) {
             const int row_i = i % rows, c = i / rows * 2;
             const uint32_t from = smem_u32(sums + (int(rank) * chunks + c) * kBM + row_i);

@@ -1,0 +1,25 @@
+"""The MoE layer at few rows per expert, on either side of each line of the weight-streaming kernel's dispatch: one, two or
+four token tiles of eight, experts with more rows than an item holds, K split over a CTA's warps or not (with the
+quantisation in a kernel of its own), one and two activation terms, routing and placement in one kernel (up to 32 tokens)
+or two, and the tcgen05 core just beyond.  Oracle and tolerance of test_gpu_moe.py's layer test."""
+import pytest
+import torch
+
+import open_cake_ir_b200 as cake
+from oracle import compare, moe as oracle_moe
+from test_gpu_moe import run_layer
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens,hidden,inter,experts,local,offset,act", [
+    (1, 1024, 256, 64, 64, 0, "split"), (3, 512, 128, 64, 16, 32, "fp8"), (20, 1024, 256, 64, 64, 0, "fp8"),      # one token tile
+    (30, 1024, 512, 64, 64, 0, "split"), (32, 2048, 256, 32, 8, 8, "fp8"), (33, 1024, 256, 32, 32, 0, "split"),   # two
+    (60, 1024, 256, 32, 32, 0, "split"), (80, 256, 384, 32, 4, 28, "fp8"), (81, 256, 384, 32, 4, 28, "fp8")])     # four; the core
+def test_few_rows_per_expert(tokens, hidden, inter, experts, local, offset, act):
+    cpu = cake.workloads.moe_inputs(tokens, hidden, inter, experts, local, offset, routing="softmax", device="cpu")
+    # every token goes to one expert of this rank, which so has more rows than an item or a tile holds
+    cpu["routing_logits"][:, offset] += 8.0
+    out, _ = run_layer(cpu, experts=experts, routing="softmax", act_mode=act)
+    want = oracle_moe.moe_reference(cpu, routing="softmax", act_quant="fp8" if act == "fp8" else "none", dtype=torch.float32)
+    assert compare.rel_frobenius(out, want["output"]) <= (1e-2 if act == "fp8" else 4e-3)
