@@ -458,6 +458,48 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, float* v) {
       : "memory");
 }
 
+// ---- pairs of CTAs (clusters of two that share products) ------------------------------------------------
+// A rendezvous of a cluster's CTAs.  A hardware barrier: every CTA gets to it, since every wait before is bounded.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// An arrival on CTA `rank`'s barrier at the same place as `bar` here.  What it announces lies in this CTA's shared memory and is
+// read by the tensor core, in front of which every writer has put a proxy fence; a release at cluster scope on top of that
+// took 1060 clocks.
+__device__ __forceinline__ void arrive_at(uint64_t* bar, uint32_t rank) {
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tmbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
+               ::"r"(smem_u32(bar)), "r"(rank) : "memory");
+}
+// The whole warp runs the issuing loop and one lane of it (`leader`) issues: with uniform control flow the compiler keeps
+// addresses in uniform registers, where these instructions want them (750 clocks for the 36 products of S otherwise).
+__device__ __forceinline__ void mma_pair(uint32_t leader, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+// Arrives on `bar` of both CTAs when every product issued so far has completed.
+__device__ __forceinline__ void commit_pair(uint32_t leader, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+               ::"r"(smem_u32(bar)), "h"(uint16_t(3)), "r"(leader) : "memory");
+}
+// All 512 columns of both SMs; one warp of each CTA.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t columns) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(columns) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t columns) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
 // Exclusive scan over the 1024 threads of a CTA (every thread must call); `total` receives the sum
 // and `warp_sums` is 32 elements of shared memory.
 template <typename T>

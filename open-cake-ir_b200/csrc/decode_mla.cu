@@ -294,32 +294,6 @@ __device__ __forceinline__ bool next_piece(const Params& p, int range_end, Curso
   return false;
 }
 
-__device__ __forceinline__ void cluster_sync() {           // hardware barrier: every CTA gets to it, since every wait before is bounded
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-// An arrival on CTA `rank`'s barrier at the same place as `bar` here.  What it announces lies in this CTA's shared memory and is
-// read by the tensor core, in front of which every writer has put a proxy fence; a release at cluster scope on top of that
-// took 1060 clocks.
-__device__ __forceinline__ void arrive_at(uint64_t* bar, uint32_t rank) {
-  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tmbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
-               ::"r"(smem_u32(bar)), "r"(rank) : "memory");
-}
-// The whole warp runs the issuing loop and one lane of it (`leader`) issues: with uniform control flow the compiler keeps
-// addresses in uniform registers, where these instructions want them (750 clocks for the 36 products of S otherwise).
-__device__ __forceinline__ void mma_pair(uint32_t leader, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
-      : "memory");
-}
-// Arrives on `bar` of both CTAs when every product issued so far has completed.
-__device__ __forceinline__ void commit_pair(uint32_t leader, uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
-      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
-               ::"r"(smem_u32(bar)), "h"(uint16_t(3)), "r"(leader) : "memory");
-}
 // 32 bytes at once: a lane has a row of its own, and a whole sector per store leaves twice as fast as halves of one.
 __device__ __forceinline__ void store_32(void* dst, const uint32_t (&v)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
@@ -332,8 +306,7 @@ mla_decode_kernel(const Params p) {
   extern __shared__ uint8_t smem_raw[];
   // launched as a programmatic dependent of the plan kernel: resident early, reads the plan after that grid has completed
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  uint32_t rank;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const uint32_t rank = cluster_rank();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head_blocks = (p.rows + kHeads - 1) / kHeads;
   const int cluster = blockIdx.x >> 1, hb = cluster % head_blocks, worker = cluster / head_blocks;
@@ -379,8 +352,7 @@ mla_decode_kernel(const Params p) {
     fence_barrier_init();
   }
   if (warp == kMmaWarp) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem_base)), "r"(kTmemColumns) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    tmem_alloc_pair(&sh->tmem_base, kTmemColumns);
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -714,7 +686,7 @@ mla_decode_kernel(const Params p) {
   __syncthreads();
   cluster_sync();                                  // neither CTA leaves while the other may still reach into it
   tcgen05_fence_after();
-  if (warp == kMmaWarp) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemColumns) : "memory");
+  if (warp == kMmaWarp) tmem_dealloc_pair(tmem_base, kTmemColumns);
 }
 
 // Merges the pieces of the cut sequences: CTA (x, y) two rows of the y-th, 128 threads x 4 dims each, the results of four

@@ -150,10 +150,6 @@ __device__ __forceinline__ bool locate(const Shared* sh, const Params& p, int n_
   return true;
 }
 
-// Two CTA-wide rendezvous of a cluster.  Hardware barriers: every CTA gets to them, since every wait before is bounded.
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
 __device__ __forceinline__ float4 load_cluster(uint32_t local_addr, uint32_t rank) {
   float4 v;
   asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"

@@ -73,6 +73,7 @@ static __global__ void __launch_bounds__(1024)
 plan_kernel(const Params p) {
   __shared__ int sums[32];
   __shared__ int bucket[kCostBuckets];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x;
   const int per = 2 * (kRows / p.group);
@@ -303,13 +304,19 @@ prefill_kernel(const Params p) {
       Work w;
       for (int k = 0; ok && get_work(p, units, k, &w); ++k) {
         if (w.n == 0) continue;
-        auto lookup = [&](int j) {
+        struct Lookup { int page, offset; };       // offset -1: no such token
+        auto lookup = [&](int j) -> Lookup {
           const int token = j * kTile + lw * 32 + lane;
-          if (token >= w.kv_len) return -1;
-          if (!p.kv_indices) return w.page_base + token;
-          return __ldg(p.kv_indices + w.page_base + token / p.page_size) * p.page_size + token % p.page_size;      // < 2^31 rows
+          if (token >= w.kv_len) return {0, -1};
+          if (!p.kv_indices) return {0, w.page_base + token};
+          const int page = token / p.page_size;
+          return {__ldg(p.kv_indices + w.page_base + page), token - page * p.page_size};
         };
-        int row = lookup(0);
+        auto resolve = [&](Lookup l) {
+          asm volatile("" : "+r"(l.page));         // the page number is not worked on before this point, so the lookup is not waited for
+          return l.offset < 0 ? -1 : l.page * p.page_size + l.offset;      // < 2^31 rows
+        };
+        Lookup ahead = lookup(0);
         // Q rows: token q0 + x * per_half + r / G, head kvh * G + r % G; rows without a token are zeros
         for (int x = 0; ok && x < 2; ++x) {
           if (w.n_kv[x] == 0) continue;
@@ -326,7 +333,8 @@ prefill_kernel(const Params p) {
         }
         for (int j = 0; ok && j < w.n; ++j, ++it) {
           const int s = it % kStages;
-          const int next = j + 1 < w.n ? lookup(j + 1) : -1;
+          const int row = resolve(ahead);
+          ahead = j + 1 < w.n ? lookup(j + 1) : Lookup{0, -1};
 #pragma unroll
           for (int kv = 0; kv < 2; ++kv) {
             ok = mbar_wait(kv ? &sh->v_empty[s] : &sh->k_empty[s], ((it / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
@@ -342,7 +350,6 @@ prefill_kernel(const Params p) {
             cp_async_arrive_noinc(kv ? &sh->v_full[s] : &sh->k_full[s]);
           }
           if (!ok) break;
-          row = next;
         }
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
