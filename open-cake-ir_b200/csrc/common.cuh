@@ -580,6 +580,21 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
   __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3);
   return uint32_t(lo) | (uint32_t(hi) << 16);
 }
+__device__ __forceinline__ float2 e4m3x2_to_float2(uint16_t v) {
+  const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(v, __NV_E4M3);
+  return __half22float2(*reinterpret_cast<const __half2*>(&h));
+}
+// x * sigmoid(x).  The quotient is an approximate one, corrected once by what it leaves of x: the correction squares the
+// relative error of a couple of ulp, so that the last rounding is all that is left of it.  Unlike the `/` operator it has no
+// branch for the ends of the range, so that a thread's many values overlap: 64 of them, with `/` one after another, took
+// an epilogue of the MoE layer 5000 clocks.  The denominator stays below 2^126, where the approximation still holds:
+// below -87 the result is x * 1.6e-38 instead of something smaller yet.
+__device__ __forceinline__ float silu(float x) {
+  const float d = 1.f + __expf(fminf(-x, 87.f));
+  const float r = __fdividef(1.f, d);
+  const float q = x * r;
+  return fmaf(fmaxf(fmaf(-q, d, x), -3.4e38f), r, q);      // the limit is for an infinite x, which leaves inf - inf
+}
 __device__ __forceinline__ float e4m3_to_float(uint8_t v) {
   __half_raw h = __nv_cvt_fp8_to_halfraw(v, __NV_E4M3);
   return __half2float(*reinterpret_cast<__half*>(&h));

@@ -92,13 +92,13 @@ struct Params {
 
 struct Shared {
   uint4 out_rows[kEpilogueWarps][128];                      // per epilogue warp: 32 rows of 64 bytes on their way out
+  int4 item[kItemSlots];                                    // group (-1: no further item), first row, rows, n tile
   uint64_t full[kStages];
   uint64_t empty[kStages];
   uint64_t tmem_full[kTmemStages];
   uint64_t tmem_empty[kTmemStages];
   uint64_t exchange_done;                                   // kGateUp: all epilogue warps have published their amax
-  uint64_t item_full[kItemSlots], item_empty[kItemSlots];   // hand-over of drawn work items from the TMA warp to the other roles
-  int item_q[kItemSlots];
+  uint64_t item_full[kItemSlots], item_empty[kItemSlots];   // hand-over of work items from the TMA warp to the other roles
   float scale_a[kScaleSlots][kBM];                          // sfa of the tile's rows for one K block
   float scale_b[kScaleSlots][2];                            // sfb of the tile's two 128-column halves
   uint32_t tmem_base;
@@ -223,6 +223,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   tcgen05_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   volatile int* abort_flag = &sh->wait.abort_flag;
+  // With groups, or where items are drawn, the TMA warp, which is ahead of the others, finds an item's group and rows and
+  // hands them on: the search of the prefix and the two offsets behind it cost the epilogue 1400 clocks an item (a K block
+  // takes it 800), in which no product was taken up.  One group without a queue has nothing to search.
+  const bool handed = p.queue || p.offsets;
 
   if (warp < kControlWarps) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kControlRegs));
@@ -244,13 +248,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       while (ok) {
         const bool valid = locate(sh, p, n_tiles, g, &item);
         int drawn = g + int(gridDim.x);
-        if (p.queue) {
+        if (handed) {
           const int slot = k % kItemSlots;
           ok = mbar_wait(&sh->item_empty[slot], ((k / kItemSlots) & 1) ^ 1, abort_flag, p.status, kStatusWaitFlag);
           if (!ok) break;
-          sh->item_q[slot] = valid ? g : -1;
+          sh->item[slot] = valid ? make_int4(item.group, item.row0, item.rows_valid, item.n_tile) : make_int4(-1, 0, 0, 0);
           mbar_arrive(&sh->item_full[slot]);
-          if (valid) drawn = int(gridDim.x) + atomicAdd(p.queue, 1);
+          if (p.queue && valid) drawn = int(gridDim.x) + atomicAdd(p.queue, 1);
         }
         if (!valid) break;
         const int b_row0 = item.group * p.b_rows_per_group;
@@ -292,15 +296,16 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       bool ok = true;
       Item item;
       for (int g = first_item; ok; g += gridDim.x, ++k) {
-        if (p.queue) {                 // the k-th item of this CTA, as drawn by the TMA warp
+        if (handed) {                  // the k-th item of this CTA, from the TMA warp
           const int slot = k % kItemSlots;
           ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
           if (!ok) break;
-          g = sh->item_q[slot];
+          const bool any = sh->item[slot].x >= 0;
           mbar_arrive(&sh->item_empty[slot]);
-          if (g < 0) break;
+          if (!any) break;
+        } else if (!locate(sh, p, n_tiles, g, &item)) {
+          break;
         }
-        if (!locate(sh, p, n_tiles, g, &item)) break;
         for (int kb = 0; kb < k_count; ++kb, ++it) {
           const int s = it % kStages;
           const int t = it % kTmemStages;
@@ -335,16 +340,18 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     bool ok = true;
     Item item;
     for (int g = first_item; ok; g += gridDim.x, ++k) {
-      if (p.queue) {                   // the k-th item of this CTA, as drawn by the TMA warp
+      if (handed) {                    // the k-th item of this CTA, from the TMA warp
         const int slot = k % kItemSlots;
         ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
         if (!ok) break;
-        g = sh->item_q[slot];
+        const int4 v = sh->item[slot];
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->item_empty[slot]);
-        if (g < 0) break;
+        if (v.x < 0) break;
+        item.group = v.x; item.row0 = v.y; item.rows_valid = v.z; item.n_tile = v.w;
+      } else if (!locate(sh, p, n_tiles, g, &item)) {
+        break;
       }
-      if (!locate(sh, p, n_tiles, g, &item)) break;
       // lanes 0 and 1 also fetch sfb: of x1 and x2 in the gate/up mode, else of the tile's two 128-column halves
       const int sfb_row = MODE == kGateUp ? item.n_tile + (lane & 1) * (p.n / 128) : SPLIT ? item.n_tile : min(item.n_tile * 2 + (lane & 1), sfb_rows - 1);
       const float* sfb = p.sfb + (size_t(item.group) * sfb_rows + sfb_row) * p.b_k_blocks;
@@ -388,17 +395,21 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     bool ok = true, met = false;               // met: SPLIT, this thread has been at the cluster's barriers
     Item item;
     for (int g = first_item; ok; g += gridDim.x, parity ^= 1, ++k) {
-      if (p.queue) {                   // the k-th item of this CTA, as drawn by the TMA warp
+      if (handed) {                    // the k-th item of this CTA, from the TMA warp
         const int slot = k % kItemSlots;
         ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
         if (!ok) break;
-        g = sh->item_q[slot];
+        const int4 v = sh->item[slot];
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->item_empty[slot]);
-        if (g < 0) break;
+        if (v.x < 0) break;
+        item.group = v.x; item.row0 = v.y; item.rows_valid = v.z; item.n_tile = v.w;
+      } else if (!locate(sh, p, n_tiles, g, &item)) {
+        break;
       }
-      if (!locate(sh, p, n_tiles, g, &item)) break;
       const int row = item.row0 + r;
+      float w = 1.f;                            // asked for here, a round trip to L2 before the K blocks end
+      if (MODE == kDown && r < item.rows_valid) w = __ldg(p.row_weight + row);
       uint64_t acc2[64];                        // 128 fp32 accumulators as packed pairs
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc2[i] = 0;
@@ -487,7 +498,6 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const bool valid = r < item.rows_valid && columns_exist;
 
       if (MODE == kDense || MODE == kDown) {
-        const float w = MODE == kDown && valid ? __ldg(p.row_weight + row) : 1.f;
         uint8_t* out = reinterpret_cast<uint8_t*>(reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(item.row0 + quad * 32) * p.n + item.n_tile * kBN + cg * 128);
         const int rows = columns_exist ? item.rows_valid - quad * 32 : 0;
 #pragma unroll
@@ -504,11 +514,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       } else {
         // SwiGLU on the 64 (x1, x2) pairs this thread holds, then e4m3 quantisation of the 128-wide
         // group it shares with the thread of the same row in the other column group.
+        // Nothing overlaps it but the two blocks the tensor core is ahead, so its length counts in full: 8700 clocks (11100
+        // with the second term) with the gate's quotient by `/` and one e4m3 value taken back at a time, against 900 a K
+        // block.  The first GEMM of 2500 tokens, hidden 2048, 128 experts of 768, two terms: 204 us then, 163 now.
         float amax = 0.f;
 #pragma unroll
         for (int i = 0; i < 64; ++i) {
-          const float gate = acc[64 + i];
-          acc[i] = acc[i] * (gate / (1.f + __expf(-gate)));
+          acc[i] *= silu(acc[64 + i]);
           amax = fmaxf(amax, fabsf(acc[i]));
         }
         const int out_kb = p.n / 128;                      // K blocks of one term of the output
@@ -537,10 +549,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           if (term + 1 < terms) {        // residual after the first term becomes the value to quantise
             amax = 0.f;
 #pragma unroll
-            for (int i = 0; i < 64; ++i) {
-              const uint32_t word = packed[i >> 2];
-              acc[i] -= e4m3_to_float(uint8_t(word >> ((i & 3) * 8))) * scale;
-              amax = fmaxf(amax, fabsf(acc[i]));
+            for (int i = 0; i < 64; i += 2) {
+              const float2 first = e4m3x2_to_float2(uint16_t(packed[i >> 2] >> ((i & 2) * 8)));
+              acc[i] -= first.x * scale;
+              acc[i + 1] -= first.y * scale;
+              amax = fmaxf(amax, fmaxf(fabsf(acc[i]), fabsf(acc[i + 1])));
             }
           }
         }

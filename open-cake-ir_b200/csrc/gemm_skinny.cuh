@@ -275,7 +275,7 @@ skinny_kernel(const Params p) {
       if (!exists || token >= it.rows) return;
       const size_t at = size_t(it.row0 + token) * p.n + f + g8 + 8 * (e >> 1);
       if (MODE == kGateUp) {
-        reinterpret_cast<float*>(p.out)[at] = v0 * (v1 / (1.f + __expf(-v1)));
+        reinterpret_cast<float*>(p.out)[at] = v0 * silu(v1);
       } else {
         reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(v0 * w);
         reinterpret_cast<__nv_bfloat16*>(p.out)[at + 16] = __float2bfloat16_rn(v1 * w);
@@ -318,7 +318,7 @@ skinny_kernel(const Params p) {
       for (int n = 0; n < NT; ++n) {
         if (n >= tiles) break;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[0][n][e] *= acc[1][n][e] / (1.f + __expf(-acc[1][n][e]));
+        for (int e = 0; e < 4; ++e) acc[0][n][e] *= silu(acc[1][n][e]);
       }
       for (int term = 0; term < p.terms; ++term, flip ^= 1) {
 #pragma unroll

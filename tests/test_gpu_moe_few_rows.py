@@ -23,3 +23,16 @@ def test_few_rows_per_expert(tokens, hidden, inter, experts, local, offset, act)
     out, _ = run_layer(cpu, experts=experts, routing="softmax", act_mode=act)
     want = oracle_moe.moe_reference(cpu, routing="softmax", act_quant="fp8" if act == "fp8" else "none", dtype=torch.float32)
     assert compare.rel_frobenius(out, want["output"]) <= (1e-2 if act == "fp8" else 4e-3)
+
+
+@pytest.mark.parametrize("act", ["fp8", "split"])
+@pytest.mark.parametrize("tokens", [12, 200])          # the weight-streaming kernel; the tcgen05 core, tiles of 128 and 72 rows
+def test_gates_at_the_ends_of_the_sigmoid(tokens, act):
+    """Gates of several hundred either way: the sigmoid is 0 or 1 to the last bit, and nothing overflows on the way there."""
+    experts, offset = 8, 0
+    cpu = cake.workloads.moe_inputs(tokens, 512, 256, experts, experts, offset, routing="softmax", device="cpu")
+    cpu["gemm1_weights_scale"] = cpu["gemm1_weights_scale"] * 300
+    out, _ = run_layer(cpu, experts=experts, routing="softmax", act_mode=act)
+    want = oracle_moe.moe_reference(cpu, routing="softmax", act_quant="fp8" if act == "fp8" else "none", dtype=torch.float32)
+    assert torch.isfinite(out.float()).all()
+    assert compare.rel_frobenius(out, want["output"]) <= (1e-2 if act == "fp8" else 4e-3)
