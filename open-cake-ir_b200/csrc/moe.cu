@@ -412,14 +412,18 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
   l.act = take(size_t(l.capacity) * c.intermediate * l.terms);
   l.act_scale = take(size_t(c.intermediate / 128) * l.terms * l.capacity * 4);
   l.y = take(size_t(l.capacity) * c.hidden * 2);
-  // The weight-streaming kernel up to 20 rows per expert on average (beyond, an expert needs a second tile of 32 rows often
-  // enough, and products begin to cost more than the weights' way from memory).
+  // The weight-streaming kernel where an expert has few rows: it gathers nothing and keeps more loads in flight, but its
+  // products grow with the rows, and a second tile of an expert streams the weights again.  The tcgen05 core's time hardly
+  // depends on the rows up to 128.  They meet at 7 to 8 rows per expert on average (hidden 7168, 64 experts of 2048: 523 us
+  // and 545 at 7 rows, 552 and 543 at 8, 678 and 545 at 19; hidden 2048, 128 experts of 768: 137 and 146 at 5, 162 and
+  // 145 at 8), and at 10 to 12 where the core's tiles are fewer than the SMs and it leaves some idle (hidden 7168, 4 experts
+  // of 2048: 69 and 72 us at 10 rows, 91 and 77 at 19; of 768, hidden 2048: 30 and 35 at 10).
   const double per_expert = double(pairs) / c.experts;
-  if (per_expert <= 20) {
+  double missed = 1;                     // experts that get a row: those not missed by every token
+  for (int64_t t = 0; t < c.tokens && missed > 1e-3; ++t) missed *= 1.0 - double(c.top_k) / c.experts;
+  const double touched = c.local_experts * (1 - missed);
+  if (per_expert <= (touched * (c.intermediate / 128) < 148 ? 11.0 : 7.5)) {
     l.token_tiles = skinny::token_tiles(per_expert);
-    double missed = 1;                   // experts that get a row: those not missed by every token
-    for (int64_t t = 0; t < c.tokens && missed > 1e-3; ++t) missed *= 1.0 - double(c.top_k) / c.experts;
-    const double touched = c.local_experts * (1 - missed);
     l.split1 = skinny::choose_split_gate_up(touched > 1 ? touched : 1, c.intermediate, c.hidden / 128, 148);
     l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128, 148);
     if (l.split1 > 1) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation

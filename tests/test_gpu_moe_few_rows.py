@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("tokens,hidden,inter,experts,local,offset,act", [
     (1, 1024, 256, 64, 64, 0, "split"), (3, 512, 128, 64, 16, 32, "fp8"), (20, 1024, 256, 64, 64, 0, "fp8"),      # one token tile
     (30, 1024, 512, 64, 64, 0, "split"), (32, 2048, 256, 32, 8, 8, "fp8"), (33, 1024, 256, 32, 32, 0, "split"),   # two
-    (60, 1024, 256, 32, 32, 0, "split"), (80, 256, 384, 32, 4, 28, "fp8"), (81, 256, 384, 32, 4, 28, "fp8")])     # four; the core
+    (42, 1024, 256, 32, 32, 0, "split"), (44, 256, 384, 32, 4, 28, "fp8"), (45, 256, 384, 32, 4, 28, "fp8"),      # four; the core
+    (60, 512, 512, 64, 64, 0, "fp8"), (61, 512, 512, 64, 64, 0, "split")])        # more tiles than SMs: two; the core
 def test_few_rows_per_expert(tokens, hidden, inter, experts, local, offset, act):
     cpu = cake.workloads.moe_inputs(tokens, hidden, inter, experts, local, offset, routing="softmax", device="cpu")
     # every token goes to one expert of this rank, which so has more rows than an item or a tile holds
