@@ -340,7 +340,7 @@ def moe_single(steps, warmup, peaks, cohorts):
     return {"ms": statistics.median(samples), "cohorts": cohort_stats(samples), "flops": flops, "clocks": summary,
             "stage_ms": dict(zip(cake.Fp8Moe.STAGES, stage_ms)),
             "stage_cycles": {name: ms * 1e-3 * mhz * 1e6 for name, ms in zip(cake.Fp8Moe.STAGES, stage_ms)},
-            "roofline": roofline, "e2e_ms": e2e_ms, "h2d": h2d, "d2h": d2h, "launches": 8 * steps, "contract_mode": contract}
+            "roofline": roofline, "e2e_ms": e2e_ms, "h2d": h2d, "d2h": d2h, "launches": 6 * steps, "contract_mode": contract}
 
 
 def moe_compute_bound(steps, peaks):

@@ -247,8 +247,8 @@ int cake_b200_moe_intermediate(void* handle, int which, void** device_pointer_ou
  * buffers: q bf16 [B,Hq,D], k_cache bf16 [pages,page_size,Hkv,D], v_cache (same), kv_indptr int32 [B+1] (pages),
  *          kv_indices int32 [*], kv_last_page_len int32 [B] (extension for page_size > 1; the reference has page_size 1),
  *          sm_scale fp32 [1], output bf16 [B,Hq,D], lse fp32 [B,Hq], workspace.  D == 128; Hq/Hkv in 1..8;
- *          batch <= 65535; max_kv_len <= 2^21.  A launch is two kernels (work list, then decode + merge); the
- *          work is cut on the device from the sequence lengths, so max_kv_len does not enter the workspace size.
+ *          batch <= 65535; max_kv_len <= 2^21.  A launch is two kernels (work list, decode), and a third that
+ *          merges where few sequences are cut into many pieces; the work is cut on the device from the sequence lengths, so max_kv_len does not enter the workspace size.
  * ---------------------------------------------------------------------------------------- */
 typedef struct {
   int64_t batch;
@@ -289,9 +289,9 @@ size_t cake_b200_gqa_decode_noalloc_scratch_limit(void);
  * buffers: q_nope bf16 [B,H,512], q_pe bf16 [B,H,64], ckv_cache bf16 [pages,page_size,512],
  *          kpe_cache bf16 [pages,page_size,64], kv_indptr int32 [B+1], kv_indices int32 [*],
  *          kv_last_page_len int32 [B], sm_scale fp32 [1], output bf16 [B,H,512], lse fp32 [B,H], workspace.
- *          Any H (128 heads per CTA, the last block padded); batch <= 65535.  A launch is three kernels (tile
- *          prefix, decode, merge of the partial results); the work is cut on the device from the sequence
- *          lengths, so max_kv_len does not enter the workspace size.
+ *          Any H (128 heads per pair of CTAs, the last block padded); batch <= 65535.  A launch is three kernels
+ *          (work list, decode, merge of the sequences that were cut); the work is cut on the device from the
+ *          sequence lengths, so max_kv_len does not enter the workspace size.
  * ---------------------------------------------------------------------------------------- */
 typedef struct {
   int64_t batch;
@@ -315,7 +315,8 @@ int cake_b200_mla_decode_destroy(void* handle);
  *          qo_indptr int32 [S+1], kv_indptr int32 [S+1], kv_indices int32 [*] (null when ragged),
  *          kv_last_page_len int32 [S] (null: every page full; null when ragged), sm_scale fp32 [1],
  *          output bf16 [total_q,Hq,D], lse fp32 [total_q,Hq], workspace.  D == 128; Hq/Hkv in 1..8; total_q <= 65535.
- * Every query token is run as a decode sequence of its own over a prefix of its segment's rows.
+ * Tiles of query rows share tiles of KV rows on the tensor core; a few query rows behind a long prefix are run as decode
+ * sequences instead, each over its own prefix (the choice is made from the config, max_kv_len included).
  * ---------------------------------------------------------------------------------------- */
 typedef struct {
   int64_t total_q;
@@ -360,8 +361,8 @@ int cake_b200_mla_prefill_destroy(void* handle);
  * buffers: q_nope bf16 [T,H,512], q_pe bf16 [T,H,64], ckv_cache bf16 [pages,page_size,512],
  *          kpe_cache bf16 [pages,page_size,64], sparse_indices int32 [T,top_k], output bf16 [T,H,512], workspace.
  * sm_scale is a number of the contract (0.1352337788608801), not a tensor, so it is part of the config.
- * The kernel is the paged MLA decode kernel with the page walk replaced by the index list (16 heads of the
- * contract occupy 16 of its 128 head rows).
+ * The kernel is the paged MLA decode kernel with the page walk replaced by the index list (the contract's 16 heads
+ * occupy 16 of its 128 rows).
  * ---------------------------------------------------------------------------------------- */
 typedef struct {
   int64_t num_tokens;      /* query rows */

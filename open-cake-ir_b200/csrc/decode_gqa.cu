@@ -1,4 +1,4 @@
-// Paged GQA decode for sm_100a: split-KV flash-decode + reduce.
+// Paged GQA decode for sm_100a: split-KV flash-decode and merge.
 //
 // Operator: src/open_cake_ir/tasks/solx_fib/attention.py:132-183 (decode branch), tensor ABI
 // attention_specs.py:44-84.  One query token per sequence; out = bf16(softmax(K q * scale) V),
@@ -18,8 +18,9 @@
 // MMA for S = Q K^T (ldmatrix on the K tile; rows beyond G are zero) and the columns of
 // O^T += V^T P^T (ldmatrix.trans on the V tile; P as two bf16 terms, so the weights keep ~16
 // significant bits); the online softmax runs in base 2 with warp shuffles.  The pair merges through
-// shared memory and writes one partial result per piece; the pair that finishes the last piece of
-// a (sequence, KV head) merges the pieces and writes the output, so there is no reduce launch.
+// shared memory; a sequence that no range boundary cuts is written straight to the output, a piece of
+// one that is cut leaves a partial result.  The pair that finishes the last piece of a (sequence, KV
+// head) merges the pieces, or, where few sequences have many pieces, gqa_merge_kernel does.
 #include "common.cuh"
 #include "prefill.cuh"
 #include "prefill_gqa.cuh"

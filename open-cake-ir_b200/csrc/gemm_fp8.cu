@@ -80,7 +80,7 @@ extern "C" int cake_b200_block_scaled_gemm_create(void** buffers, const cake_b20
     if (rc) { delete h; return rc; }
   }
   h->grid = h->split ? int(narrow) * h->split : int(items < sms ? items : sms);
-  // At most 16 rows go through the weight-streaming kernel (4096 x 7168: 8.9 us at 1 row, 10.5 at 16; 14.4 for a split tile
+  // At most 16 rows go through the weight-streaming kernel (4096 x 7168: 8.9 us at 1 row, 10.5 at 16; 12.1 for a split tile
   // of the core).  Beyond, its second tile of 16 rows reads the weights again.
   h->skinny_tiles = m > 16 ? 0 : m <= 8 ? 1 : 2;
   h->skinny_split = skinny::choose_split(1.0, int(n), p.k_blocks, sms);

@@ -2,8 +2,9 @@
 // GEMM1 + SwiGLU (+ e4m3 requantisation), grouped GEMM2 * route weight, weighted combine.
 //
 // Operator and layouts: src/open_cake_ir/tasks/solx_fib/moe.py:13-20 (tensor ABI), :122-155
-// (oracle), :275-287 (routing).  The grouped GEMMs run on the tcgen05 core in gemm_fp8.cuh; the
-// small integer kernels here are warp-level (top-k by 64-bit ordered keys, ballot prefix scans).
+// (oracle), :275-287 (routing).  The grouped GEMMs run on the tcgen05 core in gemm_fp8.cuh, or, at a few
+// rows per expert, on the weight-streaming kernel in gemm_skinny.cuh, which takes token rows where they
+// lie; the small integer kernels here are warp-level (top-k by ordered keys, ballot prefix scans).
 #include "gemm_skinny.cuh"
 #include "../../include/cake_b200.h"
 #include <new>

@@ -1,4 +1,4 @@
-// Causal prefill over a paged or ragged KV store, expressed as decode over one sequence per query token.
+// Causal GQA prefill over a paged or ragged KV store, expressed as decode over one sequence per query token.
 //
 // Operator (src/open_cake_ir/tasks/solx_fib/attention.py:132-183, the branches with `not spec['decode']`; specs
 // attention_specs.py:85-248 and :293-338): segment b holds query rows [qo_indptr[b], qo_indptr[b+1]) and KV rows
@@ -9,10 +9,10 @@
 // ragged and MLA tasks, attention.py:47) and zeros otherwise; its lse is -inf either way (:171-173).
 //
 // `prefill_plan_kernel` writes, per query token, where its KV list starts and how many rows it sees; the decode
-// kernels then treat every token as a sequence of its own (their explicit sequence table), and
+// kernel then treats every token as a sequence of its own (its explicit sequence table), and
 // `prefill_mark_kernel` writes the NaN rows.  Every query token therefore streams its own prefix of the
-// segment's KV rows: correct for any shape, and sized for the short suffix prefills of a serving step, not for
-// long prompts, where a kernel that shares KV tiles between query rows is the right tool.
+// segment's KV rows, over the whole GPU: the better form for a few query rows behind a long prefix only.
+// Everything else runs on the query tiles of prefill_gqa.cuh.
 #pragma once
 #include "common.cuh"
 

@@ -210,8 +210,8 @@ class NativeExpertParallelMoe:
         if code:
             raise _lib.CakeError("cake_b200_ep_exchange_create", code)
         self._lib = _lib
-        # kernels of this library launched per step: routing 1, exchange 4, rank-local layer 7
-        self.launches_per_step = 12
+        # kernels of this library launched per step: routing 1, exchange 4, rank-local layer 5
+        self.launches_per_step = 10
 
     def _stage(self, stage: int):
         code = self._lib.library().cake_b200_ep_exchange_launch_stage(self._handle, stage, torch.cuda.current_stream().cuda_stream)
@@ -381,8 +381,8 @@ class PushExpertParallelMoe:
         self._lib = _lib
         if self.world > 1 and virtual is None:
             dist.barrier(group)            # every rank's buffers are zeroed and mapped before anyone pushes
-        # kernels of this library launched per step: routing 1, exchange 6, rank-local layer stages 0..2: 6
-        self.launches_per_step = 13
+        # kernels of this library launched per step: routing 1, exchange 6, rank-local layer stages 0..2: 4
+        self.launches_per_step = 11
         self.slot_of = None
 
     def _stage(self, stage: int):
