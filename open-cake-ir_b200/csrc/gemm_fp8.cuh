@@ -238,25 +238,29 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       tma_prefetch_descriptor(&map_b);
       const uint64_t keep = l2_policy_evict_last();    // activations: re-read by every n tile
       // Work items.  With a queue, this thread draws them (the first is the CTA's index, every later
-      // one comes from the device counter, asked for one item ahead) and hands each to the MMA and
-      // epilogue warps through a small ring, so that an SM that runs slower simply takes fewer
-      // items; without one, item i belongs to CTA i mod grid.
+      // one comes from the device counter, asked for one item ahead) and hands each to the other
+      // roles through a small ring, so that an SM that runs slower simply takes fewer
+      // items; without one, item i belongs to CTA i mod grid.  The next item is found and handed on
+      // half-way through the K blocks of the one before, while this thread is ahead of the ring anyway
+      // (found between two items it delays the next one's first loads; second GEMM of 2500 tokens, two terms, hidden 2048, 128
+      // experts of 768: 137 us then, 128 now).
       uint32_t it = 0, k = 0;
-      bool ok = true;
+      bool ok = true, valid;
       Item item;
       int g = first_item;
-      while (ok) {
-        const bool valid = locate(sh, p, n_tiles, g, &item);
-        int drawn = g + int(gridDim.x);
-        if (handed) {
-          const int slot = k % kItemSlots;
-          ok = mbar_wait(&sh->item_empty[slot], ((k / kItemSlots) & 1) ^ 1, abort_flag, p.status, kStatusWaitFlag);
-          if (!ok) break;
-          sh->item[slot] = valid ? make_int4(item.group, item.row0, item.rows_valid, item.n_tile) : make_int4(-1, 0, 0, 0);
-          mbar_arrive(&sh->item_full[slot]);
-          if (p.queue && valid) drawn = int(gridDim.x) + atomicAdd(p.queue, 1);
-        }
-        if (!valid) break;
+      auto find = [&](int index, uint32_t nth) {         // item `index`, the nth of this CTA
+        valid = locate(sh, p, n_tiles, index, &item);
+        if (!handed) return;
+        const int slot = nth % kItemSlots;
+        ok = mbar_wait(&sh->item_empty[slot], ((nth / kItemSlots) & 1) ^ 1, abort_flag, p.status, kStatusWaitFlag);
+        if (!ok) return;
+        sh->item[slot] = valid ? make_int4(item.group, item.row0, item.rows_valid, item.n_tile) : make_int4(-1, 0, 0, 0);
+        mbar_arrive(&sh->item_full[slot]);
+      };
+      find(g, 0);
+      const int find_at = (k_count - 1) / 2;
+      while (ok && valid) {
+        g = p.queue ? int(gridDim.x) + atomicAdd(p.queue, 1) : g + int(gridDim.x);
         const int b_row0 = item.group * p.b_rows_per_group;
         // A tile of at most kTailRows valid rows (the second tile of a group a little over 128 rows) brings in those
         // rows only, through a map with a smaller box: such a tile streams its weights from L2 at what one SM can
@@ -264,9 +268,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // there; their products land in accumulator rows that no one reads.
         const bool tail = item.rows_valid <= kTailRows;
         const uint32_t stage_tx = uint32_t((tail ? kTailRows * kBK : kBytesA) + kCols * kBK);
+        const int a_row0 = item.row0, n_tile = item.n_tile;
         for (int kb = 0; kb < k_count; ++kb, ++it) {
           const int s = it % kStages;
           ok = mbar_wait(&sh->empty[s], ((it / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
+          if (!ok) break;
+          if (kb == find_at) find(g, k + 1);                            // (this item is in the variables above)
           if (!ok) break;
           if (p.skip_load && blockIdx.x == 0 && it == 1) continue;      // test hook: this ring slot is never filled
           uint8_t* a_dst = tiles + s * kStageBytes;
@@ -274,16 +281,15 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           int a_col = k_begin + kb, b_col = k_begin + kb;
           if (p.interleave_hi_lo) { a_col = (kb & 1) * (p.k_blocks >> 1) + (kb >> 1); b_col = kb >> 1; }
           mbar_arrive_expect_tx(&sh->full[s], stage_tx);
-          tma_load_2d_hint(a_dst, tail ? &map_a_tail : &map_a, a_col * kBK, item.row0, &sh->full[s], keep);
+          tma_load_2d_hint(a_dst, tail ? &map_a_tail : &map_a, a_col * kBK, a_row0, &sh->full[s], keep);
           if (MODE == kGateUp) {
             // gate/up: 128 rows of the first half (x1) and the matching 128 rows of the second half (x2)
-            tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + item.n_tile * 128, &sh->full[s]);
-            tma_load_2d(b_dst + 128 * kBK, &map_b, b_col * kBK, b_row0 + p.n + item.n_tile * 128, &sh->full[s]);
+            tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + n_tile * 128, &sh->full[s]);
+            tma_load_2d(b_dst + 128 * kBK, &map_b, b_col * kBK, b_row0 + p.n + n_tile * 128, &sh->full[s]);
           } else {
-            tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + item.n_tile * kCols, &sh->full[s]);
+            tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + n_tile * kCols, &sh->full[s]);
           }
         }
-        g = drawn;
         ++k;
       }
       if (p.drawn_out && atomicAdd(p.drawn_out, 1) == int(gridDim.x) - 1) { *p.queue = 0; *p.drawn_out = 0; }
