@@ -315,8 +315,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         for (int kb = 0; kb < k_count; ++kb, ++it) {
           const int s = it % kStages;
           const int t = it % kTmemStages;
-          ok = mbar_wait(&sh->full[s], (it / kStages) & 1, abort_flag, p.status, kStatusWaitSmemFull) &&
-               mbar_wait(&sh->tmem_empty[t], ((it / kTmemStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitTmemEmpty);
+          ok = mbar_wait_both(&sh->full[s], (it / kStages) & 1, kStatusWaitSmemFull, &sh->tmem_empty[t],
+                              ((it / kTmemStages) & 1) ^ 1, kStatusWaitTmemEmpty, abort_flag, p.status);
           if (!ok) break;
           tcgen05_fence_after();
           const uint32_t a_addr = smem_u32(tiles + s * kStageBytes);
