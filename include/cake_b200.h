@@ -25,6 +25,9 @@
  * cake_b200_read_status after synchronising the stream).  The first 256 bytes of a workspace
  * are the library's (the status word, then the counters its kernels draw work items from);
  * `launch` clears what it uses on the stream, so a workspace needs no initialisation.
+ * Output alignment: the attention operators write `output` eight bytes at a time or wider, as its address
+ * allows, so it must lie on an 8-byte boundary (create refuses it otherwise); every other bf16 or e4m3 buffer
+ * on a 16-byte one.
  * Workspace alignment: 4 bytes for the decode operators and the dense GEMM (16 there), which
  * align what follows the status block themselves inside the size they ask for; 256 bytes for
  * the MoE layer, whose workspace holds TMA-addressed tiles (create returns

@@ -181,7 +181,7 @@ gqa_plan_kernel(const Params p) {
       if (len == 0) {
         for (int h = 0; h < p.hq; ++h) {
           p.lse[size_t(b) * p.hq + h] = -INFINITY;
-          for (int d = 0; d < kD; d += 8) *reinterpret_cast<uint4*>(p.out + (size_t(b) * p.hq + h) * kD + d) = make_uint4(0u, 0u, 0u, 0u);
+          for (int d = 0; d < kD; d += 4) *reinterpret_cast<uint2*>(p.out + (size_t(b) * p.hq + h) * kD + d) = make_uint2(0u, 0u);
         }
       }
     }
@@ -655,6 +655,7 @@ inline int fill_params(Params& p, void** buffers, const cake_b200_gqa_decode_con
     if (!buffers[i]) return kErrBadArgument;
     if (i <= 2 && (reinterpret_cast<uintptr_t>(buffers[i]) & 15)) return kErrBadArgument;
   }
+  if (c.batch > 0 && (reinterpret_cast<uintptr_t>(buffers[7]) & 7)) return kErrBadArgument;      // rows leave eight bytes at a time
   p.q = static_cast<const __nv_bfloat16*>(buffers[0]);
   p.k_cache = static_cast<const __nv_bfloat16*>(buffers[1]);
   p.v_cache = static_cast<const __nv_bfloat16*>(buffers[2]);

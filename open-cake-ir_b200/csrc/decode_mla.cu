@@ -87,6 +87,7 @@ struct Params {
   int* segment_prefix;
   const int* qo_indptr;
   int segments, total_q, nan_for_masked;
+  int out_align;          // the widest store that the address of `out` allows: 32, 16 or 8 bytes
   int wait_kiloclocks;    // budget of a bounded wait in units of 1024 clocks (0: the default, about a second)
   int skip_load;          // test hook: a CTA's loader warps leave out the third tile of the first sequence they work on
 };
@@ -299,6 +300,18 @@ __device__ __forceinline__ void store_32(void* dst, const uint32_t (&v)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
+// The same 32 bytes of the caller's output, which may lie on any 8-byte boundary.
+__device__ __forceinline__ void store_32_aligned(void* dst, const uint32_t (&v)[8], int align) {
+  if (align == 32) {
+    store_32(dst, v);
+  } else if (align == 16) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) static_cast<uint4*>(dst)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) static_cast<uint2*>(dst)[i] = make_uint2(v[2 * i], v[2 * i + 1]);
+  }
+}
 
 template <bool SPARSE>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -324,8 +337,8 @@ mla_decode_kernel(const Params p) {
         const int4 s = p.seq ? p.seq[b] : make_int4(b, 1, 0, 0);
         const uint32_t word = p.nan_for_masked && s.w > 0 ? 0x7fc07fc0u : 0u;
         const size_t row0 = size_t(s.x) * p.heads;
-        for (int i = lane; i < s.y * p.heads * (kCkv / 8); i += 32)
-          reinterpret_cast<uint4*>(p.out + row0 * kCkv)[i] = make_uint4(word, word, word, word);
+        for (int i = lane; i < s.y * p.heads * (kCkv / 4); i += 32)
+          reinterpret_cast<uint2*>(p.out + row0 * kCkv)[i] = make_uint2(word, word);
         if (p.lse) for (int i = lane; i < s.y * p.heads; i += 32) p.lse[row0 + i] = -INFINITY;
       }
     }
@@ -663,7 +676,7 @@ mla_decode_kernel(const Params p) {
             uint32_t v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = pack_bf16x2(o[h + 2 * i] * by, o[h + 2 * i + 1] * by);
-            store_32(p.out + out_row * kCkv + dim + h, v);
+            store_32_aligned(p.out + out_row * kCkv + dim + h, v, p.out_align);
           }
         } else {
 #pragma unroll
@@ -784,6 +797,9 @@ inline uint8_t* carve(Params& p, void* buffer) {
 
 inline int finish_create(Handle* h) {
   Params& p = h->p;
+  const uintptr_t out = reinterpret_cast<uintptr_t>(p.out);
+  if (p.sequences > 0 && (out & 7)) return kErrBadArgument;
+  p.out_align = (out & 31) == 0 ? 32 : (out & 15) == 0 ? 16 : 8;
   int sms = 0;
   CAKE_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
   p.workers = sms / (2 * head_blocks(p.rows));               // a cluster per pair of SMs

@@ -366,6 +366,7 @@ prefill_kernel(const Params p) {
     const float pre = scale_positive ? 1.f : scale2, post = scale_positive ? scale2 : 1.f;
     const int token = x * per_half + r / p.group, head_in_group = r % p.group;
     const bool slot = r < per_half * p.group;
+    const bool out_aligned = !(reinterpret_cast<uintptr_t>(p.out) & 15);      // the caller's output may lie on any 8-byte boundary
     uint4* scratch = reinterpret_cast<uint4*>(out_rows + (warp - kSoftmaxWarp0) * (32 * 128));
     bool ok = true;
     uint32_t done = 0;                             // KV tiles so far
@@ -488,9 +489,16 @@ prefill_kernel(const Params p) {
         for (int i = 0; i < 8; ++i) {
           const int rr = i * 4 + (lane >> 3), chunk = lane & 7;
           const int row_r = quad * 32 + rr, row_token = x * per_half + row_r / p.group;
-          if (row_r < per_half * p.group && row_token < w.rows)
-            *reinterpret_cast<uint4*>(p.out + (size_t(w.q0 + row_token) * p.hq + w.kvh * p.group + row_r % p.group) * kD + h + chunk * 8) =
-                scratch[rr * 8 + (chunk ^ (rr & 7))];
+          if (row_r < per_half * p.group && row_token < w.rows) {
+            const uint4 v = scratch[rr * 8 + (chunk ^ (rr & 7))];
+            __nv_bfloat16* dst = p.out + (size_t(w.q0 + row_token) * p.hq + w.kvh * p.group + row_r % p.group) * kD + h + chunk * 8;
+            if (out_aligned) {
+              *reinterpret_cast<uint4*>(dst) = v;
+            } else {
+              reinterpret_cast<uint2*>(dst)[0] = make_uint2(v.x, v.y);
+              reinterpret_cast<uint2*>(dst)[1] = make_uint2(v.z, v.w);
+            }
+          }
         }
         __syncwarp();
       }
