@@ -27,7 +27,8 @@
  * `launch` clears what it uses on the stream, so a workspace needs no initialisation.
  * Output alignment: the attention operators write `output` eight bytes at a time or wider, as its address
  * allows, so it must lie on an 8-byte boundary (create refuses it otherwise); every other bf16 or e4m3 buffer
- * on a 16-byte one.
+ * on a 16-byte one (the MoE layer's output: looked at when it is written, by launch or stage 3, since a caller that
+ * combines the rows itself runs stages 0..2 only).
  * Workspace alignment: 4 bytes for the decode operators and the dense GEMM (16 there), which
  * align what follows the status block themselves inside the size they ask for; 256 bytes for
  * the MoE layer, whose workspace holds TMA-addressed tiles (create returns

@@ -718,6 +718,7 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
     }
     case 3:
     {
+      if (reinterpret_cast<uintptr_t>(h->output) & 15) return kErrBadArgument;      // rows leave 16 bytes at a time
       const int parts = (c.hidden + 2047) / 2048;
       return launch_dependent(moe::combine_kernel, dim3(unsigned(tokens) * parts), dim3(256), 0, s, reinterpret_cast<const __nv_bfloat16*>(h->ws + l.y),
                               pa.inv_perm, h->output, c.hidden, c.top_k, parts);

@@ -73,3 +73,14 @@ def test_views_into_a_larger_buffer(name, make):
     for offset in (2, 4):
         with pytest.raises(cake._lib.CakeError):
             make(dev, at(offset)[1], lse)
+
+
+def test_moe_output_has_to_be_aligned():
+    """The rows that combine the experts' contributions are written 16 bytes at a time."""
+    dev = {k: v.cuda() for k, v in cake.workloads.moe_inputs(3, 512, 128, 16, 16, routing="softmax", device="cpu").items()}
+    raw = torch.zeros(3 * 512 + 8, dtype=torch.bfloat16, device="cuda")
+    op = cake.Fp8Moe(dev, raw[4:4 + 3 * 512].reshape(3, 512), experts=16, routing="softmax")
+    with pytest.raises(cake._lib.CakeError):
+        op.launch()
+    torch.cuda.synchronize()
+    assert not bool(raw.any())
