@@ -649,9 +649,10 @@ mla_decode_kernel(const Params p) {
       if (!ok) break;
       tcgen05_fence_after();
       const bool exists = row < w.rows;
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      const float lse = l > 0.f ? m + log2f(l) : -INFINITY;
-      const bool nan = p.nan_for_masked && !(l > 0.f);       // only a row that sees nothing has no weight (its segment has KV rows)
+      const bool none = l == 0.f;                  // the row sees nothing; a sum that is NaN goes on as one
+      const float inv = none ? 0.f : 1.f / l;
+      const float lse = none ? -INFINITY : m + log2f(l);
+      const bool nan = p.nan_for_masked && none;             // (its segment has KV rows)
       const size_t slot_row = size_t(slot_of(worker, w.seq_begin, per_worker)) * p.rows + row, out_row = size_t(w.first_row) + row;
 #pragma unroll 1
       for (int c = 0; c < 256; c += 32) {
@@ -664,13 +665,13 @@ mla_decode_kernel(const Params p) {
           if (lane == 0) arrive_at(&sh->o_empty, 0);
         }
         const int dim = (c >> 7) * 256 + half * 128 + (c & 127);
-        if (!(l > 0.f)) {
+        if (none) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] = w.whole && nan ? __int_as_float(0x7fc00000) : 0.f;
         }
         if (!exists) continue;
         if (w.whole) {
-          const float by = l > 0.f ? inv : 1.f;
+          const float by = none ? 1.f : inv;
 #pragma unroll
           for (int h = 0; h < 32; h += 16) {
             uint32_t v[8];
@@ -729,9 +730,11 @@ mla_reduce_kernel(const Params p) {
         v[i] = __ldcg(reinterpret_cast<const float4*>(p.part_o + at * kCkv + d));
       }
     float m_new = mm;
+    bool seen = mm != -INFINITY;                   // a piece of NaN counts: the maximum leaves it out, its weight is NaN
 #pragma unroll
-    for (int i = 0; i < 4; ++i) if (k0 + i <= last) m_new = fmaxf(m_new, ls[i]);
-    if (m_new == -INFINITY) continue;              // nothing seen so far
+    for (int i = 0; i < 4; ++i)
+      if (k0 + i <= last) { m_new = fmaxf(m_new, ls[i]); seen |= ls[i] != -INFINITY; }
+    if (!seen) continue;
     const float rescale = exp2f(mm - m_new);       // 0 the first time
     mm = m_new;
     weight *= rescale;
@@ -746,14 +749,14 @@ mla_reduce_kernel(const Params p) {
   }
   const size_t out_row = size_t(s.x) * p.heads + row;
   uint2 packed = make_uint2(0u, 0u);
-  if (weight > 0.f) {
+  if (weight != 0.f) {
     const float inv = 1.f / weight;
     packed = make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
   } else if (p.nan_for_masked) {
     packed = make_uint2(0x7fc07fc0u, 0x7fc07fc0u);
   }
   *reinterpret_cast<uint2*>(p.out + out_row * kCkv + d) = packed;
-  if (d == 0 && p.lse) p.lse[out_row] = weight > 0.f ? mm + log2f(weight) : -INFINITY;
+  if (d == 0 && p.lse) p.lse[out_row] = weight != 0.f ? mm + log2f(weight) : -INFINITY;
 }
 
 struct Handle {

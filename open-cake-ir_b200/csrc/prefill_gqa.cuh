@@ -463,8 +463,11 @@ prefill_kernel(const Params p) {
       if (ok && tiles > 0) ok = mbar_wait(&sh->o_done[x], (done - 1) & 1, abort_flag, p.status, kStatusWaitFlag);
       if (!ok) break;
       tcgen05_fence_after();
+      // A sum that is NaN (a NaN, or infinities that met, in what the row sees) goes on as one.  A row that sees KV rows has a
+      // weight of at least 2^-8, unless every logit is -inf: 0 / 0, as in the decode form.  Else a zero sum means that it sees nothing.
+      if (visible > 0 && l == 0.f) l = __int_as_float(0x7fc00000);
       // rows leave through shared memory, 128 bytes of a row at a time
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const float inv = l == 0.f ? 0.f : 1.f / l;
       const bool nan = p.nan_for_masked && w.kv_len > 0 && visible <= 0;
 #pragma unroll 1
       for (int h = 0; h < kD; h += 64) {
@@ -480,7 +483,7 @@ prefill_kernel(const Params p) {
             uint4 v;
             v.x = pack_bf16x2(o[8 * i] * inv, o[8 * i + 1] * inv); v.y = pack_bf16x2(o[8 * i + 2] * inv, o[8 * i + 3] * inv);
             v.z = pack_bf16x2(o[8 * i + 4] * inv, o[8 * i + 5] * inv); v.w = pack_bf16x2(o[8 * i + 6] * inv, o[8 * i + 7] * inv);
-            if (!(l > 0.f)) v = nan ? make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u) : make_uint4(0u, 0u, 0u, 0u);
+            if (l == 0.f) v = nan ? make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u) : make_uint4(0u, 0u, 0u, 0u);
             scratch[lane * 8 + ((c / 8 + i) ^ (lane & 7))] = v;
           }
         }
@@ -502,7 +505,7 @@ prefill_kernel(const Params p) {
         }
         __syncwarp();
       }
-      if (exists) p.lse[size_t(w.q0 + token) * p.hq + w.kvh * p.group + head_in_group] = l > 0.f ? m_ref + log2f(l) : -INFINITY;
+      if (exists) p.lse[size_t(w.q0 + token) * p.hq + w.kvh * p.group + head_in_group] = l == 0.f ? -INFINITY : m_ref + log2f(l);
     }
   }
 

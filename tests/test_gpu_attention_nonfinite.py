@@ -1,0 +1,64 @@
+"""NaN and infinities in attention inputs: a result that depends on one is NaN, whatever form the operator takes and
+wherever the work list cuts a sequence, and no other result changes."""
+import pytest
+import torch
+
+import open_cake_ir_b200 as cake
+from test_gpu_decode import run_mla
+from test_gpu_mla_tiles import paged
+from test_gpu_prefill import run
+from test_gpu_prefill_tiles import problem
+
+pytestmark = pytest.mark.gpu
+NAN, INF = float("nan"), float("inf")
+
+
+def expect(out, lse, clean, hit_out, hit_lse):
+    """``hit``: [rows, heads] the results that are NaN; the others have the bits of the clean inputs' results."""
+    out, lse, hit_out, hit_lse = out.float().cpu(), lse.cpu(), hit_out.bool(), hit_lse.bool()
+    assert torch.equal(torch.isnan(out).any(2), hit_out) and torch.equal(torch.isnan(lse), hit_lse)
+    assert torch.equal(out[~hit_out], clean[0].float().cpu()[~hit_out]) and torch.equal(lse[~hit_lse], clean[1].cpu()[~hit_lse])
+
+
+@pytest.mark.parametrize("tensor", ["q", "k"])
+@pytest.mark.parametrize("q_lens,kv_lens,kv_heads", [([70, 5], [200, 5], 2), ([2, 1], [6000, 40], 1)])      # tiles; a sequence per row
+def test_gqa_prefill(tensor, q_lens, kv_lens, kv_heads):
+    cpu = problem(3, q_lens, kv_lens, 8, kv_heads, 0)
+    args = dict(mla=False, paged=False, nan=True, max_kv_len=max(kv_lens))
+    clean = run(cpu, **args)
+    hit = torch.zeros(sum(q_lens), 8)
+    if tensor == "q":
+        cpu["q"][1, 3, 7] = NAN
+        hit[1, 3] = 1
+    else:                                       # the first row of the second segment, KV head 0: all of its query rows see it
+        cpu["k"][kv_lens[0], 0, 7] = NAN
+        hit[q_lens[0]:, :8 // kv_heads] = 1
+    expect(*run(cpu, **args), clean, hit, hit)
+
+
+def test_gqa_prefill_row_of_infinite_logits():
+    """Every logit of a row -inf: 0 / 0."""
+    cpu = problem(4, [3], [3], 4, 1, 0)
+    args = dict(mla=False, paged=False, nan=True, max_kv_len=3)
+    clean = run(cpu, **args)
+    cpu["q"][0, 2] = 0
+    cpu["q"][0, 2, 0], cpu["k"][0, 0, 0] = -INF, 1.0        # only query row 0 sees nothing else
+    clean = run(dict(cpu, q=torch.where(torch.isinf(cpu["q"]), 0.0, cpu["q"])), **args)
+    hit = torch.zeros(3, 4)
+    hit[0, 2] = 1
+    expect(*run(cpu, **args), clean, hit, hit)
+
+
+@pytest.mark.parametrize("lens", [[20, 20, 20], [3000, 3000, 3000]])                       # whole; cut into many pieces
+@pytest.mark.parametrize("tensor", ["q_nope", "q_pe", "ckv_cache", "kpe_cache"])
+def test_mla_decode(lens, tensor):
+    cpu = paged(torch.Generator().manual_seed(5), lens, 1, 16, 3)
+    clean = run_mla(cpu, max(lens))
+    hit = torch.zeros(3, 16)
+    if tensor.startswith("q"):
+        cpu[tensor][1, 4, 7] = NAN
+        hit[1, 4] = 1
+    else:                                       # one of the second sequence's rows
+        cpu[tensor][cpu["kv_indices"][lens[0] + 7].long(), 0, 7] = NAN
+        hit[1] = 1
+    expect(*run_mla(cpu, max(lens)), clean, hit, hit)
