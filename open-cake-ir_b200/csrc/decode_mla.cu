@@ -313,9 +313,62 @@ __device__ __forceinline__ void store_32_aligned(void* dst, const uint32_t (&v)[
   }
 }
 
+// The tensor core multiplies every row of a tile with a weight, the masked ones with 0, and 0 times an infinity or a NaN is NaN.
+// For a row whose O is not finite this looks at the rows of its piece that it does not see, tokens [visible, end), and where
+// one of them is not finite, writes the row again from tokens [begin, visible), with the same maximum: to `whole` (the output
+// row), else `part`.  By a whole warp: lane i has dims [4 i, 4 i + 4) of either 128 of this half's dims.  (Sequences of several
+// query tokens only.)  Rare, and out of line for the registers of the loops.
+static __device__ __noinline__ void without_masked_tokens(const Params& p, size_t q_row, int page_base, int begin, int visible, int end, int half,
+                                                          float scale2, float m, float by, __nv_bfloat16* whole, float* part) {
+  const int lane = threadIdx.x & 31;
+  auto row4 = [&](const __nv_bfloat16* at) {
+    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(at));
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  };
+  auto token = [&](int t) { return size_t(__ldg(p.kv_indices + page_base + t / p.page_size)) * p.page_size + t % p.page_size; };
+  float spread = 0.f;                              // NaN once an element is not finite
+  for (int t = visible; t < end; ++t) {
+    const size_t at = token(t);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float4 v = row4(p.ckv + at * kCkv + c * 256 + half * 128 + lane * 4);
+      spread = fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, fmaf(v.w, 0.f, spread))));
+    }
+  }
+  if (!__any_sync(0xffffffffu, spread != spread)) return;
+  float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int t = begin; t < visible; ++t) {
+    const size_t at = token(t);
+    float dot = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float4 q = row4(p.q_nope + q_row * kCkv + c * 128 + lane * 4), k = row4(p.ckv + at * kCkv + c * 128 + lane * 4);
+      dot += q.x * k.x + q.y * k.y + q.z * k.z + q.w * k.w;
+    }
+    if (lane < kKpe / 4) {
+      const float4 q = row4(p.q_pe + q_row * kKpe + lane * 4), k = row4(p.kpe + at * kKpe + lane * 4);
+      dot += q.x * k.x + q.y * k.y + q.z * k.z + q.w * k.w;
+    }
+    const float w = ex2_approx(fmaf(warp_sum(dot), scale2, -m));
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float4 v = row4(p.ckv + at * kCkv + c * 256 + half * 128 + lane * 4);
+      o[4 * c] = fmaf(w, v.x, o[4 * c]); o[4 * c + 1] = fmaf(w, v.y, o[4 * c + 1]);
+      o[4 * c + 2] = fmaf(w, v.z, o[4 * c + 2]); o[4 * c + 3] = fmaf(w, v.w, o[4 * c + 3]);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int dim = c * 256 + half * 128 + lane * 4;
+    if (whole) *reinterpret_cast<uint2*>(whole + dim) = make_uint2(pack_bf16x2(o[4 * c] * by, o[4 * c + 1] * by), pack_bf16x2(o[4 * c + 2] * by, o[4 * c + 3] * by));
+    else *reinterpret_cast<float4*>(part + dim) = make_float4(o[4 * c] * by, o[4 * c + 1] * by, o[4 * c + 2] * by, o[4 * c + 3] * by);
+  }
+}
+
 template <bool SPARSE>
 __global__ void __launch_bounds__(kThreads, 1)
-mla_decode_kernel(const Params p) {
+mla_decode_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   // launched as a programmatic dependent of the plan kernel: resident early, reads the plan after that grid has completed
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -653,6 +706,10 @@ mla_decode_kernel(const Params p) {
       const float inv = none ? 0.f : 1.f / l;
       const float lse = none ? -INFINITY : m + log2f(l);
       const bool nan = p.nan_for_masked && none;             // (its segment has KV rows)
+      // tokens of the piece that the row sees, and whether the piece has others
+      const int visible = p.pack > 1 ? min(w.end, min(w.kv_len, w.first_visible + min(row, w.rows - 1) / p.heads)) : w.end;
+      const bool some_masked = !SPARSE && exists && !none && visible < w.end;
+      float spread = 0.f;                          // NaN once an element of O is not finite
       const size_t slot_row = size_t(slot_of(worker, w.seq_begin, per_worker)) * p.rows + row, out_row = size_t(w.first_row) + row;
 #pragma unroll 1
       for (int c = 0; c < 256; c += 32) {
@@ -665,6 +722,10 @@ mla_decode_kernel(const Params p) {
           if (lane == 0) arrive_at(&sh->o_empty, 0);
         }
         const int dim = (c >> 7) * 256 + half * 128 + (c & 127);
+        if (some_masked) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) spread = fmaf(o[i], 0.f, spread);
+        }
         if (none) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] = w.whole && nan ? __int_as_float(0x7fc00000) : 0.f;
@@ -688,6 +749,16 @@ mla_decode_kernel(const Params p) {
             store_32(p.part_o + slot_row * kCkv + dim + h, v);
           }
         }
+      }
+      uint32_t again = __ballot_sync(0xffffffffu, spread != spread && l == l);
+      while (again) {                              // (the row's first result has been written, by this warp)
+        const int src = __ffs(again) - 1;
+        again &= again - 1;
+        const float scale2 = (p.sm_scale ? __ldg(p.sm_scale) : p.sm_scale_value) * kLog2e;
+        const float by = __shfl_sync(0xffffffffu, inv, src);
+        const size_t q_row = __shfl_sync(0xffffffffu, out_row, src), slot = __shfl_sync(0xffffffffu, slot_row, src);
+        without_masked_tokens(p, q_row, w.page_base, w.begin, __shfl_sync(0xffffffffu, visible, src), w.end, half, scale2,
+                              __shfl_sync(0xffffffffu, m, src), by, w.whole ? p.out + q_row * kCkv : nullptr, p.part_o + slot * kCkv);
       }
       if (exists && half == 0) {
         if (!w.whole) p.part_lse[slot_row] = lse;

@@ -180,8 +180,40 @@ __device__ __forceinline__ bool get_work(const Params& p, int units, int k, Work
   return true;
 }
 
+// The tensor core multiplies every V row of a tile with a weight, the masked ones with 0, and 0 times an infinity or a NaN is
+// NaN.  For a row whose O is not finite this looks at the V rows that its tiles hold and it does not see, [visible, loaded),
+// and where one of them is not finite, writes the row again from the KV rows that it does see, with the same maximum.  By a whole
+// warp: lane i has dims [4 i, 4 i + 4).  Rare, and out of line for the registers of the loop.
+static __device__ __noinline__ void without_masked_rows(const Params& p, int q_row, int head, int kvh, int page_base, int visible, int loaded,
+                                                        float scale2, float m, float by) {
+  const int lane = threadIdx.x & 31;
+  auto row4 = [&](const __nv_bfloat16* rows, size_t row) {
+    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(rows + row * kD) + lane);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  };
+  auto kv_row = [&](int t) {
+    return size_t(p.kv_indices ? __ldg(p.kv_indices + page_base + t / p.page_size) * p.page_size + t % p.page_size : page_base + t) * p.hkv + kvh;
+  };
+  float spread = 0.f;                              // NaN once an element is not finite
+  for (int t = visible; t < loaded; ++t) {
+    const float4 v = row4(p.v, kv_row(t));
+    spread = fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, fmaf(v.w, 0.f, spread))));
+  }
+  if (!__any_sync(0xffffffffu, spread != spread)) return;
+  const float4 q = row4(p.q, size_t(q_row) * p.hq + head);
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int t = 0; t < visible; ++t) {
+    const size_t at = kv_row(t);
+    const float4 k = row4(p.k, at), v = row4(p.v, at);
+    const float w = ex2(fmaf(warp_sum(q.x * k.x + q.y * k.y + q.z * k.z + q.w * k.w), scale2, -m));
+    o.x = fmaf(w, v.x, o.x); o.y = fmaf(w, v.y, o.y); o.z = fmaf(w, v.z, o.z); o.w = fmaf(w, v.w, o.w);
+  }
+  reinterpret_cast<uint2*>(p.out + (size_t(q_row) * p.hq + head) * kD)[lane] = make_uint2(pack_bf16x2(o.x * by, o.y * by), pack_bf16x2(o.z * by, o.w * by));
+}
+
 static __global__ void __launch_bounds__(kThreads, 1)
-prefill_kernel(const Params p) {
+prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t q_addr = smem_u32(base), k_addr = q_addr + 2 * kTileBytes, v_addr = k_addr + kStages * kTileBytes;
@@ -469,6 +501,9 @@ prefill_kernel(const Params p) {
       // rows leave through shared memory, 128 bytes of a row at a time
       const float inv = l == 0.f ? 0.f : 1.f / l;
       const bool nan = p.nan_for_masked && w.kv_len > 0 && visible <= 0;
+      const int loaded = min(w.kv_len, tiles * kTile);       // KV rows in the row's products
+      const bool some_masked = visible > 0 && visible < loaded;
+      float spread = 0.f;                          // NaN once an element of O is not finite
 #pragma unroll 1
       for (int h = 0; h < kD; h += 64) {
 #pragma unroll
@@ -477,6 +512,10 @@ prefill_kernel(const Params p) {
           if (tiles > 0) {
             tmem_ld_32x32b_x32(o_col + h + c, o);
             tcgen05_wait_ld();
+          }
+          if (some_masked) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) spread = fmaf(o[i], 0.f, spread);
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -504,6 +543,13 @@ prefill_kernel(const Params p) {
           }
         }
         __syncwarp();
+      }
+      uint32_t again = __ballot_sync(0xffffffffu, spread != spread && l == l);
+      while (again) {                              // (the row's first result has been written, by this warp)
+        const int src = __ffs(again) - 1, row_r = quad * 32 + src, q_row = w.q0 + x * per_half + row_r / p.group, head = w.kvh * p.group + row_r % p.group;
+        again &= again - 1;
+        without_masked_rows(p, q_row, head, w.kvh, w.page_base, __shfl_sync(0xffffffffu, visible, src), loaded, scale2,
+                            __shfl_sync(0xffffffffu, m_ref, src), __shfl_sync(0xffffffffu, inv, src));
       }
       if (exists) p.lse[size_t(w.q0 + token) * p.hq + w.kvh * p.group + head_in_group] = l == 0.f ? -INFINITY : m_ref + log2f(l);
     }

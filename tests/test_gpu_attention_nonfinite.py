@@ -62,3 +62,40 @@ def test_mla_decode(lens, tensor):
         cpu[tensor][cpu["kv_indices"][lens[0] + 7].long(), 0, 7] = NAN
         hit[1] = 1
     expect(*run_mla(cpu, max(lens)), clean, hit, hit)
+
+
+def rows_before(out, lse, clean, first, columns):
+    """Rows before ``first`` see nothing of what is not finite (their sums may come in another order); every row behind it is NaN
+    in ``columns`` [heads, dims]."""
+    tolerance = dict(atol=2.0 ** -16, rtol=2.0 ** -7)
+    torch.testing.assert_close(out[:first].float(), clean[0][:first].float(), **tolerance)
+    assert torch.equal(lse[:first], clean[1][:first])
+    assert not torch.isfinite(out[first:].float())[:, columns].any()
+
+
+@pytest.mark.parametrize("value", [NAN, INF])
+@pytest.mark.parametrize("q_len,kv_len,page,at", [(70, 70, 0, 5), (300, 300, 16, 130), (20, 400, 5, 385)])
+def test_gqa_prefill_value_that_earlier_rows_do_not_see(value, q_len, kv_len, page, at):
+    cpu = problem(6, [q_len], [kv_len], 8, 2, page)
+    args = dict(mla=False, paged=page > 0, nan=True, max_kv_len=kv_len)
+    clean = run(cpu, **args)
+    if page:
+        cpu["v_cache"][cpu["kv_indices"][at // page].long(), at % page, 1, 9] = value
+    else:
+        cpu["v"][at, 1, 9] = value
+    columns = torch.zeros(8, 128, dtype=torch.bool)
+    columns[4:, 9] = True
+    rows_before(*run(cpu, **args), clean, at - (kv_len - q_len), columns)
+
+
+@pytest.mark.parametrize("value", [NAN, INF])
+@pytest.mark.parametrize("q_len,kv_len,heads,at", [(20, 20, 16, 5), (8, 3000, 16, 2996), (9, 9, 48, 5)])      # whole; cut; two tokens to a tile
+def test_mla_prefill_row_that_earlier_tokens_do_not_see(value, q_len, kv_len, heads, at):
+    cpu = paged(torch.Generator().manual_seed(7), [kv_len], 16, heads, q_len)
+    cpu["qo_indptr"] = torch.tensor([0, q_len], dtype=torch.int32)
+    args = dict(mla=True, paged=True, nan=True, max_kv_len=kv_len)
+    clean = run(cpu, **args)
+    cpu["ckv_cache"][cpu["kv_indices"][at // 16].long(), at % 16, 9] = value
+    columns = torch.zeros(heads, 512, dtype=torch.bool)
+    columns[:, 9] = True
+    rows_before(*run(cpu, **args), clean, at - (kv_len - q_len), columns)
