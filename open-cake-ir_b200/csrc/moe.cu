@@ -100,7 +100,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
   // Ordered score bits, 0 = absent or taken; the largest over the warp by one reduction, its lowest expert id by another.
   uint32_t keys[EPL];
 #pragma unroll
-  for (int j = 0; j < EPL; ++j) keys[j] = j * 32 + lane < experts ? ordered_bits(choice[j]) : 0u;
+  for (int j = 0; j < EPL; ++j) keys[j] = j * 32 + lane < experts ? max(ordered_bits(choice[j]), 1u) : 0u;      // (a NaN of all ones would be 0)
   float picked = 0.f;      // lane k keeps the raw value of the k-th selection
   picked_id = 0;
   for (int k = 0; k < top_k; ++k) {

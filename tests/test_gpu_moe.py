@@ -62,6 +62,17 @@ def test_routing_known_answers():
     assert ids.cpu().tolist() == want.tolist()
 
 
+@pytest.mark.parametrize("mode,experts", [("softmax", 64), ("softmax", 300), ("ds", 64)])
+def test_rows_of_all_one_bits_select_distinct_experts(mode, experts):
+    """Padding tokens whose logits are 0xff bytes (a NaN that ranks below everything else): expert ids are distinct and lowest first."""
+    logits = torch.full((40, experts), -1, dtype=torch.int32).view(torch.float32)
+    zeros = torch.zeros(experts, dtype=torch.bfloat16)
+    ids, _ = cake.moe_routing(logits.cuda(), zeros.cuda(), torch.tensor([1.0]).cuda(), mode=mode, n_group=4, topk_group=2)
+    if mode == "softmax":
+        assert ids.cpu().tolist() == [list(range(8))] * 40
+    assert all(len(set(row)) == 8 and 0 <= min(row) and max(row) < experts for row in ids.cpu().tolist())
+
+
 @pytest.mark.parametrize("tokens,experts,offset,local", [(4096, 256, 0, 256), (4096, 256, 96, 32), (1, 256, 224, 32),
                                                           (50, 64, 0, 1), (300, 64, 60, 4)])
 def test_permute_bit_exact(tokens, experts, offset, local):
