@@ -221,15 +221,25 @@ inline TestHooks& test_hooks() {
   return hooks;
 }
 
+// Time of the bounded waits, in units of 1024 clocks: 32 bits of it come round after more than half an hour, so that a look at it is
+// late by no more than that however rarely it comes (32 bits of single clocks come round in two seconds, beside the double of
+// the default budget).
+__device__ __forceinline__ uint32_t kiloclock() { return uint32_t(clock64() >> 10); }
+// Whether a wait that began at `start` has used up its budget (`kiloclocks`, 0 = the default) by `now`.  A producer that waits for a free
+// slot waits for a consumer, which may itself be waiting: twice the budget, so that the consumer reports first.
+constexpr __host__ __device__ bool wait_over(uint32_t start, uint32_t now, int kiloclocks, bool producer) {
+  const uint32_t budget = kiloclocks > 0 ? uint32_t(kiloclocks) : uint32_t(kWaitClockBudget >> 10);
+  return now - start > (producer ? 2 * budget : budget);
+}
+static_assert(wait_over(7, 7 + 0x80000000u, 0, true) && wait_over(0xffffff00u, 0xffffff00u + 4000000u, 0, true) && wait_over(0, 2000000u, 0, false) &&
+              !wait_over(0xffffff00u, 0xffffff00u + 3800000u, 0, true) && !wait_over(0, 1900000u, 0, false) && !wait_over(0, 2047, 2048, false) &&
+              wait_over(0xfffffff0u, 0xfffffff0u + 2049, 2048, false) && !wait_over(0, 4096, 2048, true), "a wait's end would be missed");
+
 // The rare part of a bounded wait, out of line on purpose: inlined, its atomic and its clock arithmetic cost the loops
 // around a wait their register allocation (GEMM core: 1030 clocks per K block against 880, same source otherwise).
 static __device__ __noinline__ bool mbar_wait_expired(uint32_t start, volatile int* abort_flag, int* status, int code) {
   if (*abort_flag) return true;
-  const int kiloclocks = abort_flag[1];
-  uint32_t budget = kiloclocks > 0 ? uint32_t(min(kiloclocks, 1 << 20)) << 10 : uint32_t(kWaitClockBudget);
-  // a producer that waits for a free slot waits for a consumer, which may itself be waiting: let the consumer report first
-  if (code == kStatusWaitSmemEmpty) budget *= 2;
-  if (uint32_t(clock()) - start <= budget) return false;
+  if (!wait_over(start, kiloclock(), abort_flag[1], code == kStatusWaitSmemEmpty)) return false;
   *abort_flag = 1;
   if (status) atomicCAS(status, 0, code);
   return true;
@@ -240,7 +250,7 @@ static __device__ __noinline__ bool mbar_wait_expired(uint32_t start, volatile i
 // flag, records `code` in the global status word and returns false so that the caller can unwind.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code) {
-  const uint32_t start = clock();
+  const uint32_t start = kiloclock();
   for (uint32_t spins = 0; !mbar_try_wait(bar, parity);) {
     if (++spins == 1024) {
       if (mbar_wait_expired(start, abort_flag, status, code)) return false;
