@@ -260,6 +260,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
+// After a wait ran out, with all of a CTA's roles back: time (about a millisecond) for the copies and products in flight to land
+// before the shared and tensor memory they read or write, and the barriers they arrive on, go to another CTA.
+__device__ __forceinline__ void settle_after_abort() {
+  const long long start = clock64();
+  while (clock64() - start < 2000000LL) { __nanosleep(1000); }
+}
+
 // Both of two phases, asked for together: a wait that is already over still takes a round trip to shared memory, about 220
 // clocks behind the tensor core's operand reads, and one after the other these add
 // up (GEMM core, operands and accumulator stage of a K block: 64 x 4096 x 7168 11.9 us apart, 11.25 together).

@@ -982,6 +982,7 @@ extern "C" int cake_b200_gqa_prefill_launch(void* handle, void* cuda_stream) {
   if (h->tiled) {
     gqa_prefill::Params t = h->t;
     t.wait_kiloclocks = test_hooks().budget_kiloclocks;
+    t.skip_load = test_hooks().skip_load;
     if (int rc = launch_dependent(gqa_prefill::plan_kernel, dim3(1), dim3(1024), 0, s, t)) return rc;
     const unsigned units = unsigned(t.capacity) * t.hkv;               // an upper bound: the list is made on the device
     return launch_dependent(gqa_prefill::prefill_kernel, dim3(units < unsigned(h->sms) ? units : unsigned(h->sms)), dim3(gqa_prefill::kThreads), gqa_prefill::kSmemBytes, s, t);

@@ -769,6 +769,7 @@ mla_decode_kernel(const __grid_constant__ Params p) {
 
   tcgen05_fence_before();
   __syncthreads();
+  if (sh->wait.abort_flag) settle_after_abort();   // (the CTA that issues gives up where the other one does: it waits for that one's rows and weights)
   cluster_sync();                                  // neither CTA leaves while the other may still reach into it
   tcgen05_fence_after();
   if (warp == kMmaWarp) tmem_dealloc_pair(tmem_base, kTmemColumns);

@@ -573,10 +573,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   tcgen05_fence_before();
   __syncthreads();
   if (sh->wait.abort_flag) {
-    // A wait ran out somewhere: give copies still in flight time to land before the shared
-    // memory they target is released with the CTA.
-    const long long start = clock64();
-    while (clock64() - start < 2000000LL) { __nanosleep(1000); }
+    settle_after_abort();
     __syncthreads();
   }
   if (warp == 1) {

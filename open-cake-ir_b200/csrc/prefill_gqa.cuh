@@ -52,6 +52,7 @@ struct Params {
   int* prefix;                                   // [segments + 3] tiles before a segment
   int* status;
   int total_q, segments, hq, hkv, group, page_size, nan_for_masked, capacity, wait_kiloclocks;
+  int skip_load;                                 // test hook: CTA 0's loader warps leave out the second K tile of their first unit
 };
 
 struct Shared {
@@ -371,6 +372,7 @@ prefill_kernel(const __grid_constant__ Params p) {
           for (int kv = 0; kv < 2; ++kv) {
             ok = mbar_wait(kv ? &sh->v_empty[s] : &sh->k_empty[s], ((it / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
             if (!ok) break;
+            if (p.skip_load && blockIdx.x == 0 && it == 1 && kv == 0) continue;      // test hook: never filled
             const __nv_bfloat16* src = (kv ? p.v : p.k) + size_t(w.kvh) * kD + chunk * 8;
             const uint32_t dst = (kv ? v_addr : k_addr) + s * kTileBytes;
 #pragma unroll
@@ -557,6 +559,10 @@ prefill_kernel(const __grid_constant__ Params p) {
 
   tcgen05_fence_before();
   __syncthreads();
+  if (sh->wait.abort_flag) {
+    settle_after_abort();
+    __syncthreads();
+  }
   if (warp == 0) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, kTmemColumns);

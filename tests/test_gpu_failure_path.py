@@ -10,6 +10,7 @@ import torch
 
 import open_cake_ir_b200 as cake
 from oracle import attention, block_scaled_gemm, compare
+from test_gpu_prefill_tiles import problem
 
 pytestmark = pytest.mark.gpu
 
@@ -49,6 +50,24 @@ def test_mla_decode_wait_runs_out_and_the_handle_stays_usable(hooks):
     op.launch()
     assert op.status() == 0
     want = attention.paged_decode_reference(cpu, mla=True, page_size=64, per_head_loop=False)
+    assert compare.compare(out, want["output"], atol=2.0 ** -16, rtol=2.0 ** -7)[0]
+    assert compare.compare(lse, want["lse"], atol=1e-4, rtol=1e-5, ieee=True)[0]
+
+
+def test_gqa_prefill_wait_runs_out_and_the_handle_stays_usable(hooks):
+    cpu = problem(9, [300, 200], [700, 200], 8, 2, 16)                  # the longest units come first: CTA 0 has several KV tiles
+    dev = {k: v.cuda() for k, v in cpu.items()}
+    out = torch.zeros_like(dev["q"]); lse = torch.zeros(dev["q"].shape[:2], dtype=torch.float32, device="cuda")
+    op = cake.GqaCausalPrefill(dev["q"], dev["k_cache"], dev["v_cache"], dev["qo_indptr"], dev["kv_indptr"], dev["kv_indices"],
+                               dev["kv_last_page_len"], dev["sm_scale"], out, lse, max_kv_len=700)
+    assert hooks(2048, 1) == 0                 # CTA 0 never receives its second K tile
+    op.launch()
+    op.launch()                                # what the first one had in flight does not reach the second
+    assert op.status() != 0
+    assert hooks(0, 0) == 0
+    op.launch()
+    assert op.status() == 0
+    want = attention.causal_prefill_reference(cpu, mla=False, paged=True, page_size=16, nan_for_masked=False, per_head_loop=False)
     assert compare.compare(out, want["output"], atol=2.0 ** -16, rtol=2.0 ** -7)[0]
     assert compare.compare(lse, want["lse"], atol=1e-4, rtol=1e-5, ieee=True)[0]
 
