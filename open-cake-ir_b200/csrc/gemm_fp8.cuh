@@ -77,6 +77,8 @@ struct Params {
   int interleave_hi_lo;        // 1: A K-block kb -> A column block (kb&1)*(k_blocks/2) + kb/2, B block kb/2
   const int* offsets;          // [groups+1] device row offsets into A; null = one group of dense_rows rows
   int dense_rows;
+  const int* enabled;          // grouped modes: device word, 0 = there is nothing to do here (null: there is)
+  int min_rows;                // groups of at most so many rows are left out: another kernel's (0: none are)
   const float* sfa;            // [k_blocks, row_capacity]
   const float* sfb;            // [groups, b_rows_per_group/128, b_k_blocks]
   void* out;                   // see Mode
@@ -164,6 +166,11 @@ template <int MODE, bool SPLIT = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a_tail,
                 const __grid_constant__ CUtensorMap map_b, const Params p) {
+  if (MODE != kDense && p.enabled) {               // the usual case is to leave, so before anything is set up
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (*p.enabled == 0) return;
+  }
   extern __shared__ uint8_t smem_raw[];
   // by an offset, not by rounding the pointer as an integer: the compiler then still knows that it is shared memory
   uint8_t* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -205,7 +212,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       int tiles_g = 0;
       if (g < p.groups) {
         int cnt = p.offsets ? p.offsets[g + 1] - p.offsets[g] : p.dense_rows;
-        tiles_g = (cnt + kBM - 1) / kBM;
+        tiles_g = cnt > p.min_rows ? (cnt + kBM - 1) / kBM : 0;
       }
       int incl = tiles_g;
 #pragma unroll

@@ -18,6 +18,7 @@
 // so that fragments of all four k-steps are two 16-byte shared-memory reads per row instead of eight 4-byte ones.
 #pragma once
 #include "gemm_fp8.cuh"
+#include <climits>
 #include <type_traits>
 
 namespace cake {
@@ -43,6 +44,8 @@ struct Params {
   void* out;                   // kGateUp: e4m3 [rows, n * terms] (WK = 1) or fp32 [rows, n]; else bf16 [rows, n]
   float* out_scale;            // kGateUp, WK = 1: [n / 128 * terms, row_capacity]
   int* status;                 // status word to clear (null: someone else does); nothing here waits, so nothing ever sets it
+  int max_rows;                // groups of more rows are the tcgen05 core's where that pays (0: none are)
+  const int* core;             // max_rows > 0: device word that says whether it does
   int n, k_blocks, w_rows, groups, dense_rows, x_stride, sx_stride, map_div, row_capacity, terms;
 };
 
@@ -113,11 +116,12 @@ skinny_kernel(const Params p) {
   if (p.status && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;
 
   if (warp == 0) {
+    const int max_rows = p.max_rows && *p.core ? p.max_rows : INT_MAX;
     int running = 0;
     for (int base = 0; base < p.groups; base += 32) {
       const int g = base + lane;
       const int count = g < p.groups ? (p.offsets ? p.offsets[g + 1] - p.offsets[g] : p.dense_rows) : 0;
-      const int tiles = (count + S::kTokens - 1) / S::kTokens;
+      const int tiles = count > max_rows ? 0 : (count + S::kTokens - 1) / S::kTokens;
       int incl = tiles;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {

@@ -154,20 +154,52 @@ routing_kernel(const float* __restrict__ logits, const __nv_bfloat16* __restrict
   }
 }
 
+// What gathering the rows of an expert takes: each routed row (e4m3 hidden state + its K-block scales + its route weight) goes to
+// its sorted position.
+struct Gather {
+  const uint8_t* hidden;
+  const float *hidden_scale, *route_weights;
+  uint8_t* x_perm;
+  float *sx_perm, *row_weight;
+  int tokens, hidden_width, top_k, capacity;
+  int above, item_rows;          // place_kernel: experts of more rows than `above` may be the core's (0: none); rows of a weight-streaming item
+  int* core;                     // place_kernel: whether they are
+};
+// Items whose weights the core has to save to be worth its two launches' latency (hidden 7168, experts of 2048: about 10 us an item, 60 us).
+constexpr int kCorePays = 8;
+// One row, by a warp: eight 16-byte loads of a lane in flight.
+__device__ __forceinline__ void gather_row(const Gather& g, int pair, int pos) {
+  const int lane = threadIdx.x & 31, token = pair / g.top_k;
+  const uint4* src = reinterpret_cast<const uint4*>(g.hidden + size_t(token) * g.hidden_width);
+  uint4* dst = reinterpret_cast<uint4*>(g.x_perm + size_t(pos) * g.hidden_width);
+  const int vectors = g.hidden_width / 16;
+  for (int base = lane; base < vectors; base += 8 * 32) {
+    uint4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = base + 32 * i < vectors ? __ldg(src + base + 32 * i) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) if (base + 32 * i < vectors) dst[base + 32 * i] = v[i];
+  }
+  for (int kb = lane; kb < g.hidden_width / 128; kb += 32) g.sx_perm[size_t(kb) * g.capacity + pos] = __ldg(g.hidden_scale + size_t(kb) * g.tokens + token);
+  if (lane == 0) g.row_weight[pos] = __ldg(g.route_weights + pair);
+}
+
 // ---- permute: stable placement ---------------------------------------------------------------
 // One CTA of eight warps per local expert, and nothing before it: the CTA counts the pairs of its expert and those of the
 // local experts before it (its offset) in one pass over the ids, so no histogram, scan or counter to clear is needed.  Each
 // warp owns a contiguous eighth of the pairs; a prefix over the warps gives every warp its starting position, and a second
 // pass places the pairs by ballot rank -- ascending pair order inside the expert, so the permutation is the stable sort
 // by expert.  Eight loads per lane are in flight per step.  Pairs of other ranks get inv_perm -1 (each step's by one CTA).
-// `clear` (may be null): `clear_words` counters of the kernels that follow.
+// `clear` (may be null): `clear_words` counters of the kernels that follow.  `gather.above` > 0 (a layer on the weight-streaming kernel): the
+// experts of many rows go to the tcgen05 core where the weights that they would have streamed again are worth its launches.  Every
+// CTA that it concerns counts all experts' rows to find out; an expert of the core's has its rows gathered here, by its CTA.
 constexpr int kPlaceWarps = 8;
 constexpr int kPlaceStep = 256;      // pairs one warp looks at per step
 __global__ void __launch_bounds__(kPlaceWarps * 32)
 place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_ptr, int* __restrict__ counts,
              int* __restrict__ offsets, int* __restrict__ sorted_pairs, int* __restrict__ inv_perm, int pairs, int local_experts,
-             int* __restrict__ clear, int clear_words) {
-  __shared__ int warp_count[kPlaceWarps], warp_before[kPlaceWarps];
+             int* __restrict__ clear, int clear_words, const Gather gather) {
+  __shared__ int warp_count[kPlaceWarps], warp_before[kPlaceWarps], rows_of[gemm::kMaxGroups], streamed_again;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int e = blockIdx.x;
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -212,8 +244,7 @@ place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_
     offsets[e] = first;
     if (e == local_experts - 1) offsets[local_experts] = first + total;
   }
-  if (count == 0) return;
-  for (int base = begin; base < end; base += kPlaceStep) {
+  for (int base = begin; count > 0 && base < end; base += kPlaceStep) {
     int ids[kPlaceStep / 32];
 #pragma unroll
     for (int i = 0; i < kPlaceStep / 32; ++i) {
@@ -233,6 +264,22 @@ place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_
       cursor += __popc(mask);
     }
   }
+  if (gather.above == 0 || (e != 0 && total <= gather.above)) return;
+  for (int g = threadIdx.x; g < local_experts; g += kPlaceWarps * 32) rows_of[g] = 0;
+  if (threadIdx.x == 0) streamed_again = 0;
+  __syncthreads();                             // (the expert's pairs are placed, too)
+  for (int p = threadIdx.x; p < pairs; p += kPlaceWarps * 32) {
+    const int g = expert_ids[p] - offset;
+    if (g >= 0 && g < local_experts) atomicAdd(rows_of + g, 1);
+  }
+  __syncthreads();
+  for (int g = threadIdx.x; g < local_experts; g += kPlaceWarps * 32)
+    if (rows_of[g] > gather.above) atomicAdd(&streamed_again, (rows_of[g] - 1) / gather.item_rows);
+  __syncthreads();
+  const bool core = streamed_again >= kCorePays;
+  if (e == 0 && threadIdx.x == 0) *gather.core = core;
+  if (!core || total <= gather.above) return;
+  for (int pos = first + warp; pos < first + total; pos += kPlaceWarps) gather_row(gather, sorted_pairs[pos], pos);
 }
 
 // Routing and permute of a step of at most 32 tokens in one CTA, a warp per token: two launches less, and the pairs never
@@ -284,28 +331,13 @@ route_place_kernel(const float* __restrict__ logits, const __nv_bfloat16* __rest
   }
 }
 
-// Copies each routed row (e4m3 hidden state + its K-block scales + its route weight) to its
-// sorted position.  One warp per destination row.
+// Gathers the rows of every local expert.  One warp per destination row.
 __global__ void __launch_bounds__(256)
-gather_kernel(const uint8_t* __restrict__ hidden, const float* __restrict__ hidden_scale,
-              const float* __restrict__ route_weights, const int* __restrict__ sorted_pairs,
-              const int* __restrict__ offsets, uint8_t* __restrict__ x_perm, float* __restrict__ sx_perm,
-              float* __restrict__ row_weight, int tokens, int hidden_width, int top_k, int local_experts,
-              int capacity) {
-  const int lane = threadIdx.x & 31;
+gather_kernel(const int* __restrict__ sorted_pairs, const int* __restrict__ offsets, int local_experts, const Gather gather) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int n_local = offsets[local_experts];
-  for (int pos = blockIdx.x * 8 + (threadIdx.x >> 5); pos < n_local; pos += gridDim.x * 8) {
-    const int pair = __ldg(sorted_pairs + pos);
-    const int token = pair / top_k;
-    const uint4* src = reinterpret_cast<const uint4*>(hidden + size_t(token) * hidden_width);
-    uint4* dst = reinterpret_cast<uint4*>(x_perm + size_t(pos) * hidden_width);
-    for (int i = lane; i < hidden_width / 16; i += 32) dst[i] = __ldg(src + i);
-    for (int kb = lane; kb < hidden_width / 128; kb += 32)
-      sx_perm[size_t(kb) * capacity + pos] = __ldg(hidden_scale + size_t(kb) * tokens + token);
-    if (lane == 0) row_weight[pos] = __ldg(route_weights + pair);
-  }
+  for (int pos = blockIdx.x * 8 + (threadIdx.x >> 5); pos < n_local; pos += gridDim.x * 8) gather_row(gather, __ldg(sorted_pairs + pos), pos);
 }
 
 // out[t,:] = bf16( fp32 sum over the token's local slots, in slot order, of the bf16 rows y[inv_perm[t,slot],:] ).  A thread
@@ -370,9 +402,9 @@ struct PermuteArgs {
   int *counts, *offsets, *sorted_pairs, *inv_perm;
   int pairs, local_experts;
 };
-inline int launch_permute(const PermuteArgs& a, cudaStream_t s, int* clear = nullptr, int clear_words = 0) {
+inline int launch_permute(const PermuteArgs& a, cudaStream_t s, int* clear = nullptr, int clear_words = 0, const Gather& gather = Gather{}) {
   return launch_dependent(place_kernel, dim3(a.local_experts), dim3(kPlaceWarps * 32), 0, s, a.expert_ids, a.local_offset, a.counts,
-                          a.offsets, a.sorted_pairs, a.inv_perm, a.pairs, a.local_experts, clear, clear_words);
+                          a.offsets, a.sorted_pairs, a.inv_perm, a.pairs, a.local_experts, clear, clear_words, gather);
 }
 
 struct RoutingHandle {
@@ -391,6 +423,7 @@ struct Layout {     // byte offsets inside the workspace
   size_t status, expert_ids, route_weights, counts, offsets, sorted_pairs, inv_perm, row_weight, x_perm, sx_perm,
       act, act_scale, y, act32, total;
   int capacity, terms;
+  int core_above;                        // weight-streaming kernel: experts of more rows than this take the tcgen05 core (0: none can hurt)
   int token_tiles, split1, split2;       // few rows per expert: token tiles of eight and K splits of the weight-streaming kernel (0: the tcgen05 core)
 };
 inline Layout make_layout(const cake_b200_moe_config& c) {
@@ -428,6 +461,15 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
     l.split1 = skinny::choose_split_gate_up(touched > 1 ? touched : 1, c.intermediate, c.hidden / 128, 148);
     l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128, 148);
     if (l.split1 > 1) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation
+    // The routing may be anything but even: the padding of a batch, or a batch of one prompt, goes to the same top_k experts.  The
+    // weight-streaming kernel then reads their weights once per item of 8 token_tiles rows, so experts of many rows (four times the
+    // average, which chance does not reach) go to the core: 96 equal tokens, hidden 7168, 256 experts of 2048: 684 us without,
+    // 163 with.  The core's two launches cost 3 us where no expert takes them, so not where such tokens would read
+    // less than 400 MB again (64 us at the copy rate): there the weight-streaming kernel is the faster one even so (96 equal
+    // tokens, hidden 2048, 128 experts of 768, 189 MB: 74 us, 82 on the core alone).
+    const double items = double((c.tokens + 8 * l.token_tiles - 1) / (8 * l.token_tiles)), chosen = c.top_k < c.local_experts ? c.top_k : c.local_experts;
+    const int above = per_expert <= 4 ? 16 : int(4 * per_expert);
+    if (c.tokens > above && (items - 1) * chosen * 3 * c.hidden * c.intermediate > 4e8) l.core_above = above;
   }
   l.total = at;
   return l;
@@ -523,6 +565,7 @@ extern "C" int cake_b200_moe_permute_destroy(void* handle) {
 }
 
 // ------------------------------------------------------------------------------------------
+constexpr int kCoreWord = 12;                 // of the status block: experts of many rows are on the tcgen05 core
 static bool moe_config_ok(const cake_b200_moe_config& c) {
   if (c.tokens < 0 || c.tokens * int64_t(c.top_k > 0 ? c.top_k : 1) > (int64_t(1) << 28)) return false;
   if (c.hidden <= 0 || c.hidden % 128 || c.intermediate <= 0 || c.intermediate % 128) return false;
@@ -591,6 +634,7 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
   p1.b_rows_per_group = 2 * inter;
   p1.groups = c.local_experts;
   p1.row_capacity = l.capacity;
+  p1.min_rows = l.core_above;
   p1.offsets = offsets;
   p1.sfa = reinterpret_cast<const float*>(h->ws + l.sx_perm);
   p1.sfb = static_cast<const float*>(buffers[5]);
@@ -610,6 +654,7 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
   p2.b_rows_per_group = hidden;
   p2.groups = c.local_experts;
   p2.row_capacity = l.capacity;
+  p2.min_rows = l.core_above;
   p2.offsets = offsets;
   p2.sfa = reinterpret_cast<const float*>(h->ws + l.act_scale);
   p2.sfb = static_cast<const float*>(buffers[7]);
@@ -641,6 +686,8 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
     s1.sx_stride = int(c.tokens);
     s1.row_capacity = l.capacity;
     s1.terms = l.terms;
+    s1.max_rows = l.core_above;
+    s1.core = status + kCoreWord;
     skinny::Params& s2 = h->s2;
     s2 = skinny::Params{};
     s2.w = static_cast<const uint8_t*>(buffers[6]);
@@ -658,6 +705,9 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
     s2.x_stride = inter * l.terms;
     s2.sx_stride = s2.row_capacity = l.capacity;
     s2.terms = 1;
+    s2.max_rows = l.core_above;
+    s2.core = status + kCoreWord;
+    if (l.core_above) p1.enabled = p2.enabled = status + kCoreWord;
     rc = skinny::prepare_any<gemm::kGateUp>(l.token_tiles, l.split1, 1);
     if (!rc) rc = skinny::prepare_any<gemm::kDown>(l.token_tiles, l.split2, l.terms);
     if (rc) { delete h; return rc; }
@@ -678,7 +728,10 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
   switch (stage) {
     case 0: {
       int* const clear = reinterpret_cast<int*>(h->ws + l.status);      // the status word and the GEMMs' counters start at 0
-      if (!c.external_routing && tokens <= moe::kSmallTokens && l.token_tiles) {
+      const moe::Gather gather{h->hidden, h->hidden_scale, h->route_weights, h->ws + l.x_perm, reinterpret_cast<float*>(h->ws + l.sx_perm),
+                               reinterpret_cast<float*>(h->ws + l.row_weight), tokens, c.hidden, c.top_k, l.capacity,
+                               l.core_above, 8 * l.token_tiles, clear + kCoreWord};
+      if (!c.external_routing && tokens <= moe::kSmallTokens && l.token_tiles && !l.core_above) {
         const int epl = (c.experts + 31) / 32;
         auto* kernel = epl <= 2 ? moe::route_place_kernel<2> : epl <= 4 ? moe::route_place_kernel<4> : epl <= 8 ? moe::route_place_kernel<8> : moe::route_place_kernel<16>;
         return launch_dependent(kernel, dim3(1), dim3(32 * tokens), 0, s, h->logits, h->bias, h->factor, h->local_offset, h->expert_ids, h->route_weights,
@@ -689,32 +742,36 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
         if (int rc = moe::launch_routing(h->logits, h->bias, h->factor, h->expert_ids, h->route_weights, tokens, c.experts, c.top_k,
                                          c.n_group, c.topk_group, c.routing_mode, s))
           return rc;
-      if (int rc = moe::launch_permute(pa, s, clear, 64)) return rc;
+      if (int rc = moe::launch_permute(pa, s, clear, 64, gather)) return rc;
       if (l.token_tiles) return 0;
       const int gather_blocks = (l.capacity + 7) / 8;
-      return launch_dependent(moe::gather_kernel, dim3(gather_blocks < 4096 ? gather_blocks : 4096), dim3(256), 0, s,
-                              h->hidden, h->hidden_scale, h->route_weights, pa.sorted_pairs, pa.offsets, h->ws + l.x_perm,
-                              reinterpret_cast<float*>(h->ws + l.sx_perm), reinterpret_cast<float*>(h->ws + l.row_weight), tokens, c.hidden,
-                              c.top_k, c.local_experts, l.capacity);
+      return launch_dependent(moe::gather_kernel, dim3(gather_blocks < 4096 ? gather_blocks : 4096), dim3(256), 0, s, pa.sorted_pairs, pa.offsets,
+                              c.local_experts, gather);
     }
     case 1: {
       if (l.token_tiles) {
         if (int rc = skinny::launch_any<gemm::kGateUp>(l.token_tiles, l.split1, 1, h->s1, h->grid, s)) return rc;
-        if (l.split1 == 1) return 0;
-        const int64_t rows = int64_t(l.capacity) * (c.intermediate / 128);
-        return launch_dependent(skinny::quantize_kernel, dim3(unsigned(rows < 8 * 592 ? (rows + 7) / 8 : 592)), dim3(256), 0, s,
-                                reinterpret_cast<const float*>(h->ws + l.act32), pa.offsets + c.local_experts, h->ws + l.act,
-                                h->p1.out_scale, c.intermediate, l.terms, l.capacity);
+        if (l.split1 > 1) {                    // (rows of the core's experts among them, which it writes afterwards)
+          const int64_t rows = int64_t(l.capacity) * (c.intermediate / 128);
+          if (int rc = launch_dependent(skinny::quantize_kernel, dim3(unsigned(rows < 8 * 592 ? (rows + 7) / 8 : 592)), dim3(256), 0, s,
+                                        reinterpret_cast<const float*>(h->ws + l.act32), pa.offsets + c.local_experts, h->ws + l.act,
+                                        h->p1.out_scale, c.intermediate, l.terms, l.capacity))
+            return rc;
+        }
+        if (!l.core_above) return 0;
       }
       gemm::Params p = h->p1;
       p.wait_kiloclocks = test_hooks().budget_kiloclocks;
       return launch_dependent(gemm::gemm_fp8_kernel<gemm::kGateUp>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a1, h->map_a1_tail, h->map_b1, p);
     }
     case 2: {
-      if (l.token_tiles) return skinny::launch_any<gemm::kDown>(l.token_tiles, l.split2, l.terms, h->s2, h->grid, s);
-      gemm::Params p = h->p2;
-      p.wait_kiloclocks = test_hooks().budget_kiloclocks;
-      return launch_dependent(gemm::gemm_fp8_kernel<gemm::kDown>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a2, h->map_a2_tail, h->map_b2, p);
+      if (!l.token_tiles || l.core_above) {
+        gemm::Params p = h->p2;
+        p.wait_kiloclocks = test_hooks().budget_kiloclocks;
+        if (int rc = launch_dependent(gemm::gemm_fp8_kernel<gemm::kDown>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a2, h->map_a2_tail, h->map_b2, p))
+          return rc;
+      }
+      return l.token_tiles ? skinny::launch_any<gemm::kDown>(l.token_tiles, l.split2, l.terms, h->s2, h->grid, s) : 0;
     }
     case 3:
     {

@@ -2,6 +2,8 @@
 four token tiles of eight, experts with more rows than an item holds, K split over a CTA's warps or not (with the
 quantisation in a kernel of its own), one and two activation terms, routing and placement in one kernel (up to 32 tokens)
 or two, and the tcgen05 core just beyond.  Oracle and tolerance of test_gpu_moe.py's layer test."""
+import functools
+
 import pytest
 import torch
 
@@ -36,4 +38,30 @@ def test_gates_at_the_ends_of_the_sigmoid(tokens, act):
     out, _ = run_layer(cpu, experts=experts, routing="softmax", act_mode=act)
     want = oracle_moe.moe_reference(cpu, routing="softmax", act_quant="fp8" if act == "fp8" else "none", dtype=torch.float32)
     assert torch.isfinite(out.float()).all()
+    assert compare.rel_frobenius(out, want["output"]) <= (1e-2 if act == "fp8" else 4e-3)
+
+
+@functools.lru_cache(maxsize=1)
+def large_experts():
+    """16 of 64 experts, large enough that streaming one several times costs more than the core's launches."""
+    return cake.workloads.moe_inputs(56, 4096, 2304, 64, 16, 0, routing="softmax", device="cpu")
+
+
+@pytest.mark.parametrize("act", ["fp8", "split"])
+@pytest.mark.parametrize("tokens,equal,offset", [
+    (24, 17, 0), (24, 16, 0),         # one row above the line and on it; up to 32 tokens
+    (24, 20, 5),                      # three of the experts of many rows are this rank's: not worth the core's launches
+    (56, 56, 0),                      # every row is the core's
+    (56, 29, 0), (56, 28, 0)])        # both kernels have experts; on the line
+def test_uneven_routing(tokens, equal, offset, act):
+    """Tokens that all go to the same experts, as a batch of one prompt or the padding of one does, among others: on either side
+    of each line that sends experts of many rows to the tcgen05 core."""
+    cpu = dict(large_experts(), local_expert_offset=torch.tensor([offset], dtype=torch.int32))
+    for name in ("routing_logits", "hidden_states"):
+        cpu[name] = cpu[name][:tokens].clone()
+    cpu["hidden_states_scale"] = cpu["hidden_states_scale"][:, :tokens].contiguous()
+    cpu["routing_logits"][:equal, :8] += 20.0
+    cpu["routing_logits"][equal:, :8] -= 20.0
+    out, _ = run_layer(cpu, experts=64, routing="softmax", act_mode=act)
+    want = oracle_moe.moe_reference(cpu, routing="softmax", act_quant="fp8" if act == "fp8" else "none", dtype=torch.float32)
     assert compare.rel_frobenius(out, want["output"]) <= (1e-2 if act == "fp8" else 4e-3)
