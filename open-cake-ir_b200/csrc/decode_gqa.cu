@@ -27,6 +27,7 @@
 #include "../../include/cake_b200.h"
 #include <mutex>
 #include <new>
+#include <type_traits>
 
 namespace cake {
 namespace gqa {
@@ -143,7 +144,7 @@ __device__ __forceinline__ void load_half(const __nv_bfloat16* __restrict__ cach
 // resets the counters and writes the results of empty sequences (zeros, lse = -inf), which no
 // piece covers.
 constexpr int kPieceCost = 32;
-constexpr int kMaxSms = 192;             // SM count the workspace is sized for
+constexpr int kMaxSms = gqa_prefill::kMaxSms;      // SM count the workspace is sized for
 constexpr int kMaxRanges = kMaxSms * kHeads;
 __global__ void __launch_bounds__(1024)
 gqa_plan_kernel(const Params p) {
@@ -862,19 +863,50 @@ struct PrefillHandle {
 };
 
 // Which of the two forms a launch takes, from what the host knows (lengths live on the device; max_kv_len bounds them).
-// The tiled form works through ceil(kv / 128) KV tiles one after another, about 1.9 us each, on as many SMs as there are
-// (query tile, KV head) pairs; the decode form reads the KV rows once per query token, at about 7 TB/s once L2 holds
-// them, but spreads any amount of work over the whole GPU.  So the decode form stays the better one for a few query
-// rows behind a long prefix.
-inline bool use_tiles(const cake_b200_gqa_prefill_config& c) {
-  const double tiles = double((c.total_q + gqa_prefill::tokens_per_tile(c.num_qo_heads / c.num_kv_heads) - 1) / gqa_prefill::tokens_per_tile(c.num_qo_heads / c.num_kv_heads) + c.segments - 1) * c.num_kv_heads;
-  const double tiled_us = (tiles > 148 ? tiles / 148 : 1.0) * double((c.max_kv_len + 127) / 128) * 1.9;
-  const double decode_us = 10.0 + double(c.total_q) * double(c.max_kv_len) * c.num_kv_heads * 512 / 7e6;
+// The tiled form shares its (query tile, KV head) units' KV tiles out over the SMs, at least two to one, 2.6 us each, or 4.1 where a unit
+// has one query tile only and its softmax nothing to run beside; a cut unit's pieces take the merge 0.2 us each.  The decode form reads
+// the KV rows once per query token, at about 9 TB/s once L2 holds them, and spreads any amount of work over the whole GPU: the
+// better one up to about three query rows a segment.  (32 query heads, 8 KV heads, us tiled / decode: 8 segments of 2 rows, 3000
+// KV rows 57 / 37; of 4 rows 58 / 72; 16 rows, 4096 KV rows 24 / 43; 64 rows 31 / 115; one KV head, 16 rows, 16384 KV rows 33 / 31.)
+inline bool use_tiles(const cake_b200_gqa_prefill_config& c, int sms) {
+  const int group = c.num_qo_heads / c.num_kv_heads, per = gqa_prefill::tokens_per_tile(group);
+  const double units = double((c.total_q + per - 1) / per + c.segments - 1) * c.num_kv_heads;
+  const double kv_tiles = double((c.max_kv_len + gqa_prefill::kTile - 1) / gqa_prefill::kTile);
+  const double least = kv_tiles < gqa_prefill::kMinPiece ? kv_tiles : gqa_prefill::kMinPiece, share = units * kv_tiles / sms;
+  const double pieces = kv_tiles >= gqa_prefill::kMinPiece + gqa_prefill::kMinGain && share < kv_tiles / 2 ? kv_tiles / (share > least ? share : least) : 0;
+  const double tiled_us = 10.0 + (share > least ? share : least) * (c.total_q * group > c.segments * gqa_prefill::kRows ? 2.6 : 4.1) + 0.2 * pieces;
+  const double decode_us = 15.0 + double(c.total_q) * double(c.max_kv_len) * c.num_kv_heads * 512 / 9e6;
   return tiled_us <= decode_us;
 }
-inline size_t tile_list_bytes(const cake_b200_gqa_prefill_config& c) {
-  const size_t n = size_t(gqa_prefill::tile_capacity(c.total_q, c.segments, c.num_qo_heads / c.num_kv_heads));
-  return align256(n * sizeof(int4)) + align256((n + 1) * sizeof(int)) + align256(size_t(c.segments + 3) * sizeof(int));
+// Pieces of cut tiles at most, see plan_kernel.  The kernel that knows pieces is the slower one for whole tiles (2000 query rows of 8 segments,
+// 800 KV rows: 63 us, 59 without), and the merge is one launch more, so it is not taken where there is too much other work for one long
+// unit to matter: where reading the KV rows once per query token of segments that are all query would take longer than
+// the longest unit.  None either where no tile is long enough.
+inline int cut_capacity(const cake_b200_gqa_prefill_config& c) {
+  const int64_t kv_tiles = (c.max_kv_len + gqa_prefill::kTile - 1) / gqa_prefill::kTile;
+  const double rows_us = 20.0 + double(c.total_q) * double(c.total_q) / c.segments / 2 * c.num_kv_heads * 512 / 7e6;
+  if (kv_tiles < gqa_prefill::kMinPiece + gqa_prefill::kMinGain || 14.0 + 2.6 * double(kv_tiles) < rows_us) return 0;
+  return gqa_prefill::kMaxSms / c.num_kv_heads;
+}
+// What the tiled form keeps behind the status block; returns its bytes.  `t`: filled with its sizes and, from `ws` on, its addresses.
+inline size_t carve_tiles(const cake_b200_gqa_prefill_config& c, gqa_prefill::Params& t, uint8_t* ws) {
+  const int group = c.num_qo_heads / c.num_kv_heads;
+  t.cut_capacity = cut_capacity(c);
+  t.capacity = gqa_prefill::tile_capacity(c.total_q, c.segments, group, t.cut_capacity);
+  t.part_rows = gqa_prefill::part_rows(c.total_q, group);
+  size_t at = 0;
+  auto take = [&](auto*& pointer, size_t count) {
+    pointer = reinterpret_cast<std::remove_reference_t<decltype(pointer)>>(reinterpret_cast<uintptr_t>(ws) + at);
+    at += align256(count * sizeof(*pointer));
+  };
+  take(t.tiles, size_t(t.capacity));
+  take(t.spans, size_t(t.capacity));
+  take(t.cuts, 2 * size_t(t.cut_capacity));
+  take(t.tile_count, 2);
+  take(t.prefix, size_t(c.segments) + 3);
+  take(t.part_o, size_t(t.cut_capacity) * c.num_kv_heads * t.part_rows * kD);
+  take(t.part_lse, size_t(t.cut_capacity) * c.num_kv_heads * t.part_rows);
+  return at;
 }
 }  // namespace gqa
 }  // namespace cake
@@ -896,7 +928,8 @@ extern "C" size_t cake_b200_gqa_prefill_workspace_bytes(const cake_b200_gqa_pref
   cake_b200_gqa_decode_config d;
   if (!c || !gqa_prefill_config_ok(*c, &d)) return 0;
   const size_t decode_form = cake_b200_gqa_decode_workspace_bytes(&d) + cake::prefill::table_bytes(c->total_q);
-  const size_t tiled_form = 512 + cake::gqa::tile_list_bytes(*c);
+  cake::gqa_prefill::Params t{};
+  const size_t tiled_form = 512 + cake::gqa::carve_tiles(*c, t, nullptr);
   return decode_form > tiled_form ? decode_form : tiled_form;
 }
 
@@ -944,7 +977,6 @@ extern "C" int cake_b200_gqa_prefill_create(void** buffers, const cake_b200_gqa_
   h->total_q = int(config->total_q);
   h->kv_unit = d.page_size;
   h->nan_for_masked = config->nan_for_masked;
-  h->tiled = gqa::use_tiles(*config);
   gqa_prefill::Params& t = h->t;
   t = gqa_prefill::Params{p.q, p.k_cache, p.v_cache, h->qo_indptr, h->kv_indptr_segments, p.kv_indices, h->last_page_len, p.sm_scale, p.out, p.lse};
   t.status = p.status;
@@ -955,17 +987,15 @@ extern "C" int cake_b200_gqa_prefill_create(void** buffers, const cake_b200_gqa_
   t.group = p.hq / p.hkv;
   t.page_size = p.page_size;
   t.nan_for_masked = h->nan_for_masked;
-  t.capacity = gqa_prefill::tile_capacity(t.total_q, t.segments, t.group);
-  t.tiles = reinterpret_cast<int4*>(ws);
-  t.tile_page = reinterpret_cast<int*>(ws + gqa::align256(size_t(t.capacity) * sizeof(int4)));
-  t.tile_count = t.tile_page + t.capacity;
-  t.prefix = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(t.tile_page) + gqa::align256(size_t(t.capacity + 1) * sizeof(int)));
+  gqa::carve_tiles(*config, t, ws);
   int sms = 0;
   int rc = gqa_sm_count(device, &sms);
   if (!rc) rc = int(cudaFuncSetAttribute(gqa::gqa_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gqa::kSmemBytes));
-  if (!rc) rc = int(cudaFuncSetAttribute(gqa_prefill::prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gqa_prefill::kSmemBytes)));
+  if (!rc) rc = int(cudaFuncSetAttribute(t.cut_capacity ? gqa_prefill::prefill_kernel<true> : gqa_prefill::prefill_kernel<false>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(gqa_prefill::kSmemBytes)));
   if (rc) { delete h; return rc; }
-  h->sms = sms < gqa::kMaxSms ? sms : gqa::kMaxSms;
+  h->sms = t.sms = sms < gqa::kMaxSms ? sms : gqa::kMaxSms;
+  h->tiled = gqa::use_tiles(*config, h->sms);
   *handle_out = h;
   return 0;
 }
@@ -985,7 +1015,10 @@ extern "C" int cake_b200_gqa_prefill_launch(void* handle, void* cuda_stream) {
     t.skip_load = test_hooks().skip_load;
     if (int rc = launch_dependent(gqa_prefill::plan_kernel, dim3(1), dim3(1024), 0, s, t)) return rc;
     const unsigned units = unsigned(t.capacity) * t.hkv;               // an upper bound: the list is made on the device
-    return launch_dependent(gqa_prefill::prefill_kernel, dim3(units < unsigned(h->sms) ? units : unsigned(h->sms)), dim3(gqa_prefill::kThreads), gqa_prefill::kSmemBytes, s, t);
+    auto* kernel = t.cut_capacity ? gqa_prefill::prefill_kernel<true> : gqa_prefill::prefill_kernel<false>;
+    if (int rc = launch_dependent(kernel, dim3(units < unsigned(h->sms) ? units : unsigned(h->sms)), dim3(gqa_prefill::kThreads), gqa_prefill::kSmemBytes, s, t)) return rc;
+    if (!t.cut_capacity) return 0;
+    return launch_dependent(gqa_prefill::merge_kernel, dim3(2 * h->sms), dim3(gqa_prefill::kMergeWarps * 32), 0, s, t);
   }
   prefill::prefill_plan_kernel<<<(h->total_q + 255) / 256, 256, 0, s>>>(h->qo_indptr, h->kv_indptr_segments, h->last_page_len, h->segments,
                                                                        h->kv_unit, h->total_q, h->seq_start, h->seq_tokens, h->masked);

@@ -1,4 +1,4 @@
-// Causal GQA prefill for sm_100a: query tiles against shared KV tiles on tcgen05 (flash attention, no split).
+// Causal GQA prefill for sm_100a: query tiles against shared KV tiles on tcgen05 (flash attention).
 //
 // Operator: the prefill branches of src/open_cake_ir/tasks/solx_fib/attention.py:132-183 (attention_specs.py:85-248), see
 // prefill.cuh for the masking rules.  A unit of work is one KV head and a tile of consecutive query tokens of one segment; the
@@ -14,6 +14,9 @@
 // and about 750 issue slots per warp.  Two row tiles with a softmax warpgroup each keep the pipe busy: the products of
 // one run while the other's softmax does ([P V of A(j), S of A(j+1)], [P V of B(j), S of B(j+1)], ...).
 // Running each query token as a decode sequence of its own read every KV row once per query token instead.
+// A unit goes through its KV tiles one after another (2 to 3 us each), so a unit that alone would take longer than an even share of
+// the launch's KV tiles, a few query rows behind a long prefix, is cut into pieces of consecutive KV tiles; these leave partial results,
+// which merge_kernel puts together.
 // Roles: warp 0 issues the products, warps 4..7 gather Q, K and V rows (cp.async through the page table, any page size; the
 // copies announce themselves on the stage's barrier), warps 8..11 and 12..15 are the softmax of tiles A and B.  Every wait
 // is bounded and reports through the status word.
@@ -39,6 +42,9 @@ constexpr uint32_t kColS = 0, kColO = 256, kTmemColumns = 512;        // tile X:
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleThreshold = 8.f;         // log2 units: O is rescaled when the running maximum grows by more
 constexpr int kCostBuckets = 1024;
+// KV tiles of a piece at least, and by how many a piece has to be shorter than its tile: the merge takes 5 us and more.
+constexpr int kMinPiece = 2, kMinGain = 4;
+constexpr int kMaxSms = 192;                     // what the workspace is sized for
 
 struct Params {
   const __nv_bfloat16 *q, *k, *v;                // [total_q, Hq, D], [rows, Hkv, D]
@@ -47,11 +53,14 @@ struct Params {
   __nv_bfloat16* out;
   float* lse;
   int4* tiles;                                   // [capacity] {first query row, rows, KV rows the first one sees (may be < 1), KV rows of the segment}
-  int* tile_page;                                // [capacity] where the segment's page list starts
-  int* tile_count;                               // [1]
+  int4* spans;                                   // [capacity] {where the segment's page list starts, first KV tile, KV tile behind the last, slot of the partial result (-1: whole)}
+  int4* cuts;                                    // [2 * cut_capacity] tiles that are cut: {as in `tiles`}, {first slot, pieces}
+  int* tile_count;                               // [2] entries of `tiles`, cut tiles
+  float *part_o, *part_lse;                      // [cut_capacity, Hkv, part_rows, D] normalised, [cut_capacity, Hkv, part_rows] base 2
   int* prefix;                                   // [segments + 3] tiles before a segment
   int* status;
   int total_q, segments, hq, hkv, group, page_size, nan_for_masked, capacity, wait_kiloclocks;
+  int sms, cut_capacity, part_rows;              // cut_capacity: pieces of cut tiles at most (0: nothing is cut)
   int skip_load;                                 // test hook: CTA 0's loader warps leave out the second K tile of their first unit
 };
 
@@ -66,14 +75,18 @@ constexpr size_t kSmemBytes = size_t(2 + 2 * kStages) * kTileBytes + kOutBytes +
 static_assert(kSmemBytes <= 232448, "the kernel's shared memory exceeds what a CTA may have on sm_100");
 
 inline int tokens_per_tile(int group) { return 2 * (kRows / group); }
-inline int tile_capacity(int64_t total_q, int64_t segments, int group) { return int(total_q / tokens_per_tile(group) + segments + 3); }
+inline int tile_capacity(int64_t total_q, int64_t segments, int group, int cuts) { return int(total_q / tokens_per_tile(group) + segments + 3) + cuts; }
+inline int part_rows(int64_t total_q, int group) { return total_q <= kRows / group ? int(total_q) * group : 2 * kRows; }      // one query tile or two
 
 // One CTA: cuts the query rows of every segment into tiles and lists them, most KV tiles first, so that the CTAs that start
-// last are the short ones.  Rows outside every segment form two more segments without KV rows (they become zeros).
+// last are the short ones.  Rows outside every segment form two more segments without KV rows (they become zeros).  With `sms`
+// CTAs and N KV tiles in all, for each KV head, a tile of n goes to floor(n sms / (N Hkv)) pieces, about an even share each, where that
+// is shorter by enough to pay for the merge; no more pieces than sms / Hkv in all.
 static __global__ void __launch_bounds__(1024)
 plan_kernel(const Params p) {
   __shared__ int sums[32];
   __shared__ int bucket[kCostBuckets];
+  __shared__ int cut_tile[kMaxSms], cut_first[kMaxSms], cut_size[kMaxSms], cut_count;      // cut_count: cut tiles << 16 | their pieces
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x;
@@ -86,6 +99,7 @@ plan_kernel(const Params p) {
   };
   const int count = p.segments + 2;
   bucket[tid] = 0;
+  if (tid == 0) cut_count = 0;
   int before = 0;
   for (int base = 0; base < count; base += 1024) {
     const int b = base + tid;
@@ -96,9 +110,9 @@ plan_kernel(const Params p) {
     if (b < count) p.prefix[b] = mine;
     before += all;
   }
-  const int total = min(before, p.capacity);
+  const int total = min(before, p.capacity - p.cut_capacity);
   __syncthreads();
-  auto describe = [&](int t, int4* tile, int* page) {
+  auto describe = [&](int t, int4* tile, int* page) {      // returns the tile's KV tiles
     int lo = 0, hi = count;                      // largest b with prefix[b] <= t
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
@@ -116,23 +130,63 @@ plan_kernel(const Params p) {
     }
     *tile = make_int4(qs + i, min(per, qe - qs - i), i + 1 + kv_len - (qe - qs), kv_len);
     const int last = min(kv_len, tile->z + tile->y - 1);
-    return kCostBuckets - 1 - min(kCostBuckets - 1, last > 0 ? (last + kTile - 1) / kTile : 0);
+    return last > 0 ? (last + kTile - 1) / kTile : 0;
   };
-  int4 tile;
-  int page;
-  for (int t = tid; t < total; t += 1024) atomicAdd(bucket + describe(t, &tile, &page), 1);
+  int4 tile, tile0;
+  int page, page0;
+  const int n0 = tid < total ? describe(tid, &tile0, &page0) : 0;      // the first 1024 tiles stay in registers
+  float share = 0;                               // KV tiles of the launch, over all heads, to an SM
+  if (p.cut_capacity) {
+    int mine = n0, all;
+    for (int t = tid + 1024; t < total; t += 1024) mine += describe(t, &tile, &page);
+    cta1024_exclusive_scan(mine, sums, all);
+    share = float(all) * float(p.hkv) / float(p.sms) * 1.0001f;        // (rounding may leave a piece out, never make one more)
+  }
+  auto size_of = [&](int n) {                    // KV tiles of a tile's pieces
+    if (share == 0.f || float(n) < 2.f * share) return n;
+    const int k = min(int(float(n) / share), n / kMinPiece), size = (n + k - 1) / k;
+    return n - size >= kMinGain ? size : n;
+  };
+  auto bucket_of = [&](int n) { return kCostBuckets - 1 - min(kCostBuckets - 1, n); };
+  auto count_tile = [&](int t, int n, const int4& tile) {
+    const int size = size_of(n), pieces = n > size ? (n + size - 1) / size : 1;
+    atomicAdd(bucket + bucket_of(size), pieces);
+    if (pieces > 1) {
+      const int at = atomicAdd(&cut_count, (1 << 16) + pieces), c = at >> 16;
+      cut_tile[c] = t; cut_first[c] = at & 0xffff; cut_size[c] = size;
+      p.cuts[2 * c] = tile;
+      p.cuts[2 * c + 1] = make_int4(at & 0xffff, pieces, 0, 0);
+    }
+  };
+  if (tid < total) count_tile(tid, n0, tile0);
+  for (int t = tid + 1024; t < total; t += 1024) { const int n = describe(t, &tile, &page); count_tile(t, n, tile); }
   __syncthreads();
   int all;
   const int mine = bucket[tid];
   const int start = cta1024_exclusive_scan(mine, sums, all);
   bucket[tid] = start;
   __syncthreads();
-  for (int t = tid; t < total; t += 1024) {
-    const int at = atomicAdd(bucket + describe(t, &tile, &page), 1);
+  auto list_tile = [&](int n, const int4& tile, int page) {
+    if (size_of(n) < n) return;
+    const int at = atomicAdd(bucket + bucket_of(n), 1);
     p.tiles[at] = tile;
-    p.tile_page[at] = page;
+    p.spans[at] = make_int4(page, 0, n, -1);
+  };
+  if (tid < total) list_tile(n0, tile0, page0);
+  for (int t = tid + 1024; t < total; t += 1024) { const int n = describe(t, &tile, &page); list_tile(n, tile, page); }
+  const int cuts = cut_count >> 16, pieces = cut_count & 0xffff;
+  for (int e = tid; e < pieces; e += 1024) {     // the pieces of the cut tiles, a thread each
+    int lo = 0, hi = cuts;                       // largest c with cut_first[c] <= e
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (cut_first[mid] <= e) lo = mid; else hi = mid;
+    }
+    const int n = describe(cut_tile[lo], &tile, &page), size = cut_size[lo], first = (e - cut_first[lo]) * size;
+    const int at = atomicAdd(bucket + bucket_of(size), 1);
+    p.tiles[at] = tile;
+    p.spans[at] = make_int4(page, first, min(n, first + size), e);
   }
-  if (tid == 0) { *p.tile_count = total; *p.status = 0; }
+  if (tid == 0) { p.tile_count[0] = all; p.tile_count[1] = cuts; *p.status = 0; }
 }
 
 __device__ __forceinline__ float ex2(float x) {
@@ -157,10 +211,12 @@ __device__ __forceinline__ uint32_t row_off(int row, int chunk) {
 // One unit of work as every role reads it from the list.
 struct Work {
   int q0, rows, first_visible, kv_len, page_base, kvh;
-  int n_kv[2], n;                                  // KV tiles each query tile sees; the larger of the two
+  int begin, slot;                                 // first KV tile; where a piece of a cut tile leaves its result (-1: whole)
+  int n_kv[2], n;                                  // KV tiles of it that each query tile sees; the larger of the two
 };
 // The k-th unit of this CTA, false past the end.  CTA c takes entries c, 2g-1-c, 2g+c, ... of the (tile, KV head) list, which
 // is sorted by length: turning round every other time evens out what a CTA gets.
+template <bool CUT>
 __device__ __forceinline__ bool get_work(const Params& p, int units, int k, Work* w) {
   const int g = gridDim.x;
   const int u = k * g + ((k & 1) ? g - 1 - int(blockIdx.x) : int(blockIdx.x));
@@ -168,7 +224,10 @@ __device__ __forceinline__ bool get_work(const Params& p, int units, int k, Work
   const int index = u / p.hkv;
   w->kvh = u - index * p.hkv;
   const int4 tile = __ldg(p.tiles + index);
-  w->page_base = __ldg(p.tile_page + index);
+  int4 span = make_int4(0, 0, INT_MAX, -1);
+  if (CUT) span = __ldg(p.spans + index);
+  else span.x = __ldg(&p.spans[index].x);
+  w->page_base = span.x; w->begin = span.y; w->slot = span.w;
   w->q0 = tile.x; w->rows = tile.y; w->first_visible = tile.z; w->kv_len = tile.w;
   const int per_half = kRows / p.group;
 #pragma unroll
@@ -176,6 +235,7 @@ __device__ __forceinline__ bool get_work(const Params& p, int units, int k, Work
     const int mine = min(w->rows - x * per_half, per_half);
     const int last = mine > 0 ? min(w->kv_len, w->first_visible + x * per_half + mine - 1) : 0;
     w->n_kv[x] = last > 0 ? (last + kTile - 1) / kTile : 0;
+    if (CUT) w->n_kv[x] = max(0, min(span.z, w->n_kv[x]) - span.y);
   }
   w->n = max(w->n_kv[0], w->n_kv[1]);
   return true;
@@ -183,10 +243,10 @@ __device__ __forceinline__ bool get_work(const Params& p, int units, int k, Work
 
 // The tensor core multiplies every V row of a tile with a weight, the masked ones with 0, and 0 times an infinity or a NaN is
 // NaN.  For a row whose O is not finite this looks at the V rows that its tiles hold and it does not see, [visible, loaded),
-// and where one of them is not finite, writes the row again from the KV rows that it does see, with the same maximum.  By a whole
-// warp: lane i has dims [4 i, 4 i + 4).  Rare, and out of line for the registers of the loop.
-static __device__ __noinline__ void without_masked_rows(const Params& p, int q_row, int head, int kvh, int page_base, int visible, int loaded,
-                                                        float scale2, float m, float by) {
+// and where one of them is not finite, writes the row again from the KV rows that it does see, [begin, visible), with the same maximum
+// (to `part` where it is a piece's).  By a whole warp: lane i has dims [4 i, 4 i + 4).  Rare, and out of line for the registers of the loop.
+static __device__ __noinline__ void without_masked_rows(const Params& p, int q_row, int head, int kvh, int page_base, int begin, int visible, int loaded,
+                                                        float scale2, float m, float by, float* part) {
   const int lane = threadIdx.x & 31;
   auto row4 = [&](const __nv_bfloat16* rows, size_t row) {
     const uint2 raw = __ldg(reinterpret_cast<const uint2*>(rows + row * kD) + lane);
@@ -204,16 +264,48 @@ static __device__ __noinline__ void without_masked_rows(const Params& p, int q_r
   if (!__any_sync(0xffffffffu, spread != spread)) return;
   const float4 q = row4(p.q, size_t(q_row) * p.hq + head);
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int t = 0; t < visible; ++t) {
+  for (int t = begin; t < visible; ++t) {
     const size_t at = kv_row(t);
     const float4 k = row4(p.k, at), v = row4(p.v, at);
     const float w = ex2(fmaf(warp_sum(q.x * k.x + q.y * k.y + q.z * k.z + q.w * k.w), scale2, -m));
     o.x = fmaf(w, v.x, o.x); o.y = fmaf(w, v.y, o.y); o.z = fmaf(w, v.z, o.z); o.w = fmaf(w, v.w, o.w);
   }
-  reinterpret_cast<uint2*>(p.out + (size_t(q_row) * p.hq + head) * kD)[lane] = make_uint2(pack_bf16x2(o.x * by, o.y * by), pack_bf16x2(o.z * by, o.w * by));
+  if (part) reinterpret_cast<float4*>(part)[lane] = make_float4(o.x * by, o.y * by, o.z * by, o.w * by);
+  else reinterpret_cast<uint2*>(p.out + (size_t(q_row) * p.hq + head) * kD)[lane] = make_uint2(pack_bf16x2(o.x * by, o.y * by), pack_bf16x2(o.z * by, o.w * by));
 }
 
-static __global__ void __launch_bounds__(kThreads, 1)
+// The sum of 32 values on top of a pair of sums: not finite once a value is not.
+__device__ __forceinline__ uint64_t sum_32(const float (&o)[32], uint64_t sum) {
+  uint64_t s[4] = {sum, 0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < 16; ++i) s[i & 3] = add_f32x2(s[i & 3], pack_f32x2(o[2 * i], o[2 * i + 1]));
+  return add_f32x2(add_f32x2(s[0], s[1]), add_f32x2(s[2], s[3]));
+}
+
+// The rows of a cut tile's piece, each lane its own (null: no such row); returns the sum as sum_32 does.  Out of line: most units are whole.
+static __device__ __noinline__ uint64_t write_part(uint32_t o_col, int tiles, float* part, float inv) {
+  uint64_t sum = 0;
+#pragma unroll 1
+  for (int c = 0; c < kD; c += 32) {
+    float o[32];
+    if (tiles > 0) {
+      tmem_ld_32x32b_x32(o_col + c, o);
+      tcgen05_wait_ld();
+    }
+    sum = sum_32(o, sum);
+    if (part) {
+#pragma unroll
+      for (int i = 0; i < 32; i += 4)
+        *reinterpret_cast<float4*>(part + c + i) = inv == 0.f ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
+    }
+    __syncwarp();
+  }
+  return sum;
+}
+
+// CUT: some tiles may be cut.
+template <bool CUT>
+__global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -274,7 +366,7 @@ prefill_kernel(const __grid_constant__ Params p) {
           fence_proxy_async_smem();                // the rows were written through the generic proxy
           tcgen05_fence_after();
         };
-        for (int k = 0; ok && get_work(p, units, k, &w); ++k) {
+        for (int k = 0; ok && get_work<CUT>(p, units, k, &w); ++k) {
           if (w.n == 0) continue;
           k_ready(it);
 #pragma unroll 1
@@ -335,11 +427,11 @@ prefill_kernel(const __grid_constant__ Params p) {
       bool ok = true;
       uint32_t it = 0, loads[2] = {0, 0};
       Work w;
-      for (int k = 0; ok && get_work(p, units, k, &w); ++k) {
+      for (int k = 0; ok && get_work<CUT>(p, units, k, &w); ++k) {
         if (w.n == 0) continue;
         struct Lookup { int page, offset; };       // offset -1: no such token
         auto lookup = [&](int j) -> Lookup {
-          const int token = j * kTile + lw * 32 + lane;
+          const int token = (w.begin + j) * kTile + lw * 32 + lane;
           if (token >= w.kv_len) return {0, -1};
           if (!p.kv_indices) return {0, w.page_base + token};
           const int page = token / p.page_size;
@@ -405,9 +497,10 @@ prefill_kernel(const __grid_constant__ Params p) {
     bool ok = true;
     uint32_t done = 0;                             // KV tiles so far
     Work w;
-    for (int k = 0; ok && get_work(p, units, k, &w); ++k) {
+    for (int k = 0; ok && get_work<CUT>(p, units, k, &w); ++k) {
       const bool exists = slot && token < w.rows;
       const int visible = exists ? min(w.kv_len, w.first_visible + token) : 0;      // KV rows this row sees
+      const int seen = visible - w.begin * kTile;  // of the unit's
       const int tiles = x ? w.n_kv[1] : w.n_kv[0];
       float m_ref = -INFINITY, l = 0.f;
       for (int j = 0; j < tiles; ++j, ++done) {
@@ -416,7 +509,7 @@ prefill_kernel(const __grid_constant__ Params p) {
         tcgen05_fence_after();
         // The logits are read twice, once for the maximum and once for the weights, 32 columns at a time: all 128 in
         // registers spill.  P of 32 KV rows (16 columns of values, 16 of residuals) goes over the logits it comes from.
-        const int limit = visible - j * kTile;     // columns at and past it are masked
+        const int limit = seen - j * kTile;        // columns at and past it are masked
         const bool plain = !__any_sync(0xffffffffu, limit < kTile) && scale_positive;
         float t4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -498,16 +591,23 @@ prefill_kernel(const __grid_constant__ Params p) {
       if (!ok) break;
       tcgen05_fence_after();
       // A sum that is NaN (a NaN, or infinities that met, in what the row sees) goes on as one.  A row that sees KV rows has a
-      // weight of at least 2^-8, unless every logit is -inf: 0 / 0, as in the decode form.  Else a zero sum means that it sees nothing.
-      if (visible > 0 && l == 0.f) l = __int_as_float(0x7fc00000);
+      // weight of at least 2^-8, unless every logit is -inf: 0 / 0, as in the decode form.  Else a zero sum means that it sees nothing (of this piece).
+      if (visible > 0 && l == 0.f && w.slot < 0) l = __int_as_float(0x7fc00000);
       // rows leave through shared memory, 128 bytes of a row at a time
       const float inv = l == 0.f ? 0.f : 1.f / l;
       const bool nan = p.nan_for_masked && w.kv_len > 0 && visible <= 0;
-      const int loaded = min(w.kv_len, tiles * kTile);       // KV rows in the row's products
-      const bool some_masked = visible > 0 && visible < loaded;
-      float spread = 0.f;                          // NaN once an element of O is not finite
+      float* part = nullptr;                       // where the row of a cut tile's piece goes
+      if (CUT && w.slot >= 0) {
+        const size_t row = (size_t(w.slot) * p.hkv + w.kvh) * p.part_rows + x * kRows + r;
+        part = p.part_o + row * kD;
+        if (exists) p.part_lse[row] = l == 0.f ? -INFINITY : m_ref + log2f(l);
+      } else if (exists) {
+        p.lse[size_t(w.q0 + token) * p.hq + w.kvh * p.group + head_in_group] = l == 0.f ? -INFINITY : m_ref + log2f(l);
+      }
+      uint64_t sum = 0;                            // of the row's O, as a pair: not finite once an element is not
+      if (CUT && part) sum = write_part(o_col, tiles, exists ? part : nullptr, inv);
 #pragma unroll 1
-      for (int h = 0; h < kD; h += 64) {
+      for (int h = CUT && part ? kD : 0; h < kD; h += 64) {
 #pragma unroll
         for (int c = 0; c < 64; c += 32) {
           float o[32];
@@ -515,10 +615,7 @@ prefill_kernel(const __grid_constant__ Params p) {
             tmem_ld_32x32b_x32(o_col + h + c, o);
             tcgen05_wait_ld();
           }
-          if (some_masked) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) spread = fmaf(o[i], 0.f, spread);
-          }
+          sum = sum_32(o, sum);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             uint4 v;
@@ -546,14 +643,16 @@ prefill_kernel(const __grid_constant__ Params p) {
         }
         __syncwarp();
       }
-      uint32_t again = __ballot_sync(0xffffffffu, spread != spread && l == l);
+      const int loaded = min(w.kv_len, (w.begin + tiles) * kTile);      // KV row behind the last in the row's products
+      float sum_a, sum_b;
+      unpack_f32x2(sum, sum_a, sum_b);
+      uint32_t again = __ballot_sync(0xffffffffu, seen > 0 && visible < loaded && l == l && !(fabsf(sum_a + sum_b) <= 3.4e38f));
       while (again) {                              // (the row's first result has been written, by this warp)
         const int src = __ffs(again) - 1, row_r = quad * 32 + src, q_row = w.q0 + x * per_half + row_r / p.group, head = w.kvh * p.group + row_r % p.group;
         again &= again - 1;
-        without_masked_rows(p, q_row, head, w.kvh, w.page_base, __shfl_sync(0xffffffffu, visible, src), loaded, scale2,
-                            __shfl_sync(0xffffffffu, m_ref, src), __shfl_sync(0xffffffffu, inv, src));
+        without_masked_rows(p, q_row, head, w.kvh, w.page_base, w.begin * kTile, __shfl_sync(0xffffffffu, visible, src), loaded, scale2,
+                            __shfl_sync(0xffffffffu, m_ref, src), __shfl_sync(0xffffffffu, inv, src), part ? part + (src - lane) * kD : nullptr);
       }
-      if (exists) p.lse[size_t(w.q0 + token) * p.hq + w.kvh * p.group + head_in_group] = l == 0.f ? -INFINITY : m_ref + log2f(l);
     }
   }
 
@@ -566,6 +665,60 @@ prefill_kernel(const __grid_constant__ Params p) {
   if (warp == 0) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, kTmemColumns);
+  }
+}
+
+// Puts the pieces of cut tiles together: a warp to a row of a (tile, KV head), four dims to a lane, the results of four pieces in flight.
+constexpr int kMergeWarps = 8;
+static __global__ void __launch_bounds__(kMergeWarps * 32)
+merge_kernel(const Params p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int lane = threadIdx.x & 31, per_half = kRows / p.group;
+  const int rows = p.tile_count[1] * p.hkv * p.part_rows;       // <= (sms / Hkv) Hkv 256
+  for (int i = blockIdx.x * kMergeWarps + (threadIdx.x >> 5); i < rows; i += gridDim.x * kMergeWarps) {
+    const int row = i % p.part_rows, kvh = i / p.part_rows % p.hkv, cut = i / p.part_rows / p.hkv;
+    const int4 tile = p.cuts[2 * cut], pieces = p.cuts[2 * cut + 1];
+    const int r = row % kRows, token = row / kRows * per_half + r / p.group;
+    if (r >= per_half * p.group || token >= tile.y) continue;
+    const size_t first = (size_t(pieces.x) * p.hkv + kvh) * p.part_rows + row, stride = size_t(p.hkv) * p.part_rows;
+    float mm = -INFINITY, weight = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k0 = 0; k0 < pieces.y; k0 += 4) {
+      float ls[4];
+      float4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const size_t at = first + size_t(min(k0 + k, pieces.y - 1)) * stride;
+        ls[k] = k0 + k < pieces.y ? __ldcg(p.part_lse + at) : -INFINITY;
+        v[k] = __ldcg(reinterpret_cast<const float4*>(p.part_o + at * kD) + lane);
+      }
+      const float m_new = fmaxf(fmaxf(fmaxf(ls[0], ls[1]), fmaxf(ls[2], ls[3])), mm);
+      const float rescale = mm == m_new ? 1.f : exp2f(mm - m_new);
+      mm = m_new;
+      weight *= rescale;
+      acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float w = ls[k] == -INFINITY ? 0.f : exp2f(ls[k] - mm);      // -inf: the row sees nothing of the piece; NaN goes on as one
+        weight += w;
+        acc.x = fmaf(w, v[k].x, acc.x); acc.y = fmaf(w, v[k].y, acc.y); acc.z = fmaf(w, v[k].z, acc.z); acc.w = fmaf(w, v[k].w, acc.w);
+      }
+    }
+    const size_t out_row = size_t(tile.x + token) * p.hq + kvh * p.group + r % p.group;
+    const bool sees = min(tile.w, tile.z + token) > 0;
+    uint2 packed = make_uint2(0u, 0u);
+    float lse = -INFINITY;
+    if (weight != 0.f) {
+      const float inv = 1.f / weight;
+      packed = make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
+      lse = mm + log2f(weight);
+    } else if (sees || (p.nan_for_masked && tile.w > 0)) {                 // every logit is -inf; or the row sees nothing
+      packed = make_uint2(0x7fc07fc0u, 0x7fc07fc0u);
+      if (sees) lse = __int_as_float(0x7fc00000);
+    }
+    reinterpret_cast<uint2*>(p.out + out_row * kD)[lane] = packed;
+    if (lane == 0) p.lse[out_row] = lse;
   }
 }
 

@@ -41,6 +41,10 @@ def problem(seed, q_lens, kv_lens, heads, kv_heads, page):
     ([26, 51], [26, 385], 5, 1, 16, True), ([21, 43], [400, 43], 6, 1, 0, True), ([19, 37], [129, 700], 14, 2, 16, False),
     ([16, 33], [513, 64], 16, 2, 16, True),                       # G = 8
     ([2, 1], [6000, 4097], 8, 1, 16, True),                       # one decode sequence per query row
+    # tiles that are cut into pieces of KV tiles: rows that see every piece and the first ones only, few rows, rows that see nothing
+    ([64], [3000], 8, 2, 16, False), ([40, 3, 0], [2500, 900, 0], 16, 2, 5, True), ([5], [1300], 64, 8, 64, False),
+    ([130, 20, 200], [100, 2000, 300], 4, 4, 0, True), ([300, 7, 64], [290, 1025, 1024], 8, 1, 0, True), ([70], [4000], 3, 3, 16, True),
+    ([900], [800], 4, 2, 0, True),                                # pieces of which some rows see nothing
 ])
 def test_tile_edges(q_lens, kv_lens, heads, kv_heads, page, nan):
     cpu = problem(len(q_lens) * 100 + heads, q_lens, kv_lens, heads, kv_heads, page)
