@@ -1,4 +1,4 @@
-// RMSNorm for sm_100a: one CTA per row (one warp up to 2048 elements), the row held in registers between
+// RMSNorm for sm_100a: one CTA per row (one warp for narrow rows), the row held in registers between
 // the reduction and the scaling, 128-bit loads and stores, fp32 arithmetic, one bf16 rounding of the result.
 //
 // Operators:
@@ -156,7 +156,7 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
   }
 }
 
-// Narrow rows (at most 2048 elements): one warp per row, four rows to a CTA, no barrier; a row's vectors are all in flight
+// Narrow rows (at most 2048 elements, see choose_shape): one warp per row, four rows to a CTA, no barrier; a row's vectors are all in flight
 // at once.  A CTA per row leaves most of its threads without a vector (64 of 256 at 512 columns).
 template <int VPL, int MODE>
 __global__ void __launch_bounds__(128)
@@ -225,10 +225,14 @@ struct Handle {
 
 inline void choose_shape(Handle* h, int device) {
   const int vectors = h->width / 8;
-  // shape class: 0 = a warp per row; 1..4 = 512 threads x 1, 2, 4, 8 vectors
-  h->vpt = vectors <= 256 ? 0 : vectors <= 512 ? 1 : vectors <= 1024 ? 2 : vectors <= 2048 ? 3 : 4;
+  // Shape class: 0 = a warp per row; 1..4 = 512 threads x 1, 2, 4, 8 vectors; 5 = 256 threads x 1.  A warp with eight vectors to a lane has
+  // too few rows in flight where a row brings little else: x alone above 1024 elements (4096 x 2048, from HBM: 14.4 us as warps, 12.4
+  // as CTAs; 4096 x 1032 12.3, 10.8), the two-output form above 1536 (8192 x 2048 30.7, 28.8).  With the residual the warps stay ahead
+  // up to 2048 (8192 x 1536 17.2 to 19.9, 18.8 to 20.9), since its loads do not wait for the row before.
+  const bool as_ctas = vectors <= 256 && vectors > (h->residual_out ? 192 : h->residual ? 256 : 128);
+  h->vpt = as_ctas ? 5 : vectors <= 256 ? 0 : vectors <= 512 ? 1 : vectors <= 1024 ? 2 : vectors <= 2048 ? 3 : 4;
   // persistent CTAs: as many as are resident at once, each walking rows with a stride of the grid
-  const int resident = sm_count(device) * (h->vpt == 1 ? 3 : h->vpt == 2 ? 2 : 1);
+  const int resident = sm_count(device) * (h->vpt == 5 ? 6 : h->vpt == 1 ? 3 : h->vpt == 2 ? 2 : 1);
   if (h->vpt == 0) h->grid = (h->rows + 3) / 4;
   else h->grid = h->rows < 1 ? 1 : (h->rows < resident ? h->rows : resident);
 }
@@ -290,6 +294,7 @@ static int rmsnorm_launch_any(void* handle, void* cuda_stream) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(cuda_stream);
   switch (h->vpt) {
     case 0: return h->width <= 512 ? launch_warps<2>(h, stream) : h->width <= 1024 ? launch_warps<4>(h, stream) : launch_warps<8>(h, stream);
+    case 5: return launch<256, 1>(h, stream);
     case 1: return launch<512, 1>(h, stream);
     case 2: return launch<512, 2>(h, stream);
     case 3: return launch<512, 4>(h, stream);

@@ -6,7 +6,7 @@ import torch
 
 import open_cake_ir_b200 as cake
 from gpu_util import poison, snapshot, unchanged
-from oracle import compare, rmsnorm
+from oracle import add_rmsnorm, compare, rmsnorm
 
 pytestmark = pytest.mark.gpu
 ATOL, RTOL = 2.0 ** -16, 2.0 ** -7
@@ -42,6 +42,31 @@ def test_serving_and_edge_shapes(rows, width):
     torch.cuda.synchronize()
     guard()
     ok, bad, err = compare.compare(out, want, atol=ATOL, rtol=RTOL)
+    assert ok, f"{bad} mismatches, max abs err {err}"
+
+
+@pytest.mark.parametrize("form", ["plain", "residual", "add"])
+@pytest.mark.parametrize("width", [1024, 1032, 1536, 1544, 2048, 2056])        # where rows go from warps to CTAs
+@pytest.mark.parametrize("rows", [1, 2000])                                    # more rows than CTAs
+def test_either_side_of_the_narrow_rows(form, width, rows):
+    g = torch.Generator().manual_seed(rows + width)
+    x, residual = (torch.randn((rows, width), generator=g).to(torch.bfloat16) for _ in range(2))
+    weight = (1 + 0.1 * torch.randn(width, generator=g)).to(torch.bfloat16)
+    out, guard = poison((rows, width), torch.bfloat16)
+    if form == "add":
+        total, guard2 = poison((rows, width), torch.bfloat16)
+        cake.AddRmsNorm(x.cuda(), residual.cuda(), weight.cuda(), out, total, 1e-6).launch()
+        want = add_rmsnorm.add_rmsnorm_reference(x, residual, weight, 1e-6)
+        want_out, want_total = want["out"], want["residual_out"]
+        torch.cuda.synchronize()
+        guard2()
+        assert torch.equal(total.cpu().view(torch.int16), want_total.view(torch.int16))
+    else:
+        cake.RmsNorm(x.cuda(), weight.cuda(), out, 1e-6, residual.cuda() if form == "residual" else None).launch()
+        want_out = rmsnorm.rmsnorm_reference(x, weight, 1e-6, residual if form == "residual" else None)
+        torch.cuda.synchronize()
+    guard()
+    ok, bad, err = compare.compare(out, want_out, atol=ATOL, rtol=RTOL)
     assert ok, f"{bad} mismatches, max abs err {err}"
 
 
