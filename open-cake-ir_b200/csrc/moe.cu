@@ -195,7 +195,7 @@ __device__ __forceinline__ void gather_row(const Gather& g, int pair, int pos) {
 // CTA that it concerns counts all experts' rows to find out; an expert of the core's has its rows gathered here, by its CTA.
 constexpr int kPlaceWarps = 8;
 constexpr int kPlaceStep = 256;      // pairs one warp looks at per step
-__global__ void __launch_bounds__(kPlaceWarps * 32)
+__global__ void __launch_bounds__(kPlaceWarps * 32, 8)
 place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_ptr, int* __restrict__ counts,
              int* __restrict__ offsets, int* __restrict__ sorted_pairs, int* __restrict__ inv_perm, int pairs, int local_experts,
              int* __restrict__ clear, int clear_words, const Gather gather) {
@@ -219,8 +219,8 @@ place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_
     }
 #pragma unroll
     for (int i = 0; i < kPlaceStep / 32; ++i) {
-      count += __popc(__ballot_sync(0xffffffffu, ids[i] == want));
-      before += __popc(__ballot_sync(0xffffffffu, ids[i] >= offset && ids[i] < want));
+      count += ids[i] == want;                                // of this lane: added up once, a vote per 32 pairs takes longer
+      before += uint32_t(ids[i] - offset) < uint32_t(e);
     }
     if ((base / kPlaceStep) % local_experts == e) {
 #pragma unroll
@@ -230,6 +230,8 @@ place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_
       }
     }
   }
+  count = __reduce_add_sync(0xffffffffu, count);
+  before = __reduce_add_sync(0xffffffffu, before);
   if (lane == 0) { warp_count[warp] = count; warp_before[warp] = before; }
   __syncthreads();
   int first = 0, total = 0, cursor = 0;
