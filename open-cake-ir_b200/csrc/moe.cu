@@ -191,11 +191,12 @@ __device__ __forceinline__ void gather_row(const Gather& g, int pair, int pos) {
 // pass places the pairs by ballot rank -- ascending pair order inside the expert, so the permutation is the stable sort
 // by expert.  Eight loads per lane are in flight per step.  Pairs of other ranks get inv_perm -1 (each step's by one CTA).
 // `clear` (may be null): `clear_words` counters of the kernels that follow.  `gather.above` > 0 (a layer on the weight-streaming kernel): the
-// experts of many rows go to the tcgen05 core where the weights that they would have streamed again are worth its launches.  Every
-// CTA that it concerns counts all experts' rows to find out; an expert of the core's has its rows gathered here, by its CTA.
+// experts of many rows go to the tcgen05 core where the weights that they would have streamed again are worth its launches.  The CTA of
+// such an expert counts all experts' rows to find out and, if so, gathers its own here.  `gather.core` says how that came out, and is
+// written only where there is such an expert: where there is none nothing hangs on it.
 constexpr int kPlaceWarps = 8;
 constexpr int kPlaceStep = 256;      // pairs one warp looks at per step
-__global__ void __launch_bounds__(kPlaceWarps * 32, 8)
+__global__ void __launch_bounds__(kPlaceWarps * 32)
 place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_ptr, int* __restrict__ counts,
              int* __restrict__ offsets, int* __restrict__ sorted_pairs, int* __restrict__ inv_perm, int pairs, int local_experts,
              int* __restrict__ clear, int clear_words, const Gather gather) {
@@ -266,7 +267,7 @@ place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_
       cursor += __popc(mask);
     }
   }
-  if (gather.above == 0 || (e != 0 && total <= gather.above)) return;
+  if (gather.above == 0 || total <= gather.above) return;
   for (int g = threadIdx.x; g < local_experts; g += kPlaceWarps * 32) rows_of[g] = 0;
   if (threadIdx.x == 0) streamed_again = 0;
   __syncthreads();                             // (the expert's pairs are placed, too)
@@ -279,8 +280,8 @@ place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_
     if (rows_of[g] > gather.above) atomicAdd(&streamed_again, (rows_of[g] - 1) / gather.item_rows);
   __syncthreads();
   const bool core = streamed_again >= kCorePays;
-  if (e == 0 && threadIdx.x == 0) *gather.core = core;
-  if (!core || total <= gather.above) return;
+  if (threadIdx.x == 0) *gather.core = core;   // (the same from each of these CTAs)
+  if (!core) return;
   for (int pos = first + warp; pos < first + total; pos += kPlaceWarps) gather_row(gather, sorted_pairs[pos], pos);
 }
 
@@ -346,9 +347,10 @@ gather_kernel(const int* __restrict__ sorted_pairs, const int* __restrict__ offs
 // owns eight columns of a token; the rows of eight slots are asked for before the first is added.
 __global__ void __launch_bounds__(256)
 combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ inv_perm, __nv_bfloat16* __restrict__ out,
-               int hidden_width, int top_k, int parts) {
+               int hidden_width, int top_k, int parts, int* __restrict__ core) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (core && blockIdx.x == 0 && threadIdx.x == 0) *core = 0;       // the next step's core kernels leave at once again
   const int token = blockIdx.x / parts, c = ((blockIdx.x % parts) * 256 + threadIdx.x) * 8;
   if (c >= hidden_width) return;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -433,6 +435,7 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
   const size_t pairs = size_t(c.tokens) * c.top_k;
   l.capacity = int(pairs < 1 ? 1 : pairs);
   l.terms = c.act_mode == 1 ? 2 : 1;
+  constexpr int sms = 148;               // of a B200: the layout is asked for before there is a device, and create has to find the same
   size_t at = 0;
   auto take = [&](size_t bytes) { size_t here = at; at += align_up(bytes); return here; };
   l.status = take(256);
@@ -458,10 +461,10 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
   double missed = 1;                     // experts that get a row: those not missed by every token
   for (int64_t t = 0; t < c.tokens && missed > 1e-3; ++t) missed *= 1.0 - double(c.top_k) / c.experts;
   const double touched = c.local_experts * (1 - missed);
-  if (per_expert <= (touched * (c.intermediate / 128) < 148 ? 11.0 : 7.5)) {
+  if (per_expert <= (touched * (c.intermediate / 128) < sms ? 11.0 : 7.5)) {
     l.token_tiles = skinny::token_tiles(per_expert);
-    l.split1 = skinny::choose_split_gate_up(touched > 1 ? touched : 1, c.intermediate, c.hidden / 128, 148);
-    l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128, 148);
+    l.split1 = skinny::choose_split_gate_up(touched > 1 ? touched : 1, c.intermediate, c.hidden / 128, sms);
+    l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128, sms);
     if (l.split1 > 1) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation
     // The routing may be anything but even: the padding of a batch, or a batch of one prompt, goes to the same top_k experts.  The
     // weight-streaming kernel then reads their weights once per item of 8 token_tiles rows, so experts of many rows (four times the
@@ -744,7 +747,7 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
         if (int rc = moe::launch_routing(h->logits, h->bias, h->factor, h->expert_ids, h->route_weights, tokens, c.experts, c.top_k,
                                          c.n_group, c.topk_group, c.routing_mode, s))
           return rc;
-      if (int rc = moe::launch_permute(pa, s, clear, 64, gather)) return rc;
+      if (int rc = moe::launch_permute(pa, s, clear, kCoreWord, gather)) return rc;
       if (l.token_tiles) return 0;
       const int gather_blocks = (l.capacity + 7) / 8;
       return launch_dependent(moe::gather_kernel, dim3(gather_blocks < 4096 ? gather_blocks : 4096), dim3(256), 0, s, pa.sorted_pairs, pa.offsets,
@@ -780,7 +783,8 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
       if (reinterpret_cast<uintptr_t>(h->output) & 15) return kErrBadArgument;      // rows leave 16 bytes at a time
       const int parts = (c.hidden + 2047) / 2048;
       return launch_dependent(moe::combine_kernel, dim3(unsigned(tokens) * parts), dim3(256), 0, s, reinterpret_cast<const __nv_bfloat16*>(h->ws + l.y),
-                              pa.inv_perm, h->output, c.hidden, c.top_k, parts);
+                              pa.inv_perm, h->output, c.hidden, c.top_k, parts,
+                              l.core_above ? reinterpret_cast<int*>(h->ws + l.status) + kCoreWord : static_cast<int*>(nullptr));
     }
     default:
       return kErrBadArgument;
