@@ -8,7 +8,7 @@ import pytest
 import torch
 
 import open_cake_ir_b200 as cake
-from oracle import compare, moe as oracle_moe
+from oracle import compare, moe as oracle_moe, routing as oracle_routing
 from test_gpu_moe import run_layer
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +65,22 @@ def test_uneven_routing(tokens, equal, offset, act):
     out, _ = run_layer(cpu, experts=64, routing="softmax", act_mode=act)
     want = oracle_moe.moe_reference(cpu, routing="softmax", act_quant="fp8" if act == "fp8" else "none", dtype=torch.float32)
     assert compare.rel_frobenius(out, want["output"]) <= (1e-2 if act == "fp8" else 4e-3)
+
+
+@pytest.mark.parametrize("tokens,hidden,inter,experts,local,offset,act", [
+    (5, 1024, 256, 64, 16, 16, "fp8"),           # K split over warps, quantisation in a kernel of its own
+    (40, 512, 256, 64, 64, 0, "split"),          # one warp to a sub-tile; no pairs of other ranks
+    (40, 512, 256, 64, 16, 32, "fp8")])
+def test_external_routing_at_few_rows(tokens, hidden, inter, experts, local, offset, act):
+    """Selections and weights from outside, as an expert-parallel step hands them over: some of other ranks, some rows absent (-1)."""
+    cpu = cake.workloads.moe_inputs(tokens, hidden, inter, experts, local, offset, routing="softmax", device="cpu")
+    ids, weights = oracle_routing.routing_softmax_topk(cpu["routing_logits"])
+    ids, weights = ids.int(), weights.float() * 2.5
+    absent = torch.arange(tokens) % 5 == 4
+    ids[absent] = -1
+    inputs = {k: v for k, v in cpu.items() if k not in ("routing_logits", "routing_bias")}
+    out, _ = run_layer(dict(inputs, expert_ids=ids, route_weights=weights), experts=experts, act_mode=act, external_routing=True)
+    want = oracle_moe.moe_reference(dict(cpu, routed_scaling_factor=torch.tensor([2.5])), routing="softmax", act_quant="fp8" if act == "fp8" else "none",
+                                    dtype=torch.float32)["output"]
+    assert not bool(out[absent.cuda()].any())
+    assert compare.rel_frobenius(out[~absent.cuda()], want[~absent]) <= (1e-2 if act == "fp8" else 4e-3)
