@@ -68,13 +68,17 @@ int cake_b200_read_status(const void* workspace, void* cuda_stream, int* status_
 int cake_b200_launch_facts(const char* kernel, int* threads_per_cta, int* dynamic_shared_bytes);
 
 /* For tests of the failure path only; never needed by a caller.  Every device-side wait of the tensor-core kernels
- * (block-scaled GEMM, MoE grouped GEMMs, MLA decode) is bounded; these hooks let a test make one run out
+ * (block-scaled GEMM, MoE grouped GEMMs, MLA attention, GQA prefill tiles) is bounded; these hooks let a test make one run out
  * without hanging or faulting anything: `wait_budget_kiloclocks` > 0 shortens the budget of every wait of later
  * launches to that many x 1024 SM clocks (0 restores the default of about a second), and `skip_load` != 0 makes
- * a later dense-GEMM launch (its first CTA) or MLA-decode launch (every CTA with three tiles or more) leave one
- * operand load out, so that the consumer's wait runs out, the kernel unwinds and returns, and the status word is
+ * a later launch of the dense GEMM or the GQA prefill tiles (its first CTA) or of the MLA kernel (every CTA with three
+ * tiles or more) leave one operand load out, so that the consumer's wait runs out, the kernel unwinds and returns, and the status word is
  * set.  Process-wide host state. */
 int cake_b200_test_hooks(int wait_budget_kiloclocks, int skip_load);
+
+/* Test accessor: the gate function of the MoE layer, x * sigmoid(x), as its kernels compute it (y), and with the compiler's
+ * division in place of theirs (by_division), for n fp32 values on the device. */
+int cake_b200_test_silu(const void* x, void* y, void* by_division, int64_t n, void* cuda_stream);
 
 /* Test accessor: where the plan kernel of a decode handle (kind "gqa_decode" or "mla_decode", the handle of the
  * matching _create) leaves the work plan of its latest launch, as a device pointer into the caller's workspace.

@@ -409,12 +409,6 @@ __device__ __forceinline__ void tcgen05_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 // 32 lanes x 16 consecutive 32-bit columns, registers -> tensor memory.
-__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-      : "memory");
-}
 __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -423,20 +417,6 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
-// 32 lanes x 32 consecutive 32-bit columns, registers -> tensor memory.
-__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const float* v) {
-  const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-
 // 32 lanes x 32 consecutive fp32 columns: thread i of the warp receives lane (base lane + i).
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, float* v) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);
@@ -619,9 +599,10 @@ __device__ __forceinline__ float2 e4m3x2_to_float2(uint16_t v) {
   const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(v, __NV_E4M3);
   return __half22float2(*reinterpret_cast<const __half2*>(&h));
 }
-// x * sigmoid(x).  The quotient is an approximate one, corrected once by what it leaves of x: the correction squares the
-// relative error of a couple of ulp, so that the last rounding is all that is left of it.  Unlike the `/` operator it has no
-// branch for the ends of the range, so that a thread's many values overlap: 64 of them, with `/` one after another, took
+// x * sigmoid(x).  The quotient is an approximate one, corrected once by its residual (a Newton step on the quotient, as in Markstein's
+// "IA-64 and Elementary Functions"): that squares the relative error of a couple of ulp, so that the last rounding is all that
+// is left of it; cake_b200_test_silu shows it beside the `/` operator, within an ulp.  Unlike `/` it has no branch for the ends
+// of the range, so that a thread's many values overlap: 64 of them, with `/` one after another, took
 // an epilogue of the MoE layer 5000 clocks.  The denominator stays below 2^126, where the approximation still holds:
 // below -87 the result is x * 1.6e-38 instead of something smaller yet.
 __device__ __forceinline__ float silu(float x) {

@@ -13,8 +13,9 @@
 //                                                    two instructions of N = 256 to which each CTA brings 128
 // The accumulators lie so that a CTA's 128 TMEM lanes are its 64 rows twice: lanes 0..63 hold the lower half of an
 // instruction's columns, lanes 64..127 the upper half, so O takes 256 columns and S 32.  In this form nothing is computed
-// twice and both operands come from shared memory at the arithmetic rate (25 clocks a step of S, 64 of O; a single CTA
-// takes 66 to 77 and 173 with A in shared memory).  One CTA per head block and half of the dims, the form before this one,
+// twice and both operands come from shared memory: 64 clocks a step of O, which is the arithmetic rate of M = 128, N = 256 on two
+// SMs, and 25 of S, where N = 64 would be worth 16 but the operand reads take longer (a single CTA takes 66 to 77 and 173 with A
+// in shared memory).  One CTA per head block and half of the dims, the form before this one,
 // repeated S and the softmax in both halves and had room for 32-token tiles only: 1770 clocks of tensor pipe per 32 tokens
 // on each of two SMs, against 1940 per 64 here.
 //
@@ -779,7 +780,7 @@ mla_decode_kernel(const __grid_constant__ Params p) {
 // pieces in flight (most sequences have two to four; eight in flight take registers from half of the resident rows).
 static __global__ void __launch_bounds__(256, 4)
 mla_reduce_kernel(const Params p) {
-  // launched as a programmatic dependent of the decode kernel: resident early, reads after it has completed
+  // launched as a programmatic dependent of the decode kernel, which never lets it in early: it starts as that one's CTAs leave
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (int(blockIdx.y) >= *p.cut_count) return;

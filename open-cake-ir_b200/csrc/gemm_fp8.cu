@@ -50,7 +50,7 @@ extern "C" int cake_b200_block_scaled_gemm_create(void** buffers, const cake_b20
   const int sms = sm_count(device), row_tiles = int((m + gemm::kBM - 1) / gemm::kBM);
   const int64_t narrow = row_tiles * (n / 128);
   h->split = 0;
-  for (int s = 4; s > 1 && !h->split; s >>= 1)
+  for (int s = gemm::kMaxSplit; s > 1 && !h->split; s >>= 1)
     if (narrow * s <= sms && k / gemm::kBK >= 4 * s) h->split = s;
   if (!rc) rc = make_tensor_map_u8_sw128(&h->map_b, buffers[2], uint64_t(n), uint64_t(k), h->split ? 128 : gemm::kBN);
   if (!rc) rc = int(cudaFuncSetAttribute(gemm::gemm_fp8_kernel<gemm::kDense>,

@@ -51,6 +51,7 @@ constexpr int kEpilogueRegs = 224;
 static_assert(kControlWarps * 32 * kControlRegs + kEpilogueWarps * 32 * kEpilogueRegs <= (65536 / kThreads / 8 * 8) * kThreads,
               "setmaxnreg budget exceeds the registers the launch allocates");
 constexpr int kMaxGroups = 512;
+constexpr int kMaxSplit = 4;      // CTAs that share a tile's K
 constexpr int kItemSlots = 4;
 // The scales of block it + kScaleAhead are announced with the operands of block it, so that the epilogue can read a
 // block's scales from shared memory while it still works on the block before.  A slot is refilled when the shared-memory
@@ -479,9 +480,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           for (int i = threadIdx.x - kControlWarps * 32; i < rows * chunks / 2; i += kEpilogueWarps * 32) {
             const int row_i = i % rows, c = i / rows * 2;
             const uint32_t from = smem_u32(sums + (int(rank) * chunks + c) * kBM + row_i);
-            float4 v[8][2];
+            float4 v[kMaxSplit][2];
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
+            for (int k = 0; k < kMaxSplit; ++k)
               if (k < int(split)) {
                 const uint32_t peer = (rank + k) & (split - 1);
                 v[k][0] = load_cluster(from, peer);
@@ -489,7 +490,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               }
             float4 sum[2] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
+            for (int k = 0; k < kMaxSplit; ++k)
               if (k < int(split))
 #pragma unroll
                 for (int h = 0; h < 2; ++h) { sum[h].x += v[k][h].x; sum[h].y += v[k][h].y; sum[h].z += v[k][h].z; sum[h].w += v[k][h].w; }

@@ -402,7 +402,8 @@ inline int with_shape(int nt, int wk, int terms, F f) {
     if constexpr (MODE != kGateUp) { if (wk == 4) return by_terms(tiles, std::integral_constant<int, 4>()); }
     return by_terms(tiles, std::integral_constant<int, 8>());
   };
-  return nt == 1 ? by_split(std::integral_constant<int, 1>()) : nt == 2 ? by_split(std::integral_constant<int, 2>()) : by_split(std::integral_constant<int, 4>());
+  if constexpr (MODE != kDense) { if (nt == 4) return by_split(std::integral_constant<int, 4>()); }      // the dense GEMM: 16 rows at most
+  return nt == 1 ? by_split(std::integral_constant<int, 1>()) : by_split(std::integral_constant<int, 2>());
 }
 template <int MODE>
 inline int launch_any(int nt, int wk, int terms, const Params& p, int grid, cudaStream_t s) {

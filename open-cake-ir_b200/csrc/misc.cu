@@ -23,6 +23,21 @@ extern "C" int cake_b200_decode_plan_view(const char* kind, void* handle, int wh
   return cake::kErrBadArgument;
 }
 
+static __global__ void silu_test_kernel(const float* __restrict__ x, float* __restrict__ y, float* __restrict__ by_division, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  y[i] = cake::silu(x[i]);
+  by_division[i] = x[i] / (1.f + __expf(-x[i]));
+}
+
+extern "C" int cake_b200_test_silu(const void* x, void* y, void* by_division, int64_t n, void* cuda_stream) {
+  if (n < 0 || n > (int64_t(1) << 30) || !x || !y || !by_division) return cake::kErrBadArgument;
+  if (n == 0) return 0;
+  silu_test_kernel<<<unsigned((n + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(cuda_stream)>>>(
+      static_cast<const float*>(x), static_cast<float*>(y), static_cast<float*>(by_division), n);
+  return int(cudaGetLastError());
+}
+
 extern "C" int cake_b200_test_hooks(int wait_budget_kiloclocks, int skip_load) {
   if (wait_budget_kiloclocks < 0) return cake::kErrBadArgument;
   cake::test_hooks().budget_kiloclocks = wait_budget_kiloclocks;
