@@ -803,19 +803,16 @@ mla_reduce_kernel(const Params p) {
         v[i] = __ldcg(reinterpret_cast<const float4*>(p.part_o + at * kCkv + d));
       }
     float m_new = mm;
-    bool seen = mm != -INFINITY;                   // a piece of NaN counts: the maximum leaves it out, its weight is NaN
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (k0 + i <= last) { m_new = fmaxf(m_new, ls[i]); seen |= ls[i] != -INFINITY; }
-    if (!seen) continue;
-    const float rescale = exp2f(mm - m_new);       // 0 the first time
+    for (int i = 0; i < 4; ++i) if (k0 + i <= last) m_new = fmaxf(m_new, ls[i]);
+    const float rescale = mm == m_new ? 1.f : exp2f(mm - m_new);       // 0 the first time that anything is seen
     mm = m_new;
     weight *= rescale;
     acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       if (k0 + i <= last) {
-        const float wt = exp2f(ls[i] - mm);
+        const float wt = ls[i] == -INFINITY ? 0.f : exp2f(ls[i] - mm);      // -inf: nothing seen; a NaN, which the maximum leaves out, goes on as one
         weight += wt;
         acc.x += wt * v[i].x; acc.y += wt * v[i].y; acc.z += wt * v[i].z; acc.w += wt * v[i].w;
       }
