@@ -226,10 +226,11 @@ struct Handle {
 inline void choose_shape(Handle* h, int device) {
   const int vectors = h->width / 8;
   // Shape class: 0 = a warp per row; 1..4 = 512 threads x 1, 2, 4, 8 vectors; 5 = 256 threads x 1.  A warp with eight vectors to a lane has
-  // too few rows in flight where a row brings little else: x alone above 1024 elements (4096 x 2048, from HBM: 14.4 us as warps, 12.4
-  // as CTAs; 4096 x 1032 12.3, 10.8), the two-output form above 1536 (8192 x 2048 30.7, 28.8).  With the residual the warps stay ahead
-  // up to 2048 (8192 x 1536 17.2 to 19.9, 18.8 to 20.9), since its loads do not wait for the row before.
-  const bool as_ctas = vectors <= 256 && vectors > (h->residual_out ? 192 : h->residual ? 256 : 128);
+  // too few rows in flight for HBM where a row brings little else: x alone above 1024 elements (4096 x 2048 14.4 us as warps, 12.4
+  // as CTAs; 8192 x 1536 18.4, 16.4), the two-output form above 1536 (8192 x 2048 30.7, 28.8).  From L2, where an input of less than
+  // 16 MB mostly lies, the warps are ahead (1507 x 2048 3.1, 3.7).  With the residual they stay ahead up to 2048 (8192 x 1536
+  // 19.9, 20.9), since its loads do not wait for the row before.
+  const bool as_ctas = vectors <= 256 && vectors > (h->residual_out ? 192 : h->residual ? 256 : 128) && int64_t(h->rows) * vectors >= (1 << 20);
   h->vpt = as_ctas ? 5 : vectors <= 256 ? 0 : vectors <= 512 ? 1 : vectors <= 1024 ? 2 : vectors <= 2048 ? 3 : 4;
   // persistent CTAs: as many as are resident at once, each walking rows with a stride of the grid
   const int resident = sm_count(device) * (h->vpt == 5 ? 6 : h->vpt == 1 ? 3 : h->vpt == 2 ? 2 : 1);
