@@ -116,12 +116,13 @@ skinny_kernel(const Params p) {
   if (p.status && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;
 
   if (warp == 0) {
-    const int max_rows = p.max_rows && *p.core ? p.max_rows : INT_MAX;
+    int max_rows = INT_MAX;
+    if (MODE != kDense && p.max_rows && *p.core) max_rows = p.max_rows;
     int running = 0;
     for (int base = 0; base < p.groups; base += 32) {
       const int g = base + lane;
       const int count = g < p.groups ? (p.offsets ? p.offsets[g + 1] - p.offsets[g] : p.dense_rows) : 0;
-      const int tiles = count > max_rows ? 0 : (count + S::kTokens - 1) / S::kTokens;
+      const int tiles = MODE != kDense && count > max_rows ? 0 : (count + S::kTokens - 1) / S::kTokens;
       int incl = tiles;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
