@@ -372,6 +372,17 @@ __device__ __forceinline__ void umma_f8f6f4(uint32_t d_tmem, uint64_t a_desc, ui
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The weight-stationary form, which also has tiles of 64 and 32 rows: D's columns then lie in two or four parts beside one another
+// in the lanes (64 rows: lanes 0..63 hold the rows' first N/2 columns, lanes 64..127 the others; 32 rows: lanes 32 i..32 i + 31 hold
+// columns [i N/4, (i + 1) N/4)), so that N = 256 takes 128 or 64 columns of tensor memory.
+__device__ __forceinline__ void umma_f8f6f4_ws(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.ws.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(
@@ -458,6 +469,24 @@ __device__ __forceinline__ void tmem_ld_wait_64(uint32_t taddr, uint64_t* v) {
         "=l"(v[16]), "=l"(v[17]), "=l"(v[18]), "=l"(v[19]), "=l"(v[20]), "=l"(v[21]), "=l"(v[22]), "=l"(v[23]),
         "=l"(v[24]), "=l"(v[25]), "=l"(v[26]), "=l"(v[27]), "=l"(v[28]), "=l"(v[29]), "=l"(v[30]), "=l"(v[31])
       : "r"(taddr), "r"(taddr + 32)
+      : "memory");
+}
+
+// The same with two runs of 16 columns.
+__device__ __forceinline__ void tmem_ld_wait_2x16(uint32_t taddr0, uint32_t taddr1, uint64_t* v) {
+  asm volatile(
+      "{\n\t.reg .b32 r<32>;\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {r0, r1, r2, r3, r4, r5, r6, r7, r8, r9, r10, r11, r12, r13, r14, r15}, [%16];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {r16, r17, r18, r19, r20, r21, r22, r23, r24, r25, r26, r27, r28, r29, r30, r31}, [%17];\n\t"
+      "tcgen05.wait::ld.sync.aligned;\n\t"
+      "mov.b64 %0, {r0, r1}; mov.b64 %1, {r2, r3}; mov.b64 %2, {r4, r5}; mov.b64 %3, {r6, r7};\n\t"
+      "mov.b64 %4, {r8, r9}; mov.b64 %5, {r10, r11}; mov.b64 %6, {r12, r13}; mov.b64 %7, {r14, r15};\n\t"
+      "mov.b64 %8, {r16, r17}; mov.b64 %9, {r18, r19}; mov.b64 %10, {r20, r21}; mov.b64 %11, {r22, r23};\n\t"
+      "mov.b64 %12, {r24, r25}; mov.b64 %13, {r26, r27}; mov.b64 %14, {r28, r29}; mov.b64 %15, {r30, r31};\n\t"
+      "}"
+      : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]), "=l"(v[4]), "=l"(v[5]), "=l"(v[6]), "=l"(v[7]),
+        "=l"(v[8]), "=l"(v[9]), "=l"(v[10]), "=l"(v[11]), "=l"(v[12]), "=l"(v[13]), "=l"(v[14]), "=l"(v[15])
+      : "r"(taddr0), "r"(taddr1)
       : "memory");
 }
 

@@ -24,6 +24,7 @@
 // hands them to the other roles through a four-slot ring (Params::queue).
 #pragma once
 #include "common.cuh"
+#include <type_traits>
 
 namespace cake {
 namespace gemm {
@@ -107,7 +108,7 @@ struct Shared {
   uint32_t tmem_base;
   WaitControl wait;
   int tile_prefix[kMaxGroups + 1];     // m tiles before group g
-  float exchange[2][2][2][kBM];        // [item parity][term][column group][row] amax exchange for kGateUp
+  float exchange[2][2][2 * kBM];       // [item parity][term][part of the row's 128 features][row] amax exchange for kGateUp
 };
 
 // A warp's 32 rows of 64 bytes (lane i holds row i) to global memory.  Through shared memory, so that a store instruction
@@ -130,6 +131,16 @@ __device__ __forceinline__ void warp_store_64(uint4* scratch, const uint4 (&v)[4
 struct Item {
   int group, row0, rows_valid, n_tile;
 };
+
+// Rows of the product that a tile takes.  Groups seldom end on 128 rows: an expert of 128 rows on average has a few in a second
+// tile half of the time, and in a step of some hundred tokens it has ten or thirty in all.  A tile of 32 or 64 rows (the
+// weight-stationary products) takes 318 or 334 clocks of tensor pipe a K block instead of 512, a quarter or half of the
+// promotion and less of A; under the power cap what it does not do is time for the others (hidden 7168, 256 experts of 2048, all
+// with as many rows: 2380 -> 1830 us at 32, 2566 -> 2090 at 64, 4116 -> 3660 at 137; at 128 there is nothing to gain).
+template <int MODE>
+__host__ __device__ constexpr int tile_rows(int rows_valid) {
+  return MODE == kDense ? kBM : rows_valid <= 32 ? 32 : rows_valid <= 64 ? 64 : kBM;
+}
 
 // Work item `g` -> (group, m tile, n tile); items of one group are ordered n tile major,
 // m tile minor.  Returns false past the end.
@@ -166,7 +177,7 @@ __device__ __forceinline__ float4 load_cluster(uint32_t local_addr, uint32_t ran
 template <int MODE, bool SPLIT = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a_tail,
-                const __grid_constant__ CUtensorMap map_b, const Params p) {
+                const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b_narrow, const Params p) {
   if (MODE != kDense && p.enabled) {               // the usual case is to leave, so before anything is set up
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -244,6 +255,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       tma_prefetch_descriptor(&map_a);
       tma_prefetch_descriptor(&map_a_tail);
       tma_prefetch_descriptor(&map_b);
+      if (MODE == kGateUp) tma_prefetch_descriptor(&map_b_narrow);
       const uint64_t keep = l2_policy_evict_last();    // activations: re-read by every n tile
       // Work items.  With a queue, this thread draws them (the first is the CTA's index, every later
       // one comes from the device counter, asked for one item ahead) and hands each to the other
@@ -270,12 +282,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       while (ok && valid) {
         g = p.queue ? int(gridDim.x) + atomicAdd(p.queue, 1) : g + int(gridDim.x);
         const int b_row0 = item.group * p.b_rows_per_group;
-        // A tile of at most kTailRows valid rows (the second tile of a group a little over 128 rows) brings in those
-        // rows only, through a map with a smaller box: such a tile streams its weights from L2 at what one SM can
-        // draw, so every byte not fetched shortens it.  Rows of the stage beyond them keep what an earlier tile left
-        // there; their products land in accumulator rows that no one reads.
-        const bool tail = item.rows_valid <= kTailRows;
-        const uint32_t stage_tx = uint32_t((tail ? kTailRows * kBK : kBytesA) + kCols * kBK);
+        const int m = MODE == kDense ? (item.rows_valid <= kTailRows ? kTailRows : kBM) : tile_rows<MODE>(item.rows_valid);       // rows of A to bring in
+        const uint32_t stage_tx = uint32_t(m * kBK + kCols * kBK);
         const int a_row0 = item.row0, n_tile = item.n_tile;
         for (int kb = 0; kb < k_count; ++kb, ++it) {
           const int s = it % kStages;
@@ -289,8 +297,16 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           int a_col = k_begin + kb, b_col = k_begin + kb;
           if (p.interleave_hi_lo) { a_col = (kb & 1) * (p.k_blocks >> 1) + (kb >> 1); b_col = kb >> 1; }
           mbar_arrive_expect_tx(&sh->full[s], stage_tx);
-          tma_load_2d_hint(a_dst, tail ? &map_a_tail : &map_a, a_col * kBK, a_row0, &sh->full[s], keep);
-          if (MODE == kGateUp) {
+          tma_load_2d_hint(a_dst, m < kBM ? &map_a_tail : &map_a, a_col * kBK, a_row0, &sh->full[s], keep);
+          if (MODE != kDense && m == 64) tma_load_2d_hint(a_dst + kTailRows * kBK, &map_a_tail, a_col * kBK, a_row0 + kTailRows, &sh->full[s], keep);
+          if (MODE == kGateUp && m < kBM) {
+            // 32 rows of x1, the matching 32 of x2, the next 32 of x1, ...: an epilogue thread of a narrow tile holds both of a feature
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              tma_load_2d(b_dst + (2 * i) * 32 * kBK, &map_b_narrow, b_col * kBK, b_row0 + n_tile * 128 + 32 * i, &sh->full[s]);
+              tma_load_2d(b_dst + (2 * i + 1) * 32 * kBK, &map_b_narrow, b_col * kBK, b_row0 + p.n + n_tile * 128 + 32 * i, &sh->full[s]);
+            }
+          } else if (MODE == kGateUp) {
             // gate/up: 128 rows of the first half (x1) and the matching 128 rows of the second half (x2)
             tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + n_tile * 128, &sh->full[s]);
             tma_load_2d(b_dst + 128 * kBK, &map_b, b_col * kBK, b_row0 + p.n + n_tile * 128, &sh->full[s]);
@@ -305,7 +321,6 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------------------
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc(0 /* e4m3 */, kBM, kCols);
       uint32_t it = 0, k = 0;
       bool ok = true;
       Item item;
@@ -314,31 +329,39 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           const int slot = k % kItemSlots;
           ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
           if (!ok) break;
-          const bool any = sh->item[slot].x >= 0;
+          const int4 v = sh->item[slot];
           mbar_arrive(&sh->item_empty[slot]);
-          if (!any) break;
+          if (v.x < 0) break;
+          item.rows_valid = v.z;
         } else if (!locate(sh, p, n_tiles, g, &item)) {
           break;
         }
-        for (int kb = 0; kb < k_count; ++kb, ++it) {
-          const int s = it % kStages;
-          const int t = it % kTmemStages;
-          ok = mbar_wait_both(&sh->full[s], (it / kStages) & 1, kStatusWaitSmemFull, &sh->tmem_empty[t],
-                              ((it / kTmemStages) & 1) ^ 1, kStatusWaitTmemEmpty, abort_flag, p.status);
-          if (!ok) break;
-          tcgen05_fence_after();
-          const uint32_t a_addr = smem_u32(tiles + s * kStageBytes);
-          const uint64_t a_desc = umma_desc_sw128(a_addr);
-          const uint64_t b_desc = umma_desc_sw128(a_addr + kBytesA);
-          const uint32_t d = tmem_base + t * kBN;
+        auto products = [&](auto narrow, uint32_t idesc) {
+          for (int kb = 0; kb < k_count; ++kb, ++it) {
+            const int s = it % kStages;
+            const int t = it % kTmemStages;
+            ok = mbar_wait_both(&sh->full[s], (it / kStages) & 1, kStatusWaitSmemFull, &sh->tmem_empty[t],
+                                ((it / kTmemStages) & 1) ^ 1, kStatusWaitTmemEmpty, abort_flag, p.status);
+            if (!ok) break;
+            tcgen05_fence_after();
+            const uint32_t a_addr = smem_u32(tiles + s * kStageBytes);
+            const uint64_t a_desc = umma_desc_sw128(a_addr);
+            const uint64_t b_desc = umma_desc_sw128(a_addr + kBytesA);
+            const uint32_t d = tmem_base + t * kBN;
 #pragma unroll
-          for (int j = 0; j < kBK / kUmmaK; ++j) {
-            // advancing K inside the 128-byte swizzle row: +32 bytes = +2 in the 16-byte address field
-            umma_f8f6f4(d, a_desc + uint64_t(j * (kUmmaK >> 4)), b_desc + uint64_t(j * (kUmmaK >> 4)), idesc, j > 0);
+            for (int j = 0; j < kBK / kUmmaK; ++j) {
+              // advancing K inside the 128-byte swizzle row: +32 bytes = +2 in the 16-byte address field
+              const uint64_t step = j * (kUmmaK >> 4);
+              if constexpr (decltype(narrow)::value) umma_f8f6f4_ws(d, a_desc + step, b_desc + step, idesc, j > 0);
+              else umma_f8f6f4(d, a_desc + step, b_desc + step, idesc, j > 0);
+            }
+            tcgen05_commit(&sh->empty[s]);       // the ring slot is free once these MMAs have read it
+            tcgen05_commit(&sh->tmem_full[t]);   // and the partial product is complete
           }
-          tcgen05_commit(&sh->empty[s]);       // the ring slot is free once these MMAs have read it
-          tcgen05_commit(&sh->tmem_full[t]);   // and the partial product is complete
-        }
+        };
+        const int m = tile_rows<MODE>(item.rows_valid);
+        if (MODE != kDense && m < kBM) products(std::true_type(), umma_idesc(0 /* e4m3 */, m, kCols));
+        else products(std::false_type(), umma_idesc(0 /* e4m3 */, kBM, kCols));
       }
     }
   } else if (warp == 2) {
@@ -379,7 +402,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const int slot = it % kScaleSlots;
 #pragma unroll
         for (int j = 0; j < kBM; j += 32)
-          cp_async_4(&sh->scale_a[slot][j + lane], sfa + min(item.row0 + j + lane, p.row_capacity - 1));
+          if (MODE == kDense || j < item.rows_valid) cp_async_4(&sh->scale_a[slot][j + lane], sfa + min(item.row0 + j + lane, p.row_capacity - 1));
         if (lane < 2) cp_async_4(&sh->scale_b[slot][lane], sfb + b_col);
         if (it >= kScaleAhead) cp_async_arrive_noinc(&sh->full[(it - kScaleAhead) % kStages]);
       }
@@ -397,40 +420,29 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int ew = warp - kControlWarps;
     const int quad = warp & 3;                 // TMEM lanes a warp may read: 32*(warp id % 4)
     const int cg = ew >> 2;                    // column group 0..1
-    const int r = quad * 32 + lane;            // row inside the tile
     const uint32_t lane_base = tmem_base + (uint32_t(quad * 32) << 16);
-    // Two 64-column segments per thread: gate/up takes 64 x1 columns and the matching 64 x2
-    // columns; the other modes take 128 consecutive columns.
-    const int seg_col0 = (MODE == kGateUp || SPLIT) ? cg * 64 : cg * 128;
-    const int seg_col1 = (MODE == kGateUp) ? 128 + cg * 64 : cg * 128 + 64;
     uint32_t it = 0, k = 0;
     uint32_t exchanges = 0;                    // amax exchanges so far (phase of Shared::exchange_done)
     int parity = 0;
     bool ok = true, met = false;               // met: SPLIT, this thread has been at the cluster's barriers
     Item item;
-    for (int g = first_item; ok; g += gridDim.x, parity ^= 1, ++k) {
-      if (handed) {                    // the k-th item of this CTA, from the TMA warp
-        const int slot = k % kItemSlots;
-        ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
-        if (!ok) break;
-        const int4 v = sh->item[slot];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->item_empty[slot]);
-        if (v.x < 0) break;
-        item.group = v.x; item.row0 = v.y; item.rows_valid = v.z; item.n_tile = v.w;
-      } else if (!locate(sh, p, n_tiles, g, &item)) {
-        break;
-      }
+    // One item of a tile of R rows.  256 / R threads share a row, R columns each: thread `part` has the tile's columns
+    // [part R, part R + R), or, gate/up, x1 and x2 of features [part R / 2, part R / 2 + R / 2).
+    auto run_item = [&](auto rows_tag) {
+      constexpr int R = decltype(rows_tag)::value;
+      const int r = R == 128 ? quad * 32 + lane : R == 64 ? (quad & 1) * 32 + lane : lane;       // row inside the tile
+      const int part = R == 128 ? cg : R == 64 ? (quad >> 1) * 2 + cg : quad * 2 + cg;
+      const int first_r = r - lane;            // the warp's first row
       const int row = item.row0 + r;
       float w = 1.f;                            // asked for here, a round trip to L2 before the K blocks end
       if (MODE == kDown && r < item.rows_valid) w = __ldg(p.row_weight + row);
-      uint64_t acc2[64];                        // 128 fp32 accumulators as packed pairs
+      uint64_t acc2[R / 2];                     // R fp32 accumulators as packed pairs
 #pragma unroll
-      for (int i = 0; i < 64; ++i) acc2[i] = 0;
+      for (int i = 0; i < R / 2; ++i) acc2[i] = 0;
       float sa = 0.f, sb0 = 0.f, sb1 = 0.f;    // scales of the coming block
       auto read_scales = [&](uint32_t block) {
         sa = sh->scale_a[block % kScaleSlots][r];
-        sb0 = sh->scale_b[block % kScaleSlots][MODE == kGateUp || SPLIT ? 0 : cg];
+        sb0 = sh->scale_b[block % kScaleSlots][MODE == kGateUp || SPLIT ? 0 : part * R / 128];
         if (MODE == kGateUp) sb1 = sh->scale_b[block % kScaleSlots][1];
       };
       if (it > 0) read_scales(it);
@@ -440,23 +452,37 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (!ok) break;
         tcgen05_fence_after();
         const uint32_t stage_addr = lane_base + t * kBN;
-        // two round trips to tensor memory per K block, 64 columns each
-        uint64_t v[32];
         if (it == 0) read_scales(0);
         const float s0 = sa * sb0, s1 = MODE == kGateUp ? sa * sb1 : s0;
-        tmem_ld_wait_64(stage_addr + seg_col0, v);
-        const uint64_t s0p = pack_f32x2(s0, s0);
+        const uint64_t s0p = pack_f32x2(s0, s0), s1p = pack_f32x2(s1, s1);
+        if constexpr (R == 128) {
+          // two round trips to tensor memory per K block, 64 columns each: gate/up takes 64 x1 columns and the matching 64 x2
+          // columns; the other modes take 128 consecutive columns (64 where CTAs share K)
+          const int seg_col0 = MODE == kGateUp || SPLIT ? cg * 64 : cg * 128;
+          const int seg_col1 = MODE == kGateUp ? 128 + cg * 64 : cg * 128 + 64;
+          uint64_t v[32];
+          tmem_ld_wait_64(stage_addr + seg_col0, v);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) acc2[i] = fma_f32x2(v[i], s0p, acc2[i]);
-        if (!SPLIT) tmem_ld_wait_64(stage_addr + seg_col1, v);
-        tcgen05_fence_before();            // everything this warp needs has left tensor memory
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->tmem_empty[t]);
-        if (kb + 1 < k_count) read_scales(it + 1);
-        if (SPLIT) continue;                   // 64 columns to a thread
-        const uint64_t s1p = pack_f32x2(s1, s1);
+          for (int i = 0; i < 32; ++i) acc2[i] = fma_f32x2(v[i], s0p, acc2[i]);
+          if (!SPLIT) tmem_ld_wait_64(stage_addr + seg_col1, v);
+          tcgen05_fence_before();            // everything this warp needs has left tensor memory
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh->tmem_empty[t]);
+          if (kb + 1 < k_count) read_scales(it + 1);
+          if (SPLIT) continue;                   // 64 columns to a thread
 #pragma unroll
-        for (int i = 0; i < 32; ++i) acc2[32 + i] = fma_f32x2(v[i], s1p, acc2[32 + i]);
+          for (int i = 0; i < 32; ++i) acc2[32 + i] = fma_f32x2(v[i], s1p, acc2[32 + i]);
+        } else {
+          uint64_t v[R / 2];
+          if constexpr (R == 64) tmem_ld_wait_64(stage_addr + cg * 64, v);
+          else tmem_ld_wait_2x16(stage_addr + cg * (MODE == kGateUp ? 16 : 32), stage_addr + (MODE == kGateUp ? 32 + cg * 16 : cg * 32 + 16), v);
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh->tmem_empty[t]);
+          if (kb + 1 < k_count) read_scales(it + 1);
+#pragma unroll
+          for (int i = 0; i < R / 2; ++i) acc2[i] = fma_f32x2(v[i], i < R / 4 ? s0p : s1p, acc2[i]);
+        }
       }
       if (SPLIT) {
         // This CTA's products are done, so its operand ring is idle: the sums go there, [chunk of 4 columns][row], and every
@@ -501,21 +527,18 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
         cluster_sync();                          // the sums stay until every CTA of the cluster has read them
         met = true;
-        break;
+        return;
       }
-      if (!ok) break;
-      float acc[128];
+      if (!ok) return;
+      float acc[R];
 #pragma unroll
-      for (int i = 0; i < 64; ++i) unpack_f32x2(acc2[i], acc[2 * i], acc[2 * i + 1]);
-      // rows past the group's end and, where N is an odd multiple of 128, the tile's second column group hold nothing
-      const bool columns_exist = MODE == kGateUp || item.n_tile * kBN + cg * 128 < p.n;
-      const bool valid = r < item.rows_valid && columns_exist;
-
+      for (int i = 0; i < R / 2; ++i) unpack_f32x2(acc2[i], acc[2 * i], acc[2 * i + 1]);
       if (MODE == kDense || MODE == kDown) {
-        uint8_t* out = reinterpret_cast<uint8_t*>(reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(item.row0 + quad * 32) * p.n + item.n_tile * kBN + cg * 128);
-        const int rows = columns_exist ? item.rows_valid - quad * 32 : 0;
+        uint8_t* out = reinterpret_cast<uint8_t*>(reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(item.row0 + first_r) * p.n + item.n_tile * kBN + part * R);
+        // rows past the group's end and, where N is an odd multiple of 128, the tile's second 128 columns hold nothing
+        const int rows = item.n_tile * kBN + part * R < p.n ? item.rows_valid - first_r : 0;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {            // 32 columns = 64 bytes of each row at a time
+        for (int c = 0; c < R / 32; ++c) {       // 32 columns = 64 bytes of each row at a time
           uint4 v[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -526,44 +549,53 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           warp_store_64(sh->out_rows[ew], v, out + c * 64, size_t(p.n) * 2, rows, lane);
         }
       } else {
-        // SwiGLU on the 64 (x1, x2) pairs this thread holds, then e4m3 quantisation of the 128-wide
-        // group it shares with the thread of the same row in the other column group.
+        // SwiGLU on the R / 2 (x1, x2) pairs this thread holds, then e4m3 quantisation of the 128-wide
+        // group it shares with the other threads of the same row.
         // Nothing overlaps it but the two blocks the tensor core is ahead, so its length counts in full: 8700 clocks (11100
         // with the second term) with the gate's quotient by `/` and one e4m3 value taken back at a time, against 900 a K
         // block.  The first GEMM of 2500 tokens, hidden 2048, 128 experts of 768, two terms: 204 us then, 163 now.
         float amax = 0.f;
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          acc[i] *= silu(acc[64 + i]);
+        for (int i = 0; i < R / 2; ++i) {
+          acc[i] *= silu(acc[R / 2 + i]);
           amax = fmaxf(amax, fabsf(acc[i]));
         }
         const int out_kb = p.n / 128;                      // K blocks of one term of the output
         const int terms = p.split_act ? 2 : 1;
         const size_t out_stride = size_t(p.n) * terms;
-        uint8_t* out = reinterpret_cast<uint8_t*>(p.out) + size_t(item.row0 + quad * 32) * out_stride + item.n_tile * 128 + cg * 64;
+        uint8_t* out = reinterpret_cast<uint8_t*>(p.out) + size_t(item.row0 + first_r) * out_stride + item.n_tile * 128 + part * (R / 2);
         for (int term = 0; term < terms; ++term, ++exchanges) {
-          // The two column groups of a row meet through shared memory.  The hand-over is an mbarrier wait like
+          // The threads of a row meet through shared memory.  The hand-over is an mbarrier wait like
           // every other wait of the kernel: bounded, and given up when another role has raised the abort flag.
-          sh->exchange[parity][term][cg][r] = amax;
+          float* const exchange = sh->exchange[parity][term];
+          exchange[part * R + r] = amax;
           __syncwarp();
           if (lane == 0) mbar_arrive(&sh->exchange_done);
           ok = mbar_wait(&sh->exchange_done, exchanges & 1, abort_flag, p.status, kStatusWaitFlag);
           if (!ok) break;
-          const float group_amax = fmaxf(amax, sh->exchange[parity][term][cg ^ 1][r]);
+          float group_amax = amax;
+#pragma unroll
+          for (int i = 0; i < 256 / R; ++i) group_amax = fmaxf(group_amax, exchange[i * R + r]);
           const float scale = group_amax > 0.f ? group_amax / 448.f : 1.f;
           const float inv = 1.f / scale;
-          uint32_t packed[16];
+          uint32_t packed[R / 8];
 #pragma unroll
-          for (int i = 0; i < 64; i += 4) packed[i >> 2] = pack_e4m3x4(acc[i] * inv, acc[i + 1] * inv, acc[i + 2] * inv, acc[i + 3] * inv);
-          uint4 v[4];
+          for (int i = 0; i < R / 2; i += 4) packed[i >> 2] = pack_e4m3x4(acc[i] * inv, acc[i + 1] * inv, acc[i + 2] * inv, acc[i + 3] * inv);
+          uint4 v[R / 32];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) v[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
-          warp_store_64(sh->out_rows[ew], v, out + size_t(term) * p.n, out_stride, item.rows_valid - quad * 32, lane);
-          if (valid && cg == 0) p.out_scale[size_t(term * out_kb + item.n_tile) * p.row_capacity + row] = scale;
+          for (int i = 0; i < R / 32; ++i) v[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+          uint8_t* const dst = out + size_t(term) * p.n;
+          if constexpr (R == 128) {
+            warp_store_64(sh->out_rows[ew], v, dst, out_stride, item.rows_valid - first_r, lane);
+          } else if (r < item.rows_valid) {
+#pragma unroll
+            for (int i = 0; i < R / 32; ++i) reinterpret_cast<uint4*>(dst + size_t(lane) * out_stride)[i] = v[i];
+          }
+          if (r < item.rows_valid && part == 0) p.out_scale[size_t(term * out_kb + item.n_tile) * p.row_capacity + row] = scale;
           if (term + 1 < terms) {        // residual after the first term becomes the value to quantise
             amax = 0.f;
 #pragma unroll
-            for (int i = 0; i < 64; i += 2) {
+            for (int i = 0; i < R / 2; i += 2) {
               const float2 first = e4m3x2_to_float2(uint16_t(packed[i >> 2] >> ((i & 2) * 8)));
               acc[i] -= first.x * scale;
               acc[i + 1] -= first.y * scale;
@@ -571,7 +603,26 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             }
           }
         }
+      }
+    };
+    for (int g = first_item; ok && !met; g += gridDim.x, parity ^= 1, ++k) {
+      if (handed) {                    // the k-th item of this CTA, from the TMA warp
+        const int slot = k % kItemSlots;
+        ok = mbar_wait(&sh->item_full[slot], (k / kItemSlots) & 1, abort_flag, p.status, kStatusWaitFlag);
         if (!ok) break;
+        const int4 v = sh->item[slot];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->item_empty[slot]);
+        if (v.x < 0) break;
+        item.group = v.x; item.row0 = v.y; item.rows_valid = v.z; item.n_tile = v.w;
+      } else if (!locate(sh, p, n_tiles, g, &item)) {
+        break;
+      }
+      const int m = tile_rows<MODE>(item.rows_valid);
+      if (m == kBM) run_item(std::integral_constant<int, 128>());
+      if constexpr (MODE != kDense) {
+        if (m == 64) run_item(std::integral_constant<int, 64>());
+        if (m == 32) run_item(std::integral_constant<int, 32>());
       }
     }
     if (SPLIT && !met) { cluster_sync(); cluster_sync(); }

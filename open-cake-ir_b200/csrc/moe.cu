@@ -489,7 +489,7 @@ struct MoeHandle {
   const int* local_offset; const float* factor;
   __nv_bfloat16* output;
   int* expert_ids; float* route_weights;       // in the workspace, or the caller's when routing is external
-  CUtensorMap map_a1, map_a1_tail, map_b1, map_a2, map_a2_tail, map_b2;
+  CUtensorMap map_a1, map_a1_tail, map_b1, map_b1_narrow, map_a2, map_a2_tail, map_b2;
   gemm::Params p1, p2;
   skinny::Params s1, s2;
   int grid;
@@ -625,6 +625,7 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
   if (!rc) rc = make_tensor_map_u8_sw128(&h->map_a1_tail, h->ws + l.x_perm, uint64_t(l.capacity), uint64_t(hidden), gemm::kTailRows);
   if (!rc) rc = make_tensor_map_u8_sw128(&h->map_a2_tail, h->ws + l.act, uint64_t(l.capacity), uint64_t(inter) * l.terms, gemm::kTailRows);
   if (!rc) rc = make_tensor_map_u8_sw128(&h->map_b1, buffers[4], uint64_t(c.local_experts) * 2 * inter, uint64_t(hidden), 128);
+  if (!rc) rc = make_tensor_map_u8_sw128(&h->map_b1_narrow, buffers[4], uint64_t(c.local_experts) * 2 * inter, uint64_t(hidden), 32);
   if (!rc) rc = make_tensor_map_u8_sw128(&h->map_a2, h->ws + l.act, uint64_t(l.capacity), uint64_t(inter) * l.terms, gemm::kBM);
   if (!rc) rc = make_tensor_map_u8_sw128(&h->map_b2, buffers[6], uint64_t(c.local_experts) * hidden, uint64_t(inter), gemm::kBN);
   if (!rc) rc = int(cudaFuncSetAttribute(gemm::gemm_fp8_kernel<gemm::kGateUp>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemm::kSmemBytes)));
@@ -767,13 +768,13 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
       }
       gemm::Params p = h->p1;
       p.wait_kiloclocks = test_hooks().budget_kiloclocks;
-      return launch_dependent(gemm::gemm_fp8_kernel<gemm::kGateUp>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a1, h->map_a1_tail, h->map_b1, p);
+      return launch_dependent(gemm::gemm_fp8_kernel<gemm::kGateUp>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a1, h->map_a1_tail, h->map_b1, h->map_b1_narrow, p);
     }
     case 2: {
       if (!l.token_tiles || l.core_above) {
         gemm::Params p = h->p2;
         p.wait_kiloclocks = test_hooks().budget_kiloclocks;
-        if (int rc = launch_dependent(gemm::gemm_fp8_kernel<gemm::kDown>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a2, h->map_a2_tail, h->map_b2, p))
+        if (int rc = launch_dependent(gemm::gemm_fp8_kernel<gemm::kDown>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a2, h->map_a2_tail, h->map_b2, h->map_b2, p))
           return rc;
       }
       return l.token_tiles ? skinny::launch_any<gemm::kDown>(l.token_tiles, l.split2, l.terms, h->s2, h->grid, s) : 0;
