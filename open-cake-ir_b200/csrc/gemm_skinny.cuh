@@ -1,10 +1,10 @@
 // Block-scaled FP8 (e4m3) GEMM for few rows per group on sm_100a: weights stream through, a handful of tokens stays.
 //
 // The same products as gemm_fp8.cuh, C[m, n] = sum_kb (sum_{k in kb} A[m, k] B[n, k]) sfa[kb, m] sfb[n/128, kb], for decode
-// steps, where a group (an expert, or the whole dense problem) has at most a few dozen rows.  What bounds it is the weight
-// stream: 2 x 32 rows of products per weight byte at most.  The tcgen05 core pays for 128 rows whatever the group holds, in
-// tensor time, in tensor-memory round trips per K block (about 0.4 us, one after another) and in power, and needs 256
-// columns to a CTA, so a small problem occupies a few SMs.  Here every warp is on its own: it streams 32 weight rows
+// steps whose groups (experts, or the whole dense problem) have a handful of rows and are few themselves.  What bounds it is
+// the weight stream: 2 x 16 rows of products per weight byte at most.  The tcgen05 core takes a tile's K blocks one after
+// another (0.25 to 0.4 us each) and 256 columns to a CTA, so a small problem occupies a few SMs for long; from about a tile to an SM
+// on its narrow row tiles are the faster ones.  Here every warp is on its own: it streams 32 weight rows
 // through a ring of its own (cp.async, one 128-wide K block of weights, token rows and scales per slot, several slots in
 // flight, no CTA-wide barrier in the main loop), multiplies with mma.m16n8k32 (weights are the 16 rows, tokens the 8
 // columns; exact products, fp32 sums, 1.06 clocks per instruction and SM) into a fresh partial sum per K block and
@@ -391,7 +391,7 @@ quantize_kernel(const float* __restrict__ in, const int* __restrict__ rows_ptr, 
   }
 }
 
-// A kernel's entry points by run-time numbers: token tiles of eight, K split, terms (two in the down mode only).
+// A kernel's entry points by run-time numbers: token tiles of eight (one or two), K split, terms (two in the down mode only).
 template <int MODE, typename F>
 inline int with_shape(int nt, int wk, int terms, F f) {
   auto by_terms = [&](auto tiles, auto split) {
@@ -403,7 +403,6 @@ inline int with_shape(int nt, int wk, int terms, F f) {
     if constexpr (MODE != kGateUp) { if (wk == 4) return by_terms(tiles, std::integral_constant<int, 4>()); }
     return by_terms(tiles, std::integral_constant<int, 8>());
   };
-  if constexpr (MODE != kDense) { if (nt == 4) return by_split(std::integral_constant<int, 4>()); }      // the dense GEMM: 16 rows at most
   return nt == 1 ? by_split(std::integral_constant<int, 1>()) : by_split(std::integral_constant<int, 2>());
 }
 template <int MODE>
@@ -418,9 +417,6 @@ inline int prepare_any(int nt, int wk, int terms) {
     return int(cudaFuncSetAttribute(skinny_kernel<MODE, tiles(), split(), t()>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<tiles(), split(), t()>::kSmemBytes));
   });
 }
-
-// Token tiles of eight per item, so that most groups of a layer fit one item: 8, 16 or 32 rows for an average of 3, 9 or more.
-inline int token_tiles(double rows_per_group) { return rows_per_group <= 3 ? 1 : rows_per_group <= 9 ? 2 : 4; }
 
 // Time of a launch in units of a warp's K block (32 weight rows x 128): rounds of the GPU times an item's K blocks and what
 // it costs beside them.  `features`: of an item, `row_tiles`: row tiles of all groups together.

@@ -451,18 +451,20 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
   l.act = take(size_t(l.capacity) * c.intermediate * l.terms);
   l.act_scale = take(size_t(c.intermediate / 128) * l.terms * l.capacity * 4);
   l.y = take(size_t(l.capacity) * c.hidden * 2);
-  // The weight-streaming kernel where an expert has few rows: it gathers nothing and keeps more loads in flight, but its
-  // products grow with the rows, and a second tile of an expert streams the weights again.  The tcgen05 core's time hardly
-  // depends on the rows up to 128.  They meet at 7 to 8 rows per expert on average (hidden 7168, 64 experts of 2048: 523 us
-  // and 545 at 7 rows, 552 and 543 at 8, 678 and 545 at 19; hidden 2048, 128 experts of 768: 137 and 146 at 5, 162 and
-  // 145 at 8), and at 10 to 12 where the core's tiles are fewer than the SMs and it leaves some idle (hidden 7168, 4 experts
-  // of 2048: 69 and 72 us at 10 rows, 91 and 77 at 19; of 768, hidden 2048: 30 and 35 at 10).
+  // The weight-streaming kernel where the core has few tiles (of the gate/up product, 128 features of an expert each): it gathers
+  // nothing, and shares an expert's K among warps where the core runs it one block after another on a part of the SMs.  Beyond about a
+  // tile to an SM the core's narrow tiles keep up with HBM better (weight-streaming kernel, core, us; hidden 7168, experts of 2048:
+  // 61 tiles 42 and 55, 115 tiles 65 and 65, 162 tiles 87 and 91, 204 tiles 99 and 95, 3600 tiles 1648 and 1509; hidden 2048,
+  // experts of 768: 135 tiles 40 and 44, 175 tiles 52 and 52, 490 tiles 97 and 88).  With two terms the core reads a weight block of the
+  // second product once per term (162 tiles 90 and 97, 241 tiles 136 and 134; 768: 247 tiles 61 and 63, 310 tiles 70 and 71).  Rows: an
+  // item of the weight-streaming kernel has 8 or 16, products in proportion (4 experts of 2048: 57 and 62 at 4 rows on average, 61 and
+  // 63 at 6, 73 and 66 at 10; 8 experts: 83 and 82 at 4, 91 and 85 at 6).
   const double per_expert = double(pairs) / c.experts;
   double missed = 1;                     // experts that get a row: those not missed by every token
   for (int64_t t = 0; t < c.tokens && missed > 1e-3; ++t) missed *= 1.0 - double(c.top_k) / c.experts;
   const double touched = c.local_experts * (1 - missed);
-  if (per_expert <= (touched * (c.intermediate / 128) < sms ? 11.0 : 7.5)) {
-    l.token_tiles = skinny::token_tiles(per_expert);
+  if (per_expert <= 5 && touched * (c.intermediate / 128) <= (l.terms == 2 ? 2.1 : 1.2) * sms) {
+    l.token_tiles = per_expert <= 3 ? 1 : 2;
     l.split1 = skinny::choose_split_gate_up(touched > 1 ? touched : 1, c.intermediate, c.hidden / 128, sms);
     l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128, sms);
     if (l.split1 > 1) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation

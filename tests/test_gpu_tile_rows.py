@@ -44,3 +44,15 @@ def test_last_tile_of_a_dense_product(m, n):
     ok, bad, err = compare.compare(c, want, atol=2e-2, rtol=2e-2)
     assert ok, f"{bad} mismatches, max abs err {err}"
     assert compare.rel_frobenius(c, want) <= 1e-2
+
+
+@pytest.mark.parametrize("tokens,experts,inter,act", [
+    (20, 32, 256, "fp8"), (21, 32, 256, "fp8"),                # five rows an expert; beyond
+    (12, 32, 256, "split"), (13, 32, 256, "split"),            # three: an item of 8 rows, of 16
+    (16, 128, 256, "fp8"), (20, 128, 256, "fp8"),              # tiles to 148 SMs: 1.1 and 1.26
+    (28, 256, 256, "split"), (31, 256, 256, "split")])         # with two terms: 2.04 and 2.17
+def test_lines_of_the_dispatch(tokens, experts, inter, act):
+    cpu = cake.workloads.moe_inputs(tokens, 512, inter, experts, experts, 0, routing="softmax", device="cpu")
+    out, _ = run_layer(cpu, experts=experts, routing="softmax", act_mode=act)
+    want = oracle_moe.moe_reference(cpu, routing="softmax", act_quant="fp8" if act == "fp8" else "none", dtype=torch.float32)
+    assert compare.rel_frobenius(out, want["output"]) <= (1e-2 if act == "fp8" else 4e-3)
