@@ -544,10 +544,10 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   return r;
 }
 
-// Exclusive scan over the 1024 threads of a CTA (every thread must call); `total` receives the sum
-// and `warp_sums` is 32 elements of shared memory.
-template <typename T>
-__device__ __forceinline__ T cta1024_exclusive_scan(T value, T* warp_sums, T& total) {
+// Exclusive scan over the WARPS x 32 threads of a CTA (every thread must call); `total` receives the sum
+// and `warp_sums` is WARPS elements of shared memory.
+template <int WARPS, typename T>
+__device__ __forceinline__ T cta_exclusive_scan(T value, T* warp_sums, T& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   T inc = value;
 #pragma unroll
@@ -557,17 +557,17 @@ __device__ __forceinline__ T cta1024_exclusive_scan(T value, T* warp_sums, T& to
   }
   if (lane == 31) warp_sums[warp] = inc;
   __syncthreads();
-  if (warp == 0) {                      // the 32 warp totals: inclusive scan in place
-    T w = warp_sums[lane];
+  if (warp == 0) {                      // the warp totals: inclusive scan in place
+    T w = lane < WARPS ? warp_sums[lane] : T(0);
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
+    for (int d = 1; d < WARPS; d <<= 1) {
       const T up = __shfl_up_sync(0xffffffffu, w, d);
       if (lane >= d) w += up;
     }
-    warp_sums[lane] = w;
+    if (lane < WARPS) warp_sums[lane] = w;
   }
   __syncthreads();
-  total = warp_sums[31];
+  total = warp_sums[WARPS - 1];
   const T before = warp > 0 ? warp_sums[warp - 1] : T(0);
   __syncthreads();                      // warp_sums may be reused by the next scan
   return before + inc - value;

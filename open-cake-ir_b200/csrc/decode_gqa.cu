@@ -6,8 +6,8 @@
 //
 // The kernel is bound by the HBM stream of K and V (2 * Hkv * D * 2 bytes per token) and never
 // writes logits or probabilities to memory.  The tokens of all sequences, in order, form one list,
-// and it is cut into as many equal consecutive ranges as there are SMs (a one-CTA plan kernel
-// lists the pieces of sequences each range holds).  The decode kernel is persistent, one CTA of
+// and it is cut into as many equal consecutive ranges as there are SMs (each CTA lists the pieces of sequences
+// its range holds; beyond 1024 sequences a one-CTA plan kernel does).  The decode kernel is persistent, one CTA of
 // sixteen warps per SM: the CTA takes one range and each PAIR of warps (w, w+8) one KV head of it,
 // so the eight pairs stream whole pages (page_size * Hkv * 256 B contiguous) and every SM moves
 // the same number of bytes whatever the sequence lengths are.  The two warps of a pair take
@@ -65,6 +65,7 @@ struct Params {
   int* done;                     // [B, Hkv] finished items
   int* status;                   // library status word (may be null)
   int batch, hq, hkv, page_size, capacity, ranges;
+  int plan_here;                 // every CTA of the decode kernel makes the plan of its ranges itself
   int merge_kernel;              // pieces are merged by gqa_merge_kernel instead of the pair that finishes a sequence's last one
   // Explicit sequence table (causal prefill, where every query token is a sequence of its own over a prefix of its
   // segment's rows): sequence b holds seq_tokens[b] tokens whose page list starts at kv_indices[seq_start[b]];
@@ -161,7 +162,7 @@ gqa_plan_kernel(const Params p) {
   const int len0 = tid < p.batch ? seq_len(p, tid) : 0;              // the first 1024 lengths stay in registers
   long long mine = len0 > 0 ? len0 + kPieceCost : 0, all_units = 0;
   for (int b = tid + 1024; b < p.batch; b += 1024) { const int n = seq_len(p, b); mine += n > 0 ? n + kPieceCost : 0; }
-  cta1024_exclusive_scan(mine, sums64, all_units);                    // (its barriers also publish the defaults above)
+  cta_exclusive_scan<32>(mine, sums64, all_units);                    // (its barriers also publish the defaults above)
   const long long per = max(16LL, (((all_units + p.ranges - 1) / p.ranges) + 15) & ~15LL);
 
   long long units_before = 0;
@@ -170,10 +171,10 @@ gqa_plan_kernel(const Params p) {
     const int b = base + tid;
     const int len = base == 0 ? len0 : (b < p.batch ? seq_len(p, b) : 0);
     long long batch_units;
-    const long long start = units_before + cta1024_exclusive_scan((long long)(len > 0 ? len + kPieceCost : 0), sums64, batch_units) + kPieceCost;
+    const long long start = units_before + cta_exclusive_scan<32>((long long)(len > 0 ? len + kPieceCost : 0), sums64, batch_units) + kPieceCost;
     const int n = len > 0 ? int((start + len - 1) / per) - int(start / per) + 1 : 0;
     int batch_entries;
-    const int first = entries_before + cta1024_exclusive_scan(n, sums32, batch_entries);
+    const int first = entries_before + cta_exclusive_scan<32>(n, sums32, batch_entries);
     starts[tid] = start; lens[tid] = len; firsts[tid] = first;
     if (b < p.batch) {
       // finished pieces per KV head; for the merge kernel the sequence's first piece and their number instead
@@ -212,6 +213,83 @@ gqa_plan_kernel(const Params p) {
     p.range_first[r] = range_first[r];
     p.range_count[r] = range_last[r] < 0 ? 0 : range_last[r] - range_first[r] + 1;
   }
+}
+
+// The same plan inside the decode kernel, for up to 1024 sequences: every CTA looks at all lengths and lists the pieces of its own ranges.
+// A plan kernel in front costs its 5 to 6 us, most of it the way through its launch and its memory round trips, before any CTA can
+// start; here the same round trips take about two (sequences of 9000 to 32768 tokens, 3 of them: 50.6 -> 48.6 us; 64 of 512 to 4096: 105.3 -> 103.2;
+// 1 of 430: 12.2 -> 9.6; 21 of 239 to 958: 23.3 -> 22.2).
+// Counters of a launch that merges in the decode kernel are cleared by gqa_reset_kernel, beside which this runs.
+constexpr int kPlanHere = 2 * kWarps * 32;
+struct RangeStart { int4 rec; int first, last, page; };      // first piece of a range, list index of it and of the last, its page list
+__device__ __forceinline__ void plan_here(const Params& p, uint8_t* scratch, int range0, int ranges, RangeStart* range_start) {
+  constexpr int kCtaWarps = kWarps;
+  long long* sums64 = reinterpret_cast<long long*>(scratch);
+  int* sums32 = reinterpret_cast<int*>(scratch + 64 * sizeof(long long));
+  const int tid = threadIdx.x;
+  int len[2], n[2], first[2];
+  long long start[2], all_units;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) len[i] = 2 * tid + i < p.batch ? seq_len(p, 2 * tid + i) : 0;
+  const long long units0 = len[0] > 0 ? len[0] + kPieceCost : 0, units1 = len[1] > 0 ? len[1] + kPieceCost : 0;
+  start[0] = cta_exclusive_scan<kCtaWarps>(units0 + units1, sums64, all_units) + kPieceCost;
+  start[1] = start[0] + units0;
+  const long long per = max(16LL, (((all_units + p.ranges - 1) / p.ranges) + 15) & ~15LL);
+  int range_first[2], range_last[2];                // of a sequence
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    range_first[i] = int(start[i] / per);
+    range_last[i] = len[i] > 0 ? int((start[i] + len[i] - 1) / per) : range_first[i] - 1;
+    n[i] = range_last[i] - range_first[i] + 1;
+  }
+  int all;
+  first[0] = cta_exclusive_scan<kCtaWarps>(n[0] + n[1], sums32, all);
+  first[1] = first[0] + n[0];
+  if (tid < ranges) { range_start[tid].first = 0x7fffffff; range_start[tid].last = -1; }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    for (int r = max(range_first[i], range0); r <= min(range_last[i], range0 + ranges - 1); ++r) {
+      atomicMin(&range_start[r - range0].first, first[i] + r - range_first[i]);
+      atomicMax(&range_start[r - range0].last, first[i] + r - range_first[i]);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int b = 2 * tid + i;
+    for (int r = max(range_first[i], range0); r <= min(range_last[i], range0 + ranges - 1); ++r) {
+      const int e = first[i] + r - range_first[i];
+      const long long begin = max(start[i], r * per), end = min(start[i] + len[i], (r + 1) * per);
+      const int4 rec = make_int4(b | (n[i] << 16), int(begin - start[i]), first[i], int(end - start[i]));
+      const int page = p.seq_start ? p.seq_start[b] : p.kv_indptr[b];
+      p.items[e] = rec;
+      p.item_page[e] = page;
+      if (e == range_start[r - range0].first) { range_start[r - range0].rec = rec; range_start[r - range0].page = page; }
+    }
+    if (b < p.batch && p.merge_kernel && blockIdx.x == 0) p.done[size_t(b) * p.hkv] = first[i] | (n[i] << 17);
+    if (b < p.batch && len[i] == 0 && b % int(gridDim.x) == int(blockIdx.x)) {
+      for (int h = 0; h < p.hq; ++h) {
+        p.lse[size_t(b) * p.hq + h] = -INFINITY;
+        for (int d = 0; d < kD; d += 4) *reinterpret_cast<uint2*>(p.out + (size_t(b) * p.hq + h) * kD + d) = make_uint2(0u, 0u);
+      }
+    }
+  }
+  if (tid < ranges) {
+    p.range_first[range0 + tid] = range_start[tid].first;
+    p.range_count[range0 + tid] = range_start[tid].last < 0 ? 0 : range_start[tid].last - range_start[tid].first + 1;
+  }
+  if (blockIdx.x == 0 && tid == 0 && p.status) *p.status = 0;
+  __syncthreads();                                  // the list is written; the scratch goes to the rings
+}
+
+// Clears the counters of a launch whose decode kernel makes the plan and merges the pieces.
+__global__ void __launch_bounds__(1024)
+gqa_reset_kernel(int* done, int count) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // everything in front of this launch is complete: the decode kernel may plan
+  const int i = blockIdx.x * 1024 + threadIdx.x;
+  if (i < count) done[i] = 0;
 }
 
 __device__ __forceinline__ void pair_barrier(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); }
@@ -282,14 +360,13 @@ __device__ __forceinline__ void merge_chunks(const Params& p, int b, int kvh, in
 }
 
 __global__ void __launch_bounds__(kWarps * 32, 1)
-gqa_decode_kernel(const Params p) {
+gqa_decode_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pair = warp % kHeads, part = warp / kHeads;
   const int group = p.hq / p.hkv;
   const int row = lane >> 2;            // query head inside the group held by this lane's rows of S
   const int quad = lane & 3;
-  const float scale2 = __ldg(p.sm_scale) * kLog2e;
   const uint32_t ring = smem_u32(smem) + warp * kWarpSmem;
   float* park = reinterpret_cast<float*>(smem + kRingBytes + pair * kParkBytes);
 
@@ -312,20 +389,35 @@ gqa_decode_kernel(const Params p) {
     kvh_mine = pair;
     active = pair < p.hkv && range_id < p.ranges;
   }
-  // Launched as a programmatic dependent of the plan kernel: everything above overlaps it, the
-  // list and the counters are read only after it has completed.
+  // Launched as a programmatic dependent.  Behind a plan kernel everything above overlaps it, the list and the counters are read
+  // only after it has completed.  Behind gqa_reset_kernel, which lets this grid in once all work before it has completed, the plan is made
+  // beside it; with neither in front nothing is read before the grids before have completed.
+  __shared__ RangeStart range_start[kHeads];
+  const int range0 = p.hkv >= kHeads || kHeads % p.hkv ? range_id : int(blockIdx.x) * (kHeads / p.hkv);
+  if (p.plan_here) {
+    if (p.merge_kernel) asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int here = p.hkv >= kHeads || kHeads % p.hkv ? 1 : kHeads / p.hkv;
+    plan_here(p, smem, range0, min(here, p.ranges - range0), range_start);
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  const float scale2 = __ldg(p.sm_scale) * kLog2e;
   // Items are numbered piece * Hkv + KV head; this pair's run from idx up to (not including) total.
   int idx = 0, total = 0;
-  if (active && p.range_count[range_id] > 0) {
-    idx = p.range_first[range_id] * p.hkv + kvh_mine;
-    total = (p.range_first[range_id] + p.range_count[range_id]) * p.hkv;
-  }
   int4 rec = make_int4(0, 0, 0, 0);
   int page_base = 0;
-  if (idx < total) {
-    rec = __ldg(p.items + idx / p.hkv);
-    page_base = __ldg(p.item_page + idx / p.hkv);
+  if (p.plan_here) {
+    const RangeStart& mine = range_start[range_id - range0];
+    if (active && mine.last >= 0) {
+      idx = mine.first * p.hkv + kvh_mine;
+      total = (mine.last + 1) * p.hkv;
+      rec = mine.rec;
+      page_base = mine.page;
+    }
+  } else if (active && p.range_count[range_id] > 0) {
+    idx = p.range_first[range_id] * p.hkv + kvh_mine;
+    total = (p.range_first[range_id] + p.range_count[range_id]) * p.hkv;
+    rec = __ldcg(p.items + idx / p.hkv);
+    page_base = __ldcg(p.item_page + idx / p.hkv);
   }
   auto tiles_of = [&](int item, const int4& r) {    // tiles of an item that fall to this warp
     return item < total ? ((r.w - r.y + kTile - 1) / kTile - part + kParts - 1) / kParts : 0;
@@ -362,8 +454,8 @@ gqa_decode_kernel(const Params p) {
     int4 nxt_rec = make_int4(0, 0, 0, 0);
     int nxt_page = 0;
     if (nxt_idx < total) {
-      nxt_rec = __ldg(p.items + nxt_idx / p.hkv);
-      nxt_page = __ldg(p.item_page + nxt_idx / p.hkv);
+      nxt_rec = __ldcg(p.items + nxt_idx / p.hkv);      // (this CTA may have written them)
+      nxt_page = __ldcg(p.item_page + nxt_idx / p.hkv);
     }
     if (my_tiles > 0 && !primed) {      // cold start: nothing of this item is in flight yet
       const int v_slot = k_slot == 2 ? 0 : k_slot + 1;
@@ -683,8 +775,13 @@ inline int launch(Params& p, int sms, cudaStream_t s) {
   // the decode kernel reads four pieces at a time, 14 us for the 50 to 90 pieces of each of three long sequences, against
   // 3 us for the launch.  At eight ranges a sequence the two cost the same.
   p.merge_kernel = p.batch * 8 <= p.ranges;
-  if (int rc = launch_dependent(gqa_plan_kernel, dim3(1), dim3(1024), 0, s, p)) return rc;
-  // The decode grid is a programmatic dependent: it may start while the plan kernel runs and waits
+  p.plan_here = p.batch <= kPlanHere;
+  if (!p.plan_here) {
+    if (int rc = launch_dependent(gqa_plan_kernel, dim3(1), dim3(1024), 0, s, p)) return rc;
+  } else if (!p.merge_kernel) {
+    if (int rc = launch_dependent(gqa_reset_kernel, dim3((p.batch * p.hkv + 1023) / 1024), dim3(1024), 0, s, p.done, p.batch * p.hkv)) return rc;
+  }
+  // The decode grid is a programmatic dependent: it may start while the kernel in front runs and waits
   // for it on the device, which takes the second launch latency off the critical path.
   if (int rc = launch_dependent(gqa_decode_kernel, dim3(grid), dim3(kWarps * 32), kSmemBytes, s, p)) return rc;
   if (!p.merge_kernel) return 0;

@@ -185,7 +185,7 @@ mla_plan_kernel(const Params p) {
     const int tiles = b < p.sequences ? (seq_len(p, b) + kUnit - 1) / kUnit : 0;
     const int n = tiles > 0 ? tiles + p.seq_cost : 0;
     int batch_total;
-    const int mine = before + cta1024_exclusive_scan(n, sums, batch_total);
+    const int mine = before + cta_exclusive_scan<32>(n, sums, batch_total);
     if (b < p.sequences) p.tile_prefix[b] = mine;
     before += batch_total;
   }
@@ -213,7 +213,7 @@ mla_prefill_plan_kernel(const Params p) {
     const int b = base + tid;
     int qs = 0, qe = 0, all;
     if (b < segments) segment(b, &qs, &qe);
-    const int mine = before + cta1024_exclusive_scan(qe > qs ? (qe - qs + p.pack - 1) / p.pack : 0, sums, all);
+    const int mine = before + cta_exclusive_scan<32>(qe > qs ? (qe - qs + p.pack - 1) / p.pack : 0, sums, all);
     if (b < segments) p.segment_prefix[b] = mine;
     before += all;
   }
@@ -243,7 +243,7 @@ mla_prefill_plan_kernel(const Params p) {
       n = seen > 0 ? (seen + kUnit - 1) / kUnit + p.seq_cost : 0;
     }
     int all;
-    const int mine = units + cta1024_exclusive_scan(n, sums, all);
+    const int mine = units + cta_exclusive_scan<32>(n, sums, all);
     if (t < count) p.tile_prefix[t] = mine;
     units += all;
   }

@@ -106,7 +106,7 @@ plan_kernel(const Params p) {
     int qs = 0, qe = 0, all;
     if (b < count) segment(b, &qs, &qe);
     const int n = qe > qs ? (qe - qs + per - 1) / per : 0;
-    const int mine = before + cta1024_exclusive_scan(n, sums, all);
+    const int mine = before + cta_exclusive_scan<32>(n, sums, all);
     if (b < count) p.prefix[b] = mine;
     before += all;
   }
@@ -139,7 +139,7 @@ plan_kernel(const Params p) {
   if (p.cut_capacity) {
     int mine = n0, all;
     for (int t = tid + 1024; t < total; t += 1024) mine += describe(t, &tile, &page);
-    cta1024_exclusive_scan(mine, sums, all);
+    cta_exclusive_scan<32>(mine, sums, all);
     share = float(all) * float(p.hkv) / float(p.sms) * 1.0001f;        // (rounding may leave a piece out, never make one more)
   }
   auto size_of = [&](int n) {                    // KV tiles of a tile's pieces
@@ -163,7 +163,7 @@ plan_kernel(const Params p) {
   __syncthreads();
   int all;
   const int mine = bucket[tid];
-  const int start = cta1024_exclusive_scan(mine, sums, all);
+  const int start = cta_exclusive_scan<32>(mine, sums, all);
   bucket[tid] = start;
   __syncthreads();
   auto list_tile = [&](int n, const int4& tile, int page) {
