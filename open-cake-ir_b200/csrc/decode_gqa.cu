@@ -57,7 +57,7 @@ struct Params {
   float* lse;                    // [B, Hq]
   float* part_o;                 // [capacity, Hq, D] normalised partial outputs, one slot per entry of `items`
   float* part_lse;               // [capacity, Hq]    base-2 partial log-sum-exp
-  int4* items;                   // [capacity] pieces of sequences in token order, written by the plan kernel:
+  int4* items;                   // [capacity] pieces of sequences in token order, from the plan:
                                  //   x = b | (pieces of b << 16), y = first token, z = list index of b's first piece, w = end token
   int* item_page;                // [capacity] kv_indptr[b] of the piece
   int* range_first;              // [ranges] list index of the first piece of each range

@@ -70,7 +70,7 @@ struct Params {
   float* part_lse;        // [2 * workers, rows]
   int4* cuts;             // [workers] sequences that a range boundary cuts: {sequence, first and last range, slot of its first piece}
   int* cut_count;
-  int* tile_prefix;       // [sequences + 1] work units (tiles + start-up shares) before a sequence, written by the plan kernel
+  int* tile_prefix;       // [sequences + 1] work units (tiles + start-up shares) before a sequence, from the plan
   int* status;
   int sequences, heads, page_size, workers;
   int rows;               // result rows of a sequence: all heads of a token, of `pack` tokens in the prefill form
@@ -81,11 +81,12 @@ struct Params {
   const int* sparse_indices;
   int top_k;
   // Causal prefill: sequence b is up to `pack` consecutive query tokens of a segment, {first query row, tokens, KV rows the
-  // first one sees (may be < 1), KV rows of the segment}, its page list starts at kv_indices[seq_page[b]].  Made by the plan kernel.
+  // first one sees (may be < 1), KV rows of the segment}, its page list starts at kv_indices[seq_page[b]].  From the plan.
   int4* seq;
   int* seq_page;
   int* seq_count;
   int* segment_prefix;
+  int plan_here;          // every CTA of the decode kernel makes the plan itself
   const int* qo_indptr;
   int segments, total_q, nan_for_masked;
   int out_align;          // the widest store that the address of `out` allows: 32, 16 or 8 bytes
@@ -147,29 +148,29 @@ __device__ __forceinline__ int units_per_worker(const Params& p, int total) {
 // sequences: the one the range begins in (slot 2 w) and the one it ends in, if that starts inside the range (2 w + 1).
 __device__ __forceinline__ int slot_of(int w, int seq_begin, int per) { return 2 * w + (seq_begin > w * per ? 1 : 0); }
 // Largest b with prefix[b] <= unit.
-__device__ __forceinline__ int sequence_at(const Params& p, int count, int unit) {
+__device__ __forceinline__ int sequence_at(const int* prefix, int count, int unit) {
   int lo = 0, hi = count;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (p.tile_prefix[mid] <= unit) lo = mid; else hi = mid;
+    if (prefix[mid] <= unit) lo = mid; else hi = mid;
   }
   return lo;
 }
 
 // Lists the cut sequences for the reduce kernel (all threads of a plan CTA, once the prefix is complete).
-__device__ __forceinline__ void list_cuts(const Params& p, int count, int total) {
-  __shared__ int listed;
-  if (threadIdx.x == 0) listed = 0;
+// `listed`: a word of shared memory.
+__device__ __forceinline__ void list_cuts(const Params& p, const int* prefix, int count, int total, int* listed) {
+  if (threadIdx.x == 0) *listed = 0;
   __syncthreads();                                 // also makes the prefix visible
   const int per = units_per_worker(p, total);
   for (int b = threadIdx.x; b < count; b += blockDim.x) {
-    const int begin = p.tile_prefix[b], end = p.tile_prefix[b + 1];
+    const int begin = prefix[b], end = prefix[b + 1];
     if (end == begin) continue;
     const int first = (begin + p.seq_cost) / per, last = (end - 1) / per;
-    if (first < last) p.cuts[atomicAdd(&listed, 1)] = make_int4(b, first, last, slot_of(first, begin, per));
+    if (first < last) p.cuts[atomicAdd(listed, 1)] = make_int4(b, first, last, slot_of(first, begin, per));
   }
   __syncthreads();
-  if (threadIdx.x == 0) *p.cut_count = listed;
+  if (threadIdx.x == 0) *p.cut_count = *listed;
 }
 
 // One CTA: tile_prefix[b] = units before sequence b (exclusive scan), tile_prefix[B] = all units.
@@ -190,29 +191,47 @@ mla_plan_kernel(const Params p) {
     before += batch_total;
   }
   if (threadIdx.x == 0) p.tile_prefix[p.sequences] = before;
-  list_cuts(p, p.sequences, before);
+  list_cuts(p, p.tile_prefix, p.sequences, before, sums);
 }
 
-// The same for a causal prefill: cuts the query rows of every segment into sequences of up to `pack` tokens first.  Rows
-// outside every segment form two more segments without KV rows (they become zeros).
+// Causal prefill: the query rows [qs, qe) of segment b; rows outside every segment form two more segments without KV rows (they
+// become zeros).
+__device__ __forceinline__ void segment_rows(const Params& p, int b, int* qs, int* qe) {
+  const int rows_end = p.qo_indptr[p.segments];
+  if (b < p.segments) { *qs = p.qo_indptr[b]; *qe = p.qo_indptr[b + 1]; }
+  else if (b == p.segments) { *qs = rows_end; *qe = p.total_q; }
+  else { *qs = 0; *qe = p.qo_indptr[0]; }
+}
+// Sequence t of a causal prefill, from the number of sequences before each segment; returns its units.
+__device__ __forceinline__ int describe(const Params& p, const int* segment_prefix, int t, int4* seq, int* page) {
+  const int segment = sequence_at(segment_prefix, p.segments + 2, t);
+  int qs, qe, kv_len = 0;
+  segment_rows(p, segment, &qs, &qe);
+  *page = 0;
+  if (segment < p.segments) {
+    *page = p.kv_indptr[segment];
+    const int pages = p.kv_indptr[segment + 1] - *page;
+    kv_len = pages <= 0 ? 0 : p.kv_last_page_len ? (pages - 1) * p.page_size + p.kv_last_page_len[segment] : pages * p.page_size;
+  }
+  const int i = (t - segment_prefix[segment]) * p.pack, tokens = min(p.pack, qe - qs - i), first = i + 1 + kv_len - (qe - qs);
+  *seq = make_int4(qs + i, tokens, first, kv_len);
+  const int seen = min(kv_len, first + tokens - 1);
+  return seen > 0 ? (seen + kUnit - 1) / kUnit + p.seq_cost : 0;
+}
+
+// The same for a causal prefill: cuts the query rows of every segment into sequences of up to `pack` tokens first.
 static __global__ void __launch_bounds__(1024)
 mla_prefill_plan_kernel(const Params p) {
   __shared__ int sums[32];
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x;
-  const int rows_end = p.qo_indptr[p.segments];
-  auto segment = [&](int b, int* qs, int* qe) {
-    if (b < p.segments) { *qs = p.qo_indptr[b]; *qe = p.qo_indptr[b + 1]; }
-    else if (b == p.segments) { *qs = rows_end; *qe = p.total_q; }
-    else { *qs = 0; *qe = p.qo_indptr[0]; }
-  };
   const int segments = p.segments + 2;
   int before = 0;
   for (int base = 0; base < segments; base += 1024) {
     const int b = base + tid;
     int qs = 0, qe = 0, all;
-    if (b < segments) segment(b, &qs, &qe);
+    if (b < segments) segment_rows(p, b, &qs, &qe);
     const int mine = before + cta_exclusive_scan<32>(qe > qs ? (qe - qs + p.pack - 1) / p.pack : 0, sums, all);
     if (b < segments) p.segment_prefix[b] = mine;
     before += all;
@@ -222,33 +241,79 @@ mla_prefill_plan_kernel(const Params p) {
   int units = 0;
   for (int base = 0; base < count; base += 1024) {
     const int t = base + tid;
-    int n = 0;
-    if (t < count) {
-      int lo = 0, hi = segments;                   // largest segment with prefix <= t
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (p.segment_prefix[mid] <= t) lo = mid; else hi = mid;
-      }
-      int qs, qe, kv_len = 0, page = 0;
-      segment(lo, &qs, &qe);
-      if (lo < p.segments) {
-        page = p.kv_indptr[lo];
-        const int pages = p.kv_indptr[lo + 1] - page;
-        kv_len = pages <= 0 ? 0 : p.kv_last_page_len ? (pages - 1) * p.page_size + p.kv_last_page_len[lo] : pages * p.page_size;
-      }
-      const int i = (t - p.segment_prefix[lo]) * p.pack, tokens = min(p.pack, qe - qs - i), first = i + 1 + kv_len - (qe - qs);
-      p.seq[t] = make_int4(qs + i, tokens, first, kv_len);
-      p.seq_page[t] = page;
-      const int seen = min(kv_len, first + tokens - 1);
-      n = seen > 0 ? (seen + kUnit - 1) / kUnit + p.seq_cost : 0;
-    }
+    const int n = t < count ? describe(p, p.segment_prefix, t, p.seq + t, p.seq_page + t) : 0;
     int all;
     const int mine = units + cta_exclusive_scan<32>(n, sums, all);
     if (t < count) p.tile_prefix[t] = mine;
     units += all;
   }
   if (tid == 0) { p.tile_prefix[count] = units; *p.seq_count = count; *p.status = 0; }
-  list_cuts(p, count, units);
+  list_cuts(p, p.tile_prefix, count, units, sums);
+}
+
+// The plan inside the decode kernel, for up to 1024 sequences (2048 of a prefill of up to 510 segments): every CTA makes all of it in
+// shared memory (`scratch`: the prefix first) and writes out what its roles read, the sequences of its range; CTA 0 writes all, and the cuts.
+// A plan kernel in front costs its 4 to 5 us before any CTA can start, most of it launch and memory round trips; made here, behind
+// a set-up that now runs beside the grid in front, it takes 1 to 2 us less: 105 sequences of 73 to 586 tokens, 16 heads, 35.3 -> 33.7 us, one of
+// 7000, 64 heads, 26.7 -> 25.6; nothing on launches of 80 us and more (84 either way).
+constexpr int kEach = 4;                           // sequences of a thread
+constexpr int kPlanSequences = 2 * kThreads, kPlanPrefill = kEach * kThreads, kPlanSegments = kThreads - 2;
+static __device__ __noinline__ int2 plan_here(const Params& p, int* scratch, int worker) {
+  int* const prefix = scratch;
+  int* const segment_prefix = scratch + kPlanPrefill + 1;
+  int* const sums = segment_prefix + kThreads;
+  const int tid = threadIdx.x;
+  int count = p.sequences;
+  if (p.seq) {
+    int qs = 0, qe = 0, all;
+    if (tid < p.segments + 2) segment_rows(p, tid, &qs, &qe);
+    const int mine = cta_exclusive_scan<kThreads / 32>(qe > qs ? (qe - qs + p.pack - 1) / p.pack : 0, sums, all);
+    segment_prefix[tid] = mine;
+    count = min(all, p.sequences);
+    __syncthreads();
+  }
+  int4 seq[kEach];
+  int page[kEach], before[kEach], n[kEach], sum = 0, total;
+#pragma unroll
+  for (int i = 0; i < kEach; ++i) {
+    const int t = tid * kEach + i;
+    n[i] = 0;
+    if (t < count) {
+      if (p.seq) {
+        n[i] = describe(p, segment_prefix, t, &seq[i], &page[i]);
+      } else {
+        const int tiles = (seq_len(p, t) + kUnit - 1) / kUnit;
+        n[i] = tiles > 0 ? tiles + p.seq_cost : 0;
+      }
+    }
+    before[i] = sum;
+    sum += n[i];
+  }
+  const int mine = cta_exclusive_scan<kThreads / 32>(sum, sums, total);
+  const int per = units_per_worker(p, total), range_begin = worker * per, range_end = min(total, range_begin + per);
+#pragma unroll
+  for (int i = 0; i < kEach; ++i) {
+    const int t = tid * kEach + i;
+    if (t >= count) continue;
+    const int start = mine + before[i], stop = start + n[i];
+    prefix[t] = start;
+    // (the warps that write the results of sequences without units take 128 at a time, see below)
+    if (blockIdx.x == 0 || (start <= range_end && stop >= range_begin) || (n[i] == 0 && t / 128 % p.workers == worker)) {
+      p.tile_prefix[t] = start;
+      p.tile_prefix[t + 1] = stop;
+      if (p.seq) { p.seq[t] = seq[i]; p.seq_page[t] = page[i]; }
+    }
+  }
+  if (tid == 0) {
+    prefix[count] = total;
+    if (blockIdx.x == 0) {
+      p.tile_prefix[count] = total;
+      *p.status = 0;
+    }
+  }
+  if (blockIdx.x == 0) list_cuts(p, prefix, count, total, sums);
+  __syncthreads();
+  return make_int2(count, total);
 }
 
 // A piece of a sequence as every role of a cluster reads it off the list.
@@ -371,36 +436,10 @@ template <bool SPARSE>
 __global__ void __launch_bounds__(kThreads, 1)
 mla_decode_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
-  // launched as a programmatic dependent of the plan kernel: resident early, reads the plan after that grid has completed
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t rank = cluster_rank();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head_blocks = (p.rows + kHeads - 1) / kHeads;
   const int cluster = blockIdx.x >> 1, hb = cluster % head_blocks, worker = cluster / head_blocks;
-  const int count = sequence_count(p);
-  const int total = p.tile_prefix[count];
-
-  // sequences without units: zeros, lse -inf; NaN for a fully masked row of a non-empty segment where the contract says so
-  if (rank == 0 && hb == 0 && warp >= kOutWarp0) {
-    for (int base = worker * 128; base < count; base += p.workers * 128) {
-      const int mine = base + (warp - kOutWarp0) * 32 + lane;
-      uint32_t empty = __ballot_sync(0xffffffffu, mine < count && p.tile_prefix[mine + 1] == p.tile_prefix[mine]);
-      while (empty) {
-        const int b = base + (warp - kOutWarp0) * 32 + __ffs(empty) - 1;
-        empty &= empty - 1;
-        const int4 s = p.seq ? p.seq[b] : make_int4(b, 1, 0, 0);
-        const uint32_t word = p.nan_for_masked && s.w > 0 ? 0x7fc07fc0u : 0u;
-        const size_t row0 = size_t(s.x) * p.heads;
-        for (int i = lane; i < s.y * p.heads * (kCkv / 4); i += 32)
-          reinterpret_cast<uint2*>(p.out + row0 * kCkv)[i] = make_uint2(word, word);
-        if (p.lse) for (int i = lane; i < s.y * p.heads; i += 32) p.lse[row0 + i] = -INFINITY;
-      }
-    }
-  }
-  const int per_worker = units_per_worker(p, total);
-  const int range_begin = worker * per_worker, range_end = min(total, range_begin + per_worker);
-  if (range_begin >= range_end) return;            // the whole cluster leaves together
-
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t q_addr = smem_u32(base), k_addr = q_addr + kQBytes, v_addr = k_addr + kStages * kKBytes, p_addr = v_addr + kStages * kVBytes;
   Shared* sh = reinterpret_cast<Shared*>(base + kQBytes + kStages * (kKBytes + kVBytes) + 2 * kPBytes);
@@ -425,9 +464,43 @@ mla_decode_kernel(const __grid_constant__ Params p) {
   __syncthreads();
   cluster_sync();                                  // the other CTA's barriers exist
   tcgen05_fence_after();
+  // Launched as a programmatic dependent: what is above runs beside the grid in front, and nothing is read before that (the plan kernel, if
+  // there is one) has completed.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int* prefix = p.tile_prefix;               // of all sequences, until the rings take the scratch
+  int count, total;
+  if (p.plan_here) {
+    const int2 plan = plan_here(p, reinterpret_cast<int*>(base), worker);
+    count = plan.x; total = plan.y;
+    prefix = reinterpret_cast<const int*>(base);
+  } else {
+    count = sequence_count(p);
+    total = prefix[count];
+  }
+
+  // sequences without units: zeros, lse -inf; NaN for a fully masked row of a non-empty segment where the contract says so
+  if (rank == 0 && hb == 0 && warp >= kOutWarp0) {
+    for (int base = worker * 128; base < count; base += p.workers * 128) {
+      const int mine = base + (warp - kOutWarp0) * 32 + lane;
+      uint32_t empty = __ballot_sync(0xffffffffu, mine < count && prefix[mine + 1] == prefix[mine]);
+      while (empty) {
+        const int b = base + (warp - kOutWarp0) * 32 + __ffs(empty) - 1;
+        empty &= empty - 1;
+        const int4 s = p.seq ? p.seq[b] : make_int4(b, 1, 0, 0);
+        const uint32_t word = p.nan_for_masked && s.w > 0 ? 0x7fc07fc0u : 0u;
+        const size_t row0 = size_t(s.x) * p.heads;
+        for (int i = lane; i < s.y * p.heads * (kCkv / 4); i += 32)
+          reinterpret_cast<uint2*>(p.out + row0 * kCkv)[i] = make_uint2(word, word);
+        if (p.lse) for (int i = lane; i < s.y * p.heads; i += 32) p.lse[row0 + i] = -INFINITY;
+      }
+    }
+  }
+  const int per_worker = units_per_worker(p, total);
+  const int range_begin = worker * per_worker, range_end = min(total, range_begin + per_worker);
+  Cursor cursor = {range_begin, sequence_at(prefix, count, range_begin)};      // an empty range has no piece
+  __syncthreads();                                 // the scratch goes to the rings
   const uint32_t tmem_base = sh->tmem_base;
   volatile int* abort_flag = &sh->wait.abort_flag;
-  Cursor cursor = {range_begin, sequence_at(p, count, range_begin)};
   Piece w;
   bool ok = true;
   uint32_t it = 0, pieces = 0;                     // tiles and pieces so far
@@ -886,7 +959,9 @@ inline int launch(const Handle* h, cudaStream_t s) {
   Params p = h->p;
   p.wait_kiloclocks = test_hooks().budget_kiloclocks;
   p.skip_load = test_hooks().skip_load;
-  if (int rc = launch_dependent(p.seq ? mla_prefill_plan_kernel : mla_plan_kernel, dim3(1), dim3(1024), 0, s, p)) return rc;
+  p.plan_here = p.seq ? p.sequences <= kPlanPrefill && p.segments <= kPlanSegments : p.sequences <= kPlanSequences;
+  if (!p.plan_here)
+    if (int rc = launch_dependent(p.seq ? mla_prefill_plan_kernel : mla_plan_kernel, dim3(1), dim3(1024), 0, s, p)) return rc;
   const dim3 grid(p.workers * head_blocks(p.rows) * 2);
   if (int rc = launch_dependent_cluster(2, p.sparse_indices ? mla_decode_kernel<true> : mla_decode_kernel<false>, grid, dim3(kThreads), kSmemBytes, s, p))
     return rc;

@@ -125,9 +125,9 @@ extern "C" int cake_b200_block_scaled_gemm_launch(void* handle, void* cuda_strea
   p.skip_load = test_hooks().skip_load;
   if (h->split)
     return launch_dependent_cluster(h->split, gemm::gemm_fp8_kernel<gemm::kDense, true>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes,
-                                    stream, h->map_a, h->map_a_tail, h->map_b, h->map_b, p);
+                                    stream, gemm::Maps<gemm::kDense>{h->map_a, h->map_a_tail, h->map_b}, p);
   if (p.queue) CAKE_CUDA_OK(cudaMemsetAsync(h->status, 0, 8 * sizeof(int), stream));     // status word and work-item counter
-  return launch_dependent(gemm::gemm_fp8_kernel<gemm::kDense>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, stream, h->map_a, h->map_a_tail, h->map_b, h->map_b, p);
+  return launch_dependent(gemm::gemm_fp8_kernel<gemm::kDense>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, stream, gemm::Maps<gemm::kDense>{h->map_a, h->map_a_tail, h->map_b}, p);
 }
 
 extern "C" int cake_b200_block_scaled_gemm_destroy(void* handle) {

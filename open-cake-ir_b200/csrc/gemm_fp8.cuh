@@ -174,10 +174,13 @@ __device__ __forceinline__ float4 load_cluster(uint32_t local_addr, uint32_t ran
 // SPLIT (dense only): tiles of 128 columns, each shared by the CTAs of a cluster (two or four), a part of K to each.  A
 // problem of few tiles otherwise runs its K blocks, about 0.45 us each, one after another on a handful of SMs (64 x 4096 x
 // 7168: 16 SMs).  The parts meet through distributed shared memory: CTA r finishes columns [128 r / S, 128 (r + 1) / S).
+template <int MODE>
+struct Maps { CUtensorMap a, a_tail, b; };
+template <>
+struct Maps<kGateUp> { CUtensorMap a, a_tail, b, b_narrow; };        // b_narrow: boxes of 32 rows
 template <int MODE, bool SPLIT = false>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a_tail,
-                const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_b_narrow, const Params p) {
+gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
   if (MODE != kDense && p.enabled) {               // the usual case is to leave, so before anything is set up
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -252,10 +255,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   if (warp == 0) {
     // ------------------------------ TMA producer --------------------------------------
     if (elect_one()) {
-      tma_prefetch_descriptor(&map_a);
-      tma_prefetch_descriptor(&map_a_tail);
-      tma_prefetch_descriptor(&map_b);
-      if (MODE == kGateUp) tma_prefetch_descriptor(&map_b_narrow);
+      tma_prefetch_descriptor(&maps.a);
+      tma_prefetch_descriptor(&maps.a_tail);
+      tma_prefetch_descriptor(&maps.b);
+      if constexpr (MODE == kGateUp) tma_prefetch_descriptor(&maps.b_narrow);
       const uint64_t keep = l2_policy_evict_last();    // activations: re-read by every n tile
       // Work items.  With a queue, this thread draws them (the first is the CTA's index, every later
       // one comes from the device counter, asked for one item ahead) and hands each to the other
@@ -297,22 +300,22 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           int a_col = k_begin + kb, b_col = k_begin + kb;
           if (p.interleave_hi_lo) { a_col = (kb & 1) * (p.k_blocks >> 1) + (kb >> 1); b_col = kb >> 1; }
           mbar_arrive_expect_tx(&sh->full[s], stage_tx);
-          tma_load_2d_hint(a_dst, m < kBM ? &map_a_tail : &map_a, a_col * kBK, a_row0, &sh->full[s], keep);
-          if (MODE != kDense && m == 64) tma_load_2d_hint(a_dst + kTailRows * kBK, &map_a_tail, a_col * kBK, a_row0 + kTailRows, &sh->full[s], keep);
-          if (MODE == kGateUp && m < kBM) {
+          tma_load_2d_hint(a_dst, m < kBM ? &maps.a_tail : &maps.a, a_col * kBK, a_row0, &sh->full[s], keep);
+          if (MODE != kDense && m == 64) tma_load_2d_hint(a_dst + kTailRows * kBK, &maps.a_tail, a_col * kBK, a_row0 + kTailRows, &sh->full[s], keep);
+          if constexpr (MODE == kGateUp)
+          if (m < kBM) {
             // 32 rows of x1, the matching 32 of x2, the next 32 of x1, ...: an epilogue thread of a narrow tile holds both of a feature
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              tma_load_2d(b_dst + (2 * i) * 32 * kBK, &map_b_narrow, b_col * kBK, b_row0 + n_tile * 128 + 32 * i, &sh->full[s]);
-              tma_load_2d(b_dst + (2 * i + 1) * 32 * kBK, &map_b_narrow, b_col * kBK, b_row0 + p.n + n_tile * 128 + 32 * i, &sh->full[s]);
+              tma_load_2d(b_dst + (2 * i) * 32 * kBK, &maps.b_narrow, b_col * kBK, b_row0 + n_tile * 128 + 32 * i, &sh->full[s]);
+              tma_load_2d(b_dst + (2 * i + 1) * 32 * kBK, &maps.b_narrow, b_col * kBK, b_row0 + p.n + n_tile * 128 + 32 * i, &sh->full[s]);
             }
-          } else if (MODE == kGateUp) {
-            // gate/up: 128 rows of the first half (x1) and the matching 128 rows of the second half (x2)
-            tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + n_tile * 128, &sh->full[s]);
-            tma_load_2d(b_dst + 128 * kBK, &map_b, b_col * kBK, b_row0 + p.n + n_tile * 128, &sh->full[s]);
           } else {
-            tma_load_2d(b_dst, &map_b, b_col * kBK, b_row0 + n_tile * kCols, &sh->full[s]);
+            // gate/up: 128 rows of the first half (x1) and the matching 128 rows of the second half (x2)
+            tma_load_2d(b_dst, &maps.b, b_col * kBK, b_row0 + n_tile * 128, &sh->full[s]);
+            tma_load_2d(b_dst + 128 * kBK, &maps.b, b_col * kBK, b_row0 + p.n + n_tile * 128, &sh->full[s]);
           }
+          if (MODE != kGateUp) tma_load_2d(b_dst, &maps.b, b_col * kBK, b_row0 + n_tile * kCols, &sh->full[s]);
         }
         ++k;
       }

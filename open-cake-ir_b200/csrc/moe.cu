@@ -770,13 +770,13 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
       }
       gemm::Params p = h->p1;
       p.wait_kiloclocks = test_hooks().budget_kiloclocks;
-      return launch_dependent(gemm::gemm_fp8_kernel<gemm::kGateUp>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a1, h->map_a1_tail, h->map_b1, h->map_b1_narrow, p);
+      return launch_dependent(gemm::gemm_fp8_kernel<gemm::kGateUp>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, gemm::Maps<gemm::kGateUp>{h->map_a1, h->map_a1_tail, h->map_b1, h->map_b1_narrow}, p);
     }
     case 2: {
       if (!l.token_tiles || l.core_above) {
         gemm::Params p = h->p2;
         p.wait_kiloclocks = test_hooks().budget_kiloclocks;
-        if (int rc = launch_dependent(gemm::gemm_fp8_kernel<gemm::kDown>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, h->map_a2, h->map_a2_tail, h->map_b2, h->map_b2, p))
+        if (int rc = launch_dependent(gemm::gemm_fp8_kernel<gemm::kDown>, dim3(h->grid), dim3(gemm::kThreads), gemm::kSmemBytes, s, gemm::Maps<gemm::kDown>{h->map_a2, h->map_a2_tail, h->map_b2}, p))
           return rc;
       }
       return l.token_tiles ? skinny::launch_any<gemm::kDown>(l.token_tiles, l.split2, l.terms, h->s2, h->grid, s) : 0;

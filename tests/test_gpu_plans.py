@@ -1,0 +1,44 @@
+"""Attention launches on either side of the sizes up to which the kernels plan for themselves (1024 sequences; 2048 and
+510 segments of an MLA prefill), with pieces merged by a kernel of their own or not, several ranges to a CTA, and sequences without KV rows.
+Oracles and tolerances of test_gpu_decode.py and test_gpu_prefill.py."""
+import pytest
+import torch
+
+from oracle import attention
+from test_gpu_decode import check as check_decode, run_gqa, run_mla
+from test_gpu_mla_tiles import paged
+from test_gpu_prefill import check, run
+from test_gpu_prefill_tiles import problem
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("batch,heads,kv_heads,longest", [
+    (1, 8, 1, 5000), (18, 8, 8, 700), (19, 8, 8, 700), (74, 4, 2, 300), (40, 6, 3, 900), (9, 32, 16, 1500),
+    (1024, 4, 4, 40), (1025, 4, 4, 40), (1024, 2, 1, 90)])
+def test_gqa_decode(batch, heads, kv_heads, longest):
+    lens = [0 if i % 7 == 3 else 1 + (i * 37) % longest for i in range(batch - 1)] + [longest]
+    cpu = problem(batch + heads, [1] * batch, lens, heads, kv_heads, 16)
+    want = attention.paged_decode_reference(cpu, mla=False, page_size=16, per_head_loop=False)
+    out, lse = run_gqa(cpu, longest)
+    check_decode(out, lse, want)
+
+
+@pytest.mark.parametrize("batch,longest", [(2, 3000), (1024, 70), (1025, 70)])
+def test_mla_decode(batch, longest):
+    lens = [0 if i % 7 == 3 else 1 + (i * 37) % longest for i in range(batch - 1)] + [longest]
+    cpu = paged(torch.Generator().manual_seed(batch), lens, 16, 16, batch)
+    want = attention.paged_decode_reference(cpu, mla=True, page_size=16, per_head_loop=False)
+    out, lse = run_mla(cpu, longest)
+    check_decode(out, lse, want)
+
+
+@pytest.mark.parametrize("segments,rows", [(510, 1), (511, 1), (60, 37), (60, 38)])          # 510 segments and more; room for 2024 and 2077 sequences
+def test_mla_prefill(segments, rows):
+    q_lens = [0 if i % 9 == 4 else rows for i in range(segments)]
+    kv_lens = [0 if i % 11 == 5 else q + i % 3 * 20 for i, q in enumerate(q_lens)]
+    cpu = paged(torch.Generator().manual_seed(segments + rows), kv_lens, 16, 128, sum(q_lens))
+    cpu["qo_indptr"] = torch.tensor([sum(q_lens[:i]) for i in range(len(q_lens) + 1)], dtype=torch.int32)
+    want = attention.causal_prefill_reference(cpu, mla=True, paged=True, page_size=16, nan_for_masked=True, per_head_loop=False)
+    out, lse = run(cpu, mla=True, paged=True, nan=True, max_kv_len=max(kv_lens))
+    check(out, lse, want)
