@@ -80,8 +80,8 @@ int cake_b200_test_hooks(int wait_budget_kiloclocks, int skip_load);
  * division in place of theirs (by_division), for n fp32 values on the device. */
 int cake_b200_test_silu(const void* x, void* y, void* by_division, int64_t n, void* cuda_stream);
 
-/* Test accessor: where the plan kernel of a decode handle (kind "gqa_decode" or "mla_decode", the handle of the
- * matching _create) leaves the work plan of its latest launch, as a device pointer into the caller's workspace.
+/* Test accessor: where a launch of a decode handle (kind "gqa_decode" or "mla_decode", the handle of the
+ * matching _create) leaves its work plan, as a device pointer into the caller's workspace.
  *   gqa_decode: which 0 = pieces, int32 x4 each {sequence | pieces of it << 16, first token, list index of the
  *               sequence's first piece, end token}, count = capacity; 1 = list index of each range's first piece
  *               (INT_MAX where a range is empty); 2 = pieces per range; count = ranges.

@@ -182,7 +182,7 @@ def workspace_bytes(stem: str, config) -> int:
 
 
 def decode_plan_view(stem: str, handle, which: int) -> tuple[int, int]:
-    """(device pointer, element count) of part ``which`` of the work plan a decode handle's plan kernel writes
+    """(device pointer, element count) of part ``which`` of the work plan that a launch of a decode handle writes
     (``cake_b200_decode_plan_view``; a test accessor)."""
     pointer, count = c_void_p(), c_int()
     code = library().cake_b200_decode_plan_view(stem.encode(), handle, which, ctypes.byref(pointer), ctypes.byref(count))

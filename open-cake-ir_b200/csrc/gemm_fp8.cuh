@@ -33,12 +33,21 @@ constexpr int kBM = 128;          // rows per tile = UMMA M = TMEM lanes
 constexpr int kBN = 256;          // columns per tile = UMMA N
 constexpr int kBK = 128;          // e4m3 elements (= bytes) per K block = scale granularity
 constexpr int kUmmaK = 32;        // K of one tcgen05.mma for 8-bit operands
-constexpr int kStages = 4;        // shared-memory ring depth
-constexpr int kTmemStages = 2;    // accumulator stages in tensor memory
-constexpr int kTmemColumns = kTmemStages * kBN;   // 512 = all of an SM's tensor memory
+constexpr int kTmemColumns = 512;                 // all of an SM's tensor memory
 constexpr int kBytesA = kBM * kBK;                // 16 KiB
 constexpr int kBytesB = kBN * kBK;                // 32 KiB
-constexpr int kStageBytes = kBytesA + kBytesB;
+// The rings: tiles of 256 columns, and of 128 where CTAs share K (see the kernel).  The latter have few K blocks to a CTA and wait for HBM
+// on all of them, so every stage more is a block sooner (64 x 4096 x 7168, 14 blocks to a CTA: 11.5 us with four stages of 48 KB and two
+// accumulators, 10.8 with six of 32 KB and four; 48 x 9472 x 7168 19.6 and 18.3).
+template <bool SPLIT>
+struct Ring {
+  static constexpr int kCols = SPLIT ? 128 : kBN;
+  static constexpr int kStageBytes = kBytesA + kCols * kBK;
+  static constexpr int kStages = SPLIT ? 6 : 4;            // 192 KiB of shared memory
+  static constexpr int kTmemStages = kTmemColumns / kCols;
+};
+constexpr int kRingBytes = Ring<false>::kStages * Ring<false>::kStageBytes, kMaxStages = Ring<true>::kStages, kMaxTmemStages = Ring<true>::kTmemStages;
+static_assert(Ring<true>::kStages * Ring<true>::kStageBytes <= kRingBytes && kMaxStages >= Ring<false>::kStages, "the narrow ring does not fit");
 constexpr int kTailRows = 32;                    // box rows of the small A map
 constexpr int kControlWarps = 4;                  // one warpgroup: warp 0 TMA, warp 1 MMA, warp 2 scales, warp 3 idle
 constexpr int kEpilogueWarps = 8;                 // two warpgroups: 2 column groups x 4 TMEM lane quadrants
@@ -59,8 +68,8 @@ constexpr int kItemSlots = 4;
 // stage of block it is handed back, i.e. when the MMAs of block it - kStages are done; those were issued after the epilogue
 // had read the scales of block it - kStages - kTmemStages.
 constexpr int kScaleAhead = 2;
-constexpr int kScaleSlots = 8;
-static_assert(kScaleSlots >= kStages + kTmemStages + kScaleAhead, "a slot's scales could be overwritten before they are read");
+constexpr int kScaleSlots = 16;
+static_assert(kScaleSlots >= kMaxStages + kMaxTmemStages + kScaleAhead, "a slot's scales could be overwritten before they are read");
 
 enum Mode : int {
   kDense = 0,        // C bf16 [M, N]
@@ -97,10 +106,10 @@ struct Params {
 struct Shared {
   uint4 out_rows[kEpilogueWarps][128];                      // per epilogue warp: 32 rows of 64 bytes on their way out
   int4 item[kItemSlots];                                    // group (-1: no further item), first row, rows, n tile
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
-  uint64_t tmem_full[kTmemStages];
-  uint64_t tmem_empty[kTmemStages];
+  uint64_t full[kMaxStages];
+  uint64_t empty[kMaxStages];
+  uint64_t tmem_full[kMaxTmemStages];
+  uint64_t tmem_empty[kMaxTmemStages];
   uint64_t exchange_done;                                   // kGateUp: all epilogue warps have published their amax
   uint64_t item_full[kItemSlots], item_empty[kItemSlots];   // hand-over of work items from the TMA warp to the other roles
   float scale_a[kScaleSlots][kBM];                          // sfa of the tile's rows for one K block
@@ -186,10 +195,12 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (*p.enabled == 0) return;
   }
+  constexpr int kStages = Ring<SPLIT>::kStages, kTmemStages = Ring<SPLIT>::kTmemStages, kStageBytes = Ring<SPLIT>::kStageBytes;
+  constexpr int kCols = Ring<SPLIT>::kCols;        // columns of a tile
   extern __shared__ uint8_t smem_raw[];
   // by an offset, not by rounding the pointer as an integer: the compiler then still knows that it is shared memory
   uint8_t* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  Shared* sh = reinterpret_cast<Shared*>(tiles + kStages * kStageBytes);
+  Shared* sh = reinterpret_cast<Shared*>(tiles + kRingBytes);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   uint32_t rank = 0, split = 1;
@@ -200,14 +211,13 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
   const int first_item = SPLIT ? blockIdx.x / split : blockIdx.x;
   const int k_begin = SPLIT ? int(rank * uint32_t(p.k_blocks) / split) : 0;                  // this CTA's K blocks
   const int k_count = SPLIT ? int((rank + 1) * uint32_t(p.k_blocks) / split) - k_begin : p.k_blocks;
-  constexpr int kCols = SPLIT ? 128 : kBN;         // columns of a tile
   const int n_tiles = (MODE == kGateUp) ? p.n / 128 : (p.n + kCols - 1) / kCols;
 
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0) {                          // (one after another: only those that the form has)
     for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 1 + 32); mbar_init(&sh->empty[s], 1); }
     for (int s = 0; s < kTmemStages; ++s) { mbar_init(&sh->tmem_full[s], 1); mbar_init(&sh->tmem_empty[s], kEpilogueWarps); }
-    for (int s = 0; s < kItemSlots; ++s) { mbar_init(&sh->item_full[s], 1); mbar_init(&sh->item_empty[s], 2 + kEpilogueWarps); }
-    mbar_init(&sh->exchange_done, kEpilogueWarps);
+    for (int s = 0; !SPLIT && s < kItemSlots; ++s) { mbar_init(&sh->item_full[s], 1); mbar_init(&sh->item_empty[s], 2 + kEpilogueWarps); }
+    if (MODE == kGateUp) mbar_init(&sh->exchange_done, kEpilogueWarps);
     sh->wait.abort_flag = 0;
     sh->wait.budget_kiloclocks = p.wait_kiloclocks;
     fence_barrier_init();
@@ -350,7 +360,7 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
             const uint32_t a_addr = smem_u32(tiles + s * kStageBytes);
             const uint64_t a_desc = umma_desc_sw128(a_addr);
             const uint64_t b_desc = umma_desc_sw128(a_addr + kBytesA);
-            const uint32_t d = tmem_base + t * kBN;
+            const uint32_t d = tmem_base + t * kCols;
 #pragma unroll
             for (int j = 0; j < kBK / kUmmaK; ++j) {
               // advancing K inside the 128-byte swizzle row: +32 bytes = +2 in the 16-byte address field
@@ -454,7 +464,7 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
         ok = mbar_wait(&sh->tmem_full[t], (it / kTmemStages) & 1, abort_flag, p.status, kStatusWaitTmemFull);
         if (!ok) break;
         tcgen05_fence_after();
-        const uint32_t stage_addr = lane_base + t * kBN;
+        const uint32_t stage_addr = lane_base + t * kCols;
         if (it == 0) read_scales(0);
         const float s0 = sa * sb0, s1 = MODE == kGateUp ? sa * sb1 : s0;
         const uint64_t s0p = pack_f32x2(s0, s0), s1p = pack_f32x2(s1, s1);
@@ -644,7 +654,8 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
   }
 }
 
-constexpr size_t kSmemBytes = size_t(kStages) * kStageBytes + sizeof(Shared) + 1024;
+constexpr size_t kSmemBytes = size_t(kRingBytes) + sizeof(Shared) + 1024;
+static_assert(kSmemBytes <= 232448, "the kernel's shared memory exceeds what a CTA may have on sm_100");
 
 }  // namespace gemm
 }  // namespace cake
