@@ -38,13 +38,24 @@ constexpr int kBytesA = kBM * kBK;                // 16 KiB
 constexpr int kBytesB = kBN * kBK;                // 32 KiB
 // The rings: tiles of 256 columns, and of 128 where CTAs share K (see the kernel).  The latter have few K blocks to a CTA and wait for HBM
 // on all of them, so every stage more is a block sooner (64 x 4096 x 7168, 14 blocks to a CTA: 11.5 us with four stages of 48 KB and two
-// accumulators, 10.8 with six of 32 KB and four; 48 x 9472 x 7168 19.6 and 18.3).
+// accumulators, 10.7 with six of 32 KB and four; 48 x 9472 x 7168 19.7 and 18.4).
 template <bool SPLIT>
 struct Ring {
   static constexpr int kCols = SPLIT ? 128 : kBN;
   static constexpr int kStageBytes = kBytesA + kCols * kBK;
   static constexpr int kStages = SPLIT ? 6 : 4;            // 192 KiB of shared memory
   static constexpr int kTmemStages = kTmemColumns / kCols;
+};
+// Where an index of the operand ring lies.  Six is not a power of two: stepped, since a division by it takes some 20 clocks of a K block.
+template <bool SPLIT>
+struct At {
+  uint32_t index = 0, slot_ = 0, phase_ = 0;
+  __device__ __forceinline__ void next() {
+    if (!SPLIT) ++index;
+    else if (++slot_ == uint32_t(Ring<true>::kStages)) { slot_ = 0; phase_ ^= 1; }
+  }
+  __device__ __forceinline__ uint32_t slot() const { return SPLIT ? slot_ : index % Ring<false>::kStages; }
+  __device__ __forceinline__ uint32_t phase() const { return SPLIT ? phase_ : (index / Ring<false>::kStages) & 1; }
 };
 constexpr int kRingBytes = Ring<false>::kStages * Ring<false>::kStageBytes, kMaxStages = Ring<true>::kStages, kMaxTmemStages = Ring<true>::kTmemStages;
 static_assert(Ring<true>::kStages * Ring<true>::kStageBytes <= kRingBytes && kMaxStages >= Ring<false>::kStages, "the narrow ring does not fit");
@@ -278,6 +289,7 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
       // (found between two items it delays the next one's first loads; second GEMM of 2500 tokens, two terms, hidden 2048, 128
       // experts of 768: 137 us then, 128 now).
       uint32_t it = 0, k = 0;
+      At<SPLIT> at;
       bool ok = true, valid;
       Item item;
       int g = first_item;
@@ -298,9 +310,9 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
         const int m = MODE == kDense ? (item.rows_valid <= kTailRows ? kTailRows : kBM) : tile_rows<MODE>(item.rows_valid);       // rows of A to bring in
         const uint32_t stage_tx = uint32_t(m * kBK + kCols * kBK);
         const int a_row0 = item.row0, n_tile = item.n_tile;
-        for (int kb = 0; kb < k_count; ++kb, ++it) {
-          const int s = it % kStages;
-          ok = mbar_wait(&sh->empty[s], ((it / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
+        for (int kb = 0; kb < k_count; ++kb, ++it, at.next()) {
+          const int s = at.slot();
+          ok = mbar_wait(&sh->empty[s], at.phase() ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
           if (!ok) break;
           if (kb == find_at) find(g, k + 1);                            // (this item is in the variables above)
           if (!ok) break;
@@ -335,6 +347,7 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
     // ------------------------------ MMA issuer ----------------------------------------
     if (elect_one()) {
       uint32_t it = 0, k = 0;
+      At<SPLIT> at;
       bool ok = true;
       Item item;
       for (int g = first_item; ok; g += gridDim.x, ++k) {
@@ -350,10 +363,10 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
           break;
         }
         auto products = [&](auto narrow, uint32_t idesc) {
-          for (int kb = 0; kb < k_count; ++kb, ++it) {
-            const int s = it % kStages;
+          for (int kb = 0; kb < k_count; ++kb, ++it, at.next()) {
+            const int s = at.slot();
             const int t = it % kTmemStages;
-            ok = mbar_wait_both(&sh->full[s], (it / kStages) & 1, kStatusWaitSmemFull, &sh->tmem_empty[t],
+            ok = mbar_wait_both(&sh->full[s], at.phase(), kStatusWaitSmemFull, &sh->tmem_empty[t],
                                 ((it / kTmemStages) & 1) ^ 1, kStatusWaitTmemEmpty, abort_flag, p.status);
             if (!ok) break;
             tcgen05_fence_after();
@@ -387,6 +400,7 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
     // and reading them when they are needed 75 to 170, since the reads queue behind the tensor core's operand reads.)
     const int sfb_rows = p.b_rows_per_group / 128;
     uint32_t it = 0, k = 0;
+    At<SPLIT> at;                        // of block it - kScaleAhead
     bool ok = true;
     Item item;
     for (int g = first_item; ok; g += gridDim.x, ++k) {
@@ -406,8 +420,7 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
       const int sfb_row = MODE == kGateUp ? item.n_tile + (lane & 1) * (p.n / 128) : SPLIT ? item.n_tile : min(item.n_tile * 2 + (lane & 1), sfb_rows - 1);
       const float* sfb = p.sfb + (size_t(item.group) * sfb_rows + sfb_row) * p.b_k_blocks;
       for (int kb = 0; ok && kb < k_count; ++kb, ++it) {
-        ok = it < kScaleAhead || mbar_wait(&sh->empty[(it - kScaleAhead) % kStages], (((it - kScaleAhead) / kStages) & 1) ^ 1, abort_flag,
-                                           p.status, kStatusWaitSmemEmpty);
+        ok = it < kScaleAhead || mbar_wait(&sh->empty[at.slot()], at.phase() ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
         if (!ok) break;
         int a_col = k_begin + kb, b_col = k_begin + kb;
         if (p.interleave_hi_lo) { a_col = (kb & 1) * (p.k_blocks >> 1) + (kb >> 1); b_col = kb >> 1; }
@@ -417,12 +430,12 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
         for (int j = 0; j < kBM; j += 32)
           if (MODE == kDense || j < item.rows_valid) cp_async_4(&sh->scale_a[slot][j + lane], sfa + min(item.row0 + j + lane, p.row_capacity - 1));
         if (lane < 2) cp_async_4(&sh->scale_b[slot][lane], sfb + b_col);
-        if (it >= kScaleAhead) cp_async_arrive_noinc(&sh->full[(it - kScaleAhead) % kStages]);
+        if (it >= kScaleAhead) { cp_async_arrive_noinc(&sh->full[at.slot()]); at.next(); }
       }
     }
-    for (uint32_t j = it < kScaleAhead ? 0 : it - kScaleAhead; ok && j < it; ++j) {       // the last blocks announce no further scales
-      ok = mbar_wait(&sh->empty[j % kStages], ((j / kStages) & 1) ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
-      if (ok) cp_async_arrive_noinc(&sh->full[j % kStages]);
+    for (uint32_t j = it < kScaleAhead ? 0 : it - kScaleAhead; ok && j < it; ++j, at.next()) {       // the last blocks announce no further scales
+      ok = mbar_wait(&sh->empty[at.slot()], at.phase() ^ 1, abort_flag, p.status, kStatusWaitSmemEmpty);
+      if (ok) cp_async_arrive_noinc(&sh->full[at.slot()]);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   }
