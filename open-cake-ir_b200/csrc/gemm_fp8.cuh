@@ -16,8 +16,8 @@
 // (tcgen05.ld), multiply it by the block's scales and add it to fp32 registers ("promotion"),
 // which is what arbitrary fp32 1x128 / 128x128 scales need -- the hardware block-scaled kinds
 // only take power-of-two scales per 32 elements.  While the epilogue promotes block kb the
-// tensor core already works on block kb+1 in the other stage.  Operands arrive through a
-// 4-stage TMA ring (128-byte swizzle, one elected producer thread); the MMA is issued by one
+// tensor core already works on block kb+1 in the other stage.  A group's last row tile may be one of
+// 64 or 32 rows (tile_rows).  Operands arrive through a TMA ring of four stages, six where CTAs share K (128-byte swizzle, one elected producer thread); the MMA is issued by one
 // elected thread of a second warp.  Work items are (group, n tile, m tile) with the m tile
 // fastest, so CTAs that share a weight tile run at the same time and the second reader hits L2.
 // Items either go round the CTAs in turn or are drawn from a device counter by the TMA warp, which
