@@ -219,7 +219,7 @@ gqa_plan_kernel(const Params p) {
 // A plan kernel in front costs its 5 to 6 us, most of it the way through its launch and its memory round trips, before any CTA can
 // start; here the same round trips take about two (sequences of 9000 to 32768 tokens, 3 of them: 50.6 -> 48.6 us; 64 of 512 to 4096: 105.3 -> 103.2;
 // 1 of 430: 12.2 -> 9.6; 21 of 239 to 958: 23.3 -> 22.2).
-// Counters of a launch that merges in the decode kernel are cleared by gqa_reset_kernel, beside which this runs.
+// Counters of a launch that merges in the decode kernel are cleared by gqa_reset_kernel in front.
 constexpr int kPlanHere = 2 * kWarps * 32;
 struct RangeStart { int4 rec; int first, last, page; };      // first piece of a range, list index of it and of the last, its page list
 __device__ __forceinline__ void plan_here(const Params& p, uint8_t* scratch, int range0, int ranges, RangeStart* range_start) {
@@ -283,11 +283,12 @@ __device__ __forceinline__ void plan_here(const Params& p, uint8_t* scratch, int
   __syncthreads();                                  // the list is written; the scratch goes to the rings
 }
 
-// Clears the counters of a launch whose decode kernel makes the plan and merges the pieces.
+// Clears the counters of a launch whose decode kernel makes the plan and merges the pieces.  It lets the decode grid in at once, which
+// then waits for this grid's end and by that for all that came before: only a grid's own wait makes earlier writes visible to it.
 __global__ void __launch_bounds__(1024)
 gqa_reset_kernel(int* done, int count) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // everything in front of this launch is complete: the decode kernel may plan
   const int i = blockIdx.x * 1024 + threadIdx.x;
   if (i < count) done[i] = 0;
 }
@@ -389,17 +390,14 @@ gqa_decode_kernel(const __grid_constant__ Params p) {
     kvh_mine = pair;
     active = pair < p.hkv && range_id < p.ranges;
   }
-  // Launched as a programmatic dependent.  Behind a plan kernel everything above overlaps it, the list and the counters are read
-  // only after it has completed.  Behind gqa_reset_kernel, which lets this grid in once all work before it has completed, the plan is made
-  // beside it; with neither in front nothing is read before the grids before have completed.
+  // Launched as a programmatic dependent: everything above overlaps the grid in front, nothing is read or written before that has completed.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ RangeStart range_start[kHeads];
   const int range0 = p.hkv >= kHeads || kHeads % p.hkv ? range_id : int(blockIdx.x) * (kHeads / p.hkv);
   if (p.plan_here) {
-    if (p.merge_kernel) asm volatile("griddepcontrol.wait;" ::: "memory");
     const int here = p.hkv >= kHeads || kHeads % p.hkv ? 1 : kHeads / p.hkv;
     plan_here(p, smem, range0, min(here, p.ranges - range0), range_start);
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const float scale2 = __ldg(p.sm_scale) * kLog2e;
   // Items are numbered piece * Hkv + KV head; this pair's run from idx up to (not including) total.
   int idx = 0, total = 0;

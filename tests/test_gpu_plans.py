@@ -4,6 +4,7 @@ Oracles and tolerances of test_gpu_decode.py and test_gpu_prefill.py."""
 import pytest
 import torch
 
+import open_cake_ir_b200 as cake
 from oracle import attention
 from test_gpu_decode import check as check_decode, run_gqa, run_mla
 from test_gpu_mla_tiles import paged
@@ -42,3 +43,41 @@ def test_mla_prefill(segments, rows):
     want = attention.causal_prefill_reference(cpu, mla=True, paged=True, page_size=16, nan_for_masked=True, per_head_loop=False)
     out, lse = run(cpu, mla=True, paged=True, nan=True, max_kv_len=max(kv_lens))
     check(out, lse, want)
+
+
+@pytest.mark.parametrize("batch,heads,kv_heads", [(3, 8, 8), (40, 8, 8), (80, 4, 2), (9, 16, 0)])          # merge kernel, merged in place (twice), MLA
+def test_lengths_rewritten_in_front_of_each_launch(batch, heads, kv_heads):
+    """One handle, launched behind kernels of the same stream that write its lengths and page table anew; nothing waits in between."""
+    page, longest, steps = 16, 900, 6
+    g = torch.Generator().manual_seed(batch)
+    full = paged(g, [longest] * batch, page, heads, batch) if kv_heads == 0 else problem(batch, [1] * batch, [longest] * batch, heads, kv_heads, page)
+    tables = []
+    for step in range(steps):
+        lens = torch.randint(0 if step % 2 else 300, 40 if step % 2 else longest + 1, (batch,), generator=g)
+        pages = (lens + page - 1) // page
+        indices = full["kv_indices"].clone()
+        indices[:int(pages.sum())] = torch.randperm(indices.numel(), generator=g)[:int(pages.sum())].int()
+        tables.append({"kv_indptr": torch.cat([torch.zeros(1, dtype=torch.long), pages.cumsum(0)]).int(), "kv_indices": indices,
+                       "kv_last_page_len": torch.where(pages > 0, lens - (pages - 1) * page, torch.zeros_like(lens)).int()})
+    dev = {k: v.cuda() for k, v in full.items()}
+    ready = [{k: v.cuda() for k, v in table.items()} for table in tables]
+    q = dev["q_nope"] if kv_heads == 0 else dev["q"]
+    out, lse = torch.empty_like(q), torch.empty(q.shape[:2], device="cuda")
+    if kv_heads == 0:
+        op = cake.MlaPagedDecode(q, dev["q_pe"], dev["ckv_cache"], dev["kpe_cache"], dev["kv_indptr"], dev["kv_indices"], dev["kv_last_page_len"],
+                                 dev["sm_scale"], out, lse, max_kv_len=longest)
+    else:
+        op = cake.GqaPagedDecode(q, dev["k_cache"], dev["v_cache"], dev["kv_indptr"], dev["kv_indices"], dev["kv_last_page_len"], dev["sm_scale"],
+                                 out, lse, max_kv_len=longest)
+    got = [(torch.empty_like(out), torch.empty_like(lse)) for _ in range(steps)]
+    torch.cuda.synchronize()
+    for table, (o, l) in zip(ready, got):
+        for name, value in table.items():
+            torch.add(value, 0, out=dev[name])
+        op.launch()
+        torch.mul(out, 1, out=o)
+        torch.mul(lse, 1, out=l)
+    torch.cuda.synchronize()
+    for table, (o, l) in zip(tables, got):
+        want = attention.paged_decode_reference(dict(full, **table), mla=kv_heads == 0, page_size=page, per_head_loop=False)
+        check_decode(o, l, want)
