@@ -58,7 +58,7 @@ extern "C" {
 int cake_b200_abi_version(void);
 
 /* Copies the 4-byte status word at the start of `workspace` to the host (synchronous on
- * `cuda_stream`).  0 = every kernel ran to completion; otherwise the code of the first wait
+ * `cuda_stream`).  0 = every kernel ran to completion; otherwise the code of a wait
  * that gave up (1 smem-full, 2 smem-empty, 3 tmem-full, 4 tmem-empty, 5 flag). */
 int cake_b200_read_status(const void* workspace, void* cuda_stream, int* status_out);
 

@@ -203,7 +203,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 constexpr long long kWaitClockBudget = 2000000000LL;
 
 // What a kernel with bounded waits keeps in shared memory for them: the flag any role raises when its wait
-// ran out, and the budget of a wait in units of 1024 clocks (0 = the default above).
+// ran out (the code of that wait), and the budget of a wait in units of 1024 clocks (0 = the default above).
 struct WaitControl {
   int abort_flag;
   int budget_kiloclocks;
@@ -240,14 +240,14 @@ static_assert(wait_over(7, 7 + 0x80000000u, 0, true) && wait_over(0xffffff00u, 0
 static __device__ __noinline__ bool mbar_wait_expired(uint32_t start, volatile int* abort_flag, int* status, int code) {
   if (*abort_flag) return true;
   if (!wait_over(start, kiloclock(), abort_flag[1], code == kStatusWaitSmemEmpty)) return false;
-  *abort_flag = 1;
+  *abort_flag = code;
   if (status) atomicCAS(status, 0, code);
   return true;
 }
 
 // Wait for `parity` of `bar`.  Gives up when the budget runs out or when another role of the
 // CTA has already raised the abort flag (`abort_flag` points at a WaitControl); on giving up it raises the
-// flag, records `code` in the global status word and returns false so that the caller can unwind.
+// flag, records `code` in the global status word (if there is one) and returns false so that the caller can unwind.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code) {
   const uint32_t start = kiloclock();

@@ -72,6 +72,7 @@ struct Params {
   int* cut_count;
   int* tile_prefix;       // [sequences + 1] work units (tiles + start-up shares) before a sequence, from the plan
   int* status;
+  uint8_t* codes;         // [CTAs] why a CTA of the decode kernel gave up (0: it did not), from which the reduce kernel makes the status word
   int sequences, heads, page_size, workers;
   int rows;               // result rows of a sequence: all heads of a token, of `pack` tokens in the prefill form
   int pack;               // tokens of a sequence (1 unless prefill packs several)
@@ -87,6 +88,7 @@ struct Params {
   int* seq_count;
   int* segment_prefix;
   int plan_here;          // every CTA of the decode kernel makes the plan itself
+  int code_count;         // CTAs of the decode kernel
   const int* qo_indptr;
   int segments, total_q, nan_for_masked;
   int out_align;          // the widest store that the address of `out` allows: 32, 16 or 8 bytes
@@ -306,10 +308,7 @@ static __device__ __noinline__ int2 plan_here(const Params& p, int* scratch, int
   }
   if (tid == 0) {
     prefix[count] = total;
-    if (blockIdx.x == 0) {
-      p.tile_prefix[count] = total;
-      *p.status = 0;
-    }
+    if (blockIdx.x == 0) p.tile_prefix[count] = total;
   }
   if (blockIdx.x == 0) list_cuts(p, prefix, count, total, sums);
   __syncthreads();
@@ -843,6 +842,7 @@ mla_decode_kernel(const __grid_constant__ Params p) {
 
   tcgen05_fence_before();
   __syncthreads();
+  if (p.codes && threadIdx.x == 0) p.codes[blockIdx.x] = uint8_t(sh->wait.abort_flag);
   if (sh->wait.abort_flag) settle_after_abort();   // (the CTA that issues gives up where the other one does: it waits for that one's rows and weights)
   cluster_sync();                                  // neither CTA leaves while the other may still reach into it
   tcgen05_fence_after();
@@ -856,6 +856,16 @@ mla_reduce_kernel(const Params p) {
   // launched as a programmatic dependent of the decode kernel, which never lets it in early: it starts as that one's CTAs leave
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // The last row of CTAs makes the status word of the codes that the decode kernel's CTAs have left.  (With one of those clearing the word as
+  // it starts and the others reporting to it, what is reported before that one starts would be lost.)
+  if (blockIdx.y + 1 == gridDim.y) {
+    if (blockIdx.x > 0 || threadIdx.x >= 32) return;
+    int code = 0;
+    for (int i = threadIdx.x; i < p.code_count; i += 32) { const int c = p.codes[i]; code = code ? code : c; }
+    const uint32_t failed = __ballot_sync(0xffffffffu, code != 0);
+    if (int(threadIdx.x) == (failed ? __ffs(failed) - 1 : 0)) *p.status = code;
+    return;
+  }
   if (int(blockIdx.y) >= *p.cut_count) return;
   const int4 cut = p.cuts[blockIdx.y];
   const int b = cut.x, first = cut.y, last = cut.z;
@@ -909,6 +919,10 @@ struct Handle {
 
 constexpr int kMaxWorkers = 96;                            // pairs of SMs the workspace is sized for
 
+// The status block: the status word, and from byte 64 a code of every CTA of the decode kernel.
+constexpr size_t kCodesAt = 64;
+static_assert(kCodesAt + 2 * kMaxWorkers <= 256, "the codes do not fit into the status block");
+
 // Workspace behind the 256-byte status block: tile_prefix [sequences + 1] int | cuts [kMaxWorkers] int4, their number | part_o [slots, rows, 512] f32 | part_lse [slots, rows],
 // and for the prefill form seq [sequences] int4 | seq_page [sequences] | segment_prefix [segments + 3] | seq_count [1]
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -959,14 +973,20 @@ inline int launch(const Handle* h, cudaStream_t s) {
   Params p = h->p;
   p.wait_kiloclocks = test_hooks().budget_kiloclocks;
   p.skip_load = test_hooks().skip_load;
-  p.plan_here = p.seq ? p.sequences <= kPlanPrefill && p.segments <= kPlanSegments : p.sequences <= kPlanSequences;
+  if (p.workers > 1) {                                       // else there is no reduce kernel: the plan kernel clears the word, reports go there
+    p.codes = reinterpret_cast<uint8_t*>(p.status) + kCodesAt;
+    p.code_count = p.workers * head_blocks(p.rows) * 2;
+  }
+  p.plan_here = p.workers > 1 && (p.seq ? p.sequences <= kPlanPrefill && p.segments <= kPlanSegments : p.sequences <= kPlanSequences);
   if (!p.plan_here)
     if (int rc = launch_dependent(p.seq ? mla_prefill_plan_kernel : mla_plan_kernel, dim3(1), dim3(1024), 0, s, p)) return rc;
   const dim3 grid(p.workers * head_blocks(p.rows) * 2);
-  if (int rc = launch_dependent_cluster(2, p.sparse_indices ? mla_decode_kernel<true> : mla_decode_kernel<false>, grid, dim3(kThreads), kSmemBytes, s, p))
+  Params decode = p;
+  if (p.codes) decode.status = nullptr;
+  if (int rc = launch_dependent_cluster(2, p.sparse_indices ? mla_decode_kernel<true> : mla_decode_kernel<false>, grid, dim3(kThreads), kSmemBytes, s, decode))
     return rc;
   if (p.workers == 1) return 0;                              // nothing is ever cut
-  return launch_dependent(mla_reduce_kernel, dim3((p.rows + 1) / 2, p.workers - 1 < p.sequences ? p.workers - 1 : p.sequences), dim3(256), 0, s, p);
+  return launch_dependent(mla_reduce_kernel, dim3((p.rows + 1) / 2, (p.workers - 1 < p.sequences ? p.workers - 1 : p.sequences) + 1), dim3(256), 0, s, p);
 }
 
 }  // namespace mla

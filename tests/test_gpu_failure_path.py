@@ -10,6 +10,7 @@ import torch
 
 import open_cake_ir_b200 as cake
 from oracle import attention, block_scaled_gemm, compare
+from test_gpu_mla_tiles import paged
 from test_gpu_prefill_tiles import problem
 
 pytestmark = pytest.mark.gpu
@@ -49,6 +50,26 @@ def test_mla_decode_wait_runs_out_and_the_handle_stays_usable(hooks):
     assert hooks(0, 0) == 0
     op.launch()
     assert op.status() == 0
+    want = attention.paged_decode_reference(cpu, mla=True, page_size=64, per_head_loop=False)
+    assert compare.compare(out, want["output"], atol=2.0 ** -16, rtol=2.0 ** -7)[0]
+    assert compare.compare(lse, want["lse"], atol=1e-4, rtol=1e-5, ieee=True)[0]
+
+
+@pytest.mark.parametrize("lens,heads", [
+    ([6000, 9000], 128),                       # every CTA has a code of its own, the reduce kernel makes the status word of them
+    ([400], 2500)])                            # one range for all SMs, so no reduce kernel: the plan kernel clears the word, CTAs report to it
+def test_mla_status_word_whatever_it_held_before(hooks, lens, heads):
+    cpu = paged(torch.Generator().manual_seed(heads), lens, 64, heads, len(lens))
+    dev = {k: v.cuda() for k, v in cpu.items()}
+    out = torch.zeros_like(dev["q_nope"]); lse = torch.zeros((len(lens), heads), device="cuda")
+    op = cake.MlaPagedDecode(dev["q_nope"], dev["q_pe"], dev["ckv_cache"], dev["kpe_cache"], dev["kv_indptr"], dev["kv_indices"],
+                             dev["kv_last_page_len"], dev["sm_scale"], out, lse, max_kv_len=max(lens))
+    at = op.workspace_ptr - op.workspace.data_ptr()
+    for skip in (0, 1, 0):
+        op.workspace[at:at + 256] = 0xa5       # the library's block: nothing in it has to survive, or be zero
+        assert hooks(2048 if skip else 0, skip) == 0
+        op.launch()
+        assert 1 <= op.status() <= 5 if skip else op.status() == 0
     want = attention.paged_decode_reference(cpu, mla=True, page_size=64, per_head_loop=False)
     assert compare.compare(out, want["output"], atol=2.0 ** -16, rtol=2.0 ** -7)[0]
     assert compare.compare(lse, want["lse"], atol=1e-4, rtol=1e-5, ieee=True)[0]
