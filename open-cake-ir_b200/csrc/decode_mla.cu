@@ -89,6 +89,7 @@ struct Params {
   int* segment_prefix;
   int plan_here;          // every CTA of the decode kernel makes the plan itself
   int code_count;         // CTAs of the decode kernel
+  int reduce_columns;     // CTAs of the reduce kernel that share a sequence's rows
   const int* qo_indptr;
   int segments, total_q, nan_for_masked;
   int out_align;          // the widest store that the address of `out` allows: 32, 16 or 8 bytes
@@ -175,13 +176,23 @@ __device__ __forceinline__ void list_cuts(const Params& p, const int* prefix, in
   if (threadIdx.x == 0) *p.cut_count = *listed;
 }
 
+// Why this CTA gave up.  (Out of line, as its registers are those of the loops.)
+static __device__ __noinline__ void leave_code(const Params& p, int code) {
+  if (p.codes && threadIdx.x == 0) p.codes[blockIdx.x] = uint8_t(code);
+}
+// What the plan kernel in front of a launch clears.
+__device__ __forceinline__ void clear_status(const Params& p) {
+  if (threadIdx.x == 0) *p.status = 0;
+  if (int(threadIdx.x) < p.code_count) p.codes[threadIdx.x] = 0;
+}
+
 // One CTA: tile_prefix[b] = units before sequence b (exclusive scan), tile_prefix[B] = all units.
 static __global__ void __launch_bounds__(1024)
 mla_plan_kernel(const Params p) {
   __shared__ int sums[32];
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the decode grid may become resident now; it waits for this grid's end
-  if (threadIdx.x == 0) *p.status = 0;
+  clear_status(p);
   int before = 0;
   for (int base = 0; base < p.sequences; base += 1024) {
     const int b = base + threadIdx.x;
@@ -249,7 +260,8 @@ mla_prefill_plan_kernel(const Params p) {
     if (t < count) p.tile_prefix[t] = mine;
     units += all;
   }
-  if (tid == 0) { p.tile_prefix[count] = units; *p.seq_count = count; *p.status = 0; }
+  if (tid == 0) { p.tile_prefix[count] = units; *p.seq_count = count; }
+  clear_status(p);
   list_cuts(p, p.tile_prefix, count, units, sums);
 }
 
@@ -308,6 +320,7 @@ static __device__ __noinline__ int2 plan_here(const Params& p, int* scratch, int
   }
   if (tid == 0) {
     prefix[count] = total;
+    p.codes[blockIdx.x] = 0;
     if (blockIdx.x == 0) p.tile_prefix[count] = total;
   }
   if (blockIdx.x == 0) list_cuts(p, prefix, count, total, sums);
@@ -842,35 +855,47 @@ mla_decode_kernel(const __grid_constant__ Params p) {
 
   tcgen05_fence_before();
   __syncthreads();
-  if (p.codes && threadIdx.x == 0) p.codes[blockIdx.x] = uint8_t(sh->wait.abort_flag);
-  if (sh->wait.abort_flag) settle_after_abort();   // (the CTA that issues gives up where the other one does: it waits for that one's rows and weights)
+  if (sh->wait.abort_flag) {
+    leave_code(p, sh->wait.abort_flag);
+    settle_after_abort();                          // (the CTA that issues gives up where the other one does: it waits for that one's rows and weights)
+  }
   cluster_sync();                                  // neither CTA leaves while the other may still reach into it
   tcgen05_fence_after();
   if (warp == kMmaWarp) tmem_dealloc_pair(tmem_base, kTmemColumns);
 }
 
-// Merges the pieces of the cut sequences: CTA (x, y) two rows of the y-th, 128 threads x 4 dims each, the results of four
+// Merges the pieces of the cut sequences: a CTA two rows of one, 128 threads x 4 dims each, the results of four
 // pieces in flight (most sequences have two to four; eight in flight take registers from half of the resident rows).
 static __global__ void __launch_bounds__(256, 4)
 mla_reduce_kernel(const Params p) {
   // launched as a programmatic dependent of the decode kernel, which never lets it in early: it starts as that one's CTAs leave
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // The last row of CTAs makes the status word of the codes that the decode kernel's CTAs have left.  (With one of those clearing the word as
+  // The first CTA makes the status word of the codes that the decode kernel's CTAs have left.  (With one of those clearing the word as
   // it starts and the others reporting to it, what is reported before that one starts would be lost.)
-  if (blockIdx.y + 1 == gridDim.y) {
-    if (blockIdx.x > 0 || threadIdx.x >= 32) return;
-    int code = 0;
-    for (int i = threadIdx.x; i < p.code_count; i += 32) { const int c = p.codes[i]; code = code ? code : c; }
-    const uint32_t failed = __ballot_sync(0xffffffffu, code != 0);
-    if (int(threadIdx.x) == (failed ? __ffs(failed) - 1 : 0)) *p.status = code;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x >= 32) return;
+    uint32_t least = 0xff;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {                  // four codes at a time
+      const int at = 4 * (32 * j + int(threadIdx.x));
+      const uint32_t four = at < p.code_count ? *reinterpret_cast<const uint32_t*>(p.codes + at) : 0u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t code = four >> (8 * i) & 0xff;
+        if (code && at + i < p.code_count) least = min(least, code);
+      }
+    }
+    least = __reduce_min_sync(0xffffffffu, least);
+    if (threadIdx.x == 0) *p.status = least == 0xff ? 0 : int(least);
     return;
   }
-  if (int(blockIdx.y) >= *p.cut_count) return;
-  const int4 cut = p.cuts[blockIdx.y];
+  const int column = int(blockIdx.x - 1) % p.reduce_columns, nth = int(blockIdx.x - 1) / p.reduce_columns;
+  if (nth >= *p.cut_count) return;
+  const int4 cut = p.cuts[nth];
   const int b = cut.x, first = cut.y, last = cut.z;
   const int4 s = p.seq ? p.seq[b] : make_int4(b, 1, 0, 0);
-  const int row = blockIdx.x * 2 + (threadIdx.x >> 7), d = (threadIdx.x & 127) * 4;
+  const int row = column * 2 + (threadIdx.x >> 7), d = (threadIdx.x & 127) * 4;
   if (row >= s.y * p.heads) return;
   auto slot_row = [&](int k) { return size_t(k == first ? cut.w : 2 * k) * p.rows + row; };
   float mm = -INFINITY, weight = 0.f;
@@ -921,7 +946,7 @@ constexpr int kMaxWorkers = 96;                            // pairs of SMs the w
 
 // The status block: the status word, and from byte 64 a code of every CTA of the decode kernel.
 constexpr size_t kCodesAt = 64;
-static_assert(kCodesAt + 2 * kMaxWorkers <= 256, "the codes do not fit into the status block");
+static_assert(kCodesAt + 2 * kMaxWorkers <= 256 && 2 * kMaxWorkers <= 2 * 32 * 4, "the codes do not fit into the status block, or one look of a warp");
 
 // Workspace behind the 256-byte status block: tile_prefix [sequences + 1] int | cuts [kMaxWorkers] int4, their number | part_o [slots, rows, 512] f32 | part_lse [slots, rows],
 // and for the prefill form seq [sequences] int4 | seq_page [sequences] | segment_prefix [segments + 3] | seq_count [1]
@@ -986,7 +1011,8 @@ inline int launch(const Handle* h, cudaStream_t s) {
   if (int rc = launch_dependent_cluster(2, p.sparse_indices ? mla_decode_kernel<true> : mla_decode_kernel<false>, grid, dim3(kThreads), kSmemBytes, s, decode))
     return rc;
   if (p.workers == 1) return 0;                              // nothing is ever cut
-  return launch_dependent(mla_reduce_kernel, dim3((p.rows + 1) / 2, (p.workers - 1 < p.sequences ? p.workers - 1 : p.sequences) + 1), dim3(256), 0, s, p);
+  p.reduce_columns = (p.rows + 1) / 2;
+  return launch_dependent(mla_reduce_kernel, dim3(1 + p.reduce_columns * (p.workers - 1 < p.sequences ? p.workers - 1 : p.sequences)), dim3(256), 0, s, p);
 }
 
 }  // namespace mla
