@@ -117,7 +117,7 @@ OPERATORS = {
     "mla_prefill": (MlaPrefillConfig, True),
 }
 # every symbol include/cake_b200.h declares
-EXPORTS = (["cake_b200_abi_version", "cake_b200_read_status", "cake_b200_test_hooks", "cake_b200_test_silu", "cake_b200_launch_facts", "cake_b200_decode_plan_view", "cake_b200_moe_intermediate", "cake_b200_moe_launch_stage",
+EXPORTS = (["cake_b200_abi_version", "cake_b200_read_status", "cake_b200_test_hooks", "cake_b200_test_silu", "cake_b200_launch_facts", "cake_b200_decode_plan_view", "cake_b200_moe_dispatch", "cake_b200_moe_intermediate", "cake_b200_moe_launch_stage",
             "cake_b200_gqa_decode_noalloc", "cake_b200_gqa_decode_noalloc_scratch_limit",
             "cake_b200_ep_row_bytes", "cake_b200_ep_exchange_create", "cake_b200_ep_exchange_launch_stage",
             "cake_b200_ep_exchange_destroy", "cake_b200_ep_push_symmetric_bytes", "cake_b200_ep_push_scratch_bytes",
@@ -142,6 +142,7 @@ def library() -> ctypes.CDLL:
         lib.cake_b200_test_silu.argtypes = [c_void_p, c_void_p, c_void_p, ctypes.c_int64, c_void_p]
         lib.cake_b200_launch_facts.argtypes = [ctypes.c_char_p, POINTER(c_int), POINTER(c_int)]
         lib.cake_b200_decode_plan_view.argtypes = [ctypes.c_char_p, c_void_p, c_int, POINTER(c_void_p), POINTER(c_int)]
+        lib.cake_b200_moe_dispatch.argtypes = [POINTER(MoeConfig), POINTER(c_int)]
         lib.cake_b200_moe_intermediate.argtypes = [c_void_p, c_int, POINTER(c_void_p)]
         lib.cake_b200_moe_launch_stage.argtypes = [c_void_p, c_int, c_void_p]
         lib.cake_b200_gqa_decode_noalloc.argtypes = [POINTER(c_void_p), POINTER(GqaDecodeConfig), c_void_p]
@@ -189,6 +190,15 @@ def decode_plan_view(stem: str, handle, which: int) -> tuple[int, int]:
     if code != 0:
         raise CakeError("cake_b200_decode_plan_view", code)
     return int(pointer.value or 0), int(count.value)
+
+
+def moe_dispatch(config) -> dict:
+    """Which kernels a layer of this configuration takes (``cake_b200_moe_dispatch``; a test accessor)."""
+    out = (c_int * 5)()
+    code = library().cake_b200_moe_dispatch(ctypes.byref(config), out)
+    if code != 0:
+        raise CakeError("cake_b200_moe_dispatch", code)
+    return dict(zip(("token_tiles", "split_gate_up", "split_down", "core_above", "one_routing_kernel"), out))
 
 
 class NativeHandle:

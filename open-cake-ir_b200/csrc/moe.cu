@@ -459,29 +459,39 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
   // 61 tiles 42 and 55, 115 tiles 65 and 65, 162 tiles 87 and 91, 204 tiles 99 and 95, 3600 tiles 1648 and 1509; hidden 2048,
   // experts of 768: 135 tiles 40 and 44, 175 tiles 52 and 52, 490 tiles 97 and 88).  With two terms the core reads a weight block of the
   // second product once per term (162 tiles 90 and 97, 241 tiles 136 and 134; 768: 247 tiles 61 and 63, 310 tiles 70 and 71).  Rows: an
-  // item of the weight-streaming kernel has 8 or 16, products in proportion (4 experts of 2048: 57 and 62 at 4 rows on average, 61 and
-  // 63 at 6, 73 and 66 at 10; 8 experts: 83 and 82 at 4, 91 and 85 at 6).
+  // item of the weight-streaming kernel has 8 or 16, products in proportion, so that from six rows on it takes the few tiles on which the core
+  // leaves most SMs idle: up to a quarter of a tile to an SM, and of four experts as many rows and tiles as the core takes about as long for
+  // (of 256 experts, with the core's launches beside it where there are any, see below: 2 of 2048 39 and 52 us at 6 rows on average, 43 and 54 at 8, 49 and
+  // 55 at 10; 4 of them 59 and 59 at 6, 62 and 60 at 8; 8 83 and 82 at 6; 4 of 1536, hidden 4096, 38 and 40 at 6, 40 and 41 at 8, 46 and 41 at 10, 8 of them
+  // 53 and 47 at 6; 4 of 768, hidden 2048, 22 and 29 at 6, 25 and 30 at 10, 8 of them 32 and 30 at 6; 8 of 512, hidden 1024, 22 and 24 at 6 and 8).
   const double per_expert = double(pairs) / c.experts;
   double missed = 1;                     // experts that get a row: those not missed by every token
   for (int64_t t = 0; t < c.tokens && missed > 1e-3; ++t) missed *= 1.0 - double(c.top_k) / c.experts;
   const double touched = c.local_experts * (1 - missed);
-  if (per_expert <= 5 && touched * (c.intermediate / 128) <= (l.terms == 2 ? 2.1 : 1.2) * sms) {
+  const double tiles = touched * (c.intermediate / 128);
+  if (per_expert <= 5 ? tiles <= (l.terms == 2 ? 2.1 : 1.2) * sms
+                      : per_expert <= 11 && (tiles <= 0.25 * sms || (touched <= 4 && per_expert * tiles <= 2.7 * sms))) {
     l.token_tiles = per_expert <= 3 ? 1 : 2;
     l.split1 = skinny::choose_split_gate_up(touched > 1 ? touched : 1, c.intermediate, c.hidden / 128, sms);
     l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128, sms);
     if (l.split1 > 1) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation
     // The routing may be anything but even: the padding of a batch, or a batch of one prompt, goes to the same top_k experts.  The
     // weight-streaming kernel then reads their weights once per item of 8 token_tiles rows, so experts of many rows (four times the
-    // average, which chance does not reach) go to the core: 96 equal tokens, hidden 7168, 256 experts of 2048: 684 us without,
-    // 163 with.  The core's two launches cost 3 us where no expert takes them, so not where such tokens would read
-    // less than 400 MB again (64 us at the copy rate): there the weight-streaming kernel is the faster one even so (96 equal
-    // tokens, hidden 2048, 128 experts of 768, 189 MB: 74 us, 82 on the core alone).
+    // average, which chance does not reach) go to the core (hidden 7168, 8 of 256 experts of 2048, all 96 tokens equal: 595 us
+    // streamed, 130 so, 89 on the core alone; half of them equal: 333, 108, 86; none: 72, 74.5, 74).  The core's two launches cost 3 us where
+    // no expert takes them, a tenth of a step on small experts, so not where such tokens would read less than 400 MB again (64 us at the copy
+    // rate; hidden 2048, 16 of 256 experts of 768, all 64 tokens equal, 264 MB: 67 us streamed, 33 on the core alone; none: 28.5 and 32).
     const double items = double((c.tokens + 8 * l.token_tiles - 1) / (8 * l.token_tiles)), chosen = c.top_k < c.local_experts ? c.top_k : c.local_experts;
     const int above = per_expert <= 4 ? 16 : int(4 * per_expert);
     if (c.tokens > above && (items - 1) * chosen * 3 * c.hidden * c.intermediate > 4e8) l.core_above = above;
   }
   l.total = at;
   return l;
+}
+
+// Routing and placement in one kernel.
+inline bool routes_in_one(const cake_b200_moe_config& c, const Layout& l) {
+  return !c.external_routing && c.tokens <= kSmallTokens && l.token_tiles && !l.core_above;
 }
 
 struct MoeHandle {
@@ -590,6 +600,18 @@ static bool moe_config_ok(const cake_b200_moe_config& c) {
 extern "C" size_t cake_b200_moe_workspace_bytes(const cake_b200_moe_config* config) {
   if (!config || !moe_config_ok(*config)) return 0;
   return cake::moe::make_layout(*config).total;
+}
+
+extern "C" int cake_b200_moe_dispatch(const cake_b200_moe_config* config, int* out) {
+  using namespace cake;
+  if (!config || !out || !moe_config_ok(*config)) return kErrBadArgument;
+  const moe::Layout l = moe::make_layout(*config);
+  out[0] = l.token_tiles;
+  out[1] = l.split1;
+  out[2] = l.split2;
+  out[3] = l.core_above;
+  out[4] = moe::routes_in_one(*config, l);
+  return 0;
 }
 
 extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* config, void** handle_out) {
@@ -741,7 +763,7 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
       const moe::Gather gather{h->hidden, h->hidden_scale, h->route_weights, h->ws + l.x_perm, reinterpret_cast<float*>(h->ws + l.sx_perm),
                                reinterpret_cast<float*>(h->ws + l.row_weight), tokens, c.hidden, c.top_k, l.capacity,
                                l.core_above, 8 * l.token_tiles, clear + kCoreWord};
-      if (!c.external_routing && tokens <= moe::kSmallTokens && l.token_tiles && !l.core_above) {
+      if (moe::routes_in_one(c, l)) {
         const int epl = (c.experts + 31) / 32;
         auto* kernel = epl <= 2 ? moe::route_place_kernel<2> : epl <= 4 ? moe::route_place_kernel<4> : epl <= 8 ? moe::route_place_kernel<8> : moe::route_place_kernel<16>;
         return launch_dependent(kernel, dim3(1), dim3(32 * tokens), 0, s, h->logits, h->bias, h->factor, h->local_offset, h->expert_ids, h->route_weights,

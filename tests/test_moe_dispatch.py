@@ -1,0 +1,43 @@
+"""Which kernels an MoE layer takes (csrc/moe.cu, make_layout), on either side of each line of the rule, asked of the library on the host."""
+import pytest
+
+import open_cake_ir_b200 as cake
+
+
+def form(tokens, hidden, inter, experts, local, act="fp8", external=False, top_k=8):
+    cfg = cake._lib.MoeConfig(tokens, hidden, inter, experts, local, top_k, 8, 4, 1, int(act == "split"), int(external))
+    return cake._lib.moe_dispatch(cfg)
+
+
+@pytest.mark.parametrize("tokens,hidden,inter,experts,local,act,token_tiles", [
+    # up to five rows on average: by the tiles of the first product (148 SMs: 177.6, two terms 310.8)
+    (96, 7168, 2048, 256, 8, "fp8", 1), (97, 7168, 2048, 256, 8, "fp8", 2),            # three rows: items of 8, of 16
+    (160, 7168, 2048, 256, 8, "fp8", 2), (161, 7168, 2048, 256, 8, "fp8", 0),          # five rows
+    (36, 7168, 2048, 256, 16, "fp8", 1), (40, 7168, 2048, 256, 16, "fp8", 0),          # 174 and 184 tiles
+    (29, 7168, 2048, 256, 32, "split", 1), (31, 7168, 2048, 256, 32, "split", 0),      # 308 and 321
+    (64, 7168, 2048, 256, 256, "fp8", 0), (96, 2048, 768, 128, 128, "fp8", 0),
+    # six to eleven rows: few tiles, or up to four experts
+    (192, 7168, 2048, 256, 2, "fp8", 2), (352, 7168, 2048, 256, 2, "split", 2), (353, 7168, 2048, 256, 2, "split", 0),
+    (192, 2048, 768, 256, 4, "fp8", 2), (320, 2048, 768, 256, 4, "fp8", 2), (192, 2048, 768, 256, 8, "fp8", 0),
+    (192, 1024, 512, 256, 8, "split", 2), (320, 1024, 512, 256, 8, "fp8", 2),
+    (192, 7168, 2048, 256, 4, "split", 2), (256, 7168, 2048, 256, 4, "split", 0),      # 382 and 511 rows x tiles, line at 400
+    (256, 4096, 1536, 256, 4, "fp8", 2), (320, 4096, 1536, 256, 4, "fp8", 0)])
+def test_weight_streaming_or_core(tokens, hidden, inter, experts, local, act, token_tiles):
+    assert form(tokens, hidden, inter, experts, local, act)["token_tiles"] == token_tiles
+
+
+@pytest.mark.parametrize("tokens,one", [(1, 1), (8, 1), (9, 0)])
+def test_one_kernel_for_routing_and_placement(tokens, one):
+    assert form(tokens, 2048, 768, 64, 16)["one_routing_kernel"] == one
+    assert form(tokens, 2048, 768, 64, 16, external=True)["one_routing_kernel"] == 0
+
+
+@pytest.mark.parametrize("tokens,local,act,above", [
+    (16, 8, "fp8", 0), (17, 8, "fp8", 16), (160, 8, "fp8", 20), (36, 16, "fp8", 16), (29, 32, "split", 16), (40, 16, "fp8", 0)])
+def test_experts_of_many_rows_go_to_the_core(tokens, local, act, above):
+    assert form(tokens, 7168, 2048, 256, local, act)["core_above"] == above
+
+
+def test_what_no_layer_is_made_of_is_refused():
+    with pytest.raises(cake._lib.CakeError):
+        form(4, 7168 + 1, 2048, 256, 8)
