@@ -23,7 +23,7 @@
  * bakes shapes into emitted code), and a device status word at the start of the workspace
  * that a kernel sets when one of its bounded waits runs out (read it with
  * cake_b200_read_status after synchronising the stream).  The first 256 bytes of a workspace
- * are the library's (the status word, then the counters its kernels draw work items from);
+ * are the library's (the status word, then counters that its kernels draw work items from and codes that they make the word of);
  * `launch` clears what it uses on the stream, so a workspace needs no initialisation.
  * Output alignment: the attention operators write `output` eight bytes at a time or wider, as its address
  * allows, so it must lie on an 8-byte boundary (create refuses it otherwise); every other bf16 or e4m3 buffer

@@ -154,7 +154,7 @@ struct Item {
 
 // Rows of the product that a tile takes.  Groups seldom end on 128 rows: an expert of 128 rows on average has a few in a second
 // tile half of the time, and in a step of some hundred tokens it has ten or thirty in all.  A tile of 32 or 64 rows (the
-// weight-stationary products) takes 318 or 334 clocks of tensor pipe a K block instead of 512, a quarter or half of the
+// weight-stationary products) takes 307 or 323 clocks of tensor pipe a K block (429 or 449 with the two commits behind each) instead of 512, a quarter or half of the
 // promotion and less of A; under the power cap what it does not do is time for the others (hidden 7168, 256 experts of 2048, all
 // with as many rows: 2380 -> 1830 us at 32, 2566 -> 2090 at 64, 4116 -> 3660 at 137; at 128 there is nothing to gain).
 template <int MODE>
@@ -240,7 +240,9 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
   // launched as a programmatic dependent where the caller says so: everything above overlaps the kernel before
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (MODE == kDense && !p.queue && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;      // long before any wait can run out
+  // Long before any wait can run out, as the grid fits the GPU and its CTAs start together.  (Were the SMs of CTA 0 held by other work for the second that a
+  // wait takes to run out, its report would be lost; a kernel in front that clears the word takes 0.4 us of 7 to 21, 0.7 to 1.2 launched from the host.)
+  if (MODE == kDense && !p.queue && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;
   if (warp == kControlWarps) {   // m-tile prefix over groups (serial per lane chunk, then a warp scan)
     int running = 0;
     for (int base = 0; base < p.groups; base += 32) {
@@ -324,20 +326,22 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
           mbar_arrive_expect_tx(&sh->full[s], stage_tx);
           tma_load_2d_hint(a_dst, m < kBM ? &maps.a_tail : &maps.a, a_col * kBK, a_row0, &sh->full[s], keep);
           if (MODE != kDense && m == 64) tma_load_2d_hint(a_dst + kTailRows * kBK, &maps.a_tail, a_col * kBK, a_row0 + kTailRows, &sh->full[s], keep);
-          if constexpr (MODE == kGateUp)
-          if (m < kBM) {
-            // 32 rows of x1, the matching 32 of x2, the next 32 of x1, ...: an epilogue thread of a narrow tile holds both of a feature
+          if constexpr (MODE == kGateUp) {
+            if (m < kBM) {
+              // 32 rows of x1, the matching 32 of x2, the next 32 of x1, ...: an epilogue thread of a narrow tile holds both of a feature
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              tma_load_2d(b_dst + (2 * i) * 32 * kBK, &maps.b_narrow, b_col * kBK, b_row0 + n_tile * 128 + 32 * i, &sh->full[s]);
-              tma_load_2d(b_dst + (2 * i + 1) * 32 * kBK, &maps.b_narrow, b_col * kBK, b_row0 + p.n + n_tile * 128 + 32 * i, &sh->full[s]);
+              for (int i = 0; i < 4; ++i) {
+                tma_load_2d(b_dst + (2 * i) * 32 * kBK, &maps.b_narrow, b_col * kBK, b_row0 + n_tile * 128 + 32 * i, &sh->full[s]);
+                tma_load_2d(b_dst + (2 * i + 1) * 32 * kBK, &maps.b_narrow, b_col * kBK, b_row0 + p.n + n_tile * 128 + 32 * i, &sh->full[s]);
+              }
+            } else {
+              // 128 rows of the first half (x1) and the matching 128 rows of the second half (x2)
+              tma_load_2d(b_dst, &maps.b, b_col * kBK, b_row0 + n_tile * 128, &sh->full[s]);
+              tma_load_2d(b_dst + 128 * kBK, &maps.b, b_col * kBK, b_row0 + p.n + n_tile * 128, &sh->full[s]);
             }
           } else {
-            // gate/up: 128 rows of the first half (x1) and the matching 128 rows of the second half (x2)
-            tma_load_2d(b_dst, &maps.b, b_col * kBK, b_row0 + n_tile * 128, &sh->full[s]);
-            tma_load_2d(b_dst + 128 * kBK, &maps.b, b_col * kBK, b_row0 + p.n + n_tile * 128, &sh->full[s]);
+            tma_load_2d(b_dst, &maps.b, b_col * kBK, b_row0 + n_tile * kCols, &sh->full[s]);
           }
-          if (MODE != kGateUp) tma_load_2d(b_dst, &maps.b, b_col * kBK, b_row0 + n_tile * kCols, &sh->full[s]);
         }
         ++k;
       }

@@ -480,7 +480,8 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
     // average, which chance does not reach) go to the core (hidden 7168, 8 of 256 experts of 2048, all 96 tokens equal: 595 us
     // streamed, 130 so, 89 on the core alone; half of them equal: 333, 108, 86; none: 72, 74.5, 74).  The core's two launches cost 3 us where
     // no expert takes them, a tenth of a step on small experts, so not where such tokens would read less than 400 MB again (64 us at the copy
-    // rate; hidden 2048, 16 of 256 experts of 768, all 64 tokens equal, 264 MB: 67 us streamed, 33 on the core alone; none: 28.5 and 32).
+    // rate; hidden 2048, 16 of 256 experts of 768, all 64 tokens equal, 264 MB: 67 us streamed, 33 on the core alone; none: 28.5 and 32; 4 of them, all
+    // 192 tokens equal: 111 and 36, a quarter 48 and 31, none 22 and 29).
     const double items = double((c.tokens + 8 * l.token_tiles - 1) / (8 * l.token_tiles)), chosen = c.top_k < c.local_experts ? c.top_k : c.local_experts;
     const int above = per_expert <= 4 ? 16 : int(4 * per_expert);
     if (c.tokens > above && (items - 1) * chosen * 3 * c.hidden * c.intermediate > 4e8) l.core_above = above;

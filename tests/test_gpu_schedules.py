@@ -1,4 +1,4 @@
-"""The work plans the decode operators' plan kernels write on the device, read back through
+"""The work plans the decode operators write on the device, read back through
 ``cake_b200_decode_plan_view`` and held to the host-side restatement of tests/test_schedules.py (which the
 CPU suite checks for the properties the kernels rely on)."""
 import random

@@ -1,11 +1,11 @@
 """Host-side restatement of the two device-side work schedules of the decode operators, checked for
 the properties the kernels rely on (no GPU needed).
 
-* MLA (csrc/decode_mla.cu, plan kernels, next_piece, slot_of, list_cuts): the units of all sequences, a start-up share and then one
+* MLA (csrc/decode_mla.cu, plan_here and the plan kernels, next_piece, slot_of, list_cuts): the units of all sequences, a start-up share and then one
   per 32 tokens, form one list; worker w of W takes the w-th of W equal consecutive ranges.  A piece of a sequence that a range
-  boundary cuts leaves its result in slot 2 w, or 2 w + 1 if the sequence begins inside the range; the plan kernel lists the
+  boundary cuts leaves its result in slot 2 w, or 2 w + 1 if the sequence begins inside the range; the plan lists the
   cut sequences, from which alone the reduce kernel finds the pieces.
-* GQA (csrc/decode_gqa.cu, gqa_plan_kernel): the tokens of all sequences form one list, cut into equal
+* GQA (csrc/decode_gqa.cu, plan_here and gqa_plan_kernel): the tokens of all sequences form one list, cut into equal
   consecutive ranges (a multiple of the 16-token tile); the pieces of sequences the ranges hold are
   listed in token order, so the pieces of a range, and the pieces of a sequence, are consecutive.
 """
@@ -57,7 +57,7 @@ def slot_of(worker, seq_begin, per):
 
 
 def mla_cuts(prefix, per, seq_cost):
-    """The plan kernel's list: (sequence, first and last worker, slot of the first piece)."""
+    """The plan's list: (sequence, first and last worker, slot of the first piece)."""
     cuts = []
     for b in range(len(prefix) - 1):
         begin, end = prefix[b], prefix[b + 1]
