@@ -245,6 +245,8 @@ int cake_b200_moe_destroy(void* handle);
  * weight-streaming kernel (0: the tcgen05 core alone), out[1], out[2] warps that share K in its first and second product, out[3] rows
  * above which an expert goes to the core all the same (0: none does), out[4] 1 where routing and placement are one kernel. */
 int cake_b200_moe_dispatch(const cake_b200_moe_config* config, int* out);
+/* The same: 1 where cake_b200_moe_launch runs stages 1 to 3 of such a layer as one kernel (a step of few tokens). */
+int cake_b200_moe_few_tokens(const cake_b200_moe_config* config);
 /* Device pointers of intermediates inside the workspace, for tests and for expert-parallel callers:
  * which = 0 expert_ids int32 [T,top_k]; 1 route_weights fp32 [T,top_k]; 2 counts; 3 offsets; 4 sorted_pairs; 5 inv_perm;
  * 6 the weighted contribution rows bf16 [T*top_k,H] that GEMM2 writes in sorted order (row inv_perm[t,slot] belongs to

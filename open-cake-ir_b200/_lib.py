@@ -117,7 +117,7 @@ OPERATORS = {
     "mla_prefill": (MlaPrefillConfig, True),
 }
 # every symbol include/cake_b200.h declares
-EXPORTS = (["cake_b200_abi_version", "cake_b200_read_status", "cake_b200_test_hooks", "cake_b200_test_silu", "cake_b200_launch_facts", "cake_b200_decode_plan_view", "cake_b200_moe_dispatch", "cake_b200_moe_intermediate", "cake_b200_moe_launch_stage",
+EXPORTS = (["cake_b200_abi_version", "cake_b200_read_status", "cake_b200_test_hooks", "cake_b200_test_silu", "cake_b200_launch_facts", "cake_b200_decode_plan_view", "cake_b200_moe_dispatch", "cake_b200_moe_few_tokens", "cake_b200_moe_intermediate", "cake_b200_moe_launch_stage",
             "cake_b200_gqa_decode_noalloc", "cake_b200_gqa_decode_noalloc_scratch_limit",
             "cake_b200_ep_row_bytes", "cake_b200_ep_exchange_create", "cake_b200_ep_exchange_launch_stage",
             "cake_b200_ep_exchange_destroy", "cake_b200_ep_push_symmetric_bytes", "cake_b200_ep_push_scratch_bytes",
@@ -143,6 +143,7 @@ def library() -> ctypes.CDLL:
         lib.cake_b200_launch_facts.argtypes = [ctypes.c_char_p, POINTER(c_int), POINTER(c_int)]
         lib.cake_b200_decode_plan_view.argtypes = [ctypes.c_char_p, c_void_p, c_int, POINTER(c_void_p), POINTER(c_int)]
         lib.cake_b200_moe_dispatch.argtypes = [POINTER(MoeConfig), POINTER(c_int)]
+        lib.cake_b200_moe_few_tokens.argtypes = [POINTER(MoeConfig)]
         lib.cake_b200_moe_intermediate.argtypes = [c_void_p, c_int, POINTER(c_void_p)]
         lib.cake_b200_moe_launch_stage.argtypes = [c_void_p, c_int, c_void_p]
         lib.cake_b200_gqa_decode_noalloc.argtypes = [POINTER(c_void_p), POINTER(GqaDecodeConfig), c_void_p]

@@ -6,6 +6,7 @@
 // rows per expert, on the weight-streaming kernel in gemm_skinny.cuh, which takes token rows where they
 // lie; the small integer kernels here are warp-level (top-k by ordered keys, ballot prefix scans).
 #include "gemm_skinny.cuh"
+#include "moe_few.cuh"
 #include "../../include/cake_b200.h"
 #include <new>
 
@@ -206,7 +207,8 @@ place_kernel(const int* __restrict__ expert_ids, const int* __restrict__ offset_
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int offset = __ldg(offset_ptr), want = e + offset;
-  if (e == 0 && clear && threadIdx.x < clear_words) clear[threadIdx.x] = 0;
+  if (e == 0 && clear)
+    for (int i = threadIdx.x; i < clear_words; i += kPlaceWarps * 32) clear[i] = 0;
   const int per_warp = ((pairs + kPlaceWarps - 1) / kPlaceWarps + kPlaceStep - 1) / kPlaceStep * kPlaceStep;
   const int begin = warp * per_warp, end = min(pairs, begin + per_warp);
   const uint32_t below = (1u << lane) - 1u;
@@ -297,7 +299,8 @@ route_place_kernel(const float* __restrict__ logits, const __nv_bfloat16* __rest
                    int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ sorted_pairs, int* __restrict__ inv_perm,
                    int tokens, int experts, int top_k, int n_group, int topk_group, int mode, int local_experts,
                    int* __restrict__ clear, int clear_words) {
-  __shared__ int local_id[kSmallTokens * 32];        // -1: another rank's
+  __shared__ int4 local_ids[kSmallTokens * 32 / 4];      // -1: another rank's
+  int* const local_id = reinterpret_cast<int*>(local_ids);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -311,28 +314,33 @@ route_place_kernel(const float* __restrict__ logits, const __nv_bfloat16* __rest
     route_weights[p] = weight;
     local_id[p] = id >= offset && id < offset + local_experts ? id - offset : -1;
   }
+  const int pairs = tokens * top_k;
+  if (threadIdx.x < 4 && pairs + threadIdx.x < kSmallTokens * 32) local_id[pairs + threadIdx.x] = -1;      // read four at a time
   for (int i = threadIdx.x; i < clear_words; i += blockDim.x) clear[i] = 0;
   __syncthreads();
-  const int pairs = tokens * top_k;
-  if (threadIdx.x < pairs) {
-    const int p = threadIdx.x, mine = local_id[p];
-    int at = 0;
-    for (int q = 0; q < pairs; ++q) {
-      const int other = local_id[q];
-      at += other >= 0 && (other < mine || (other == mine && q < p));
+  // thread i: the place of pair i, and of the first pair of experts i, i + blockDim.x, ...
+  const int p = threadIdx.x, mine = p < pairs ? local_id[p] : -1;
+  int at = 0;
+  for (int e = p;; e += blockDim.x) {
+    int before = 0, count = 0;
+#pragma unroll 4
+    for (int q = 0; q < (pairs + 3) / 4; ++q) {
+      const int4 v = local_ids[q];
+      const int other[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        before += uint32_t(other[i]) < uint32_t(e);
+        count += other[i] == e;
+        at += e == p && (uint32_t(other[i]) < uint32_t(mine) || (other[i] == mine && q * 4 + i < p));
+      }
     }
+    if (e <= local_experts) offsets[e] = before;
+    if (e < local_experts) counts[e] = count;
+    if (e + int(blockDim.x) > local_experts) break;
+  }
+  if (p < pairs) {
     inv_perm[p] = mine < 0 ? -1 : at;
     if (mine >= 0) sorted_pairs[at] = p;
-  }
-  for (int e = threadIdx.x; e <= local_experts; e += blockDim.x) {
-    int before = 0, count = 0;
-    for (int q = 0; q < pairs; ++q) {
-      const int other = local_id[q];
-      before += other >= 0 && other < e;
-      count += other == e;
-    }
-    offsets[e] = before;
-    if (e < local_experts) counts[e] = count;
   }
 }
 
@@ -430,6 +438,7 @@ struct Layout {     // byte offsets inside the workspace
       act, act_scale, y, act32, total;
   int capacity, terms;
   int core_above;                        // weight-streaming kernel: experts of more rows than this take the tcgen05 core (0: none can hurt)
+  bool few;                              // a whole launch takes few_tokens_kernel behind the routing
   int token_tiles, split1, split2;       // few rows per expert: token tiles of eight and K splits of the weight-streaming kernel (0: the tcgen05 core)
 };
 inline Layout make_layout(const cake_b200_moe_config& c) {
@@ -440,7 +449,7 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
   constexpr int sms = 148;               // of a B200: the layout is asked for before there is a device, and create has to find the same
   size_t at = 0;
   auto take = [&](size_t bytes) { size_t here = at; at += align_up(bytes); return here; };
-  l.status = take(256);
+  l.status = take(256 + size_t(few::counter_words(int(pairs), c.hidden)) * 4);      // the counters of few_tokens_kernel behind it: cleared together
   l.expert_ids = take(pairs * 4);
   l.route_weights = take(pairs * 4);
   l.counts = take(size_t(c.local_experts) * 4);
@@ -474,7 +483,6 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
     l.token_tiles = per_expert <= 3 ? 1 : 2;
     l.split1 = skinny::choose_split_gate_up(touched > 1 ? touched : 1, c.intermediate, c.hidden / 128, sms);
     l.split2 = skinny::choose_split(touched > 1 ? touched : 1, c.hidden, c.intermediate / 128, sms);
-    if (l.split1 > 1) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation
     // The routing may be anything but even: the padding of a batch, or a batch of one prompt, goes to the same top_k experts.  The
     // weight-streaming kernel then reads their weights once per item of 8 token_tiles rows, so experts of many rows (four times the
     // average, which chance does not reach) go to the core (hidden 7168, 8 of 256 experts of 2048, all 96 tokens equal: 595 us
@@ -486,13 +494,25 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
     const int above = per_expert <= 4 ? 16 : int(4 * per_expert);
     if (c.tokens > above && (items - 1) * chosen * 3 * c.hidden * c.intermediate > 4e8) l.core_above = above;
   }
+  // A step of few tokens in one kernel behind the routing, where its fixed times (the start and end of three more kernels) are much of the step.  That goes by the
+  // local pairs and by how large an expert is: with small ones an item of that kernel is shorter than what happens beside it, with two terms
+  // the rows' quantisation counts (other form and this one, us; one term, two terms.  Hidden 7168, experts of 2048: 1 token on 64 of 256 67 and 44, 44 and 34; 8 on 32
+  // 99 and 75, 82 and 79; 8 on all 256 422 and 378, 472 and 471; 11 on 128 286 and 259, 283 and 267; 16 on 64 179 and 165, 216 and 224.  4096, 1536, 32 of 128: 4 tokens
+  // 40 and 28, 43 and 38; 11 73 and 65, 63 and 60; 16 71 and 72.  2048, 768, 128 experts: 1 token 30 and 21, 33 and 27, 4 50 and 42, 53 and 52; 6 54 and 55, 59 and 62.  1024, 512,
+  // 64 experts: 1 token 19 and 14, 4 23.0 and 21.3, 24.2 and 23.2; 6 27.6 and 28.3).  Tokens that all go to the same experts make a second row
+  // tile from nine on, which reads the weights again: not where the tcgen05 core, which does not, has the layer, or some experts of it.
+  const double rows = per_expert * c.local_experts;
+  const bool large = 3.0 * c.hidden * c.intermediate >= 32e6;
+  l.few = few::fits(int64_t(pairs)) && !l.core_above && (l.token_tiles == 1 || c.tokens <= kSmallTokens) &&
+          (large ? rows <= (l.terms == 2 ? 48 : 128) : rows <= (l.terms == 2 ? 24 : 32) && rows <= 1.5 * touched);
+  if (l.split1 > 1 || l.few) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation
   l.total = at;
   return l;
 }
 
-// Routing and placement in one kernel.
-inline bool routes_in_one(const cake_b200_moe_config& c, const Layout& l) {
-  return !c.external_routing && c.tokens <= kSmallTokens && l.token_tiles && !l.core_above;
+// Routing and placement in one kernel; `few`: in front of few_tokens_kernel.
+inline bool routes_in_one(const cake_b200_moe_config& c, const Layout& l, bool few) {
+  return !c.external_routing && c.tokens <= kSmallTokens && (few || (l.token_tiles && !l.core_above));
 }
 
 struct MoeHandle {
@@ -507,6 +527,8 @@ struct MoeHandle {
   CUtensorMap map_a1, map_a1_tail, map_b1, map_b1_narrow, map_a2, map_a2_tail, map_b2;
   gemm::Params p1, p2;
   skinny::Params s1, s2;
+  few::Maps few_maps;
+  few::Params few;
   int grid;
 };
 
@@ -611,8 +633,12 @@ extern "C" int cake_b200_moe_dispatch(const cake_b200_moe_config* config, int* o
   out[1] = l.split1;
   out[2] = l.split2;
   out[3] = l.core_above;
-  out[4] = moe::routes_in_one(*config, l);
+  out[4] = moe::routes_in_one(*config, l, false);
   return 0;
+}
+
+extern "C" int cake_b200_moe_few_tokens(const cake_b200_moe_config* config) {
+  return config && moe_config_ok(*config) && cake::moe::make_layout(*config).few;
 }
 
 extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* config, void** handle_out) {
@@ -745,12 +771,40 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
     if (!rc) rc = skinny::prepare_any<gemm::kDown>(l.token_tiles, l.split2, l.terms);
     if (rc) { delete h; return rc; }
   }
+  if (l.few) {
+    few::Params& p = h->few;
+    p = few::Params{};
+    p.s13 = p1.sfb;
+    p.s2 = p2.sfb;
+    p.x = h->hidden;
+    p.sx = h->hidden_scale;
+    p.offsets = offsets;
+    p.sorted_pairs = reinterpret_cast<const int*>(h->ws + l.sorted_pairs);
+    p.inv_perm = reinterpret_cast<const int*>(h->ws + l.inv_perm);
+    p.route_weights = h->route_weights;
+    p.act32 = reinterpret_cast<float*>(h->ws + l.act32);
+    p.y = reinterpret_cast<__nv_bfloat16*>(h->ws + l.y);
+    p.out = h->output;
+    p.status = status;
+    p.counters = status + 64;
+    p.hidden = hidden;
+    p.inter = inter;
+    p.groups = c.local_experts;
+    p.tokens = int(c.tokens);
+    p.top_k = c.top_k;
+    rc = few::weight_maps(&h->few_maps, buffers[4], buffers[6], c.local_experts, hidden, inter);
+    if (!rc)
+      rc = few::with_terms(l.terms, [](auto* kernel) {
+        return int(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, few::kSmemBytes));
+      });
+    if (rc) { delete h; return rc; }
+  }
   *handle_out = h;
   return 0;
 }
 
-// stage 0: routing + permute + gather; 1: grouped GEMM1 + SwiGLU; 2: grouped GEMM2; 3: combine
-static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) {
+// `few`: stage 0 in front of few_tokens_kernel, which gathers nothing.  stage 0: routing + permute + gather; 1: grouped GEMM1 + SwiGLU; 2: grouped GEMM2; 3: combine
+static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s, bool few = false) {
   using namespace cake;
   const cake_b200_moe_config& c = h->cfg;
   const moe::Layout& l = h->layout;
@@ -760,23 +814,24 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
                       reinterpret_cast<int*>(h->ws + l.inv_perm), tokens * c.top_k, c.local_experts};
   switch (stage) {
     case 0: {
-      int* const clear = reinterpret_cast<int*>(h->ws + l.status);      // the status word and the GEMMs' counters start at 0
+      int* const clear = reinterpret_cast<int*>(h->ws + l.status);      // the status word and the counters of the kernels behind start at 0
+      const int few_words = few ? 64 + few::counter_words(tokens * c.top_k, c.hidden) : 0;
       const moe::Gather gather{h->hidden, h->hidden_scale, h->route_weights, h->ws + l.x_perm, reinterpret_cast<float*>(h->ws + l.sx_perm),
                                reinterpret_cast<float*>(h->ws + l.row_weight), tokens, c.hidden, c.top_k, l.capacity,
                                l.core_above, 8 * l.token_tiles, clear + kCoreWord};
-      if (moe::routes_in_one(c, l)) {
+      if (moe::routes_in_one(c, l, few)) {
         const int epl = (c.experts + 31) / 32;
         auto* kernel = epl <= 2 ? moe::route_place_kernel<2> : epl <= 4 ? moe::route_place_kernel<4> : epl <= 8 ? moe::route_place_kernel<8> : moe::route_place_kernel<16>;
         return launch_dependent(kernel, dim3(1), dim3(32 * tokens), 0, s, h->logits, h->bias, h->factor, h->local_offset, h->expert_ids, h->route_weights,
                                 pa.counts, pa.offsets, pa.sorted_pairs, pa.inv_perm, tokens, c.experts, c.top_k, c.n_group, c.topk_group,
-                                c.routing_mode, c.local_experts, clear, 64);
+                                c.routing_mode, c.local_experts, clear, few ? few_words : 64);
       }
       if (!c.external_routing)
         if (int rc = moe::launch_routing(h->logits, h->bias, h->factor, h->expert_ids, h->route_weights, tokens, c.experts, c.top_k,
                                          c.n_group, c.topk_group, c.routing_mode, s))
           return rc;
-      if (int rc = moe::launch_permute(pa, s, clear, kCoreWord, gather)) return rc;
-      if (l.token_tiles) return 0;
+      if (int rc = moe::launch_permute(pa, s, clear, few ? few_words : kCoreWord, gather)) return rc;
+      if (l.token_tiles || few) return 0;
       const int gather_blocks = (l.capacity + 7) / 8;
       return launch_dependent(moe::gather_kernel, dim3(gather_blocks < 4096 ? gather_blocks : 4096), dim3(256), 0, s, pa.sorted_pairs, pa.offsets,
                               c.local_experts, gather);
@@ -819,6 +874,19 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s) 
   }
 }
 
+// A step of few tokens: stages 1 to 3 in one kernel behind the routing.
+static int moe_launch_few(cake::moe::MoeHandle* h, cudaStream_t s) {
+  using namespace cake;
+  if (reinterpret_cast<uintptr_t>(h->output) & 15) return kErrBadArgument;      // rows leave 16 bytes at a time
+  if (int rc = moe_launch_stage(h, 0, s, true)) return rc;
+  few::Params p = h->few;
+  p.wait_kiloclocks = test_hooks().budget_kiloclocks;
+  p.skip_signal = test_hooks().skip_load;
+  return few::with_terms(h->layout.terms, [&](auto* kernel) {
+    return launch_dependent(kernel, dim3(h->grid), dim3(few::kThreads), few::kSmemBytes, s, h->few_maps, p);
+  });
+}
+
 extern "C" int cake_b200_moe_launch_stage(void* handle, int stage, void* cuda_stream) {
   using namespace cake;
   if (!handle) return kErrBadArgument;
@@ -831,8 +899,16 @@ extern "C" int cake_b200_moe_launch_stage(void* handle, int stage, void* cuda_st
 }
 
 extern "C" int cake_b200_moe_launch(void* handle, void* cuda_stream) {
+  using namespace cake;
+  if (!handle) return kErrBadArgument;
+  auto* h = static_cast<moe::MoeHandle*>(handle);
+  int device = -1;
+  CAKE_CUDA_OK(cudaGetDevice(&device));
+  if (device != h->device) return kErrWrongDevice;
+  if (h->cfg.tokens == 0) return 0;
+  if (h->layout.few) return moe_launch_few(h, reinterpret_cast<cudaStream_t>(cuda_stream));
   for (int stage = 0; stage < 4; ++stage)
-    if (int rc = cake_b200_moe_launch_stage(handle, stage, cuda_stream)) return rc;
+    if (int rc = moe_launch_stage(h, stage, reinterpret_cast<cudaStream_t>(cuda_stream))) return rc;
   return 0;
 }
 

@@ -1,0 +1,524 @@
+// A step of few tokens behind its routing in one kernel: gate/up product with SwiGLU, requantisation, down product and combine.
+//
+// The arithmetic of gemm_skinny.cuh (mma.m16n8k32 on 32 weight rows and eight token rows, promotion in registers, K shared by eight warps,
+// which meet in warp order), for a layer that reads a few experts' weights and is over in tens of microseconds.  As four kernels (gate/up,
+// quantisation, down, combine) each of them began with an empty pipe and ended with an idle GPU.  Here the second product's weights, which wait for
+// nothing, are on their way while the first product ends.  One token, hidden 7168, experts of 2048: eight of 256 experts 79 us then and 65 now (352 MB, 54 us at
+// the copy rate), three of 32 48 and 39 with two terms; hidden 1024, experts of 512 19 and 14.  While it streams it reads 5.8 TB/s.
+//
+// Work items, in order: the gate/up items (16 features of 8 rows), then the down items (64 columns of 8 rows).  They are DRAWN from a
+// counter in that order, so an item that has to wait (a down item, for all gate/up items of its rows) waits only for items that a running CTA
+// has already drawn: no number of resident CTAs is assumed, and several such kernels may share the GPU.
+// A CTA: two teams of eight warps that multiply, taking its items in turn; a warp that brings the weights in, a slot of 32 KB to an instruction; two
+// that bring rows and scales; and one for what happens between CTAs: it draws and locates items, announces finished down items and, where one was the
+// last of its columns, adds the tokens' rows up (the combine step: slot order, fp32).  A gate/up item leaves its features in fp32, and the row warps of
+// the down items quantise them on the way (the same 1 x 128 groups and bits).
+#pragma once
+#include "gemm_skinny.cuh"
+
+namespace cake {
+namespace few {
+
+using skinny::kSubRows;
+using skinny::kWeightBytes;
+using skinny::kMaxGroups;
+constexpr int kSubTiles = 8;                        // of 32 weight rows and one K block, in a slot of the ring
+constexpr int kTeams = 2, kComputeWarps = kTeams * kSubTiles,      // two teams of warps, which take a CTA's items in turn
+               kDrawWarp = kComputeWarps, kLoadWarp = kDrawWarp + 1, kRowWarp = kDrawWarp + 2, kRowWarps = 2;
+constexpr int kThreads = (kRowWarp + kRowWarps) * 32;
+constexpr int kRows = 8;                            // of an item
+constexpr int kSlotBytes = kSubTiles * kWeightBytes;
+// A slot of the down product: WK K blocks of WM times 32 columns.  (Eight of one: the rows' quantisation, whose work goes with a slot's K blocks, then
+// takes longer than the weights; one token on eight experts of 2048, hidden 7168, 70.7 us, two terms 79.9; 64.7 and 72.9 so.)
+constexpr int WK = 4, WM = kSubTiles / WK, kDownFeatures = 32 * WM;
+constexpr int kParts = 4 * WM;                      // finished parts of an item
+constexpr int kSlots = 5;
+// What a slot of weights meets, in a ring of its own: the rows of its K blocks (eight of the gate/up product; four of the down product, one or two terms
+// of each block after the other; swizzled as the weights are), their scales [term][row][K block] and the weights' [K block][MMA tile].
+constexpr int kTermBytes = kRows * 128;
+constexpr int kScales = kSubTiles * kTermBytes, kWeightScales = kScales + kSubTiles * kRows * 4, kRowSlotBytes = kWeightScales + kSubTiles * 8;
+constexpr int kMaxPairs = 256;
+constexpr int kItemRing = 32;
+constexpr int kAhead = 2;                           // items drawn beyond the one whose weights are being asked for
+
+struct Params {
+  const float *s13, *s2;                   // [groups, 2 inter / 128, hidden / 128], [groups, hidden / 128, inter / 128]
+  const uint8_t* x;                        // [tokens, hidden]
+  const float* sx;                         // [hidden / 128, tokens]
+  const int *offsets, *sorted_pairs, *inv_perm;
+  const float* route_weights;
+  float* act32;                            // [pairs, inter]: SwiGLU output
+  __nv_bfloat16 *y, *out;
+  int* counters;                           // 0 at launch: items drawn; gate/up items done of each row tile; down items done of each column tile
+  int* status;
+  int hidden, inter, groups, tokens, top_k;
+  int wait_kiloclocks, skip_signal;        // test hook: a gate/up item of CTA 0 is not announced
+};
+inline int counter_words(int pairs, int hidden) { return 1 + pairs + hidden / 32; }
+
+struct Item {
+  int phase;                               // 0 gate/up, 1 down, -1: no further item
+  int group, feature0, row0, rows, tile;   // tile: row tile of all groups together
+};
+struct Shared {
+  float reduce[kComputeWarps][8][32];
+  uint64_t full[kSlots], empty[kSlots], row_full[kSlots];
+  int16_t tile_prefix[kMaxGroups + 2], row_prefix[kMaxGroups + 2];
+  int16_t pair_of[kMaxPairs], row_of[kMaxPairs];     // sorted_pairs, inv_perm
+  float weight_of[kMaxPairs];                        // route weight of a pair
+  Item item[kItemRing];
+  int drawn, opened, issued;                         // written by one side and watched by others: items drawn, items and slots whose weights have been asked for
+  int emitted[kTeams];                               // finished parts of a team's items
+  WaitControl wait;
+};
+struct Maps { CUtensorMap w13, w2; };                // boxes of a slot: see weight_map
+constexpr int kSmemBytes = 1024 + kSlots * (kSlotBytes + kRowSlotBytes) + int(sizeof(Shared));
+static_assert(kSmemBytes <= 232448, "the kernel's shared memory exceeds what a CTA may have on sm_100");
+
+// A slot of the ring is one box: of the gate/up weights 16 rows of x1 and the matching 16 of x2, of the down weights 32 WM rows, of every K
+// block it has, K block by K block and each as rows of 128 bytes in the 128-byte swizzle.  K blocks past the end are filled with zeros.
+inline int weight_map(CUtensorMap* map, const void* base, uint64_t groups, uint64_t rows, uint64_t k, uint32_t box_rows, uint32_t box_groups, uint32_t box_blocks) {
+  EncodeTiledFn encode = nullptr;
+  if (int rc = get_encode_tiled(&encode)) return rc;
+  cuuint64_t dims[4] = {128, rows, groups, k / 128}, strides[3] = {k, rows * k, 128};
+  cuuint32_t box[4] = {128, box_rows, box_groups, box_blocks}, steps[4] = {1, 1, 1, 1};
+  const CUresult st = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(base), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return st == CUDA_SUCCESS ? 0 : 10000 + int(st);
+}
+__device__ __forceinline__ void load_slot(void* dst, const CUtensorMap* map, int row, int group, int block, uint64_t* bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5}], [%6], %7;"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(0), "r"(row), "r"(group), "r"(block), "r"(smem_u32(bar)), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void team_sync(int team) { asm volatile("bar.sync %0, 256;" ::"r"(1 + team) : "memory"); }
+__device__ __forceinline__ int peek(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
+__device__ __forceinline__ void post(int* p, int v) { *reinterpret_cast<volatile int*>(p) = v; }
+__device__ __forceinline__ float lds32f(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void sts32f(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ int load_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// A look at the clock of a wait that goes on; true: the budget is used up (or another warp's was), and the status word says so.
+static __device__ __forceinline__ bool gives_up(uint32_t start, Shared* sh, int* status, bool inside) {
+  volatile int* flag = &sh->wait.abort_flag;
+  if (!inside && *flag) return true;
+  if (!wait_over(start, kiloclock(), sh->wait.budget_kiloclocks, inside)) return false;
+  *flag = kStatusWaitFlag;
+  atomicCAS(status, 0, int(kStatusWaitFlag));
+  return true;
+}
+// Until *word > value.  Words of this CTA: their writers end in bounded time, so that nobody gives up here before them.
+__device__ __forceinline__ bool wait_above(const int* word, int value, Shared* sh, int* status) {
+  if (peek(word) <= value) {
+    const uint32_t start = kiloclock();
+    for (uint32_t spins = 0; peek(word) <= value;)
+      if (++spins > 16) {                          // (the shared memory is for those that have work)
+        __nanosleep(40);
+        if (spins == 2048) {
+          if (gives_up(start, sh, status, true)) return false;
+          spins = 17;
+        }
+      }
+  }
+  __threadfence_block();
+  return true;
+}
+
+// TERMS: e4m3 terms of the SwiGLU output.
+template <int TERMS>
+__global__ void __launch_bounds__(kThreads, 1)
+few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* row_ring = ring + kSlots * kSlotBytes;
+  Shared* sh = reinterpret_cast<Shared*>(row_ring + kSlots * kRowSlotBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    sh->drawn = sh->opened = sh->issued = sh->emitted[0] = sh->emitted[1] = 0;
+    sh->wait.abort_flag = 0;
+    sh->wait.budget_kiloclocks = p.wait_kiloclocks;
+    for (int s = 0; s < kSlots; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], kSubTiles); mbar_init(&sh->row_full[s], 32); }
+    fence_barrier_init();
+  }
+  const int pairs = p.tokens * p.top_k, blocks1 = p.hidden / 128, blocks2 = p.inter / 128, n1 = p.inter / 16, n2 = p.hidden / kDownFeatures;
+  if (threadIdx.x == 0) { tma_prefetch_descriptor(&maps.w13); tma_prefetch_descriptor(&maps.w2); }
+  asm volatile("griddepcontrol.wait;" ::: "memory");         // everything above overlaps the kernel before
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // what the routing has left, all of it asked for at once
+  int first_draw = 0;
+  if (warp == 0) {
+    int first[kMaxGroups / 32], behind[kMaxGroups / 32];
+#pragma unroll
+    for (int j = 0; j < kMaxGroups / 32; ++j) {
+      const int g = j * 32 + lane;
+      first[j] = behind[j] = 0;
+      if (g < p.groups) { first[j] = p.offsets[g]; behind[j] = p.offsets[g + 1]; }
+    }
+    int running = 0;
+#pragma unroll
+    for (int j = 0; j < kMaxGroups / 32; ++j) {
+      if (j * 32 >= p.groups) break;
+      const int g = j * 32 + lane, tiles = (behind[j] - first[j] + kRows - 1) / kRows;
+      int incl = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (g < p.groups) { sh->tile_prefix[g] = running + incl - tiles; sh->row_prefix[g] = first[j]; }
+      if (g == p.groups - 1) sh->row_prefix[p.groups] = behind[j];
+      running += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) sh->tile_prefix[p.groups] = running;
+  } else if (warp == kDrawWarp) {
+    if (lane == 0) first_draw = atomicAdd(p.counters, 1);
+  } else {
+    const int thread = warp < kComputeWarps ? threadIdx.x - 32 : kMaxPairs;       // 480 threads
+    if (thread < pairs) {
+      sh->pair_of[thread] = p.sorted_pairs[thread];          // (behind the local pairs: whatever was there, not used)
+      sh->row_of[thread] = p.inv_perm[thread];
+      sh->weight_of[thread] = p.route_weights[thread];
+    }
+  }
+  __syncthreads();
+  const int tiles = sh->tile_prefix[p.groups];
+  const int items1 = tiles * n1, items = items1 + tiles * n2;
+  if (tiles == 0) {                                          // no pair is this rank's
+    for (int i = blockIdx.x * kThreads + threadIdx.x; i < p.tokens * (p.hidden / 8); i += gridDim.x * kThreads)
+      reinterpret_cast<uint4*>(p.out)[i] = make_uint4(0u, 0u, 0u, 0u);
+    return;
+  }
+  int* const done1 = p.counters + 1;
+  int* const done2 = done1 + pairs;
+
+  if (warp == kDrawWarp) {
+    // ------------------------------ what happens between CTAs ------------------------------
+    // Draws items and announces finished down items: a round trip to L2 each, both under way at a time.
+    int drawn = 0, done_even = 0, done_odd = 0;
+    bool more = true;
+    while (more || done_even + done_odd < drawn - 1) {
+      // one team's finished items, the other's, up to 16 of each
+      const int team = lane >> 4, nth = lane & 15, done = team ? done_odd : done_even;
+      const int finished = peek(&sh->emitted[team]) / kParts - done;
+      const uint32_t fresh = __ballot_sync(0xffffffffu, nth < finished);
+      bool down = false;
+      int column = 0, sum = 0;
+      if (fresh) {
+        if (nth < finished) {
+          const Item it = sh->item[((done + nth) * kTeams + team) % kItemRing];
+          down = it.phase == 1;
+          column = it.feature0;
+        }
+        if (__any_sync(0xffffffffu, down)) __threadfence();
+        if (down) sum = atomicAdd(done2 + column / kDownFeatures, 1) + 1;
+        done_even += __popc(fresh & 0xffffu);
+        done_odd += __popc(fresh >> 16);
+      }
+      const bool draw = more && drawn < peek(&sh->opened) + kAhead && drawn < min(done_even * kTeams, done_odd * kTeams + 1) + kItemRing - 1;
+      int index = first_draw;
+      if (draw && drawn > 0 && lane == 0) index = atomicAdd(p.counters, 1);
+      if (draw) {
+        index = __shfl_sync(0xffffffffu, index, 0);
+        Item it{-1, 0, 0, 0, 0, 0};
+        if (index < items) {
+          it.phase = index >= items1;
+          const int n = it.phase ? n2 : n1;
+          index -= it.phase ? items1 : 0;
+          // the last group whose items begin at or before this one, by 32 lanes at a time
+          const int stride = (p.groups + 31) / 32;
+          uint32_t before = __ballot_sync(0xffffffffu, lane * stride < p.groups && sh->tile_prefix[lane * stride] * n <= index);
+          const int base = (31 - __clz(before)) * stride;
+          before = __ballot_sync(0xffffffffu, lane < stride && base + lane < p.groups && sh->tile_prefix[base + lane] * n <= index);
+          const int g = base + 31 - __clz(before);
+          const int m_tiles = sh->tile_prefix[g + 1] - sh->tile_prefix[g], idx = index - sh->tile_prefix[g] * n, m = idx % m_tiles;
+          it.group = g;
+          it.feature0 = idx / m_tiles * (it.phase ? kDownFeatures : 16);
+          it.row0 = sh->row_prefix[g] + m * kRows;
+          it.rows = min(kRows, sh->row_prefix[g + 1] - it.row0);
+          it.tile = sh->tile_prefix[g] + m;
+        } else {
+          more = false;
+        }
+        if (lane == 0) {
+          sh->item[drawn % kItemRing] = it;
+          __threadfence_block();
+          post(&sh->drawn, drawn + 1);
+        }
+        __syncwarp();
+        ++drawn;
+      }
+      // the last item of its columns: the tokens' rows are added up
+      for (uint32_t last = __ballot_sync(0xffffffffu, down && sum == tiles); last; last &= last - 1) {
+        const int column0 = __shfl_sync(0xffffffffu, column, __ffs(last) - 1);
+        __threadfence();
+        // eight columns of a token to a lane; the rows of eight slots are asked for before the first is added
+        for (int i = lane; i < p.tokens * (kDownFeatures / 8); i += 32) {
+          const int token = i / (kDownFeatures / 8), c = column0 + i % (kDownFeatures / 8) * 8;
+          float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          for (int s0 = 0; s0 < p.top_k; s0 += 8) {
+            uint4 raw[8];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+              const int row = s0 + s < p.top_k ? sh->row_of[token * p.top_k + s0 + s] : -1;
+              raw[s] = row >= 0 ? __ldcg(reinterpret_cast<const uint4*>(p.y + size_t(row) * p.hidden + c)) : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+              const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[s]);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(h[j]);
+                acc[2 * j] += f.x;
+                acc[2 * j + 1] += f.y;
+              }
+            }
+          }
+          *reinterpret_cast<uint4*>(p.out + size_t(token) * p.hidden + c) =
+              make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
+        }
+        __syncwarp();
+      }
+    }
+    return;
+  }
+
+  if (warp == kLoadWarp) {
+    // ------------------------------ brings the weights in ------------------------------
+    // A whole slot to an instruction.  (cp.async by the warps that multiply: 80 instructions a slot, 0.65 us in which nothing was multiplied; boxes of
+    // 16 rows from one thread: 16 a slot, 1 us.)
+    if (lane == 0) {
+      const uint64_t stream = l2_policy_evict_first();
+      uint32_t step = 0;
+      for (int k = 0;; ++k) {
+        post(&sh->opened, k + 1);
+        if (!wait_above(&sh->drawn, k, sh, p.status)) return;
+        const Item it = sh->item[k % kItemRing];
+        if (it.phase < 0) return;
+        const int share = it.phase ? WK : kSubTiles, blocks = it.phase ? blocks2 : blocks1;
+        for (int kb0 = 0; kb0 < blocks; kb0 += share, ++step) {
+          const int s = step % kSlots;
+          mbar_wait(&sh->empty[s], ((step / kSlots) & 1) ^ 1, &sh->wait.abort_flag, p.status, kStatusWaitSmemEmpty);
+          mbar_arrive_expect_tx(&sh->full[s], kSlotBytes);
+          __threadfence_block();
+          post(&sh->issued, int(step) + 1);
+          if (it.phase) load_slot(ring + s * kSlotBytes, &maps.w2, it.feature0, it.group, kb0, &sh->full[s], stream);
+          else load_slot(ring + s * kSlotBytes, &maps.w13, it.feature0, 2 * it.group, kb0, &sh->full[s], stream);
+        }
+      }
+    }
+    return;
+  }
+
+  if (warp >= kRowWarp) {
+    // ------------------------------ bring the rows and all scales in, slot by slot in turn ------------------------------
+    // (Loaded into registers by the warps that multiply, two blocks ahead, they cost a round trip to L2 a block all the same.)
+    uint32_t step0 = 0;
+    int there = 0;                                           // row tiles, from the first on, whose gate/up items are known to be done
+    for (int k = 0;; ++k) {
+      if (!wait_above(&sh->drawn, k, sh, p.status)) break;
+      const Item it = sh->item[k % kItemRing];
+      if (it.phase < 0) break;
+      const bool down = it.phase == 1;
+      const int share = down ? WK : kSubTiles, blocks = down ? blocks2 : blocks1, steps = (blocks + share - 1) / share;
+      if (down && it.tile >= there) {
+        // until all gate/up items of the rows are announced (or given up: the launch then runs on without what it waited for); a look takes in 32 tiles
+        const uint32_t start = kiloclock();
+        for (uint32_t spins = 0; it.tile >= there;) {
+          const bool is = there + lane < tiles && load_acquire(done1 + there + lane) == n1;
+          const uint32_t missing = ~__ballot_sync(0xffffffffu, is);
+          there += missing ? __ffs(missing) - 1 : 32;
+          if (++spins == 64) {
+            if (__any_sync(0xffffffffu, it.tile >= there && gives_up(start, sh, p.status, false))) break;
+            spins = 0;
+          }
+        }
+      }
+      for (int j = (warp - kRowWarp + step0) % kRowWarps; j < steps; j += kRowWarps) {
+        const uint32_t step = step0 + j;
+        const int s = step % kSlots, kb0 = j * share, n = min(share, blocks - kb0);
+        const uint32_t slot = smem_u32(row_ring) + s * kRowSlotBytes;
+        if (!down) {
+          const int token_of = lane < it.rows ? sh->pair_of[it.row0 + lane] / p.top_k : 0;
+          // lane i: the scale of MMA tile i & 1 in K block i / 2 of a slot
+          const float* const sw = p.s13 + (size_t(it.group) * (2 * p.inter / 128) + it.feature0 / 128 + (lane & 1) * (p.inter / 128)) * blocks1 + kb0 + (lane >> 1);
+          wait_above(&sh->issued, int(step), sh, p.status);
+          for (int r = 0; r < it.rows; ++r) {
+            const int token = __shfl_sync(0xffffffffu, token_of, r);
+            const uint8_t* row = p.x + size_t(token) * p.hidden + size_t(kb0) * 128 + lane * 16;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {          // 16 bytes a lane, four K blocks an instruction
+              const int b = h * 4 + (lane >> 3);
+              if (b < n) skinny::cp_async_16(slot + b * kTermBytes + r * 128 + (((lane & 7) ^ r) << 4), row + h * 512);
+            }
+            if (lane < n) skinny::cp_async_4_zfill(slot + kScales + (r * kSubTiles + lane) * 4, p.sx + size_t(kb0 + lane) * p.tokens + token, true);
+          }
+          if (lane >> 1 < n) skinny::cp_async_4_zfill(slot + kWeightScales + lane * 4, sw, true);
+          cp_async_arrive_noinc(&sh->row_full[s]);
+        } else {
+          // Quantisation of the rows (skinny::quantize_kernel's arithmetic): eight lanes to a K block, each with four times four features of it, and the
+          // next rows on their way.
+          const int b = lane >> 3, c = lane & 7;
+          const float4* const act = reinterpret_cast<const float4*>(p.act32 + size_t(it.row0) * p.inter + size_t(kb0) * 128) + b * 32 + c;
+          const uint32_t block = slot + b * (TERMS * kTermBytes) + (c & 3) * 4;
+          auto ask = [&](int r, float4 (&v)[4]) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = r < it.rows && b < n ? __ldcg(act + size_t(r) * (p.inter / 4) + i * 8) : make_float4(0.f, 0.f, 0.f, 0.f);
+          };
+          auto quantise = [&](int r, float4 (&v)[4]) {
+            for (int term = 0; term < TERMS; ++term) {
+              float m = 0.f;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) m = fmaxf(m, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+#pragma unroll
+              for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+              const float scale = m > 0.f ? m / 448.f : 1.f, inv = 1.f / scale;
+              if (c == 0) sts32f(slot + kScales + ((term * kRows + r) * WK + b) * 4, scale);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const uint32_t packed = pack_e4m3x4(v[i].x * inv, v[i].y * inv, v[i].z * inv, v[i].w * inv);
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(block + term * kTermBytes + r * 128 + (((2 * i + (c >> 2)) ^ r) << 4)), "r"(packed) : "memory");
+                if (TERMS > 1) {
+                  v[i].x -= e4m3_to_float(uint8_t(packed)) * scale; v[i].y -= e4m3_to_float(uint8_t(packed >> 8)) * scale;
+                  v[i].z -= e4m3_to_float(uint8_t(packed >> 16)) * scale; v[i].w -= e4m3_to_float(uint8_t(packed >> 24)) * scale;
+                }
+              }
+            }
+          };
+          const float w = lane >> 1 < n ? __ldg(p.s2 + (size_t(it.group) * (p.hidden / 128) + it.feature0 / 128) * blocks2 + kb0 + (lane >> 1)) : 0.f;
+          constexpr int kRowsAhead = TERMS == 2 ? 2 : 3;           // what there are registers for
+          float4 v[kRowsAhead][4];
+#pragma unroll
+          for (int i = 0; i < kRowsAhead; ++i) ask(i, v[i]);
+          wait_above(&sh->issued, int(step), sh, p.status);
+          for (int r = 0; r < it.rows; r += kRowsAhead) {
+#pragma unroll
+            for (int i = 0; i < kRowsAhead; ++i) {
+              if (r + i < it.rows) quantise(r + i, v[i]);
+              ask(r + i + kRowsAhead, v[i]);
+            }
+          }
+          if (lane >> 1 < n) sts32f(slot + kWeightScales + lane * 4, w);
+          mbar_arrive(&sh->row_full[s]);
+        }
+      }
+      step0 += steps;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
+
+  // ------------------------------ products ------------------------------
+  // Two teams, as a slot's way through a warp (its wait, shared memory, four products one after another) and the meeting at an item's end are longer than the
+  // next slot takes to come.
+  const int g8 = lane >> 2, q = lane & 3, team = warp / kSubTiles, sub = warp % kSubTiles;
+  uint32_t step0 = 0;
+  for (int k = 0;; ++k) {
+    if (!wait_above(&sh->drawn, k, sh, p.status)) break;
+    const Item it = sh->item[k % kItemRing];
+    if (it.phase < 0) break;
+    const bool down = it.phase == 1;
+    const int share = down ? WK : kSubTiles, blocks = down ? blocks2 : blocks1, part = down ? sub % WK : sub, steps = (blocks + share - 1) / share;
+    if (k % kTeams != team) { step0 += steps; continue; }
+    float acc[2][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[0][e] = acc[1][e] = 0.f;
+    for (int j = 0; j < steps; ++j) {
+      const uint32_t step = step0 + j;
+      const int s = step % kSlots;
+      // The barriers tell the present phase from the one before, no more, and one team (one row warp) may be further ahead of the other: nobody looks at
+      // them, or writes rows, before the load warp, which goes from slot to slot, has seen the slot's last use end and begun this one.
+      wait_above(&sh->issued, int(step), sh, p.status);
+      mbar_wait_both(&sh->full[s], (step / kSlots) & 1, kStatusWaitSmemFull, &sh->row_full[s], (step / kSlots) & 1, kStatusWaitSmemFull,
+                     &sh->wait.abort_flag, p.status);
+      if (j * share + part < blocks) {
+        const uint32_t from = smem_u32(ring) + s * kSlotBytes + (down ? part * WM + sub / WK : sub) * kWeightBytes;
+        const uint32_t slot = smem_u32(row_ring) + s * kRowSlotBytes;
+        const float2 sw = skinny::lds64f(slot + kWeightScales + part * 8);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {              // MMA tile
+          uint32_t a[2][8];                        // [row g / g + 8][k-step pair words]
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int r = t * 16 + h * 8 + g8;
+            const uint4 lo = skinny::lds128(from + r * 128 + (((2 * q) ^ g8) << 4)), hi = skinny::lds128(from + r * 128 + (((2 * q + 1) ^ g8) << 4));
+            a[h][0] = lo.x; a[h][1] = lo.y; a[h][2] = lo.z; a[h][3] = lo.w;
+            a[h][4] = hi.x; a[h][5] = hi.y; a[h][6] = hi.z; a[h][7] = hi.w;
+          }
+#pragma unroll 1
+          for (int term = 0; term < (down ? TERMS : 1); ++term) {
+            // (rows that the item does not have hold whatever was there: their columns of the product are not used)
+            const uint32_t xr = slot + (down ? part * TERMS + term : part) * kTermBytes + g8 * 128, scales = slot + kScales + ((term * kRows + q * 2) * share + part) * 4;
+            const uint4 lo = skinny::lds128(xr + (((2 * q) ^ g8) << 4)), hi = skinny::lds128(xr + (((2 * q + 1) ^ g8) << 4));
+            const uint32_t b[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            const float w = t == 0 ? sw.x : sw.y, s0 = w * lds32f(scales), s1 = w * lds32f(scales + share * 4);
+            float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) skinny::mma_e4m3(d, a[0][2 * ks], a[1][2 * ks], a[0][2 * ks + 1], a[1][2 * ks + 1], b[2 * ks], b[2 * ks + 1]);
+            acc[t][0] = fmaf(d[0], s0, acc[t][0]); acc[t][1] = fmaf(d[1], s1, acc[t][1]);
+            acc[t][2] = fmaf(d[2], s0, acc[t][2]); acc[t][3] = fmaf(d[3], s1, acc[t][3]);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh->empty[s]);
+    }
+    step0 += steps;
+    // the warps that share K add their sums in warp order; the first four of them finish one accumulator each
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sh->reduce[warp][j][lane] = acc[j >> 2][j & 3];
+    team_sync(team);
+    const int e = part, first = warp - part;
+    float v0 = 0.f, v1 = 0.f;
+    if (e < 4) {
+#pragma unroll
+      for (int w = 0; w < kSubTiles; ++w)
+        if (w < share) { v0 += sh->reduce[first + w][e][lane]; v1 += sh->reduce[first + w][4 + e][lane]; }
+    }
+    team_sync(team);
+    if (e < 4) {
+      const int token = q * 2 + (e & 1), row = it.row0 + token;
+      if (token < it.rows) {
+        if (!down) {
+          p.act32[size_t(row) * p.inter + it.feature0 + g8 + 8 * (e >> 1)] = v0 * silu(v1);
+        } else {
+          const float w = sh->weight_of[sh->pair_of[row]];
+          __nv_bfloat16* y = p.y + size_t(row) * p.hidden + it.feature0 + sub / WK * 32 + g8 + 8 * (e >> 1);
+          y[0] = __float2bfloat16_rn(v0 * w);
+          y[16] = __float2bfloat16_rn(v1 * w);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) {
+        __threadfence_block();
+        const int add = down ? 1 : WM, sum = atomicAdd(&sh->emitted[team], add) + add;
+        // the last part of a gate/up item announces it, since down items wait for that
+        if (!down && sum % kParts == 0 && !(p.skip_signal && blockIdx.x == 0 && k == 0)) {
+          __threadfence();
+          atomicAdd(done1 + it.tile, 1);
+        }
+      }
+    }
+  }
+  if (sh->wait.abort_flag) settle_after_abort();
+}
+
+inline bool fits(int64_t pairs) { return pairs <= kMaxPairs; }
+inline int weight_maps(Maps* maps, const void* w13, const void* w2, int groups, int hidden, int inter) {
+  const int rc = weight_map(&maps->w13, w13, 2 * uint64_t(groups), inter, hidden, 16, 2, kSubTiles);
+  return rc ? rc : weight_map(&maps->w2, w2, groups, hidden, inter, kDownFeatures, 1, WK);
+}
+template <typename F>
+inline int with_terms(int terms, F f) {
+  return terms == 2 ? f(few_tokens_kernel<2>) : f(few_tokens_kernel<1>);
+}
+
+}  // namespace few
+}  // namespace cake

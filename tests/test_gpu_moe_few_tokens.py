@@ -1,0 +1,121 @@
+"""The MoE layer of a step of few tokens, whose products and combine are one kernel behind the routing (csrc/moe_few.cuh): the smallest
+and the largest it takes, K blocks that do not divide among the warps, experts with more rows than an item,
+tokens without a row here, several at a time, and its wait.  Oracle and tolerance of test_gpu_moe.py's layer test; the four kernels of the staged launches besides."""
+import ctypes
+
+import pytest
+import torch
+
+import open_cake_ir_b200 as cake
+from gpu_util import poison, snapshot, unchanged
+from oracle import compare, moe as oracle_moe
+
+pytestmark = pytest.mark.gpu
+
+
+def one_kernel(tokens, hidden, inter, experts, local, act, top_k=8):
+    cfg = cake._lib.MoeConfig(tokens, hidden, inter, experts, local, top_k, 8, 4, 1, int(act == "split"), 0)
+    return cake._lib.library().cake_b200_moe_few_tokens(ctypes.byref(cfg)) == 1
+
+
+def layer(tokens, hidden, inter, experts, local, offset, act, top_k=8, routing="softmax", change=None):
+    cpu = cake.workloads.moe_inputs(tokens, hidden, inter, experts, local, offset, routing=routing, device="cpu")
+    if change:
+        change(cpu)
+    dev = {k: v.cuda() for k, v in cpu.items()}
+    out, intact = poison((tokens, hidden), torch.bfloat16)
+    assert one_kernel(tokens, hidden, inter, experts, local, act, top_k)
+    op = cake.Fp8Moe(dev, out, experts=experts, top_k=top_k, routing=routing, act_mode=act)
+    return cpu, dev, out, intact, op
+
+
+def check(cpu, out, act, top_k=8, routing="softmax"):
+    want = oracle_moe.moe_reference(cpu, routing=routing, act_quant="fp8" if act == "fp8" else "none", dtype=torch.float32, top_k=top_k)["output"]
+    assert compare.rel_frobenius(out, want) <= (1e-2 if act == "fp8" else 4e-3)
+
+
+@pytest.mark.parametrize("act", ["fp8", "split"])
+@pytest.mark.parametrize("tokens,hidden,inter,experts,local,offset,top_k", [
+    (1, 1024, 512, 64, 64, 0, 8),
+    (1, 7168, 2048, 64, 8, 24, 8),            # a serving layer's experts
+    (2, 1152, 640, 64, 16, 16, 8),            # nine and five K blocks; an odd number of 128 columns
+    (3, 128, 128, 64, 16, 0, 8),              # fewer K blocks than warps that share them, in both products
+    (8, 1408, 1024, 128, 32, 32, 8),          # as many tokens as are routed and placed in one kernel
+    (9, 1024, 768, 128, 32, 64, 8),           # in two
+    (32, 1024, 512, 512, 48, 400, 8),         # as many pairs as it takes
+    (8, 1024, 512, 512, 48, 100, 32)])       # the same from eight tokens
+def test_few_tokens(tokens, hidden, inter, experts, local, offset, top_k, act):
+    cpu, dev, out, intact, op = layer(tokens, hidden, inter, experts, local, offset, act, top_k)
+    before = snapshot(dev)
+    op.launch()
+    check(cpu, out, act, top_k)
+    first = out.clone()
+    out.fill_(float("nan"))
+    for stage in range(4):                     # the same step as separate kernels: sums of another order, so roundings may differ
+        op.launch_stage(stage)
+    assert compare.rel_frobenius(out, first) <= 5e-3
+    for _ in range(3):                         # drawn in another order each time, added up in the same
+        out.fill_(float("nan"))
+        op.launch()
+        assert torch.equal(out, first)
+    assert op.status() == 0 and unchanged(before, dev)
+    intact()
+
+
+@pytest.mark.parametrize("act", ["fp8", "split"])
+def test_more_rows_than_an_item(act):
+    """Every token goes to one expert of this rank: three row tiles of it beside the others' one."""
+    def one(cpu):
+        cpu["routing_logits"][:, 50] += 12.0
+    cpu, dev, out, intact, op = layer(20, 1024, 512, 256, 36, 32, act, change=one)
+    op.launch()
+    assert int(op.intermediate("counts").max()) == 20
+    check(cpu, out, act)
+    intact()
+
+
+@pytest.mark.parametrize("tokens,some", [(1, False), (6, False), (6, True)])
+def test_tokens_without_a_row_here(tokens, some):
+    """Their output is zero, also where no token of the step has a row on this rank."""
+    def elsewhere(cpu):
+        cpu["routing_logits"][:, 16:32] = -30.0
+        if some:
+            cpu["routing_logits"][3, 20] = 30.0
+    cpu, dev, out, intact, op = layer(tokens, 1024, 512, 64, 16, 16, "fp8", change=elsewhere)
+    op.launch()
+    rows = out.float().abs().amax(1).cpu()
+    assert (rows > 0).tolist() == [some and t == 3 for t in range(tokens)]
+    if some:
+        check(cpu, out, "fp8")
+    intact()
+
+
+def test_wait_runs_out_and_the_handle_stays_usable():
+    lib = cake._lib.library()
+    cpu, dev, out, intact, op = layer(3, 1024, 512, 64, 64, 0, "split")
+    assert lib.cake_b200_test_hooks(2048, 1) == 0          # waits give up after 2 Mi clocks; a gate/up item is never announced
+    try:
+        op.launch()
+        assert op.status() != 0                  # (which role notices first is not fixed)
+    finally:
+        assert lib.cake_b200_test_hooks(0, 0) == 0
+    op.launch()
+    assert op.status() == 0
+    check(cpu, out, "split")
+    intact()
+
+
+def test_several_streams_at_a_time():
+    """Layers that run at the same time share the SMs: an item waits only for items that a running CTA has."""
+    layers = [layer(4, 2048, 1024, 64, 32, 0, "fp8") for _ in range(4)]
+    streams = [torch.cuda.Stream() for _ in layers]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for (_, _, _, _, op), s in zip(layers, streams):
+            with torch.cuda.stream(s):
+                op.launch()
+    torch.cuda.synchronize()
+    for cpu, _, out, intact, op in layers:
+        assert op.status() == 0
+        check(cpu, out, "fp8")
+        intact()

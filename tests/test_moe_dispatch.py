@@ -1,4 +1,6 @@
 """Which kernels an MoE layer takes (csrc/moe.cu, make_layout), on either side of each line of the rule, asked of the library on the host."""
+import ctypes
+
 import pytest
 
 import open_cake_ir_b200 as cake
@@ -41,3 +43,17 @@ def test_experts_of_many_rows_go_to_the_core(tokens, local, act, above):
 def test_what_no_layer_is_made_of_is_refused():
     with pytest.raises(cake._lib.CakeError):
         form(4, 7168 + 1, 2048, 256, 8)
+
+
+@pytest.mark.parametrize("tokens,hidden,inter,experts,local,act,one", [
+    (8, 7168, 2048, 256, 256, "fp8", 1), (9, 7168, 2048, 256, 256, "fp8", 0),          # beyond eight tokens not where the core has the layer
+    (13, 7168, 2048, 256, 32, "fp8", 1), (14, 7168, 2048, 256, 32, "fp8", 0),
+    (6, 7168, 2048, 256, 256, "split", 1), (7, 7168, 2048, 256, 256, "split", 0),      # 48 rows of two terms
+    (4, 2048, 768, 128, 128, "fp8", 1), (5, 2048, 768, 128, 128, "fp8", 0),            # 32 rows of small experts
+    (3, 2048, 768, 128, 128, "split", 1), (4, 2048, 768, 128, 128, "split", 0),
+    (9, 4096, 1536, 128, 32, "fp8", 1), (17, 4096, 1536, 128, 16, "fp8", 0),           # one and a half rows to an expert
+    (17, 7168, 2048, 256, 8, "fp8", 0),                                                # experts of many rows may be the core's
+    (32, 1024, 512, 512, 60, "fp8", 1), (33, 1024, 512, 512, 60, "fp8", 0)])           # 256 pairs
+def test_products_and_combine_in_one_kernel(tokens, hidden, inter, experts, local, act, one):
+    cfg = cake._lib.MoeConfig(tokens, hidden, inter, experts, local, 8, 8, 4, 1, int(act == "split"), 0)
+    assert cake._lib.library().cake_b200_moe_few_tokens(ctypes.byref(cfg)) == one
