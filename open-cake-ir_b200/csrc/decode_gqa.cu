@@ -771,8 +771,11 @@ inline int launch(Params& p, int sms, cudaStream_t s) {
   geometry(p.hkv, sms, &p.ranges, &grid);
   // A sequence cut into more than a handful of pieces is merged by a kernel of its own: the one warp that merges it inside
   // the decode kernel reads four pieces at a time, 14 us for the 50 to 90 pieces of each of three long sequences, against
-  // 3 us for the launch.  At eight ranges a sequence the two cost the same.
-  p.merge_kernel = p.batch * 8 <= p.ranges;
+  // 3 us for the launch; and where it is not, a kernel in front clears its counters.  Merged in place and by the kernel, us, 8 KV heads (148 ranges), 32 query
+  // heads: 19 sequences of 100 to 400 tokens 17.5 and 13.8, of 2000 to 8000 69.6 and 66.4; 34 of 75 to 300 21 and 17, of 500 to 2000 39.0 and 38.0; 50 of 128 to 512
+  // 24.0 and 23.2; 74 of 150 to 600 30.9 and 31.5, of 750 to 3000 with 64 query heads 98 and 101; 128 of 500 to 2000 107 and 111.  4 KV heads (296 ranges): 50 23.5 and
+  // 19.5, 74 25.4 and 24.0, 128 62 and 65.
+  p.merge_kernel = p.batch * 3 <= p.ranges;
   p.plan_here = p.batch <= kPlanHere;
   if (!p.plan_here) {
     if (int rc = launch_dependent(gqa_plan_kernel, dim3(1), dim3(1024), 0, s, p)) return rc;
