@@ -864,9 +864,11 @@ mla_decode_kernel(const __grid_constant__ Params p) {
   if (warp == kMmaWarp) tmem_dealloc_pair(tmem_base, kTmemColumns);
 }
 
-// Merges the pieces of the cut sequences: a CTA two rows of one, 128 threads x 4 dims each, the results of four
-// pieces in flight (most sequences have two to four; eight in flight take registers from half of the resident rows).
-static __global__ void __launch_bounds__(256, 4)
+// Merges the pieces of the cut sequences, 128 threads x 4 dims to a row.  With many sequences most have two to four pieces: a CTA two rows, four pieces in
+// flight (eight take registers from half of the resident rows).  GROUPS > 1, few sequences, which have many pieces each: a CTA one row, whose
+// pieces its GROUPS times 128 threads share, eight in flight each, so that the 60 pieces of a lone sequence are two round trips to L2 and not 15.
+template <int GROUPS>
+static __global__ void __launch_bounds__(GROUPS > 1 ? GROUPS * 128 : 256, GROUPS > 1 ? 2 : 4)
 mla_reduce_kernel(const Params p) {
   // launched as a programmatic dependent of the decode kernel, which never lets it in early: it starts as that one's CTAs leave
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -891,39 +893,61 @@ mla_reduce_kernel(const Params p) {
     return;
   }
   const int column = int(blockIdx.x - 1) % p.reduce_columns, nth = int(blockIdx.x - 1) / p.reduce_columns;
+  const int4 cut = p.cuts[nth];                    // (asked for beside their number: there is room for as many as there are CTAs)
   if (nth >= *p.cut_count) return;
-  const int4 cut = p.cuts[nth];
   const int b = cut.x, first = cut.y, last = cut.z;
   const int4 s = p.seq ? p.seq[b] : make_int4(b, 1, 0, 0);
-  const int row = column * 2 + (threadIdx.x >> 7), d = (threadIdx.x & 127) * 4;
-  if (row >= s.y * p.heads) return;
+  constexpr int kFlight = GROUPS > 1 ? 8 : 4;
+  const int group = GROUPS > 1 ? threadIdx.x >> 7 : 0;
+  const int row = GROUPS > 1 ? column : column * 2 + int(threadIdx.x >> 7), d = (threadIdx.x & 127) * 4;
+  if (row >= s.y * p.heads) return;                // (the whole CTA where its threads share a row)
   auto slot_row = [&](int k) { return size_t(k == first ? cut.w : 2 * k) * p.rows + row; };
   float mm = -INFINITY, weight = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int k0 = first; k0 <= last; k0 += 4) {
-    float ls[4];
-    float4 v[4];
+  for (int k0 = first + group; k0 <= last; k0 += kFlight * GROUPS) {
+    float ls[kFlight];
+    float4 v[kFlight];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (k0 + i <= last) {
-        const size_t at = slot_row(k0 + i);
+    for (int i = 0; i < kFlight; ++i)
+      if (k0 + i * GROUPS <= last) {
+        const size_t at = slot_row(k0 + i * GROUPS);
         ls[i] = __ldcg(p.part_lse + at);
         v[i] = __ldcg(reinterpret_cast<const float4*>(p.part_o + at * kCkv + d));
       }
     float m_new = mm;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) if (k0 + i <= last) m_new = fmaxf(m_new, ls[i]);
+    for (int i = 0; i < kFlight; ++i) if (k0 + i * GROUPS <= last) m_new = fmaxf(m_new, ls[i]);
     const float rescale = mm == m_new ? 1.f : exp2f(mm - m_new);       // 0 the first time that anything is seen
     mm = m_new;
     weight *= rescale;
     acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (k0 + i <= last) {
+    for (int i = 0; i < kFlight; ++i)
+      if (k0 + i * GROUPS <= last) {
         const float wt = ls[i] == -INFINITY ? 0.f : exp2f(ls[i] - mm);      // -inf: nothing seen; a NaN, which the maximum leaves out, goes on as one
         weight += wt;
         acc.x += wt * v[i].x; acc.y += wt * v[i].y; acc.z += wt * v[i].z; acc.w += wt * v[i].w;
       }
+  }
+  if constexpr (GROUPS > 1) {
+    __shared__ float4 sums[GROUPS][128];
+    __shared__ float2 stats[GROUPS];               // maximum, weight
+    sums[group][threadIdx.x & 127] = acc;
+    if (d == 0) stats[group] = make_float2(mm, weight);
+    __syncthreads();
+    if (group) return;
+    mm = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < GROUPS; ++k) mm = fmaxf(mm, stats[k].x);
+    weight = 0.f;
+    acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < GROUPS; ++k) {
+      const float w = stats[k].x == mm ? 1.f : exp2f(stats[k].x - mm);      // a group that has seen nothing: 0, of a weight of 0 (or NaN)
+      const float4 v = sums[k][threadIdx.x & 127];
+      weight += w * stats[k].y;
+      acc.x += w * v.x; acc.y += w * v.y; acc.z += w * v.z; acc.w += w * v.w;
+    }
   }
   const size_t out_row = size_t(s.x) * p.heads + row;
   uint2 packed = make_uint2(0u, 0u);
@@ -1011,8 +1035,14 @@ inline int launch(const Handle* h, cudaStream_t s) {
   if (int rc = launch_dependent_cluster(2, p.sparse_indices ? mla_decode_kernel<true> : mla_decode_kernel<false>, grid, dim3(kThreads), kSmemBytes, s, decode))
     return rc;
   if (p.workers == 1) return 0;                              // nothing is ever cut
-  p.reduce_columns = (p.rows + 1) / 2;
-  return launch_dependent(mla_reduce_kernel, dim3(1 + p.reduce_columns * (p.workers - 1 < p.sequences ? p.workers - 1 : p.sequences)), dim3(256), 0, s, p);
+  const int cuts = p.workers - 1 < p.sequences ? p.workers - 1 : p.sequences;
+  // Few sequences have many pieces each (of a prefill, by what there is room for): their threads share a row, as long as that does not take more CTAs than run
+  // at a time (two rows to a CTA and so, us: 128 heads, one sequence of 7000 25.4 and 20.5, two of 4000 24.0 and 21.2, three of 20000 36.2 and 34.9, four of 1000
+  // 19.2 and 21.2; 64 heads, six of 6000 28.8 and 29.6; 16 heads, one of 7000 22.9 and 17.1, six of 6000 26.7 and 25.3, 14 of 8000 44.3 and 44.9).
+  const bool shared = p.sequences * 24 <= p.workers || (p.sequences * 8 <= p.workers && p.rows * p.sequences <= 192);
+  p.reduce_columns = shared ? p.rows : (p.rows + 1) / 2;
+  if (shared) return launch_dependent(mla_reduce_kernel<4>, dim3(1 + p.reduce_columns * cuts), dim3(512), 0, s, p);
+  return launch_dependent(mla_reduce_kernel<1>, dim3(1 + p.reduce_columns * cuts), dim3(256), 0, s, p);
 }
 
 }  // namespace mla
