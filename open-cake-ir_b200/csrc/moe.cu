@@ -23,6 +23,7 @@ __device__ __forceinline__ uint32_t ordered_bits(float v) {
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 // Routing of one token by one warp; lane l holds experts j*32 + l.  Returns selection k's expert and weight in lane k.
+__device__ __forceinline__ float from_ordered_bits(uint32_t key) { return __uint_as_float((key & 0x80000000u) ? key ^ 0x80000000u : ~key); }
 template <int EPL>
 __device__ __forceinline__ void route_token(const float* __restrict__ logits, const __nv_bfloat16* __restrict__ bias, float factor,
                                             int experts, int top_k, int n_group, int topk_group, int mode,
@@ -56,21 +57,29 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
         m1 = hi; m2 = lo;
       }
     };
-    if (group_size == 32 && n_group == EPL) {     // group j is slot j of every lane: the groups' reductions are independent of one another
-      float m1[EPL], m2[EPL];
+    bool not_a_number = false;
 #pragma unroll
-      for (int j = 0; j < EPL; ++j) { m1[j] = choice[j]; m2[j] = -INFINITY; }
+    for (int j = 0; j < EPL; ++j) not_a_number |= choice[j] != choice[j];
+    // Groups of 32: group j is slot j of every lane.  Its two best by one reduction of the ordered bits each, which all groups have under way at a time, no
+    // division to find an expert's group, and the ranks unrolled: as shuffles level by level and loops over the groups this was half of the routing of a
+    // token.  (A NaN, which the maxima below leave out, would come first.)
+    if (group_size == 32 && n_group == EPL && !__any_sync(0xffffffffu, not_a_number)) {
+      float score[EPL];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int j = 0; j < EPL; ++j) {
-          const float p1 = __shfl_xor_sync(0xffffffffu, m1[j], o), p2 = __shfl_xor_sync(0xffffffffu, m2[j], o);
-          const float hi = fmaxf(m1[j], p1), lo = fmaxf(fminf(m1[j], p1), fmaxf(m2[j], p2));
-          m1[j] = hi; m2[j] = lo;
-        }
+      for (int j = 0; j < EPL; ++j) {
+        const uint32_t key = ordered_bits(choice[j]), first = __reduce_max_sync(0xffffffffu, key);
+        const int holder = __ffs(__ballot_sync(0xffffffffu, key == first)) - 1;
+        const uint32_t second = __reduce_max_sync(0xffffffffu, lane == holder ? 0u : key);
+        score[j] = from_ordered_bits(first) + from_ordered_bits(second);
       }
 #pragma unroll
-      for (int j = 0; j < EPL; ++j) if (lane == j) mine = m1[j] + m2[j];
+      for (int g = 0; g < EPL; ++g) if (lane == g) mine = score[g];
+      int rank = 0;
+#pragma unroll
+      for (int g = 0; g < EPL; ++g) rank += score[g] > mine || (score[g] == mine && g < lane);
+      const uint32_t kept = __ballot_sync(0xffffffffu, lane < EPL && rank < topk_group);
+#pragma unroll
+      for (int j = 0; j < EPL; ++j) if (!((kept >> j) & 1u)) choice[j] = -INFINITY;
     } else {
       for (int g = 0; g < n_group; ++g) {
         float m1 = -INFINITY, m2 = -INFINITY;      // this lane's two best of group g
@@ -85,17 +94,17 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, co
         best_two(m1, m2);
         if (lane == g) mine = m1 + m2;
       }
-    }
-    int rank = 0;
-    for (int g = 0; g < n_group; ++g) {
-      const float other = __shfl_sync(0xffffffffu, mine, g);
-      rank += (other > mine) || (other == mine && g < lane);
-    }
-    const uint32_t kept = __ballot_sync(0xffffffffu, lane < n_group && rank < topk_group);
+      int rank = 0;
+      for (int g = 0; g < n_group; ++g) {
+        const float other = __shfl_sync(0xffffffffu, mine, g);
+        rank += (other > mine) || (other == mine && g < lane);
+      }
+      const uint32_t kept = __ballot_sync(0xffffffffu, lane < n_group && rank < topk_group);
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) {
-      const int id = j * 32 + lane;
-      if (id < experts && !((kept >> (id / group_size)) & 1u)) choice[j] = -INFINITY;
+      for (int j = 0; j < EPL; ++j) {
+        const int id = j * 32 + lane;
+        if (id < experts && !((kept >> (id / group_size)) & 1u)) choice[j] = -INFINITY;
+      }
     }
   }
   // Ordered score bits, 0 = absent or taken; the largest over the warp by one reduction, its lowest expert id by another.
