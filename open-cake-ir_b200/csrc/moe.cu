@@ -504,16 +504,16 @@ inline Layout make_layout(const cake_b200_moe_config& c) {
     if (c.tokens > above && (items - 1) * chosen * 3 * c.hidden * c.intermediate > 4e8) l.core_above = above;
   }
   // A step of few tokens in one kernel behind the routing, where its fixed times (the start and end of three more kernels) are much of the step.  That goes by the
-  // local pairs and by how large an expert is: with small ones an item of that kernel is shorter than what happens beside it, with two terms
-  // the rows' quantisation counts (other form and this one, us; one term, two terms.  Hidden 7168, experts of 2048: 1 token on 64 of 256 67 and 44, 44 and 34; 8 on 32
-  // 99 and 75, 82 and 79; 8 on all 256 422 and 378, 472 and 471; 11 on 128 286 and 259, 283 and 267; 16 on 64 179 and 165, 216 and 224.  4096, 1536, 32 of 128: 4 tokens
-  // 40 and 28, 43 and 38; 11 73 and 65, 63 and 60; 16 71 and 72.  2048, 768, 128 experts: 1 token 30 and 21, 33 and 27, 4 50 and 42, 53 and 52; 6 54 and 55, 59 and 62.  1024, 512,
-  // 64 experts: 1 token 19 and 14, 4 23.0 and 21.3, 24.2 and 23.2; 6 27.6 and 28.3).  Tokens that all go to the same experts make a second row
-  // tile from nine on, which reads the weights again: not where the tcgen05 core, which does not, has the layer, or some experts of it.
+  // local pairs and by how large an expert is, since with small ones an item of that kernel is shorter than what happens beside it (other form and this one, us,
+  // one term, two terms.  Hidden 7168, experts of 2048: 1 token on 64 of 256 67 and 45, 44 and 32; 8 on 32 99 and 74, 82 and 72; 8 on all 256 422 and 384, 472 and
+  // 430; 11 on 128 286 and 259, 283 and 260; 16 on 64 179 and 165, 216 and 205.  4096, 1536, 32 of 128: 4 tokens 40 and 28, 43 and 36; 11 73 and 65, 63 and 58; 16 71
+  // and 72.  2048, 768, 128 experts: 1 token 30 and 21, 32 and 23; 4 50 and 41, 53 and 46; 6 54 and 55, 59 and 60.  1024, 512, 64 experts: 1 token 19 and 14, 20 and 15;
+  // 4 23.0 and 21.3, 24.2 and 22.7; 6 27.6 and 28.3).  Tokens that all go to the same experts make a second row tile from nine on, which reads the weights again: not
+  // where the tcgen05 core, which does not, has the layer, or some experts of it.  (Eight such tokens, 8 of 256 experts, 76 and 92, two terms 137 and 132 with four.)
   const double rows = per_expert * c.local_experts;
   const bool large = 3.0 * c.hidden * c.intermediate >= 32e6;
   l.few = few::fits(int64_t(pairs)) && !l.core_above && (l.token_tiles == 1 || c.tokens <= kSmallTokens) &&
-          (large ? rows <= (l.terms == 2 ? 48 : 128) : rows <= (l.terms == 2 ? 24 : 32) && rows <= 1.5 * touched);
+          (large ? rows <= 128 : rows <= 32 && rows <= 1.5 * touched);
   if (l.split1 > 1 || l.few) l.act32 = take(pairs * c.intermediate * 4);      // SwiGLU output before its quantisation
   l.total = at;
   return l;

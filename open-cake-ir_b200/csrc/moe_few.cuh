@@ -4,7 +4,7 @@
 // which meet in warp order), for a layer that reads a few experts' weights and is over in tens of microseconds.  As four kernels (gate/up,
 // quantisation, down, combine) each of them began with an empty pipe and ended with an idle GPU.  Here the second product's weights, which wait for
 // nothing, are on their way while the first product ends.  One token, hidden 7168, experts of 2048: eight of 256 experts 79 us then and 65 now (352 MB, 54 us at
-// the copy rate), three of 32 48 and 39 with two terms; hidden 1024, experts of 512 19 and 14.  While it streams it reads 5.8 TB/s.
+// the copy rate), eight of 256 with two terms 83 and 66; hidden 1024, experts of 512 19 and 14.  While it streams it reads 5.8 TB/s.
 //
 // Work items, in order: the gate/up items (16 features of 8 rows), then the down items (64 columns of 8 rows).  They are DRAWN from a
 // counter in that order, so an item that has to wait (a down item, for all gate/up items of its rows) waits only for items that a running CTA
@@ -29,7 +29,7 @@ constexpr int kThreads = (kRowWarp + kRowWarps) * 32;
 constexpr int kRows = 8;                            // of an item
 constexpr int kSlotBytes = kSubTiles * kWeightBytes;
 // A slot of the down product: WK K blocks of WM times 32 columns.  (Eight of one: the rows' quantisation, whose work goes with a slot's K blocks, then
-// takes longer than the weights; one token on eight experts of 2048, hidden 7168, 70.7 us, two terms 79.9; 64.7 and 72.9 so.)
+// takes longer than the weights: one token on eight experts of 2048, hidden 7168, 70.7 us, two terms 79.9; 64.7 and 72.9 so.)
 constexpr int WK = 4, WM = kSubTiles / WK, kDownFeatures = 32 * WM;
 constexpr int kParts = 4 * WM;                      // finished parts of an item
 constexpr int kSlots = 5;
@@ -341,14 +341,15 @@ few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
           }
         }
       }
-      for (int j = (warp - kRowWarp + step0) % kRowWarps; j < steps; j += kRowWarps) {
-        const uint32_t step = step0 + j;
-        const int s = step % kSlots, kb0 = j * share, n = min(share, blocks - kb0);
-        const uint32_t slot = smem_u32(row_ring) + s * kRowSlotBytes;
-        if (!down) {
+      const int first = (warp - kRowWarp + step0) % kRowWarps;      // slots of the item that are this warp's: first, first + kRowWarps, ...
+      if (!down) {
+        // lane i: the scale of MMA tile i & 1 in K block i / 2 of a slot
+        const float* const sw = p.s13 + (size_t(it.group) * (2 * p.inter / 128) + it.feature0 / 128 + (lane & 1) * (p.inter / 128)) * blocks1 + (lane >> 1);
+        for (int j = first; j < steps; j += kRowWarps) {
+          const uint32_t step = step0 + j;
+          const int s = step % kSlots, kb0 = j * share, n = min(share, blocks - kb0);
+          const uint32_t slot = smem_u32(row_ring) + s * kRowSlotBytes;
           const int token_of = lane < it.rows ? sh->pair_of[it.row0 + lane] / p.top_k : 0;
-          // lane i: the scale of MMA tile i & 1 in K block i / 2 of a slot
-          const float* const sw = p.s13 + (size_t(it.group) * (2 * p.inter / 128) + it.feature0 / 128 + (lane & 1) * (p.inter / 128)) * blocks1 + kb0 + (lane >> 1);
           wait_above(&sh->issued, int(step), sh, p.status);
           for (int r = 0; r < it.rows; ++r) {
             const int token = __shfl_sync(0xffffffffu, token_of, r);
@@ -360,53 +361,75 @@ few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
             }
             if (lane < n) skinny::cp_async_4_zfill(slot + kScales + (r * kSubTiles + lane) * 4, p.sx + size_t(kb0 + lane) * p.tokens + token, true);
           }
-          if (lane >> 1 < n) skinny::cp_async_4_zfill(slot + kWeightScales + lane * 4, sw, true);
+          if (lane >> 1 < n) skinny::cp_async_4_zfill(slot + kWeightScales + lane * 4, sw + kb0, true);
           cp_async_arrive_noinc(&sh->row_full[s]);
-        } else {
-          // Quantisation of the rows (skinny::quantize_kernel's arithmetic): eight lanes to a K block, each with four times four features of it, and the
-          // next rows on their way.
-          const int b = lane >> 3, c = lane & 7;
-          const float4* const act = reinterpret_cast<const float4*>(p.act32 + size_t(it.row0) * p.inter + size_t(kb0) * 128) + b * 32 + c;
-          const uint32_t block = slot + b * (TERMS * kTermBytes) + (c & 3) * 4;
-          auto ask = [&](int r, float4 (&v)[4]) {
+        }
+      } else {
+        // Quantisation of the rows (skinny::quantize_kernel's arithmetic): eight lanes to a K block, each with four times four features of it.  The next
+        // rows, of this slot or of the warp's next one, are on their way meanwhile: asked for slot by slot, a row took its trip to L2 each time, 1.3 us a
+        // slot with two terms where the weights take 0.7.
+        const int b = lane >> 3, c = lane & 7;
+        const float4* const act = reinterpret_cast<const float4*>(p.act32 + size_t(it.row0) * p.inter) + b * 32 + c;
+        const float* const sw = p.s2 + (size_t(it.group) * (p.hidden / 128) + it.feature0 / 128) * blocks2 + (lane >> 1);
+        constexpr int kRowsAhead = 2;              // (three spill, and take eight equal tokens from 92 to 99 us)
+        float4 v[kRowsAhead][4];
+        float w[kRowsAhead];
+        const int row_step = p.inter / 4;
+        int ask_j = first, ask_r = 0;
+        const float4* asked = act + first * (WK * 32);
+        bool there_is = b < blocks2 - first * WK;
+        auto ask = [&](int i) {
+          if (ask_j >= steps) return;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] = r < it.rows && b < n ? __ldcg(act + size_t(r) * (p.inter / 4) + i * 8) : make_float4(0.f, 0.f, 0.f, 0.f);
-          };
-          auto quantise = [&](int r, float4 (&v)[4]) {
+          for (int k = 0; k < 4; ++k) v[i][k] = there_is ? __ldcg(asked + k * 8) : make_float4(0.f, 0.f, 0.f, 0.f);
+          if (ask_r == 0) w[i] = lane >> 1 < blocks2 - ask_j * WK ? __ldg(sw + ask_j * WK) : 0.f;
+          asked += row_step;
+          if (++ask_r == it.rows) {
+            ask_r = 0;
+            ask_j += kRowWarps;
+            asked = act + ask_j * (WK * 32);
+            there_is = b < blocks2 - ask_j * WK;
+          }
+        };
+#pragma unroll
+        for (int i = 0; i < kRowsAhead; ++i) ask(i);
+        uint32_t s = 0, slot = 0;
+        for (int j = first, r = 0; j < steps;) {
+#pragma unroll
+          for (int i = 0; i < kRowsAhead; ++i) {
+            if (j >= steps) break;
+            if (r == 0) {
+              s = (step0 + j) % kSlots;
+              slot = smem_u32(row_ring) + s * kRowSlotBytes;
+              wait_above(&sh->issued, int(step0) + j, sh, p.status);
+              if (lane < 2 * WK) sts32f(slot + kWeightScales + lane * 4, w[i]);
+            }
             for (int term = 0; term < TERMS; ++term) {
+              float4 (&x)[4] = v[i];
               float m = 0.f;
 #pragma unroll
-              for (int i = 0; i < 4; ++i) m = fmaxf(m, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+              for (int k = 0; k < 4; ++k) m = fmaxf(m, fmaxf(fmaxf(fabsf(x[k].x), fabsf(x[k].y)), fmaxf(fabsf(x[k].z), fabsf(x[k].w))));
 #pragma unroll
               for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
               const float scale = m > 0.f ? m / 448.f : 1.f, inv = 1.f / scale;
               if (c == 0) sts32f(slot + kScales + ((term * kRows + r) * WK + b) * 4, scale);
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const uint32_t packed = pack_e4m3x4(v[i].x * inv, v[i].y * inv, v[i].z * inv, v[i].w * inv);
-                asm volatile("st.shared.b32 [%0], %1;" ::"r"(block + term * kTermBytes + r * 128 + (((2 * i + (c >> 2)) ^ r) << 4)), "r"(packed) : "memory");
-                if (TERMS > 1) {
-                  v[i].x -= e4m3_to_float(uint8_t(packed)) * scale; v[i].y -= e4m3_to_float(uint8_t(packed >> 8)) * scale;
-                  v[i].z -= e4m3_to_float(uint8_t(packed >> 16)) * scale; v[i].w -= e4m3_to_float(uint8_t(packed >> 24)) * scale;
+              for (int k = 0; k < 4; ++k) {
+                const uint32_t packed = pack_e4m3x4(x[k].x * inv, x[k].y * inv, x[k].z * inv, x[k].w * inv);
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(slot + (b * TERMS + term) * kTermBytes + r * 128 + (((2 * k + (c >> 2)) ^ r) << 4) + (c & 3) * 4), "r"(packed) : "memory");
+                if (term + 1 < TERMS) {
+                  x[k].x -= e4m3_to_float(uint8_t(packed)) * scale; x[k].y -= e4m3_to_float(uint8_t(packed >> 8)) * scale;
+                  x[k].z -= e4m3_to_float(uint8_t(packed >> 16)) * scale; x[k].w -= e4m3_to_float(uint8_t(packed >> 24)) * scale;
                 }
               }
             }
-          };
-          const float w = lane >> 1 < n ? __ldg(p.s2 + (size_t(it.group) * (p.hidden / 128) + it.feature0 / 128) * blocks2 + kb0 + (lane >> 1)) : 0.f;
-          constexpr int kRowsAhead = TERMS == 2 ? 2 : 3;           // what there are registers for
-          float4 v[kRowsAhead][4];
-#pragma unroll
-          for (int i = 0; i < kRowsAhead; ++i) ask(i, v[i]);
-          wait_above(&sh->issued, int(step), sh, p.status);
-          for (int r = 0; r < it.rows; r += kRowsAhead) {
-#pragma unroll
-            for (int i = 0; i < kRowsAhead; ++i) {
-              if (r + i < it.rows) quantise(r + i, v[i]);
-              ask(r + i + kRowsAhead, v[i]);
+            ask(i);
+            if (++r == it.rows) {
+              mbar_arrive(&sh->row_full[s]);
+              r = 0;
+              j += kRowWarps;
             }
           }
-          if (lane >> 1 < n) sts32f(slot + kWeightScales + lane * 4, w);
-          mbar_arrive(&sh->row_full[s]);
         }
       }
       step0 += steps;
@@ -427,6 +450,9 @@ few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
     const bool down = it.phase == 1;
     const int share = down ? WK : kSubTiles, blocks = down ? blocks2 : blocks1, part = down ? sub % WK : sub, steps = (blocks + share - 1) / share;
     if (k % kTeams != team) { step0 += steps; continue; }
+    // Two terms of up to four rows are the eight columns of one product, their sums added up at the end: mma.sync takes e4m3 at 37 clocks an
+    // instruction and quarter of an SM (measured), 1200 of a slot's 1400 clocks with a product for each term.
+    const bool both = TERMS == 2 && down && it.rows <= kRows / 2, apart = TERMS == 2 && down && !both;
     float acc[2][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[0][e] = acc[1][e] = 0.f;
@@ -442,30 +468,51 @@ few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
         const uint32_t from = smem_u32(ring) + s * kSlotBytes + (down ? part * WM + sub / WK : sub) * kWeightBytes;
         const uint32_t slot = smem_u32(row_ring) + s * kRowSlotBytes;
         const float2 sw = skinny::lds64f(slot + kWeightScales + part * 8);
+        // (rows that the item does not have hold whatever was there: their columns of the product are not used)
+        const int b_row = both ? g8 & 3 : g8, s_row = both ? (q >> 1) * kRows + (q & 1) * 2 : q * 2;
+        const uint32_t rows = slot + ((down ? part * TERMS : part) + (both ? g8 >> 2 : 0)) * kTermBytes + b_row * 128, scales = slot + kScales + (s_row * share + part) * 4;
+        // Both MMA tiles and terms beside one another: a sum's four products come one after another, and four such chains one after another took
+        // longer than a slot takes to come.
+        float d[2][TERMS][4];
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {              // MMA tile
-          uint32_t a[2][8];                        // [row g / g + 8][k-step pair words]
+        for (int t = 0; t < 2; ++t)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int r = t * 16 + h * 8 + g8;
-            const uint4 lo = skinny::lds128(from + r * 128 + (((2 * q) ^ g8) << 4)), hi = skinny::lds128(from + r * 128 + (((2 * q + 1) ^ g8) << 4));
-            a[h][0] = lo.x; a[h][1] = lo.y; a[h][2] = lo.z; a[h][3] = lo.w;
-            a[h][4] = hi.x; a[h][5] = hi.y; a[h][6] = hi.z; a[h][7] = hi.w;
-          }
-#pragma unroll 1
-          for (int term = 0; term < (down ? TERMS : 1); ++term) {
-            // (rows that the item does not have hold whatever was there: their columns of the product are not used)
-            const uint32_t xr = slot + (down ? part * TERMS + term : part) * kTermBytes + g8 * 128, scales = slot + kScales + ((term * kRows + q * 2) * share + part) * 4;
-            const uint4 lo = skinny::lds128(xr + (((2 * q) ^ g8) << 4)), hi = skinny::lds128(xr + (((2 * q + 1) ^ g8) << 4));
-            const uint32_t b[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-            const float w = t == 0 ? sw.x : sw.y, s0 = w * lds32f(scales), s1 = w * lds32f(scales + share * 4);
-            float d[4] = {0.f, 0.f, 0.f, 0.f};
+          for (int term = 0; term < TERMS; ++term)
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) skinny::mma_e4m3(d, a[0][2 * ks], a[1][2 * ks], a[0][2 * ks + 1], a[1][2 * ks + 1], b[2 * ks], b[2 * ks + 1]);
-            acc[t][0] = fmaf(d[0], s0, acc[t][0]); acc[t][1] = fmaf(d[1], s1, acc[t][1]);
-            acc[t][2] = fmaf(d[2], s0, acc[t][2]); acc[t][3] = fmaf(d[3], s1, acc[t][3]);
-          }
+            for (int e = 0; e < 4; ++e) d[t][term][e] = 0.f;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {     // two k-steps: a 16-byte chunk of every row
+          const uint32_t chunk = ((2 * q + half) ^ g8) << 4, b_chunk = ((2 * q + half) ^ b_row) << 4;
+          uint4 a[2][2], b[TERMS];                 // [MMA tile][row g / g + 8], [term]
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) a[t][h] = skinny::lds128(from + (t * 16 + h * 8 + g8) * 128 + chunk);
+#pragma unroll
+          for (int term = 0; term < TERMS; ++term) if (term == 0 || apart) b[term] = skinny::lds128(rows + term * kTermBytes + b_chunk);
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int term = 0; term < TERMS; ++term)
+              if (term == 0 || apart) {
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                  if (k == 0) skinny::mma_e4m3(d[t][term], a[t][0].x, a[t][1].x, a[t][0].y, a[t][1].y, b[term].x, b[term].y);
+                  else skinny::mma_e4m3(d[t][term], a[t][0].z, a[t][1].z, a[t][0].w, a[t][1].w, b[term].z, b[term].w);
+                }
+              }
         }
+#pragma unroll
+        for (int term = 0; term < TERMS; ++term)
+          if (term == 0 || apart) {
+            const float sx0 = lds32f(scales + term * (kRows * share * 4)), sx1 = lds32f(scales + term * (kRows * share * 4) + share * 4);
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+              const float w = t == 0 ? sw.x : sw.y, s0 = w * sx0, s1 = w * sx1;
+              acc[t][0] = fmaf(d[t][term][0], s0, acc[t][0]); acc[t][1] = fmaf(d[t][term][1], s1, acc[t][1]);
+              acc[t][2] = fmaf(d[t][term][2], s0, acc[t][2]); acc[t][3] = fmaf(d[t][term][3], s1, acc[t][3]);
+            }
+          }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh->empty[s]);
@@ -481,6 +528,10 @@ few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
 #pragma unroll
       for (int w = 0; w < kSubTiles; ++w)
         if (w < share) { v0 += sh->reduce[first + w][e][lane]; v1 += sh->reduce[first + w][4 + e][lane]; }
+      if (both) {                                  // the second term's columns are two lanes further
+        v0 += __shfl_down_sync(0xffffffffu, v0, 2);
+        v1 += __shfl_down_sync(0xffffffffu, v1, 2);
+      }
     }
     team_sync(team);
     if (e < 4) {

@@ -48,9 +48,10 @@ def test_what_no_layer_is_made_of_is_refused():
 @pytest.mark.parametrize("tokens,hidden,inter,experts,local,act,one", [
     (8, 7168, 2048, 256, 256, "fp8", 1), (9, 7168, 2048, 256, 256, "fp8", 0),          # beyond eight tokens not where the core has the layer
     (13, 7168, 2048, 256, 32, "fp8", 1), (14, 7168, 2048, 256, 32, "fp8", 0),
-    (6, 7168, 2048, 256, 256, "split", 1), (7, 7168, 2048, 256, 256, "split", 0),      # 48 rows of two terms
+    (8, 7168, 2048, 256, 256, "split", 1), (9, 7168, 2048, 256, 256, "split", 0),
+    (11, 7168, 2048, 256, 64, "split", 1), (12, 7168, 2048, 256, 64, "split", 0),
     (4, 2048, 768, 128, 128, "fp8", 1), (5, 2048, 768, 128, 128, "fp8", 0),            # 32 rows of small experts
-    (3, 2048, 768, 128, 128, "split", 1), (4, 2048, 768, 128, 128, "split", 0),
+    (4, 2048, 768, 128, 128, "split", 1), (5, 2048, 768, 128, 128, "split", 0),
     (9, 4096, 1536, 128, 32, "fp8", 1), (17, 4096, 1536, 128, 16, "fp8", 0),           # one and a half rows to an expert
     (17, 7168, 2048, 256, 8, "fp8", 0),                                                # experts of many rows may be the core's
     (32, 1024, 512, 512, 60, "fp8", 1), (33, 1024, 512, 512, 60, "fp8", 0)])           # 256 pairs
