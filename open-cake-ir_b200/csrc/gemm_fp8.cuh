@@ -237,12 +237,20 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
     tmem_alloc(&sh->tmem_base, kTmemColumns);
     tmem_relinquish();
   }
-  // launched as a programmatic dependent where the caller says so: everything above overlaps the kernel before
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // Long before any wait can run out, as the grid fits the GPU and its CTAs start together.  (Were the SMs of CTA 0 held by other work for the second that a
-  // wait takes to run out, its report would be lost; a kernel in front that clears the word takes 0.4 us of 7 to 21, 0.7 to 1.2 launched from the host.)
-  if (MODE == kDense && !p.queue && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;
+  if (threadIdx.x == 96) {
+    tma_prefetch_descriptor(&maps.a);
+    tma_prefetch_descriptor(&maps.a_tail);
+    tma_prefetch_descriptor(&maps.b);
+    if constexpr (MODE == kGateUp) tma_prefetch_descriptor(&maps.b_narrow);
+  }
+  // Launched as a programmatic dependent: what comes before this overlaps the kernel in front.  The dense form's items lie in the parameters, so there
+  // the roles are set up and the first item found by then as well, and each waits where it begins (its bounded waits among them; the first load
+  // came 1.2 us behind that kernel's end with the wait here; launches in turn: 64 x 4096 x 7168 11.7 and 11.0 us, 32 x 2048 x 2048 6.5 and 6.0).
+  auto behind_grid = []() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  };
+  if (MODE != kDense) behind_grid();
   if (warp == kControlWarps) {   // m-tile prefix over groups (serial per lane chunk, then a warp scan)
     int running = 0;
     for (int base = 0; base < p.groups; base += 32) {
@@ -278,10 +286,6 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
   if (warp == 0) {
     // ------------------------------ TMA producer --------------------------------------
     if (elect_one()) {
-      tma_prefetch_descriptor(&maps.a);
-      tma_prefetch_descriptor(&maps.a_tail);
-      tma_prefetch_descriptor(&maps.b);
-      if constexpr (MODE == kGateUp) tma_prefetch_descriptor(&maps.b_narrow);
       const uint64_t keep = l2_policy_evict_last();    // activations: re-read by every n tile
       // Work items.  With a queue, this thread draws them (the first is the CTA's index, every later
       // one comes from the device counter, asked for one item ahead) and hands each to the other
@@ -305,6 +309,12 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
         mbar_arrive(&sh->item_full[slot]);
       };
       find(g, 0);
+      if (MODE == kDense) {
+        behind_grid();
+        // Long before any wait can run out, as the grid fits the GPU and its CTAs start together.  (Were the SMs of CTA 0 held by other work for the second that
+        // a wait takes to run out, its report would be lost; a kernel in front that clears the word takes 0.4 us of 7 to 21, 0.7 to 1.2 launched from the host.)
+        if (!p.queue && blockIdx.x == 0) *p.status = 0;
+      }
       const int find_at = (k_count - 1) / 2;
       while (ok && valid) {
         g = p.queue ? int(gridDim.x) + atomicAdd(p.queue, 1) : g + int(gridDim.x);
@@ -350,6 +360,7 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------------------
     if (elect_one()) {
+      if (MODE == kDense) asm volatile("griddepcontrol.wait;" ::: "memory");
       uint32_t it = 0, k = 0;
       At<SPLIT> at;
       bool ok = true;
@@ -402,6 +413,7 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
     // thread loading its own scales a few blocks ahead into registers paid one round trip to L2 per block, because handing
     // a register on from block to block waits for the load behind it; a barrier of their own cost 150 clocks per block,
     // and reading them when they are needed 75 to 170, since the reads queue behind the tensor core's operand reads.)
+    if (MODE == kDense) asm volatile("griddepcontrol.wait;" ::: "memory");
     const int sfb_rows = p.b_rows_per_group / 128;
     uint32_t it = 0, k = 0;
     At<SPLIT> at;                        // of block it - kScaleAhead
@@ -447,6 +459,7 @@ gemm_fp8_kernel(const __grid_constant__ Maps<MODE> maps, const Params p) {
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
     // ------------------------------ epilogue / promotion ------------------------------
+    if (MODE == kDense) asm volatile("griddepcontrol.wait;" ::: "memory");
     const int ew = warp - kControlWarps;
     const int quad = warp & 3;                 // TMEM lanes a warp may read: 32*(warp id % 4)
     const int cg = ew >> 2;                    // column group 0..1
