@@ -314,16 +314,18 @@ route_place_kernel(const float* __restrict__ logits, const __nv_bfloat16* __rest
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int offset = __ldg(offset_ptr);
-  int id;
-  float weight;
-  route_token<EPL>(logits + size_t(warp) * experts, bias, __ldg(factor_ptr), experts, top_k, n_group, topk_group, mode, id, weight);
-  if (lane < top_k) {
-    const int p = warp * top_k + lane;
-    expert_ids[p] = id;
-    route_weights[p] = weight;
-    local_id[p] = id >= offset && id < offset + local_experts ? id - offset : -1;
-  }
   const int pairs = tokens * top_k;
+  if (warp < tokens) {                             // (the others help with what comes behind: 257 first pairs and hundreds of counters)
+    int id;
+    float weight;
+    route_token<EPL>(logits + size_t(warp) * experts, bias, __ldg(factor_ptr), experts, top_k, n_group, topk_group, mode, id, weight);
+    if (lane < top_k) {
+      const int p = warp * top_k + lane;
+      expert_ids[p] = id;
+      route_weights[p] = weight;
+      local_id[p] = id >= offset && id < offset + local_experts ? id - offset : -1;
+    }
+  }
   if (threadIdx.x < 4 && pairs + threadIdx.x < kSmallTokens * 32) local_id[pairs + threadIdx.x] = -1;      // read four at a time
   for (int i = threadIdx.x; i < clear_words; i += blockDim.x) clear[i] = 0;
   __syncthreads();
@@ -831,7 +833,7 @@ static int moe_launch_stage(cake::moe::MoeHandle* h, int stage, cudaStream_t s, 
       if (moe::routes_in_one(c, l, few)) {
         const int epl = (c.experts + 31) / 32;
         auto* kernel = epl <= 2 ? moe::route_place_kernel<2> : epl <= 4 ? moe::route_place_kernel<4> : epl <= 8 ? moe::route_place_kernel<8> : moe::route_place_kernel<16>;
-        return launch_dependent(kernel, dim3(1), dim3(32 * tokens), 0, s, h->logits, h->bias, h->factor, h->local_offset, h->expert_ids, h->route_weights,
+        return launch_dependent(kernel, dim3(1), dim3(32 * moe::kSmallTokens), 0, s, h->logits, h->bias, h->factor, h->local_offset, h->expert_ids, h->route_weights,
                                 pa.counts, pa.offsets, pa.sorted_pairs, pa.inv_perm, tokens, c.experts, c.top_k, c.n_group, c.topk_group,
                                 c.routing_mode, c.local_experts, clear, few ? few_words : 64);
       }
