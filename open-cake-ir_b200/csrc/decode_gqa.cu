@@ -632,9 +632,9 @@ gqa_decode_kernel(const __grid_constant__ Params p) {
   cp_async_wait<0>();
 }
 
-// Merges the pieces of sequences that are cut into many: one CTA per (head, sequence), each of its eight warps every eighth
+// Merges the pieces of sequences that are cut into many: one CTA per (head, sequence), each of its warps every kMergeWarps-th
 // piece, four in flight, a float4 of the row to a lane.
-constexpr int kMergeWarps = 8;
+template <int kMergeWarps>
 __global__ void __launch_bounds__(kMergeWarps * 32)
 gqa_merge_kernel(const Params p) {
   __shared__ float4 sums[kMergeWarps][32];
@@ -772,10 +772,10 @@ inline int launch(Params& p, int sms, cudaStream_t s) {
   // A sequence cut into more than a handful of pieces is merged by a kernel of its own: the one warp that merges it inside
   // the decode kernel reads four pieces at a time, 14 us for the 50 to 90 pieces of each of three long sequences, against
   // 3 us for the launch; and where it is not, a kernel in front clears its counters.  Merged in place and by the kernel, us, 8 KV heads (148 ranges), 32 query
-  // heads: 19 sequences of 100 to 400 tokens 17.5 and 13.8, of 2000 to 8000 69.6 and 66.4; 34 of 75 to 300 21 and 17, of 500 to 2000 39.0 and 38.0; 50 of 128 to 512
-  // 24.0 and 23.2; 74 of 150 to 600 30.9 and 31.5, of 750 to 3000 with 64 query heads 98 and 101; 128 of 500 to 2000 107 and 111.  4 KV heads (296 ranges): 50 23.5 and
-  // 19.5, 74 25.4 and 24.0, 128 62 and 65.
-  p.merge_kernel = p.batch * 3 <= p.ranges;
+  // heads: 19 sequences of 100 to 400 tokens 17.5 and 13.8; 50 of 128 to 512 23.8 and 21.8, with 64 query heads 28.0 and 24.8; 64 of 512 to 4096 101.2 and 100.5;
+  // 74 of 150 to 600 29.8 and 30.9, with 64 query heads 35.3 and 33.8; 128 of 500 to 2000 107.6 and 108.8, with 64 query heads 110.5 and 115.3.
+  // 4 KV heads (296 ranges): 100 23.5 and 20.6, 128 63.4 and 63.3.
+  p.merge_kernel = p.batch * 2 <= p.ranges;
   p.plan_here = p.batch <= kPlanHere;
   if (!p.plan_here) {
     if (int rc = launch_dependent(gqa_plan_kernel, dim3(1), dim3(1024), 0, s, p)) return rc;
@@ -786,7 +786,11 @@ inline int launch(Params& p, int sms, cudaStream_t s) {
   // for it on the device, which takes the second launch latency off the critical path.
   if (int rc = launch_dependent(gqa_decode_kernel, dim3(grid), dim3(kWarps * 32), kSmemBytes, s, p)) return rc;
   if (!p.merge_kernel) return 0;
-  return launch_dependent(gqa_merge_kernel, dim3(p.hq, p.batch), dim3(kMergeWarps * 32), 0, s, p);
+  // As many warps to a head as it has pieces for.  With 8 and 16, us: one sequence of 2000 tokens 11.3 and 10.7, of 32000 29.7 and 29.1; one KV head, two sequences
+  // 23.1 and 19.1; 12 sequences 42.4 and 44.1.  With 4 and 8: 19 sequences 25.6 and 26.1, 30 90.7 and 92.2, 40 with 64 query heads 43.8 and 45.6.
+  const int pieces = p.ranges / p.batch;
+  auto* merge = pieces >= 64 ? gqa_merge_kernel<16> : pieces > 10 ? gqa_merge_kernel<8> : gqa_merge_kernel<4>;
+  return launch_dependent(merge, dim3(p.hq, p.batch), dim3(pieces >= 64 ? 512 : pieces > 10 ? 256 : 128), 0, s, p);
 }
 
 }  // namespace gqa

@@ -16,7 +16,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("batch,heads,kv_heads,longest", [
     (1, 8, 1, 5000), (18, 8, 8, 700), (19, 8, 8, 700), (74, 4, 2, 300), (40, 6, 3, 900), (9, 32, 16, 1500),
-    (49, 8, 8, 700), (50, 8, 8, 700), (49, 16, 16, 700), (98, 4, 4, 300), (99, 4, 4, 300),          # on either side of the merge kernel's line
+    (49, 8, 8, 700), (50, 8, 8, 700), (49, 16, 16, 700), (98, 4, 4, 300), (99, 4, 4, 300),
+    (74, 8, 8, 700), (75, 8, 8, 700), (74, 16, 16, 700), (148, 4, 4, 300), (149, 4, 4, 300),          # on either side of the merge kernel's line
+    (2, 8, 8, 4000), (3, 8, 8, 4000), (13, 8, 8, 700), (14, 8, 8, 700),                            # and of its numbers of warps
     (1024, 4, 4, 40), (1025, 4, 4, 40), (1024, 2, 1, 90)])
 def test_gqa_decode(batch, heads, kv_heads, longest):
     lens = [0 if i % 7 == 3 else 1 + (i * 37) % longest for i in range(batch - 1)] + [longest]
@@ -48,7 +50,8 @@ def test_mla_prefill(segments, rows):
     check(out, lse, want)
 
 
-@pytest.mark.parametrize("batch,heads,kv_heads", [(3, 8, 8), (40, 8, 8), (80, 4, 2), (9, 16, 0), (60, 8, 8), (110, 4, 4)])          # merge kernel (three times), MLA, merged in place (twice)
+@pytest.mark.parametrize("batch,heads,kv_heads", [(3, 8, 8), (40, 8, 8), (80, 4, 2), (9, 16, 0), (60, 8, 8), (110, 4, 4),
+                                                    (80, 8, 8), (150, 4, 4)])          # MLA in the fourth, merged in place in the last two, else the merge kernel
 def test_lengths_rewritten_in_front_of_each_launch(batch, heads, kv_heads):
     """One handle, launched behind kernels of the same stream that write its lengths and page table anew; nothing waits in between."""
     page, longest, steps = 16, 900, 6
