@@ -4,7 +4,7 @@
 // Operator and layouts: src/open_cake_ir/tasks/solx_fib/moe.py:13-20 (tensor ABI), :122-155
 // (oracle), :275-287 (routing).  The grouped GEMMs run on the tcgen05 core in gemm_fp8.cuh, or, at a few
 // rows per expert, on the weight-streaming kernel in gemm_skinny.cuh, which takes token rows where they
-// lie; the small integer kernels here are warp-level (top-k by ordered keys, ballot prefix scans).
+// lie; a step of few tokens takes both products and the combine in one kernel (moe_few.cuh).  The small integer kernels here are warp-level (top-k by ordered keys, ballot prefix scans).
 #include "gemm_skinny.cuh"
 #include "moe_few.cuh"
 #include "../../include/cake_b200.h"

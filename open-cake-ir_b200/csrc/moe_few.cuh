@@ -29,7 +29,7 @@ constexpr int kThreads = (kRowWarp + kRowWarps) * 32;
 constexpr int kRows = 8;                            // of an item
 constexpr int kSlotBytes = kSubTiles * kWeightBytes;
 // A slot of the down product: WK K blocks of WM times 32 columns.  (Eight of one: the rows' quantisation, whose work goes with a slot's K blocks, then
-// takes longer than the weights: one token on eight experts of 2048, hidden 7168, 70.7 us, two terms 79.9; 64.7 and 72.9 so.)
+// takes longer than the weights: one token on eight experts of 2048, hidden 7168, 70.7 us, two terms 79.9, against 64.7 and 72.9 when it was chosen; 65 and 66 now.)
 constexpr int WK = 4, WM = kSubTiles / WK, kDownFeatures = 32 * WM;
 constexpr int kParts = 4 * WM;                      // finished parts of an item
 constexpr int kSlots = 5;
