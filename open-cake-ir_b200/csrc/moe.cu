@@ -805,7 +805,7 @@ extern "C" int cake_b200_moe_create(void** buffers, const cake_b200_moe_config* 
     p.top_k = c.top_k;
     rc = few::weight_maps(&h->few_maps, buffers[4], buffers[6], c.local_experts, hidden, inter);
     if (!rc)
-      rc = few::with_terms(l.terms, [](auto* kernel) {
+      rc = few::with_kernel(l.terms, few::row_warps(l.terms, p.tokens, hidden, inter), [](auto* kernel) {
         return int(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, few::kSmemBytes));
       });
     if (rc) { delete h; return rc; }
@@ -893,8 +893,9 @@ static int moe_launch_few(cake::moe::MoeHandle* h, cudaStream_t s) {
   few::Params p = h->few;
   p.wait_kiloclocks = test_hooks().budget_kiloclocks;
   p.skip_signal = test_hooks().skip_load;
-  return few::with_terms(h->layout.terms, [&](auto* kernel) {
-    return launch_dependent(kernel, dim3(h->grid), dim3(few::kThreads), few::kSmemBytes, s, h->few_maps, p);
+  const int row_warps = few::row_warps(h->layout.terms, p.tokens, p.hidden, p.inter);
+  return few::with_kernel(h->layout.terms, row_warps, [&](auto* kernel) {
+    return launch_dependent(kernel, dim3(h->grid), dim3(few::threads(row_warps)), few::kSmemBytes, s, h->few_maps, p);
   });
 }
 

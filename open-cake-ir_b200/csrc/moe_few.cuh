@@ -10,7 +10,7 @@
 // counter in that order, so an item that has to wait (a down item, for all gate/up items of its rows) waits only for items that a running CTA
 // has already drawn: no number of resident CTAs is assumed, and several such kernels may share the GPU.
 // A CTA: two teams of eight warps that multiply, taking its items in turn; a warp that brings the weights in, a slot of 32 KB to an instruction; two
-// that bring rows and scales; and one for what happens between CTAs: it draws and locates items, announces finished down items and, where one was the
+// or four that bring rows and scales; and one for what happens between CTAs: it draws and locates items, announces finished down items and, where one was the
 // last of its columns, adds the tokens' rows up (the combine step: slot order, fp32).  A gate/up item leaves its features in fp32, and the row warps of
 // the down items quantise them on the way (the same 1 x 128 groups and bits).
 #pragma once
@@ -24,8 +24,8 @@ using skinny::kWeightBytes;
 using skinny::kMaxGroups;
 constexpr int kSubTiles = 8;                        // of 32 weight rows and one K block, in a slot of the ring
 constexpr int kTeams = 2, kComputeWarps = kTeams * kSubTiles,      // two teams of warps, which take a CTA's items in turn
-               kDrawWarp = kComputeWarps, kLoadWarp = kDrawWarp + 1, kRowWarp = kDrawWarp + 2, kRowWarps = 2;
-constexpr int kThreads = (kRowWarp + kRowWarps) * 32;
+               kDrawWarp = kComputeWarps, kLoadWarp = kDrawWarp + 1, kRowWarp = kDrawWarp + 2;
+inline constexpr int threads(int row_warps) { return (kRowWarp + row_warps) * 32; }
 constexpr int kRows = 8;                            // of an item
 constexpr int kSlotBytes = kSubTiles * kWeightBytes;
 // A slot of the down product: WK K blocks of WM times 32 columns.  (Eight of one: the rows' quantisation, whose work goes with a slot's K blocks, then
@@ -133,9 +133,10 @@ __device__ __forceinline__ bool wait_above(const int* word, int value, Shared* s
 }
 
 // TERMS: e4m3 terms of the SwiGLU output.
-template <int TERMS>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int TERMS, int ROW_WARPS>
+__global__ void __launch_bounds__((kRowWarp + ROW_WARPS) * 32, 1)
 few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
+  constexpr int kThreads = (kRowWarp + ROW_WARPS) * 32;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* row_ring = ring + kSlots * kSlotBytes;
@@ -341,11 +342,11 @@ few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
           }
         }
       }
-      const int first = (warp - kRowWarp + step0) % kRowWarps;      // slots of the item that are this warp's: first, first + kRowWarps, ...
+      const int first = (warp - kRowWarp + step0) % ROW_WARPS;      // slots of the item that are this warp's: first, first + ROW_WARPS, ...
       if (!down) {
         // lane i: the scale of MMA tile i & 1 in K block i / 2 of a slot
         const float* const sw = p.s13 + (size_t(it.group) * (2 * p.inter / 128) + it.feature0 / 128 + (lane & 1) * (p.inter / 128)) * blocks1 + (lane >> 1);
-        for (int j = first; j < steps; j += kRowWarps) {
+        for (int j = first; j < steps; j += ROW_WARPS) {
           const uint32_t step = step0 + j;
           const int s = step % kSlots, kb0 = j * share, n = min(share, blocks - kb0);
           const uint32_t slot = smem_u32(row_ring) + s * kRowSlotBytes;
@@ -386,7 +387,7 @@ few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
           asked += row_step;
           if (++ask_r == it.rows) {
             ask_r = 0;
-            ask_j += kRowWarps;
+            ask_j += ROW_WARPS;
             asked = act + ask_j * (WK * 32);
             there_is = b < blocks2 - ask_j * WK;
           }
@@ -427,7 +428,7 @@ few_tokens_kernel(const __grid_constant__ Maps maps, const Params p) {
             if (++r == it.rows) {
               mbar_arrive(&sh->row_full[s]);
               r = 0;
-              j += kRowWarps;
+              j += ROW_WARPS;
             }
           }
         }
@@ -566,9 +567,14 @@ inline int weight_maps(Maps* maps, const void* w13, const void* w2, int groups, 
   const int rc = weight_map(&maps->w13, w13, 2 * uint64_t(groups), inter, hidden, 16, 2, kSubTiles);
   return rc ? rc : weight_map(&maps->w2, w2, groups, hidden, inter, kDownFeatures, 1, WK);
 }
+// Two warps take longer over the quantisation of several rows a slot than its weights take, four do not, but leave 80 registers a thread.  Two and four, us, one term: eight
+// tokens on the same eight experts of 2048, hidden 7168, 92.7 and 75.9, four tokens 77.8 and 65.6 to 70, eight at even routing 378.8 and 370 to 379; of 1536, hidden 4096, three
+// 40.1 and 38.7, one 36.5 and 37.1; of 768, hidden 2048, two at even routing 27.0 and 27.9; of 512, hidden 1024, 16.7 and 17.2.  Two terms, which spill: eight on the same
+// experts 121 and 104, but at even routing 58 and 71, four tokens 201 and 231.
+inline int row_warps(int terms, int tokens, int hidden, int inter) { return terms == 1 && tokens > 1 && 3 * int64_t(hidden) * inter >= 16000000 ? 4 : 2; }
 template <typename F>
-inline int with_terms(int terms, F f) {
-  return terms == 2 ? f(few_tokens_kernel<2>) : f(few_tokens_kernel<1>);
+inline int with_kernel(int terms, int row_warps, F f) {
+  return terms == 2 ? f(few_tokens_kernel<2, 2>) : row_warps == 4 ? f(few_tokens_kernel<1, 4>) : f(few_tokens_kernel<1, 2>);
 }
 
 }  // namespace few

@@ -38,6 +38,8 @@ def check(cpu, out, act, top_k=8, routing="softmax"):
 @pytest.mark.parametrize("tokens,hidden,inter,experts,local,offset,top_k", [
     (1, 1024, 512, 64, 64, 0, 8),
     (1, 7168, 2048, 64, 8, 24, 8),            # a serving layer's experts
+    (3, 4096, 1408, 64, 16, 16, 8),           # four row warps (one term): three slots of eleven K blocks an item
+    (8, 7168, 2048, 64, 8, 24, 8),            # the same, at an expert's full rows
     (2, 1152, 640, 64, 16, 16, 8),            # nine and five K blocks; an odd number of 128 columns
     (3, 128, 128, 64, 16, 0, 8),              # fewer K blocks than warps that share them, in both products
     (8, 1408, 1024, 128, 32, 32, 8),          # as many tokens as are routed and placed in one kernel
